@@ -115,8 +115,9 @@ typedef struct {
                                     of a shared node (an order-free sum of two terms) */
   int32_t chain_ordered;         /* with node_diag: consecutive elements follow each other along every
                                     wire (element e's node b is element e+1's node a, or the node has
-                                    one element); xk_beam_assemble32 then writes each shared node's
-                                    sum once, without zeroing or atomics */
+                                    one element); xk_beam_assemble32, and xk_beam_assemble in FP64,
+                                    then write each shared node's sum once, without zeroing or
+                                    atomics */
   int32_t beam_ctas_per_sm;      /* float kernel: 0 for one CTA per 128 threads of work, else at most
                                     this many CTAs per SM, looping (room for concurrent kernels) */
 } xk_beam_plan;

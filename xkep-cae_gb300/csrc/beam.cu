@@ -4,10 +4,10 @@
 // one element per thread, with the corotated frame in quaternion form:
 //   R_cr = R0 R_rod^T,  theta_def = log(R_cr R_node R0^T) = R0 log(q_rod^* (x) q_node)
 // which equals the reference's matrix Shepperd route for rotations below pi.
-// k_beam<P> (xk_beam_assemble) takes the frame in double in both precision modes
-// and runs everything downstream of it (local stiffness, f_cr, B, K_mat, K_geo)
-// in Prec<P>::T; k_beam32e (xk_beam_assemble32, the mixed engine) runs all of it
-// in float from the prepared element and node records.
+// k_beam64 (xk_beam_assemble in FP64) runs in double.  k_beam<XK_MIXED> (the same
+// entry, mixed) takes the frame in double and everything downstream of it (local
+// stiffness, f_cr, B, K_mat, K_geo) in float; k_beam32e (xk_beam_assemble32, the
+// mixed engine) runs all of it in float from the prepared element and node records.
 #include "xk_common.cuh"
 
 namespace {
@@ -48,9 +48,10 @@ XK_D void rotvec_of_quat(const double* qin, double* th) {
   double s2 = x * x + y * y + z * z;
   double coef;
   if (s2 < 0.0025 * w * w) {  // |v|/w < 0.05: 2 atan(r)/(r w) by its series
-    double r2 = s2 / (w * w);
+    const double iw = rcp64(w);  // w is at least 0.998 here
+    const double r2 = s2 * (iw * iw);
     double at = 1.0 + r2 * (-1.0 / 3 + r2 * (1.0 / 5 + r2 * (-1.0 / 7 + r2 * (1.0 / 9 + r2 * (-1.0 / 11 + r2 * (1.0 / 13))))));
-    coef = 2.0 * at / w;
+    coef = 2.0 * at * iw;
   } else {
     double sh = sqrt(s2);
     coef = 2.0 * atan2(sh, w) / sh;
@@ -212,8 +213,6 @@ struct KeCoef {
 // issues at the FP64 rate), the same bits as the cast.
 template <typename T>
 XK_D T sec_val(double x);
-template <>
-XK_D double sec_val<double>(double x) { return x; }
 template <>
 XK_D float sec_val<float>(double x) { return xk_d2f(x); }
 
@@ -504,6 +503,7 @@ constexpr int EL_S01 = 18, EL_S03 = 27, EL_S13 = 36;  // row-major
 constexpr int EL_G0 = 45, EL_G1 = 48, EL_G3 = 51;     // f rows: node a translation g0, rotation g1; node b -g0, g3
 constexpr int EL_BLK = 54;                            // the element's block ids aa, ab, ba, bb (int bits)
 constexpr int EL_STRIDE = 59;  // odd: the threads' slots fall in different banks
+constexpr int EL_STRIDE64 = 57;  // the same in double (the block ids take two places)
 
 XK_D int sym_index(int r, int c) {  // position of (r, c) in a symmetric 3x3 stored as 6 values
   const int i = r < c ? r : c, j = r < c ? c : r;
@@ -511,28 +511,185 @@ XK_D int sym_index(int r, int c) {  // position of (r, c) in a symmetric 3x3 sto
 }
 
 // sym(X) of a row-major 3x3 into the 6-value form
-XK_D void sym6(const float* X, float* S) {
+template <typename T>
+XK_D void sym6(const T* X, T* S) {
   S[0] = X[0];
-  S[1] = 0.5f * (X[1] + X[3]);
-  S[2] = 0.5f * (X[2] + X[6]);
+  S[1] = T(0.5) * (X[1] + X[3]);
+  S[2] = T(0.5) * (X[2] + X[6]);
   S[3] = X[4];
-  S[4] = 0.5f * (X[5] + X[7]);
+  S[4] = T(0.5) * (X[5] + X[7]);
   S[5] = X[8];
 }
 
 // M = sum of the outer products R_k (x) V_k (row-major)
-XK_D void outer2(const float* Ra, const float* Va, const float* Rb, const float* Vb, float* M) {
+template <typename T>
+XK_D void outer2(const T* Ra, const T* Va, const T* Rb, const T* Vb, T* M) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int c = 0; c < 3; ++c) M[3 * i + c] = Ra[i] * Va[c] + Rb[i] * Vb[c];
 }
-XK_D void outer3(const float* Ra, const float* Va, const float* Rb, const float* Vb, const float* Rc,
-                 const float* Vc, float* M) {
+template <typename T>
+XK_D void outer3(const T* Ra, const T* Va, const T* Rb, const T* Vb, const T* Rc, const T* Vc, T* M) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int c = 0; c < 3; ++c) M[3 * i + c] = Ra[i] * Va[c] + Rb[i] * Vb[c] + Rc[i] * Vc[c];
+}
+
+// The outputs of one element from its frame: global forces of the blocks and, with want_K, the six symmetrised
+// tangent blocks, written to the slot o as they are formed.  Rcr: the corotated frame, ex and iLd: the deformed
+// axis and 1/L, t1, t2: the local rotations, tha, thb: the nodal rotation vectors, dax: the axial stretch.
+template <typename T>
+XK_D void beam_slots(const KeCoef<T>& kc, const T* Rcr, const T* ex, T iLd, const T* t1, const T* t2, const T* tha,
+                     const T* thb, T dax, bool want_K, T* o) {
+  // local forces of blocks 0, 1, 3 (block 2 = -block 0) and their global images g_I = Rcr^T f_I
+  T g0[3], g1[3], g3[3];
+  {
+    const T f0[3] = {-kc.ea * dax, kc.k2z * (t1[2] + t2[2]), -kc.k2y * (t1[1] + t2[1])};
+    const T f1[3] = {kc.gj * (t1[0] - t2[0]), kc.k1ay * t1[1] + kc.k1by * t2[1],
+                         kc.k1az * t1[2] + kc.k1bz * t2[2]};
+    const T f3[3] = {-f1[0], kc.k1by * t1[1] + kc.k1ay * t2[1], kc.k1bz * t1[2] + kc.k1az * t2[2]};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      g0[i] = Rcr[i] * f0[0] + Rcr[3 + i] * f0[1] + Rcr[6 + i] * f0[2];
+      g1[i] = Rcr[i] * f1[0] + Rcr[3 + i] * f1[1] + Rcr[6 + i] * f1[2];
+      g3[i] = Rcr[i] * f3[0] + Rcr[3 + i] * f3[1] + Rcr[6 + i] * f3[2];
+      o[EL_G0 + i] = g0[i];
+      o[EL_G1 + i] = g1[i];
+      o[EL_G3 + i] = g3[i];
+    }
+  }
+  if (!want_K) return;
+  const T* R_0 = Rcr;
+  const T* R_1 = Rcr + 3;
+  const T* R_2 = Rcr + 6;
+  // P_s = T^-1(t_s) dpsi with dpsi = Rcr [e_x]x / L: row i of M [e_x]x is M_i x e_x, M = T^-1 Rcr;
+  // Q_s = T^-1(t_s) Rcr T(theta_node)
+  T P1[9], P2[9], Q1[9], Q2[9];
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    T Ti[9], Ts[9], M[9];
+    tangent_ops<T>(side ? t2 : t1, true, Ti);
+    tangent_ops<T>(side ? thb : tha, false, Ts);
+    mm3(Ti, Rcr, M);
+    T* P = side ? P2 : P1;
+    T* Q = side ? Q2 : Q1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      T c[3];
+      cross3(M + 3 * i, ex, c);
+      P[3 * i] = c[0] * iLd;
+      P[3 * i + 1] = c[1] * iLd;
+      P[3 * i + 2] = c[2] * iLd;
+    }
+    mm3(M, Ts, Q);
+  }
+  // G_I = Rcr^T A_I + geometric term; G1^T / 2 and G3^T / 2 go to the S01 and S03 slots at once
+  // (0.5 x + 0.5 y rounds as 0.5 (x + y)), so that P1, P2 and the forces end here
+  {
+    T v0[3], v1[3], v2[3], G[9];
+    const T d1 = dot3(g1, ex), d3 = dot3(g3, ex), d0 = dot3(g0, ex);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = kc.gj * (P1[c] - P2[c]);
+      v1[c] = kc.k1ay * P1[3 + c] + kc.k1by * P2[3 + c];
+      v2[c] = kc.k1az * P1[6 + c] + kc.k1bz * P2[6 + c];
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[EL_S01 + 3 * c + i] = T(0.5) * (G[3 * i + c] + iLd * (ex[i] * g1[c] - (i == c ? d1 : T(0))));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = -v0[c];
+      v1[c] = kc.k1by * P1[3 + c] + kc.k1ay * P2[3 + c];
+      v2[c] = kc.k1bz * P1[6 + c] + kc.k1az * P2[6 + c];
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[EL_S03 + 3 * c + i] = T(0.5) * (G[3 * i + c] + iLd * (ex[i] * g3[c] - (i == c ? d3 : T(0))));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = kc.ea * ex[c];
+      v1[c] = kc.k2z * (P1[6 + c] + P2[6 + c]);
+      v2[c] = -kc.k2y * (P1[3 + c] + P2[3 + c]);
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) G[3 * i + c] += iLd * (ex[i] * g0[c] - (i == c ? d0 : T(0)));
+    T S[6];
+    sym6(G, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
+  }
+  {
+    T a1[3], a2[3], b0[3], X[9], S[6];
+    // H0, J0: the I = 0 rows against Q1, Q2, added to the halves of G1^T, G3^T
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      a1[c] = kc.k2z * Q1[6 + c];
+      a2[c] = -kc.k2y * Q1[3 + c];
+    }
+    outer2(R_1, a1, R_2, a2, X);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S01 + i] += T(0.5) * X[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      a1[c] = kc.k2z * Q2[6 + c];
+      a2[c] = -kc.k2y * Q2[3 + c];
+    }
+    outer2(R_1, a1, R_2, a2, X);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S03 + i] += T(0.5) * X[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = kc.gj * Q1[c];
+      a1[c] = kc.k1ay * Q1[3 + c];
+      a2[c] = kc.k1az * Q1[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H1
+    sym6(X, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S11 + i] = S[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = kc.gj * Q2[c];
+      a1[c] = kc.k1ay * Q2[3 + c];
+      a2[c] = kc.k1az * Q2[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J3
+    sym6(X, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S33 + i] = S[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = -kc.gj * Q1[c];
+      a1[c] = kc.k1by * Q1[3 + c];
+      a2[c] = kc.k1bz * Q1[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H3
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = T(0.5) * X[3 * i + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = -kc.gj * Q2[c];
+      a1[c] = kc.k1by * Q2[3 + c];
+      a2[c] = kc.k1bz * Q2[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J1
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S13 + i] += T(0.5) * X[i];
+  }
 }
 
 // One element: frame (the rotation vectors of both nodes by one thread), global forces of the
@@ -596,173 +753,30 @@ XK_D void beam_elem32(const float* __restrict__ E, const float* __restrict__ NA,
       for (int j = 0; j < 3; ++j)
         Rcr[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
   }
-  const KeCoef<float> kc = ke_coef<float>(sec, L0);
-  // local forces of blocks 0, 1, 3 (block 2 = -block 0) and their global images g_I = Rcr^T f_I
-  float g0[3], g1[3], g3[3];
-  {
-    const float f0[3] = {-kc.ea * dax, kc.k2z * (t1[2] + t2[2]), -kc.k2y * (t1[1] + t2[1])};
-    const float f1[3] = {kc.gj * (t1[0] - t2[0]), kc.k1ay * t1[1] + kc.k1by * t2[1],
-                         kc.k1az * t1[2] + kc.k1bz * t2[2]};
-    const float f3[3] = {-f1[0], kc.k1by * t1[1] + kc.k1ay * t2[1], kc.k1bz * t1[2] + kc.k1az * t2[2]};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      g0[i] = Rcr[i] * f0[0] + Rcr[3 + i] * f0[1] + Rcr[6 + i] * f0[2];
-      g1[i] = Rcr[i] * f1[0] + Rcr[3 + i] * f1[1] + Rcr[6 + i] * f1[2];
-      g3[i] = Rcr[i] * f3[0] + Rcr[3 + i] * f3[1] + Rcr[6 + i] * f3[2];
-      o[EL_G0 + i] = g0[i];
-      o[EL_G1 + i] = g1[i];
-      o[EL_G3 + i] = g3[i];
-    }
-  }
-  if (!want_K) return;
-  const float* R_0 = Rcr;
-  const float* R_1 = Rcr + 3;
-  const float* R_2 = Rcr + 6;
-  // P_s = T^-1(t_s) dpsi with dpsi = Rcr [e_x]x / L: row i of M [e_x]x is M_i x e_x, M = T^-1 Rcr;
-  // Q_s = T^-1(t_s) Rcr T(theta_node)
-  float P1[9], P2[9], Q1[9], Q2[9];
-#pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    float Ti[9], Ts[9], M[9];
-    tangent_ops<float>(side ? t2 : t1, true, Ti);
-    tangent_ops<float>(side ? ub + 3 : ua + 3, false, Ts);
-    mm3(Ti, Rcr, M);
-    float* P = side ? P2 : P1;
-    float* Q = side ? Q2 : Q1;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      float c[3];
-      cross3(M + 3 * i, ex, c);
-      P[3 * i] = c[0] * iLd;
-      P[3 * i + 1] = c[1] * iLd;
-      P[3 * i + 2] = c[2] * iLd;
-    }
-    mm3(M, Ts, Q);
-  }
-  // G_I = Rcr^T A_I + geometric term; G1^T / 2 and G3^T / 2 go to the S01 and S03 slots at once
-  // (0.5 x + 0.5 y rounds as 0.5 (x + y)), so that P1, P2 and the forces end here
-  {
-    float v0[3], v1[3], v2[3], G[9];
-    const float d1 = dot3(g1, ex), d3 = dot3(g3, ex), d0 = dot3(g0, ex);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = kc.gj * (P1[c] - P2[c]);
-      v1[c] = kc.k1ay * P1[3 + c] + kc.k1by * P2[3 + c];
-      v2[c] = kc.k1az * P1[6 + c] + kc.k1bz * P2[6 + c];
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        o[EL_S01 + 3 * c + i] = 0.5f * (G[3 * i + c] + iLd * (ex[i] * g1[c] - (i == c ? d1 : 0.f)));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = -v0[c];
-      v1[c] = kc.k1by * P1[3 + c] + kc.k1ay * P2[3 + c];
-      v2[c] = kc.k1bz * P1[6 + c] + kc.k1az * P2[6 + c];
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        o[EL_S03 + 3 * c + i] = 0.5f * (G[3 * i + c] + iLd * (ex[i] * g3[c] - (i == c ? d3 : 0.f)));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = kc.ea * ex[c];
-      v1[c] = kc.k2z * (P1[6 + c] + P2[6 + c]);
-      v2[c] = -kc.k2y * (P1[3 + c] + P2[3 + c]);
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) G[3 * i + c] += iLd * (ex[i] * g0[c] - (i == c ? d0 : 0.f));
-    float S[6];
-    sym6(G, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
-  }
-  {
-    float a1[3], a2[3], b0[3], X[9], S[6];
-    // H0, J0: the I = 0 rows against Q1, Q2, added to the halves of G1^T, G3^T
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      a1[c] = kc.k2z * Q1[6 + c];
-      a2[c] = -kc.k2y * Q1[3 + c];
-    }
-    outer2(R_1, a1, R_2, a2, X);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S01 + i] += 0.5f * X[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      a1[c] = kc.k2z * Q2[6 + c];
-      a2[c] = -kc.k2y * Q2[3 + c];
-    }
-    outer2(R_1, a1, R_2, a2, X);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S03 + i] += 0.5f * X[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = kc.gj * Q1[c];
-      a1[c] = kc.k1ay * Q1[3 + c];
-      a2[c] = kc.k1az * Q1[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H1
-    sym6(X, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S11 + i] = S[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = kc.gj * Q2[c];
-      a1[c] = kc.k1ay * Q2[3 + c];
-      a2[c] = kc.k1az * Q2[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J3
-    sym6(X, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S33 + i] = S[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = -kc.gj * Q1[c];
-      a1[c] = kc.k1by * Q1[3 + c];
-      a2[c] = kc.k1bz * Q1[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H3
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = 0.5f * X[3 * i + c];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = -kc.gj * Q2[c];
-      a1[c] = kc.k1by * Q2[3 + c];
-      a2[c] = kc.k1bz * Q2[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J1
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S13 + i] += 0.5f * X[i];
-  }
+  beam_slots<float>(ke_coef<float>(sec, L0), Rcr, ex, iLd, t1, t2, ua + 3, ub + 3, dax, want_K, o);
 }
 
 // Value (r, c) of a stored 6x6 block of one element, from its slot o:
 // aa = [S00 S01; S01^T S11], bb = [S00 -S03; -S03^T S33], ab = [-S00 S03; -S01^T S13] (rows: node a).
-XK_D float blk_aa(const float* o, int r, int c) {
+template <typename T>
+XK_D T blk_aa(const T* o, int r, int c) {
   if (r < 3) return c < 3 ? o[EL_S00 + sym_index(r, c)] : o[EL_S01 + 3 * r + c - 3];
   return c < 3 ? o[EL_S01 + 3 * c + r - 3] : o[EL_S11 + sym_index(r - 3, c - 3)];
 }
-XK_D float blk_bb(const float* o, int r, int c) {
+template <typename T>
+XK_D T blk_bb(const T* o, int r, int c) {
   if (r < 3) return c < 3 ? o[EL_S00 + sym_index(r, c)] : -o[EL_S03 + 3 * r + c - 3];
   return c < 3 ? -o[EL_S03 + 3 * c + r - 3] : o[EL_S33 + sym_index(r - 3, c - 3)];
 }
-XK_D float blk_ab(const float* o, int r, int c) {
+template <typename T>
+XK_D T blk_ab(const T* o, int r, int c) {
   if (r < 3) return c < 3 ? -o[EL_S00 + sym_index(r, c)] : o[EL_S03 + 3 * r + c - 3];
   return c < 3 ? -o[EL_S01 + 3 * c + r - 3] : o[EL_S13 + 3 * (r - 3) + c - 3];
 }
 
 // block kinds of an element: 0 aa, 1 ab, 2 ba (the transpose of ab), 3 bb; 4: aa of o plus bb of p
-XK_D float blk_val(int kind, const float* o, const float* p, int r, int c) {
+template <typename T>
+XK_D T blk_val(int kind, const T* o, const T* p, int r, int c) {
   switch (kind) {
     case 0: return blk_aa(o, r, c);
     case 1: return blk_ab(o, r, c);
@@ -772,15 +786,34 @@ XK_D float blk_val(int kind, const float* o, const float* p, int r, int c) {
   }
 }
 
-// HOW: 0 store, 1 add to the stored value, 2 atomic add
-template <int KIND, int HOW>
-XK_D void put_block(float* __restrict__ dst, const float* o, const float* p) {
+// HOW: 0 store, 1 add to the stored value, 2 atomic add (float).  vec: dst is 16-byte aligned.
+template <int KIND, int HOW, typename T>
+XK_D void put_block(T* __restrict__ dst, const T* o, const T* p, bool vec) {
+  if (sizeof(T) == 8) {
+    double2* d2 = reinterpret_cast<double2*>(dst);
+#pragma unroll
+    for (int q = 0; q < 18; ++q) {
+      double v0 = blk_val<T>(KIND, o, p, (2 * q) / 6, (2 * q) % 6);
+      double v1 = blk_val<T>(KIND, o, p, (2 * q + 1) / 6, (2 * q + 1) % 6);
+      if (HOW == 1) {
+        v0 += dst[2 * q];
+        v1 += dst[2 * q + 1];
+      }
+      if (vec) {
+        d2[q] = make_double2(v0, v1);
+      } else {
+        dst[2 * q] = v0;
+        dst[2 * q + 1] = v1;
+      }
+    }
+    return;
+  }
   float4* d = reinterpret_cast<float4*>(dst);
 #pragma unroll
   for (int q = 0; q < 9; ++q) {
     float v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = blk_val(KIND, o, p, (4 * q + k) / 6, (4 * q + k) % 6);
+    for (int k = 0; k < 4; ++k) v[k] = blk_val<T>(KIND, o, p, (4 * q + k) / 6, (4 * q + k) % 6);
     float4 x = make_float4(v[0], v[1], v[2], v[3]);
     if (HOW == 2) {
       atomicAdd(d + q, x);
@@ -794,14 +827,17 @@ XK_D void put_block(float* __restrict__ dst, const float* o, const float* p) {
   }
 }
 
+XK_D double row_f64(float x) { return xk_f2d(x); }
+XK_D double row_f64(double x) { return x; }
+
 // f rows of one node: translation t (3, negated with neg_t) then rotation r (3), as doubles
-template <int HOW>  // 0 store, 1 add, 2 atomic add
-XK_D void put_rows(double* __restrict__ f, long long node, const float* t, const float* r, bool neg_t) {
+template <int HOW, typename T>  // 0 store, 1 add, 2 atomic add
+XK_D void put_rows(double* __restrict__ f, long long node, const T* t, const T* r, bool neg_t) {
   double v[6];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    v[i] = xk_f2d(neg_t ? -t[i] : t[i]);
-    v[3 + i] = xk_f2d(r[i]);
+    v[i] = row_f64(neg_t ? -t[i] : t[i]);
+    v[3 + i] = row_f64(r[i]);
   }
   double* d = f + 6 * node;
 #pragma unroll
@@ -837,10 +873,12 @@ constexpr int BEAMW_T = 128;
 constexpr int BEAM_ORDERED = 0, BEAM_ATOMIC = 1, BEAM_COLOUR = 2;
 
 // One element of the launch (t: the thread's logical index), its outputs staged in the slots.
-XK_D void beam_item(int mode, long long t, const xk_mesh& m, const xk_section& sec, const float* __restrict__ e32,
-                    const int32_t* __restrict__ order, int k0, int k1, const int32_t* __restrict__ blk,
-                    const uint8_t* __restrict__ first, const float* __restrict__ n32, double* __restrict__ f_int,
-                    float* __restrict__ Kv, float* slots) {
+// elem(e, a, b, o) computes element e between nodes a and b into its slot o.
+template <typename T, typename Elem>
+XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __restrict__ order, int k0, int k1,
+                    const int32_t* __restrict__ blk, const uint8_t* __restrict__ first, double* __restrict__ f_int,
+                    T* __restrict__ Kv, bool vec, T* slots, Elem elem) {
+  constexpr int STRIDE = sizeof(T) == 4 ? EL_STRIDE : EL_STRIDE64;
   const int lane = threadIdx.x & 31;
   const long long ne = m.n_elems;
   long long e;
@@ -855,42 +893,51 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const xk_section& s
     e = mode == BEAM_COLOUR ? order[k] : k;
   }
   const bool want_K = Kv != nullptr;
-  float* o = slots + threadIdx.x * EL_STRIDE;
+  T* o = slots + threadIdx.x * STRIDE;
   int a = -1, b = -1;
   int* ob = reinterpret_cast<int*>(o + EL_BLK);
   if (live) {
     // the block ids are loaded with the connectivity, before the element's chain, and parked in the slot
-    const int2 ab = __ldg(reinterpret_cast<const int2*>(m.conn) + e);
-    if (want_K) {
-      const int4 bi = __ldg(reinterpret_cast<const int4*>(blk) + e);
-      ob[0] = bi.x; ob[1] = bi.y; ob[2] = bi.z; ob[3] = bi.w;
+    if (sizeof(T) == 4) {
+      const int2 ab = __ldg(reinterpret_cast<const int2*>(m.conn) + e);
+      a = ab.x;
+      b = ab.y;
+    } else {  // no alignment is asked of the FP64 caller's arrays
+      a = m.conn[2 * e];
+      b = m.conn[2 * e + 1];
     }
-    a = ab.x;
-    b = ab.y;
-    beam_elem32(e32 + e * XK_ELEM32_STRIDE, n32 + (long long)a * XK_NODE32_STRIDE + 6,
-                n32 + (long long)b * XK_NODE32_STRIDE + 6, sec, want_K, o);
+    if (want_K) {
+      if (sizeof(T) == 4) {
+        const int4 bi = __ldg(reinterpret_cast<const int4*>(blk) + e);
+        ob[0] = bi.x; ob[1] = bi.y; ob[2] = bi.z; ob[3] = bi.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ob[q] = blk[4 * e + q];
+      }
+    }
+    elem(e, a, b, o);
   }
   if (mode == BEAM_ORDERED) {
     const int bp = __shfl_up_sync(0xffffffffu, b, 1);  // the predecessor's node b
     __syncwarp();
     if (lane == 0 || e > ne) return;
-    const float* p = o - EL_STRIDE;          // the predecessor's slot
+    const T* p = o - STRIDE;          // the predecessor's slot
     const bool pred = e >= 1;                // the predecessor exists (e <= ne here)
     const bool joined = live && pred && bp == a;
     if (pred && !joined) {                   // the predecessor ends its wire: its node b alone
-      if (f_int) put_rows<0>(f_int, bp, p + EL_G0, p + EL_G3, true);
-      if (want_K) put_block<3, 0>(Kv + 36LL * reinterpret_cast<const int*>(p + EL_BLK)[3], p, p);
+      if (f_int) put_rows<0, T>(f_int, bp, p + EL_G0, p + EL_G3, true);
+      if (want_K) put_block<3, 0, T>(Kv + 36LL * reinterpret_cast<const int*>(p + EL_BLK)[3], p, p, vec);
     }
     if (!live) return;
     if (f_int) {
       double v[6];
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        v[i] = xk_f2d(o[EL_G0 + i]);
-        v[3 + i] = xk_f2d(o[EL_G1 + i]);
+        v[i] = row_f64(o[EL_G0 + i]);
+        v[3 + i] = row_f64(o[EL_G1 + i]);
         if (joined) {
-          v[i] += xk_f2d(-p[EL_G0 + i]);
-          v[3 + i] += xk_f2d(p[EL_G3 + i]);
+          v[i] += row_f64(-p[EL_G0 + i]);
+          v[3 + i] += row_f64(p[EL_G3 + i]);
         }
       }
       if (((uintptr_t)f_int & 15) == 0) {
@@ -903,37 +950,37 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const xk_section& s
       }
     }
     if (!want_K) return;
-    if (joined) put_block<4, 0>(Kv + 36LL * ob[0], o, p);
-    else put_block<0, 0>(Kv + 36LL * ob[0], o, o);
-    if (ob[1] >= 0) put_block<1, 0>(Kv + 36LL * ob[1], o, o);
-    else put_block<2, 0>(Kv + 36LL * ob[2], o, o);
+    if (joined) put_block<4, 0, T>(Kv + 36LL * ob[0], o, p, vec);
+    else put_block<0, 0, T>(Kv + 36LL * ob[0], o, o, vec);
+    if (ob[1] >= 0) put_block<1, 0, T>(Kv + 36LL * ob[1], o, o, vec);
+    else put_block<2, 0, T>(Kv + 36LL * ob[2], o, o, vec);
     return;
   }
   const uint8_t fl = mode == BEAM_COLOUR ? first[e] : 0;
   if (f_int) {
     if (mode == BEAM_ATOMIC) {
-      put_rows<2>(f_int, a, o + EL_G0, o + EL_G1, false);
-      put_rows<2>(f_int, b, o + EL_G0, o + EL_G3, true);
+      put_rows<2, T>(f_int, a, o + EL_G0, o + EL_G1, false);
+      put_rows<2, T>(f_int, b, o + EL_G0, o + EL_G3, true);
     } else {
-      if (fl & 1) put_rows<0>(f_int, a, o + EL_G0, o + EL_G1, false);
-      else put_rows<1>(f_int, a, o + EL_G0, o + EL_G1, false);
-      if (fl & 8) put_rows<0>(f_int, b, o + EL_G0, o + EL_G3, true);
-      else put_rows<1>(f_int, b, o + EL_G0, o + EL_G3, true);
+      if (fl & 1) put_rows<0, T>(f_int, a, o + EL_G0, o + EL_G1, false);
+      else put_rows<1, T>(f_int, a, o + EL_G0, o + EL_G1, false);
+      if (fl & 8) put_rows<0, T>(f_int, b, o + EL_G0, o + EL_G3, true);
+      else put_rows<1, T>(f_int, b, o + EL_G0, o + EL_G3, true);
     }
   }
   if (!want_K) return;
   if (mode == BEAM_ATOMIC) {
-    put_block<0, 2>(Kv + 36LL * ob[0], o, o);
-    put_block<3, 2>(Kv + 36LL * ob[3], o, o);
+    put_block<0, 2, T>(Kv + 36LL * ob[0], o, o, vec);
+    put_block<3, 2, T>(Kv + 36LL * ob[3], o, o, vec);
   } else {
-    if (fl & 1) put_block<0, 0>(Kv + 36LL * ob[0], o, o);
-    else put_block<0, 1>(Kv + 36LL * ob[0], o, o);
-    if (fl & 8) put_block<3, 0>(Kv + 36LL * ob[3], o, o);
-    else put_block<3, 1>(Kv + 36LL * ob[3], o, o);
+    if (fl & 1) put_block<0, 0, T>(Kv + 36LL * ob[0], o, o, vec);
+    else put_block<0, 1, T>(Kv + 36LL * ob[0], o, o, vec);
+    if (fl & 8) put_block<3, 0, T>(Kv + 36LL * ob[3], o, o, vec);
+    else put_block<3, 1, T>(Kv + 36LL * ob[3], o, o, vec);
   }
   // the off-diagonal block has one writer
-  if (ob[1] >= 0) put_block<1, 0>(Kv + 36LL * ob[1], o, o);
-  else put_block<2, 0>(Kv + 36LL * ob[2], o, o);
+  if (ob[1] >= 0) put_block<1, 0, T>(Kv + 36LL * ob[1], o, o, vec);
+  else put_block<2, 0, T>(Kv + 36LL * ob[2], o, o, vec);
 }
 
 // Launch: the logical threads of the mode (32 per warp of 31 ordered elements, or one per element of
@@ -952,8 +999,129 @@ __global__ void __launch_bounds__(BEAMW_T, 6) k_beam32e(int mode, xk_mesh m, xk_
   const long long stride = (long long)gridDim.x * BEAMW_T;  // a multiple of 32
   for (long long t = (long long)blockIdx.x * BEAMW_T + threadIdx.x; t < n_threads; t += stride) {
     if (mode == BEAM_ORDERED) __syncwarp();  // the whole warp is here: n_threads is a multiple of 32 there
-    beam_item(mode, t, m, sec, e32, order, k0, k1, blk, first, n32, f_int, Kv, slots);
+    beam_item<float>(mode, t, m, order, k0, k1, blk, first, f_int, Kv, true, slots,
+                     [&](long long e, int a, int b, float* o) {
+                       beam_elem32(e32 + e * XK_ELEM32_STRIDE, n32 + (long long)a * XK_NODE32_STRIDE + 6,
+                                   n32 + (long long)b * XK_NODE32_STRIDE + 6, sec, Kv != nullptr, o);
+                     });
   }
+}
+
+// The FP64 beam: the same element outputs and write-back in double.  What bounds it is the FP64 pipe, so the
+// element takes the six-block form (about 2.4 times fewer operations than the full rows of beam_tail),
+// reciprocals by Newton-Raphson, section constants formed once on the host and the frame from the displacement
+// differences, as in the float element, and an ordered wire mesh runs in one launch instead of one per colour.
+// CTAs of one warp: a small mesh then reaches every SM (4,736 elements: 153 CTAs), where CTAs of 128 threads,
+// one launch after another, left most of them idle.
+// Measured, colour launches of beam_tail against this: 98,592 elements 406 -> 242 us, 4,736 elements
+// 157 -> 46 us (a warp issues one FP64 instruction in 64 clocks, so one warp per SM is what that mesh allows).
+constexpr int BEAM64_T = 32;
+struct BeamConst64 {  // E A, G J, E Iy, E Iz; 12 E I / (kappa G A); A / (12 I) * scf (0: off)
+  double ea, gj, eiy, eiz, py, pz, sy, sz;
+};
+
+XK_D KeCoef<double> ke_coef64(const BeamConst64& s, double iL, double L) {
+  double phy = s.py * iL * iL, phz = s.pz * iL * iL;
+  if (s.sy > 0.0) {
+    phy = phy / (1.0 + s.sy * L * L);
+    phz = phz / (1.0 + s.sz * L * L);
+  }
+  KeCoef<double> k;
+  k.ea = s.ea * iL;
+  k.gj = s.gj * iL;
+  const double ky = s.eiy * iL * rcp64(1.0 + phy), kz = s.eiz * iL * rcp64(1.0 + phz);
+  k.k3y = 12.0 * ky * iL * iL;
+  k.k2y = 6.0 * ky * iL;
+  k.k1ay = (4.0 + phy) * ky;
+  k.k1by = (2.0 - phy) * ky;
+  k.k3z = 12.0 * kz * iL * iL;
+  k.k2z = 6.0 * kz * iL;
+  k.k1az = (4.0 + phz) * kz;
+  k.k1bz = (2.0 - phz) * kz;
+  return k;
+}
+
+XK_D void beam_elem64(const xk_mesh& m, const double* __restrict__ ref, const double* __restrict__ u,
+                      const BeamConst64& sec, long long e, int a, int b, bool want_K, double* o) {
+  const long long ne = m.n_elems;
+  const double L0 = ref[e];
+  double R0[9], ua[6], ub[6], dx0[3], du[3], dx[3];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) R0[i] = ref[(1 + i) * ne + e];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    ua[i] = u[6LL * a + i];
+    ub[i] = u[6LL * b + i];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dx0[i] = m.X[3LL * b + i] - m.X[3LL * a + i];
+    du[i] = ub[i] - ua[i];
+    dx[i] = dx0[i] + du[i];
+  }
+  const double L2 = dot3(dx, dx);
+  double iL, L;
+  if (in_range64<-300, 300>(L2)) {
+    iL = rsqrt64(L2);
+    L = L2 * iL;
+    L = fma(fma(-L, L, L2), 0.5 * iL, L);
+  } else {
+    L = sqrt(L2);
+    iL = 1.0 / L;
+  }
+  const double ex[3] = {dx[0] * iL, dx[1] * iL, dx[2] * iL};
+  const double sum[3] = {dx0[0] + dx[0], dx0[1] + dx[1], dx0[2] + dx[2]};
+  const double dax = dot3(du, sum) * (in_range64<-140, 140>(L + L0) ? rcp64(L + L0) : 1.0 / (L + L0));
+  // the smallest rotation of e0 (row 0 of R0) onto ex: 1 + e0 . ex = (L + L0 + e0 . du) / L, e0 x ex = e0 x du / L
+  double qr[4];
+  const double opc = (L + L0 + dot3(R0, du)) * iL;
+  if (opc > 0.5) {
+    double v[3];
+    cross3(R0, du, v);
+    const double rw = rsqrt64(0.5 * opc);
+    const double k = 0.5 * iL * rw;
+    qr[0] = 0.5 * opc * rw;
+    qr[1] = k * v[0];
+    qr[2] = k * v[1];
+    qr[3] = k * v[2];
+  } else {
+    quat_between(R0, ex, qr);
+  }
+  const double qrc[4] = {qr[0], -qr[1], -qr[2], -qr[3]};
+  double t1[3], t2[3];
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    double qn[4], qx[4], tx[3];
+    quat_of_rotvec(side ? ub + 3 : ua + 3, qn);
+    qmul(qrc, qn, qx);
+    rotvec_of_quat(qx, tx);
+    double* t = side ? t2 : t1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) t[i] = R0[3 * i] * tx[0] + R0[3 * i + 1] * tx[1] + R0[3 * i + 2] * tx[2];
+  }
+  double Rrod[9], Rcr[9];
+  rotmat_of_quat<double>(qr, Rrod);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      Rcr[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
+  const double iL0 = in_range64<-140, 140>(L0) ? rcp64(L0) : 1.0 / L0;
+  beam_slots<double>(ke_coef64(sec, iL0, L0), Rcr, ex, iL, t1, t2, ua + 3, ub + 3, dax, want_K, o);
+}
+
+__global__ void __launch_bounds__(BEAM64_T) k_beam64(int mode, xk_mesh m, BeamConst64 sec, const double* __restrict__ ref,
+                                                     const int32_t* __restrict__ order, int k0, int k1,
+                                                     const int32_t* __restrict__ blk, const uint8_t* __restrict__ first,
+                                                     const double* __restrict__ u, double* __restrict__ f_int,
+                                                     double* __restrict__ Kv, int vec, long long n_threads) {
+  __shared__ double slots[BEAM64_T * EL_STRIDE64];
+  const long long t = (long long)blockIdx.x * BEAM64_T + threadIdx.x;
+  if (t >= n_threads) return;  // n_threads is a multiple of 32 in the ordered mode
+  beam_item<double>(mode, t, m, order, k0, k1, blk, first, f_int, Kv, vec != 0, slots,
+                    [&](long long e, int a, int b, double* o) {
+                      beam_elem64(m, ref, u, sec, e, a, b, Kv != nullptr, o);
+                    });
 }
 
 // Chain launches: zero the node rows of f_int and the diagonal blocks that the elements add into,
@@ -1026,6 +1194,19 @@ extern "C" xk_status xk_beam_reference(const xk_mesh* m, const double* v_ref, do
   return XK_OK;
 }
 
+static BeamConst64 beam_const64(const xk_section& s) {
+  BeamConst64 c;
+  c.ea = s.E * s.A;
+  c.gj = s.G * s.J;
+  c.eiy = s.E * s.Iy;
+  c.eiz = s.E * s.Iz;
+  c.py = 12.0 * c.eiy / (s.kappa_y * s.G * s.A);
+  c.pz = 12.0 * c.eiz / (s.kappa_z * s.G * s.A);
+  c.sy = s.scf > 0.0 ? s.scf * s.A / (12.0 * s.Iy) : 0.0;
+  c.sz = s.scf > 0.0 ? s.scf * s.A / (12.0 * s.Iz) : 0.0;
+  return c;
+}
+
 extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, const double* elem_ref,
                                       const xk_beam_plan* plan, const double* u, int precision, double* f_int,
                                       void* K_vals, xk_stream s) {
@@ -1033,16 +1214,26 @@ extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, c
   if (precision != XK_FP64 && precision != XK_MIXED) return xk_set_error(XK_ERR_ARG, "xk_beam_assemble: precision");
   if (!f_int && !K_vals) return XK_OK;
   cudaStream_t st = (cudaStream_t)s;
+  const BeamConst64 bc = beam_const64(*sec);
+  const int vec = ((uintptr_t)K_vals & 15) == 0;
+  if (precision == XK_FP64 && plan->node_diag && plan->chain_ordered) {  // one launch, one writer per block
+    if (m->n_elems == 0) return XK_OK;
+    const long long threads = 32 * ((long long)m->n_elems / 31 + 1);
+    k_beam64<<<xk_blocks(threads, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_ORDERED, *m, bc, elem_ref, nullptr, 0, 0, plan->blk,
+                                                               plan->first, u, f_int, (double*)K_vals, vec, threads);
+    XK_CHECK_LAUNCH();
+    return XK_OK;
+  }
   for (int c = 0; c < plan->n_colors; ++c) {
     int k0 = plan->color_ptr_host[c], k1 = plan->color_ptr_host[c + 1];
     if (k1 <= k0) continue;
-    int nb = xk_blocks(k1 - k0, BEAM_T);
     if (precision == XK_FP64)
-      k_beam<XK_FP64><<<nb, BEAM_T, 0, st>>>(*m, *sec, elem_ref, plan->elem_order, k0, k1, plan->blk, plan->first, u,
-                                              f_int, (double*)K_vals);
+      k_beam64<<<xk_blocks(k1 - k0, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_COLOUR, *m, bc, elem_ref, plan->elem_order, k0, k1,
+                                                                 plan->blk, plan->first, u, f_int, (double*)K_vals, vec,
+                                                                 k1 - k0);
     else
-      k_beam<XK_MIXED><<<nb, BEAM_T, 0, st>>>(*m, *sec, elem_ref, plan->elem_order, k0, k1, plan->blk, plan->first, u,
-                                               f_int, (float*)K_vals);
+      k_beam<XK_MIXED><<<xk_blocks(k1 - k0, BEAM_T), BEAM_T, 0, st>>>(*m, *sec, elem_ref, plan->elem_order, k0, k1,
+                                                                     plan->blk, plan->first, u, f_int, (float*)K_vals);
     XK_CHECK_LAUNCH();
   }
   return XK_OK;

@@ -206,8 +206,8 @@ XK_D double coat_compression(const xk_mesh& m, int ea, int eb, double gap) {
   return fmax(0.0, xsub(coat_total_of(m, ea, eb), gap));
 }
 
-XK_D void narrow_exact_one(const xk_mesh& m, xk_pairs& p, const double* __restrict__ u, double g_on, double g_off,
-                           int allow_deact, int update_active, int i) {
+XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __restrict__ u, double g_on,
+                           double g_off, int allow_deact, int update_active, int i) {
   const long long cap = p.cap;
   PairNodes nd = pair_nodes(m, p.ea[i], p.eb[i]);
   double x[4][3];
@@ -353,6 +353,301 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
   for (int a = 0; a < 3; ++a)
     for (int b = 0; b < 3; ++b)
       B[3 * a + b] += (t1[a] * D00 + t2[a] * D01) * t1[b] + (t1[a] * D01 + t2[a] * D11) * t2[b];
+}
+
+// ===========================================================================
+// FP64 engine: the per-iteration pair kernels in double.
+//
+// What bounds them is the FP64 pipe, about two operations per clock and SM on this GPU, not memory: every
+// double divide and square root costs some ten of them, and a dot product with separately rounded terms
+// five instead of three.  The detection needs the reference's operation order (its active sets are compared
+// bit for bit) and keeps the exact routine; the per-iteration narrowphase needs double precision only, so it
+// is written for the fewest FP64 operations: fused multiply-adds, one reciprocal or reciprocal square root
+// per normalisation (two Newton-Raphson steps from the approximate PTX instruction), range tests on the high
+// word in the integer pipe, and the frame transported as R p = c p + v x p + v (v.p) / (1 + c).  Pairs outside
+// the ordinary case (near-parallel, degenerate, without a unit frame, NaN) take the exact routine.
+// Measured at the 1027-wire strand (2.46M other pairs, 0.75M contributing ones), exact routine for every
+// pair against this one: other pairs 1757 -> 652 us, contributing pairs 936 -> 393 us (132 and 262 FP64
+// operations a pair at the pipe's measured 1.64 per clock and SM).
+// ===========================================================================
+
+XK_D bool above_one64(double x) { return __double_as_longlong(x) > 0x3ff0000000000000LL; }
+XK_D bool outside01(double x) { return __double2hiint(x) < 0 || above_one64(x); }
+XK_D double clamp01_64(double x) { return __double2hiint(x) < 0 ? 0.0 : (above_one64(x) ? 1.0 : x); }
+XK_D double fdot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
+XK_D void fcross3(const double* a, const double* b, double* c) {
+  c[0] = fma(a[1], b[2], -(a[2] * b[1]));
+  c[1] = fma(a[2], b[0], -(a[0] * b[2]));
+  c[2] = fma(a[0], b[1], -(a[1] * b[0]));
+}
+
+// Closest point, gap and transported frame of one pair at positions x; rs: the radius sum; pn, pt1: the
+// previous frame.  False (nothing written) outside the ordinary case.
+XK_D bool narrow64(const double (*x)[3], double rs, const double* pn, const double* pt1, double& s, double& t,
+                   double& gap, double* n, double* t1, double* t2) {
+  double dA[3], dB[3], w[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dA[i] = x[1][i] - x[0][i];
+    dB[i] = x[3][i] - x[2][i];
+    w[i] = x[0][i] - x[2][i];
+  }
+  const double a = fdot3(dA, dA), b = fdot3(dA, dB), c = fdot3(dB, dB), d = fdot3(dA, w), e = fdot3(dB, w);
+  const double ac = a * c, det = fma(-b, b, ac);
+  // segments longer than 2^-14 and at an angle (det > 1e-3 ac): the absolute and relative tolerances of the
+  // reference (1e-10) are far off
+  if (!(in_range64<-29, 300>(a) && in_range64<-29, 300>(c) && __double2hiint(fma(-1e-3, ac, det)) > 0)) return false;
+  const double idet = rcp64(det);
+  const double su = fma(b, e, -(c * d)) * idet, tu = fma(a, e, -(b * d)) * idet;
+  double sc = clamp01_64(su), tc = clamp01_64(tu);
+  const bool s_out = outside01(su), t_out = outside01(tu);
+  if (s_out || t_out) {
+    const double ic = rcp64(c);
+    if (s_out) tc = clamp01_64(fma(b, sc, e) * ic);
+    if (t_out) {
+      sc = clamp01_64(fma(b, tc, -d) * rcp64(a));
+      tc = clamp01_64(fma(b, sc, e) * ic);
+    }
+  }
+  double v[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) v[i] = fma(-tc, dB[i], fma(sc, dA[i], w[i]));
+  const double d2 = fdot3(v, v);
+  const double pp = fdot3(pt1, pt1), qq = fdot3(pn, pn);
+  if (!(in_range64<-190, 300>(d2) && near_one64(qq) && in_range64<-60, 60>(pp))) return false;
+  const double iv = rsqrt64(d2);
+  double dist = d2 * iv;
+  dist = fma(fma(-dist, dist, d2), 0.5 * iv, dist);
+  double nn[3], no[3], tr[3], vx[3];
+  const double iq = fma(-0.5, qq, 1.5);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    nn[i] = v[i] * iv;
+    no[i] = pn[i] * iq;
+  }
+  fcross3(no, nn, v);
+  const double cv = fdot3(no, nn);
+  if (!(__double2hiint(cv + 0.5) > 0)) return false;
+  fcross3(v, pt1, vx);
+  const double f = fdot3(v, pt1) * rcp64(1.0 + cv);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) tr[i] = fma(f, v[i], fma(cv, pt1[i], vx[i]));
+  const double dn = fdot3(tr, nn);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) tr[i] = fma(-dn, nn[i], tr[i]);
+  const double rr = fdot3(tr, tr);
+  if (!in_range64<-60, 60>(rr)) return false;
+  const double ir = near_one64(rr) ? fma(-0.5, rr, 1.5) : rsqrt64(rr);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    n[i] = nn[i];
+    t1[i] = tr[i] * ir;
+  }
+  fcross3(n, t1, t2);
+  s = sc;
+  t = tc;
+  gap = dist - rs;
+  return true;
+}
+
+// the exact routine, out of line so that its registers stay out of the common path; it writes the table
+__noinline__ __device__ void narrow64_exact(const xk_mesh& m, const xk_pairs& p, const double* __restrict__ u, int i) {
+  narrow_exact_one(m, p, u, 0.0, 0.0, 0, 0, i);
+}
+
+// Narrowphase of pair i (nodes nd, radius sum rs: the cores' on coated wires), written to the table.
+XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const int* nd, double rs,
+                        const double* __restrict__ u, double& s, double& t, double& gap, double* n, double* t1,
+                        double* t2) {
+  const long long cap = p.cap;
+  double x[4][3], pt1[3], pn[3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[k][c] = m.X[3LL * nd[k] + c] + u[6LL * nd[k] + c];
+  load3(p.t1, cap, i, pt1);
+  load3(p.normal, cap, i, pn);
+  if (narrow64(x, rs, pn, pt1, s, t, gap, n, t1, t2)) {
+    p.s[i] = s;
+    p.t[i] = t;
+    p.gap[i] = gap;
+    store3(p.normal, cap, i, n);
+    store3(p.t1, cap, i, t1);
+    store3(p.t2, cap, i, t2);
+    if (m.core_radii && p.coat_cc) p.coat_cc[i] = coat_compression(m, p.ea[i], p.eb[i], gap);
+  } else {
+    narrow64_exact(m, p, u, i);
+    s = p.s[i];
+    t = p.t[i];
+    gap = p.gap[i];
+    load3(p.normal, cap, i, n);
+    load3(p.t1, cap, i, t1);
+    load3(p.t2, cap, i, t2);
+  }
+}
+
+XK_D double narrow_radii(const xk_mesh& m, int ea, int eb) {
+  const double* r = m.core_radii ? m.core_radii : m.radii;
+  return r[ea] + r[eb];
+}
+
+constexpr int PAIR64_T = 128;
+__global__ void __launch_bounds__(PAIR64_T) k_pair_other64(const __grid_constant__ xk_mesh m,
+                                                           const __grid_constant__ xk_pairs p,
+                                                           const int32_t* __restrict__ others, int n_o,
+                                                           const double* __restrict__ u) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= n_o) return;
+  const int i = others[o];
+  const int ea = p.ea[i], eb = p.eb[i];
+  const PairNodes pn = pair_nodes(m, ea, eb);
+  double s, t, gap, n[3], t1[3], t2[3];
+  pair_narrow64(m, p, i, pn.n, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+}
+
+// Contributing pairs, all four stages, combined records.  The frame is orthonormal (just formed), so the
+// geometric friction term q0 n t1^T + q1 t2 n^T - q1 [t1]x^T is n (q0 t1 + q1 t2)^T, since
+// [t1]x = n t2^T - t2 n^T, and the record's B = n (x) ((wm + wg) n + vf / dist) - wg I - T D T^T.
+template <bool COAT>
+__global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constant__ xk_mesh m,
+                                                            const __grid_constant__ xk_pairs p,
+                                                            const int32_t* __restrict__ members,
+                                                            const int32_t* __restrict__ mnodes, int n_m,
+                                                            const double* __restrict__ u,
+                                                            const double* __restrict__ u_ref,
+                                                            const __grid_constant__ xk_contact_params cp, double dh,
+                                                            int rec_vec, double* __restrict__ rec) {
+  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (mi >= n_m) return;
+  const int i = members[mi];
+  const long long cap = p.cap;
+  int nd[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) nd[k] = mnodes[4LL * mi + k];
+  const int ea = p.ea[i], eb = p.eb[i];
+  uint8_t status = p.status[i];
+  double p_n = p.p_n[i];
+  double s, t, gap, n[3], t1[3], t2[3];
+  pair_narrow64(m, p, i, nd, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  double v[3] = {0.0, 0.0, 0.0};
+  // normal force
+  const double xpen = -cp.k_pen * gap;
+  if (status != ST_INACTIVE) {
+    p_n = huber(xpen, dh);
+    p.p_n[i] = p_n;
+    if (p_n > 1e-30) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = p_n * n[k];
+    }
+  }
+  // friction
+  const double mu_eff = m.mu ? m.mu[ea] : cp.mu_eff;
+  const bool fproc = p_n > 0.0 && mu_eff > 0.0;
+  double e[3] = {0.0, 0.0, 0.0}, g[3] = {0.0, 0.0, 0.0};  // T D T^T = t1 (x) e + t2 (x) g
+  double vf[3] = {0.0, 0.0, 0.0};
+  bool fric = false;
+  double du[4][3];
+  if (fproc || COAT) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long dof = 6LL * nd[k] + c;
+        du[k][c] = u_ref ? u[dof] - u_ref[dof] : u[dof];
+      }
+  }
+  if (fproc) {
+    double kt = p.k_t[i];
+    if (p.k_pen[i] <= 0.0) {
+      p.k_pen[i] = cp.k_pen;
+      kt = cp.k_pen * cp.k_t_ratio;
+      p.k_t[i] = kt;
+    }
+    double dr[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      dr[c] = fma(t, du[3][c] - du[2][c], du[2][c]) - fma(s, du[1][c] - du[0][c], du[0][c]);
+    const double d0 = fdot3(dr, t1), d1 = fdot3(dr, t2);
+    const double q0 = fma(kt, d0, p.z_t[i]), q1 = fma(kt, d1, p.z_t[cap + i]);
+    const double q2 = fma(q0, q0, q1 * q1);
+    const bool ord = in_range64<-190, 300>(q2);  // else (no slip at all, or out of range): the plain functions
+    const double iq = ord ? rsqrt64(q2) : 0.0;
+    double qn = q2 * iq;
+    qn = ord ? fma(fma(-qn, qn, q2), 0.5 * iq, qn) : sqrt(q2);
+    const double fy = mu_eff * p_n;
+    const bool stick = qn <= fy;
+    double r0 = q0, r1 = q1, kr = kt, h0 = 0.0, h1 = 0.0;  // D = kr (I - h h^T)
+    if (!stick) {
+      const double inv = ord ? iq : 1.0 / qn;
+      h0 = q0 * inv;
+      h1 = q1 * inv;
+      r0 = fy * h0;
+      r1 = fy * h1;
+      kr = fy * inv * kt;
+    }
+    p.z_t[i] = r0;
+    p.z_t[cap + i] = r1;
+    p.stick[i] = stick ? 1 : 0;
+    p.q_trial_norm[i] = qn;
+    p.dissipation[i] = fma(r0, d0, r1 * d1);
+    status = stick ? ST_ACTIVE : ST_SLIDING;
+    p.status[i] = status;
+    fric = (stick ? qn : fy) >= 1e-30;  // |(r0, r1)|
+    if (fric) {
+      const double D01 = -kr * h0 * h1, D00 = fma(-kr * h0, h0, kr), D11 = fma(-kr * h1, h1, kr);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        vf[k] = fma(r0, t1[k], r1 * t2[k]);
+        v[k] += vf[k];
+        e[k] = fma(D00, t1[k], D01 * t2[k]);
+        g[k] = fma(D01, t1[k], D11 * t2[k]);
+      }
+    }
+  }
+  // pair tangent
+  double B[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) B[k] = 0.0;
+  if (status != ST_INACTIVE) {
+    const double dist = (gap + m.radii[ea]) + m.radii[eb];
+    const double hd = huber_deriv(xpen, dh);
+    const bool nrm = !(hd < 1e-30 && p_n < 1e-30);
+    const double idist = in_range64<-45, 300>(dist) ? rcp64(dist) : (dist > 1e-15 ? 1.0 / dist : 0.0);
+    const double wg = nrm ? p_n * idist : 0.0, wn = nrm ? fma(hd, cp.k_pen, wg) : 0.0;
+    double w[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) w[b] = fma(idist, vf[b], wn * n[b]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) B[3 * a + b] = fma(n[a], w[b], -fma(t1[a], e[b], t2[a] * g[b]));
+    B[0] -= wg;
+    B[4] -= wg;
+    B[8] -= wg;
+  }
+  if (COAT)
+    coating_epilogue<double, double>(cp, p.coat_cc_prev, p.coat_z_t, p.coat_qtn, p.coat_diss, p.coat_stick, i, cap,
+                                     p.coat_cc[i], s, t, n, t1, t2, du, v, B);
+  double* r = rec + (long long)mi * XK_REC_STRIDE_COMBINED;
+  const double o[16] = {B[0], B[1], B[2], B[3], B[4], B[5], B[6], B[7], B[8], s, t, v[0], v[1], v[2], 0.0, 0.0};
+  static_assert(XK_REC_B == 0 && XK_REC_S == 9 && XK_REC_V == 11, "combined record layout");
+  if (rec_vec) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)  // whole 32-byte sectors
+      asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(r + 4 * k), "d"(o[4 * k]), "d"(o[4 * k + 1]),
+                   "d"(o[4 * k + 2]), "d"(o[4 * k + 3])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) r[k] = o[k];
+  }
+}
+
+// CTA size of the FP64 pair kernels: the FP64 pipe of every SM is what they need, so a small table is cut
+// into CTAs of one or two warps that reach all SMs (6,500 contributing pairs: 26 CTAs of 256 took 57 us, the same work in 204 of 32 takes 15 us).
+int pair64_block(long long n) {
+  const long long sms = xk_sm_count();
+  return n >= 4 * sms * PAIR64_T ? PAIR64_T : (n >= 2 * sms * 64 ? 64 : 32);
 }
 
 // Pairs that cannot contribute in this increment: only the frozen narrowphase,
@@ -1248,11 +1543,11 @@ extern "C" xk_status xk_pair_step(const xk_mesh* m, xk_pairs* p, const xk_contac
     return xk_set_error(XK_ERR_ARG, "xk_pair_step: pattern was built for another pair table");
   cudaStream_t st = (cudaStream_t)s;
   if ((stages & XK_STAGE_NARROW) && !(stages & XK_STAGE_NO_OTHERS) && pat->n_others > 0) {
-    const int nb = xk_blocks(pat->n_others, PAIR_T);
-    if (precision == XK_FP64)
-      k_pair_other<XK_FP64><<<nb, PAIR_T, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
-    else if (precision == XK_MIXED)
-      k_pair_other<XK_MIXED><<<nb, PAIR_T, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
+    if (precision == XK_FP64) {
+      const int bs = pair64_block(pat->n_others);
+      k_pair_other64<<<xk_blocks(pat->n_others, bs), bs, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
+    } else if (precision == XK_MIXED)
+      k_pair_other<XK_MIXED><<<xk_blocks(pat->n_others, PAIR_T), PAIR_T, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
     else
       return xk_set_error(XK_ERR_ARG, "xk_pair_step: precision");
     XK_CHECK_LAUNCH();
@@ -1261,6 +1556,20 @@ extern "C" xk_status xk_pair_step(const xk_mesh* m, xk_pairs* p, const xk_contac
   const int nb = xk_blocks(pat->n_members, PAIR_T);
   const long long rs = out_mode == XK_OUT_COMBINED ? XK_REC_STRIDE_COMBINED : XK_REC_STRIDE_SPLIT;
   const bool coat = m->core_radii && p->coat_cc;
+  // combined FP64 records after the narrowphase (the engine's case, whose frame is orthonormal as it is used)
+  if (precision == XK_FP64 && out_mode == XK_OUT_COMBINED && (stages & XK_STAGE_NARROW)) {
+    const double dh = cp->smoothing_delta > 0.0 ? cp->k_pen / cp->smoothing_delta : 0.0;
+    const int bs = pair64_block(pat->n_members), nb64 = xk_blocks(pat->n_members, bs);
+    const int rv = ((uintptr_t)rec & 31) == 0;
+    if (coat)
+      k_pair_member64<true><<<nb64, bs, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u, u_ref, *cp,
+                                                 dh, rv, (double*)rec);
+    else
+      k_pair_member64<false><<<nb64, bs, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u, u_ref,
+                                                  *cp, dh, rv, (double*)rec);
+    XK_CHECK_LAUNCH();
+    return XK_OK;
+  }
 #define XK_MEMBER_LAUNCH(PP, OO, CC, TT)                                                                        \
   k_pair_member<PP, OO, CC><<<nb, PAIR_T, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u,  \
                                                    u_ref, *cp, stages, (TT*)rec, rs)

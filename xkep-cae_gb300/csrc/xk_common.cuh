@@ -105,6 +105,32 @@ XK_D double xk_f2d(float v) {
   return __hiloint2double((int)((f & 0x80000000u) | ((e + 896u) << 20) | ((f & 0x7fffffu) >> 3)), (int)(f << 29));
 }
 
+// FP64 on the FP64 pipe is scarce (about two operations per clock and SM; a divide or a square root takes some
+// ten of them).  1/x and 1/sqrt(x) for x in the ordinary range: the approximate instruction and two Newton-Raphson steps
+// (r <- r + r (1 - x r); y <- y + y (1/2 - x y^2 / 2)), within a few units of the last place.
+XK_D double rcp64(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+XK_D double rsqrt64(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = 0.5 * x;
+  y = fma(y, fma(-h * y, y, 0.5), y);
+  return fma(y, fma(-h * y, y, 0.5), y);
+}
+// x in [2^lo, 2^hi), tested on the high word: false for zero, negative values, infinities and NaN
+template <int LO, int HI>
+XK_D bool in_range64(double x) {
+  return (unsigned)(__double2hiint(x) - ((1023 + LO) << 20)) < (unsigned)((HI - LO) << 20);
+}
+// x in [1 - 2^-32, 1 + 2^-30): a unit vector's square up to rounding, where 1/sqrt(x) = 3/2 - x/2 to 2^-61
+XK_D bool near_one64(double x) {
+  return (unsigned long long)(__double_as_longlong(x) - 0x3fefffffffe00000LL) < 0x600000ULL;
+}
+
 // Eight floats from a 32-byte aligned read-only address in one 256-bit load.
 XK_D void ldg8(const float* __restrict__ p, float* v) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
