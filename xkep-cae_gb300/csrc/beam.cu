@@ -48,10 +48,9 @@ XK_D void rotvec_of_quat(const double* qin, double* th) {
   double s2 = x * x + y * y + z * z;
   double coef;
   if (s2 < 0.0025 * w * w) {  // |v|/w < 0.05: 2 atan(r)/(r w) by its series
-    const double iw = rcp64(w);  // w is at least 0.998 here
-    const double r2 = s2 * (iw * iw);
+    double r2 = div64(s2, w * w);
     double at = 1.0 + r2 * (-1.0 / 3 + r2 * (1.0 / 5 + r2 * (-1.0 / 7 + r2 * (1.0 / 9 + r2 * (-1.0 / 11 + r2 * (1.0 / 13))))));
-    coef = 2.0 * at * iw;
+    coef = div64(2.0 * at, w);
   } else {
     double sh = sqrt(s2);
     coef = 2.0 * atan2(sh, w) / sh;
@@ -83,8 +82,8 @@ XK_D void quat_between(const double* e0, const double* e1, double* q) {
     }
     return;
   }
-  double w = sqrt(0.5 * (1.0 + c));
-  double k = 0.5 / w;
+  double w = sqrt64(0.5 * (1.0 + c));
+  double k = div64(0.5, w);
   q[0] = w; q[1] = k * v[0]; q[2] = k * v[1]; q[3] = k * v[2];
 }
 
@@ -214,16 +213,22 @@ struct KeCoef {
 template <typename T>
 XK_D T sec_val(double x);
 template <>
+XK_D double sec_val<double>(double x) { return x; }
+template <>
 XK_D float sec_val<float>(double x) { return xk_d2f(x); }
+
+// a / b: the same bits as the operator, in double on fewer FP64 operations
+XK_D float quot(float a, float b) { return a / b; }
+XK_D double quot(double a, double b) { return div64(a, b); }
 
 template <typename T>
 XK_D KeCoef<T> ke_coef(const xk_section& s, T L0) {
   T L = L0;
-  T iL = T(1) / L;
+  T iL = quot(T(1), L);
   T E = sec_val<T>(s.E), G = sec_val<T>(s.G), A = sec_val<T>(s.A), Iy = sec_val<T>(s.Iy), Iz = sec_val<T>(s.Iz),
     J = sec_val<T>(s.J);
-  T phy = T(12) * E * Iy / (sec_val<T>(s.kappa_y) * G * A * L * L);
-  T phz = T(12) * E * Iz / (sec_val<T>(s.kappa_z) * G * A * L * L);
+  T phy = quot(T(12) * E * Iy, sec_val<T>(s.kappa_y) * G * A * L * L);
+  T phz = quot(T(12) * E * Iz, sec_val<T>(s.kappa_z) * G * A * L * L);
   if (__double_as_longlong(s.scf) > 0 && __double_as_longlong(s.scf) <= 0x7ff0000000000000LL) {  // scf > 0
     T sc = sec_val<T>(s.scf);
     phy = phy / (T(1) + sc * L * L * A / (T(12) * Iy));
@@ -232,7 +237,7 @@ XK_D KeCoef<T> ke_coef(const xk_section& s, T L0) {
   KeCoef<T> k;
   k.ea = E * A * iL;
   k.gj = G * J * iL;
-  T dy = T(1) / (T(1) + phy), dz = T(1) / (T(1) + phz);
+  T dy = quot(T(1), T(1) + phy), dz = quot(T(1), T(1) + phz);
   T eiy = E * Iy * iL, eiz = E * Iz * iL;
   k.k3y = T(12) * eiy * iL * iL * dy;
   k.k2y = T(6) * eiy * iL * dy;
@@ -511,185 +516,28 @@ XK_D int sym_index(int r, int c) {  // position of (r, c) in a symmetric 3x3 sto
 }
 
 // sym(X) of a row-major 3x3 into the 6-value form
-template <typename T>
-XK_D void sym6(const T* X, T* S) {
+XK_D void sym6(const float* X, float* S) {
   S[0] = X[0];
-  S[1] = T(0.5) * (X[1] + X[3]);
-  S[2] = T(0.5) * (X[2] + X[6]);
+  S[1] = 0.5f * (X[1] + X[3]);
+  S[2] = 0.5f * (X[2] + X[6]);
   S[3] = X[4];
-  S[4] = T(0.5) * (X[5] + X[7]);
+  S[4] = 0.5f * (X[5] + X[7]);
   S[5] = X[8];
 }
 
 // M = sum of the outer products R_k (x) V_k (row-major)
-template <typename T>
-XK_D void outer2(const T* Ra, const T* Va, const T* Rb, const T* Vb, T* M) {
+XK_D void outer2(const float* Ra, const float* Va, const float* Rb, const float* Vb, float* M) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int c = 0; c < 3; ++c) M[3 * i + c] = Ra[i] * Va[c] + Rb[i] * Vb[c];
 }
-template <typename T>
-XK_D void outer3(const T* Ra, const T* Va, const T* Rb, const T* Vb, const T* Rc, const T* Vc, T* M) {
+XK_D void outer3(const float* Ra, const float* Va, const float* Rb, const float* Vb, const float* Rc,
+                 const float* Vc, float* M) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int c = 0; c < 3; ++c) M[3 * i + c] = Ra[i] * Va[c] + Rb[i] * Vb[c] + Rc[i] * Vc[c];
-}
-
-// The outputs of one element from its frame: global forces of the blocks and, with want_K, the six symmetrised
-// tangent blocks, written to the slot o as they are formed.  Rcr: the corotated frame, ex and iLd: the deformed
-// axis and 1/L, t1, t2: the local rotations, tha, thb: the nodal rotation vectors, dax: the axial stretch.
-template <typename T>
-XK_D void beam_slots(const KeCoef<T>& kc, const T* Rcr, const T* ex, T iLd, const T* t1, const T* t2, const T* tha,
-                     const T* thb, T dax, bool want_K, T* o) {
-  // local forces of blocks 0, 1, 3 (block 2 = -block 0) and their global images g_I = Rcr^T f_I
-  T g0[3], g1[3], g3[3];
-  {
-    const T f0[3] = {-kc.ea * dax, kc.k2z * (t1[2] + t2[2]), -kc.k2y * (t1[1] + t2[1])};
-    const T f1[3] = {kc.gj * (t1[0] - t2[0]), kc.k1ay * t1[1] + kc.k1by * t2[1],
-                         kc.k1az * t1[2] + kc.k1bz * t2[2]};
-    const T f3[3] = {-f1[0], kc.k1by * t1[1] + kc.k1ay * t2[1], kc.k1bz * t1[2] + kc.k1az * t2[2]};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      g0[i] = Rcr[i] * f0[0] + Rcr[3 + i] * f0[1] + Rcr[6 + i] * f0[2];
-      g1[i] = Rcr[i] * f1[0] + Rcr[3 + i] * f1[1] + Rcr[6 + i] * f1[2];
-      g3[i] = Rcr[i] * f3[0] + Rcr[3 + i] * f3[1] + Rcr[6 + i] * f3[2];
-      o[EL_G0 + i] = g0[i];
-      o[EL_G1 + i] = g1[i];
-      o[EL_G3 + i] = g3[i];
-    }
-  }
-  if (!want_K) return;
-  const T* R_0 = Rcr;
-  const T* R_1 = Rcr + 3;
-  const T* R_2 = Rcr + 6;
-  // P_s = T^-1(t_s) dpsi with dpsi = Rcr [e_x]x / L: row i of M [e_x]x is M_i x e_x, M = T^-1 Rcr;
-  // Q_s = T^-1(t_s) Rcr T(theta_node)
-  T P1[9], P2[9], Q1[9], Q2[9];
-#pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    T Ti[9], Ts[9], M[9];
-    tangent_ops<T>(side ? t2 : t1, true, Ti);
-    tangent_ops<T>(side ? thb : tha, false, Ts);
-    mm3(Ti, Rcr, M);
-    T* P = side ? P2 : P1;
-    T* Q = side ? Q2 : Q1;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      T c[3];
-      cross3(M + 3 * i, ex, c);
-      P[3 * i] = c[0] * iLd;
-      P[3 * i + 1] = c[1] * iLd;
-      P[3 * i + 2] = c[2] * iLd;
-    }
-    mm3(M, Ts, Q);
-  }
-  // G_I = Rcr^T A_I + geometric term; G1^T / 2 and G3^T / 2 go to the S01 and S03 slots at once
-  // (0.5 x + 0.5 y rounds as 0.5 (x + y)), so that P1, P2 and the forces end here
-  {
-    T v0[3], v1[3], v2[3], G[9];
-    const T d1 = dot3(g1, ex), d3 = dot3(g3, ex), d0 = dot3(g0, ex);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = kc.gj * (P1[c] - P2[c]);
-      v1[c] = kc.k1ay * P1[3 + c] + kc.k1by * P2[3 + c];
-      v2[c] = kc.k1az * P1[6 + c] + kc.k1bz * P2[6 + c];
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        o[EL_S01 + 3 * c + i] = T(0.5) * (G[3 * i + c] + iLd * (ex[i] * g1[c] - (i == c ? d1 : T(0))));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = -v0[c];
-      v1[c] = kc.k1by * P1[3 + c] + kc.k1ay * P2[3 + c];
-      v2[c] = kc.k1bz * P1[6 + c] + kc.k1az * P2[6 + c];
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        o[EL_S03 + 3 * c + i] = T(0.5) * (G[3 * i + c] + iLd * (ex[i] * g3[c] - (i == c ? d3 : T(0))));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v0[c] = kc.ea * ex[c];
-      v1[c] = kc.k2z * (P1[6 + c] + P2[6 + c]);
-      v2[c] = -kc.k2y * (P1[3 + c] + P2[3 + c]);
-    }
-    outer3(R_0, v0, R_1, v1, R_2, v2, G);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) G[3 * i + c] += iLd * (ex[i] * g0[c] - (i == c ? d0 : T(0)));
-    T S[6];
-    sym6(G, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
-  }
-  {
-    T a1[3], a2[3], b0[3], X[9], S[6];
-    // H0, J0: the I = 0 rows against Q1, Q2, added to the halves of G1^T, G3^T
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      a1[c] = kc.k2z * Q1[6 + c];
-      a2[c] = -kc.k2y * Q1[3 + c];
-    }
-    outer2(R_1, a1, R_2, a2, X);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S01 + i] += T(0.5) * X[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      a1[c] = kc.k2z * Q2[6 + c];
-      a2[c] = -kc.k2y * Q2[3 + c];
-    }
-    outer2(R_1, a1, R_2, a2, X);
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S03 + i] += T(0.5) * X[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = kc.gj * Q1[c];
-      a1[c] = kc.k1ay * Q1[3 + c];
-      a2[c] = kc.k1az * Q1[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H1
-    sym6(X, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S11 + i] = S[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = kc.gj * Q2[c];
-      a1[c] = kc.k1ay * Q2[3 + c];
-      a2[c] = kc.k1az * Q2[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J3
-    sym6(X, S);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) o[EL_S33 + i] = S[i];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = -kc.gj * Q1[c];
-      a1[c] = kc.k1by * Q1[3 + c];
-      a2[c] = kc.k1bz * Q1[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H3
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = T(0.5) * X[3 * i + c];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      b0[c] = -kc.gj * Q2[c];
-      a1[c] = kc.k1by * Q2[3 + c];
-      a2[c] = kc.k1bz * Q2[6 + c];
-    }
-    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J1
-#pragma unroll
-    for (int i = 0; i < 9; ++i) o[EL_S13 + i] += T(0.5) * X[i];
-  }
 }
 
 // One element: frame (the rotation vectors of both nodes by one thread), global forces of the
@@ -753,7 +601,154 @@ XK_D void beam_elem32(const float* __restrict__ E, const float* __restrict__ NA,
       for (int j = 0; j < 3; ++j)
         Rcr[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
   }
-  beam_slots<float>(ke_coef<float>(sec, L0), Rcr, ex, iLd, t1, t2, ua + 3, ub + 3, dax, want_K, o);
+  const KeCoef<float> kc = ke_coef<float>(sec, L0);
+  // local forces of blocks 0, 1, 3 (block 2 = -block 0) and their global images g_I = Rcr^T f_I
+  float g0[3], g1[3], g3[3];
+  {
+    const float f0[3] = {-kc.ea * dax, kc.k2z * (t1[2] + t2[2]), -kc.k2y * (t1[1] + t2[1])};
+    const float f1[3] = {kc.gj * (t1[0] - t2[0]), kc.k1ay * t1[1] + kc.k1by * t2[1],
+                         kc.k1az * t1[2] + kc.k1bz * t2[2]};
+    const float f3[3] = {-f1[0], kc.k1by * t1[1] + kc.k1ay * t2[1], kc.k1bz * t1[2] + kc.k1az * t2[2]};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      g0[i] = Rcr[i] * f0[0] + Rcr[3 + i] * f0[1] + Rcr[6 + i] * f0[2];
+      g1[i] = Rcr[i] * f1[0] + Rcr[3 + i] * f1[1] + Rcr[6 + i] * f1[2];
+      g3[i] = Rcr[i] * f3[0] + Rcr[3 + i] * f3[1] + Rcr[6 + i] * f3[2];
+      o[EL_G0 + i] = g0[i];
+      o[EL_G1 + i] = g1[i];
+      o[EL_G3 + i] = g3[i];
+    }
+  }
+  if (!want_K) return;
+  const float* R_0 = Rcr;
+  const float* R_1 = Rcr + 3;
+  const float* R_2 = Rcr + 6;
+  // P_s = T^-1(t_s) dpsi with dpsi = Rcr [e_x]x / L: row i of M [e_x]x is M_i x e_x, M = T^-1 Rcr;
+  // Q_s = T^-1(t_s) Rcr T(theta_node)
+  float P1[9], P2[9], Q1[9], Q2[9];
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    float Ti[9], Ts[9], M[9];
+    tangent_ops<float>(side ? t2 : t1, true, Ti);
+    tangent_ops<float>(side ? ub + 3 : ua + 3, false, Ts);
+    mm3(Ti, Rcr, M);
+    float* P = side ? P2 : P1;
+    float* Q = side ? Q2 : Q1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      float c[3];
+      cross3(M + 3 * i, ex, c);
+      P[3 * i] = c[0] * iLd;
+      P[3 * i + 1] = c[1] * iLd;
+      P[3 * i + 2] = c[2] * iLd;
+    }
+    mm3(M, Ts, Q);
+  }
+  // G_I = Rcr^T A_I + geometric term; G1^T / 2 and G3^T / 2 go to the S01 and S03 slots at once
+  // (0.5 x + 0.5 y rounds as 0.5 (x + y)), so that P1, P2 and the forces end here
+  {
+    float v0[3], v1[3], v2[3], G[9];
+    const float d1 = dot3(g1, ex), d3 = dot3(g3, ex), d0 = dot3(g0, ex);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = kc.gj * (P1[c] - P2[c]);
+      v1[c] = kc.k1ay * P1[3 + c] + kc.k1by * P2[3 + c];
+      v2[c] = kc.k1az * P1[6 + c] + kc.k1bz * P2[6 + c];
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[EL_S01 + 3 * c + i] = 0.5f * (G[3 * i + c] + iLd * (ex[i] * g1[c] - (i == c ? d1 : 0.f)));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = -v0[c];
+      v1[c] = kc.k1by * P1[3 + c] + kc.k1ay * P2[3 + c];
+      v2[c] = kc.k1bz * P1[6 + c] + kc.k1az * P2[6 + c];
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[EL_S03 + 3 * c + i] = 0.5f * (G[3 * i + c] + iLd * (ex[i] * g3[c] - (i == c ? d3 : 0.f)));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      v0[c] = kc.ea * ex[c];
+      v1[c] = kc.k2z * (P1[6 + c] + P2[6 + c]);
+      v2[c] = -kc.k2y * (P1[3 + c] + P2[3 + c]);
+    }
+    outer3(R_0, v0, R_1, v1, R_2, v2, G);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) G[3 * i + c] += iLd * (ex[i] * g0[c] - (i == c ? d0 : 0.f));
+    float S[6];
+    sym6(G, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
+  }
+  {
+    float a1[3], a2[3], b0[3], X[9], S[6];
+    // H0, J0: the I = 0 rows against Q1, Q2, added to the halves of G1^T, G3^T
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      a1[c] = kc.k2z * Q1[6 + c];
+      a2[c] = -kc.k2y * Q1[3 + c];
+    }
+    outer2(R_1, a1, R_2, a2, X);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S01 + i] += 0.5f * X[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      a1[c] = kc.k2z * Q2[6 + c];
+      a2[c] = -kc.k2y * Q2[3 + c];
+    }
+    outer2(R_1, a1, R_2, a2, X);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S03 + i] += 0.5f * X[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = kc.gj * Q1[c];
+      a1[c] = kc.k1ay * Q1[3 + c];
+      a2[c] = kc.k1az * Q1[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H1
+    sym6(X, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S11 + i] = S[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = kc.gj * Q2[c];
+      a1[c] = kc.k1ay * Q2[3 + c];
+      a2[c] = kc.k1az * Q2[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J3
+    sym6(X, S);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S33 + i] = S[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = -kc.gj * Q1[c];
+      a1[c] = kc.k1by * Q1[3 + c];
+      a2[c] = kc.k1bz * Q1[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // H3
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = 0.5f * X[3 * i + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      b0[c] = -kc.gj * Q2[c];
+      a1[c] = kc.k1by * Q2[3 + c];
+      a2[c] = kc.k1bz * Q2[6 + c];
+    }
+    outer3(R_0, b0, R_1, a1, R_2, a2, X);  // J1
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S13 + i] += 0.5f * X[i];
+  }
 }
 
 // Value (r, c) of a stored 6x6 block of one element, from its slot o:
@@ -1007,45 +1002,56 @@ __global__ void __launch_bounds__(BEAMW_T, 6) k_beam32e(int mode, xk_mesh m, xk_
   }
 }
 
-// The FP64 beam: the same element outputs and write-back in double.  What bounds it is the FP64 pipe, so the
-// element takes the six-block form (about 2.4 times fewer operations than the full rows of beam_tail),
-// reciprocals by Newton-Raphson, section constants formed once on the host and the frame from the displacement
-// differences, as in the float element, and an ordered wire mesh runs in one launch instead of one per colour.
+// The FP64 beam: the same element outputs and write-back in double.  What bounds it is the FP64 pipe, and
+// beam_tail spends most of it on the zeros of the local stiffness (a product with a zero constant is not
+// folded away) and on the block rows that are the negatives of others.  Here every sum keeps the terms and
+// the order that beam_tail's have once its zeros are left out, so the values are the same to the last place
+// (bit for bit at u = 0, where an increment's first tangent is formed); divides and square roots are the
+// correctly rounded ones on fewer operations (div64, sqrt64), and an ordered wire mesh runs in one launch
+// instead of one per colour.
 // CTAs of one warp: a small mesh then reaches every SM (4,736 elements: 153 CTAs), where CTAs of 128 threads,
 // one launch after another, left most of them idle.
-// Measured, colour launches of beam_tail against this: 98,592 elements 406 -> 242 us, 4,736 elements
-// 157 -> 46 us (a warp issues one FP64 instruction in 64 clocks, so one warp per SM is what that mesh allows).
+// Measured, colour launches of beam_tail against this: 98,592 elements 406 -> 265 us, 4,736 elements
+// 157 -> 52 us (a warp issues one FP64 instruction in 64 clocks, and that mesh has one warp per SM).
 constexpr int BEAM64_T = 32;
-struct BeamConst64 {  // E A, G J, E Iy, E Iz; 12 E I / (kappa G A); A / (12 I) * scf (0: off)
-  double ea, gj, eiy, eiz, py, pz, sy, sz;
-};
 
-XK_D KeCoef<double> ke_coef64(const BeamConst64& s, double iL, double L) {
-  double phy = s.py * iL * iL, phz = s.pz * iL * iL;
-  if (s.sy > 0.0) {
-    phy = phy / (1.0 + s.sy * L * L);
-    phz = phz / (1.0 + s.sz * L * L);
+// R^T A from the rows of both: fma(R2i, A2c, fma(R0i, A0c, R1i A1c)), the contraction of mtm3
+XK_D void rta3(const double* R, const double* a0, const double* a1, const double* a2, double* M) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) M[3 * i + c] = fma(R[6 + i], a2[c], fma(R[i], a0[c], R[3 + i] * a1[c]));
+}
+// the same with a zero row 0
+XK_D void rta2(const double* R, const double* a1, const double* a2, double* M) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) M[3 * i + c] = fma(R[6 + i], a2[c], R[3 + i] * a1[c]);
+}
+// A += [f]x D by rows
+XK_D void add_skew(const double* f, const double* D, double* a0, double* a1, double* a2) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] += fma(f[1], D[6 + c], -f[2] * D[3 + c]);
+    a1[c] += fma(-f[0], D[6 + c], f[2] * D[c]);
+    a2[c] += fma(-f[1], D[c], f[0] * D[3 + c]);
   }
-  KeCoef<double> k;
-  k.ea = s.ea * iL;
-  k.gj = s.gj * iL;
-  const double ky = s.eiy * iL * rcp64(1.0 + phy), kz = s.eiz * iL * rcp64(1.0 + phz);
-  k.k3y = 12.0 * ky * iL * iL;
-  k.k2y = 6.0 * ky * iL;
-  k.k1ay = (4.0 + phy) * ky;
-  k.k1by = (2.0 - phy) * ky;
-  k.k3z = 12.0 * kz * iL * iL;
-  k.k2z = 6.0 * kz * iL;
-  k.k1az = (4.0 + phz) * kz;
-  k.k1bz = (2.0 - phz) * kz;
-  return k;
+}
+XK_D void sym6d(const double* X, double* S) {
+  S[0] = X[0];
+  S[1] = 0.5 * (X[1] + X[3]);
+  S[2] = 0.5 * (X[2] + X[6]);
+  S[3] = X[4];
+  S[4] = 0.5 * (X[5] + X[7]);
+  S[5] = X[8];
 }
 
 XK_D void beam_elem64(const xk_mesh& m, const double* __restrict__ ref, const double* __restrict__ u,
-                      const BeamConst64& sec, long long e, int a, int b, bool want_K, double* o) {
+                      const xk_section& sec, long long e, int a, int b, bool want_K, double* o) {
   const long long ne = m.n_elems;
   const double L0 = ref[e];
-  double R0[9], ua[6], ub[6], dx0[3], du[3], dx[3];
+  double R0[9], ua[6], ub[6], dx[3];
 #pragma unroll
   for (int i = 0; i < 9; ++i) R0[i] = ref[(1 + i) * ne + e];
 #pragma unroll
@@ -1054,39 +1060,12 @@ XK_D void beam_elem64(const xk_mesh& m, const double* __restrict__ ref, const do
     ub[i] = u[6LL * b + i];
   }
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    dx0[i] = m.X[3LL * b + i] - m.X[3LL * a + i];
-    du[i] = ub[i] - ua[i];
-    dx[i] = dx0[i] + du[i];
-  }
-  const double L2 = dot3(dx, dx);
-  double iL, L;
-  if (in_range64<-300, 300>(L2)) {
-    iL = rsqrt64(L2);
-    L = L2 * iL;
-    L = fma(fma(-L, L, L2), 0.5 * iL, L);
-  } else {
-    L = sqrt(L2);
-    iL = 1.0 / L;
-  }
+  for (int i = 0; i < 3; ++i) dx[i] = (m.X[3LL * b + i] + ub[i]) - (m.X[3LL * a + i] + ua[i]);
+  const double L = sqrt64(dot3(dx, dx));
+  const double iL = div64(1.0, L);
   const double ex[3] = {dx[0] * iL, dx[1] * iL, dx[2] * iL};
-  const double sum[3] = {dx0[0] + dx[0], dx0[1] + dx[1], dx0[2] + dx[2]};
-  const double dax = dot3(du, sum) * (in_range64<-140, 140>(L + L0) ? rcp64(L + L0) : 1.0 / (L + L0));
-  // the smallest rotation of e0 (row 0 of R0) onto ex: 1 + e0 . ex = (L + L0 + e0 . du) / L, e0 x ex = e0 x du / L
   double qr[4];
-  const double opc = (L + L0 + dot3(R0, du)) * iL;
-  if (opc > 0.5) {
-    double v[3];
-    cross3(R0, du, v);
-    const double rw = rsqrt64(0.5 * opc);
-    const double k = 0.5 * iL * rw;
-    qr[0] = 0.5 * opc * rw;
-    qr[1] = k * v[0];
-    qr[2] = k * v[1];
-    qr[3] = k * v[2];
-  } else {
-    quat_between(R0, ex, qr);
-  }
+  quat_between(R0, ex, qr);  // R0 row 0 is e_x of the reference frame
   const double qrc[4] = {qr[0], -qr[1], -qr[2], -qr[3]};
   double t1[3], t2[3];
 #pragma unroll
@@ -1099,22 +1078,146 @@ XK_D void beam_elem64(const xk_mesh& m, const double* __restrict__ ref, const do
 #pragma unroll
     for (int i = 0; i < 3; ++i) t[i] = R0[3 * i] * tx[0] + R0[3 * i + 1] * tx[1] + R0[3 * i + 2] * tx[2];
   }
-  double Rrod[9], Rcr[9];
+  const double dax = L - L0;
+  double Rrod[9], R[9];
   rotmat_of_quat<double>(qr, Rrod);
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j)
-      Rcr[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
-  const double iL0 = in_range64<-140, 140>(L0) ? rcp64(L0) : 1.0 / L0;
-  beam_slots<double>(ke_coef64(sec, iL0, L0), Rcr, ex, iL, t1, t2, ua + 3, ub + 3, dax, want_K, o);
+      R[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
+  const KeCoef<double> k = ke_coef<double>(sec, L0);
+  const double f0[3] = {-k.ea * dax, k.k2z * (t1[2] + t2[2]), -k.k2y * (t1[1] + t2[1])};
+  const double f1[3] = {k.gj * (t1[0] - t2[0]), k.k1ay * t1[1] + k.k1by * t2[1], k.k1az * t1[2] + k.k1bz * t2[2]};
+  const double f3[3] = {-f1[0], k.k1by * t1[1] + k.k1ay * t2[1], k.k1bz * t1[2] + k.k1az * t2[2]};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    o[EL_G0 + i] = R[i] * f0[0] + R[3 + i] * f0[1] + R[6 + i] * f0[2];
+    o[EL_G1 + i] = R[i] * f1[0] + R[3 + i] * f1[1] + R[6 + i] * f1[2];
+    o[EL_G3 + i] = R[i] * f3[0] + R[3 + i] * f3[1] + R[6 + i] * f3[2];
+  }
+  if (!want_K) return;
+  // dpsi = R [e_x]x / L, P_s = T^-1(t_s) dpsi, Q_s = T^-1(t_s) R T(theta_node)
+  double D[9], P1[9], P2[9], Q1[9], Q2[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double* r = R + 3 * i;
+    D[3 * i] = fma(r[2], -ex[1], r[1] * ex[2]) * iL;
+    D[3 * i + 1] = fma(r[2], ex[0], r[0] * -ex[2]) * iL;
+    D[3 * i + 2] = fma(r[0], ex[1], r[1] * -ex[0]) * iL;
+  }
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    double Ti[9], Ts[9], M[9];
+    tangent_ops<double>(side ? t2 : t1, true, Ti);
+    tangent_ops<double>(side ? ub + 3 : ua + 3, false, Ts);
+    mm3(Ti, D, side ? P2 : P1);
+    mm3(Ti, R, M);
+    mm3(M, Ts, side ? Q2 : Q1);
+  }
+  double a0[3], a1[3], a2[3], X[9], S[6];
+  // the rows of A_I = (local stiffness against P1, P2 and the axis) + [f_I]x dpsi, then G_I = R^T A_I;
+  // G1^T / 2 and G3^T / 2 go to the S01 and S03 slots at once (0.5 x + 0.5 y rounds as 0.5 (x + y))
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = fma(k.gj, P1[c], -k.gj * P2[c]);
+    a1[c] = fma(k.k1ay, P1[3 + c], k.k1by * P2[3 + c]);
+    a2[c] = fma(k.k1az, P1[6 + c], k.k1bz * P2[6 + c]);
+  }
+  add_skew(f1, D, a0, a1, a2);
+  rta3(R, a0, a1, a2, X);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[EL_S01 + 3 * c + i] = 0.5 * X[3 * i + c];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = fma(-k.gj, P1[c], k.gj * P2[c]);
+    a1[c] = fma(k.k1by, P1[3 + c], k.k1ay * P2[3 + c]);
+    a2[c] = fma(k.k1bz, P1[6 + c], k.k1az * P2[6 + c]);
+  }
+  add_skew(f3, D, a0, a1, a2);
+  rta3(R, a0, a1, a2, X);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[EL_S03 + 3 * c + i] = 0.5 * X[3 * i + c];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = k.ea * ex[c];
+    a1[c] = fma(k.k2z, P1[6 + c], k.k2z * P2[6 + c]);
+    a2[c] = fma(-k.k2y, P1[3 + c], -k.k2y * P2[3 + c]);
+  }
+  add_skew(f0, D, a0, a1, a2);
+  rta3(R, a0, a1, a2, X);
+  sym6d(X, S);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
+  // H_I = R^T (local stiffness against Q1), J_I against Q2
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a1[c] = k.k2z * Q1[6 + c];
+    a2[c] = -k.k2y * Q1[3 + c];
+  }
+  rta2(R, a1, a2, X);  // H0
+#pragma unroll
+  for (int i = 0; i < 9; ++i) o[EL_S01 + i] = fma(0.5, X[i], o[EL_S01 + i]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a1[c] = k.k2z * Q2[6 + c];
+    a2[c] = -k.k2y * Q2[3 + c];
+  }
+  rta2(R, a1, a2, X);  // J0
+#pragma unroll
+  for (int i = 0; i < 9; ++i) o[EL_S03 + i] = fma(0.5, X[i], o[EL_S03 + i]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = k.gj * Q1[c];
+    a1[c] = k.k1ay * Q1[3 + c];
+    a2[c] = k.k1az * Q1[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);  // H1
+  sym6d(X, S);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) o[EL_S11 + i] = S[i];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = k.gj * Q2[c];
+    a1[c] = k.k1ay * Q2[3 + c];
+    a2[c] = k.k1az * Q2[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);  // J3
+  sym6d(X, S);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) o[EL_S33 + i] = S[i];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = -k.gj * Q1[c];
+    a1[c] = k.k1by * Q1[3 + c];
+    a2[c] = k.k1bz * Q1[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);  // H3
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = 0.5 * X[3 * i + c];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = -k.gj * Q2[c];
+    a1[c] = k.k1by * Q2[3 + c];
+    a2[c] = k.k1bz * Q2[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);  // J1
+#pragma unroll
+  for (int i = 0; i < 9; ++i) o[EL_S13 + i] = fma(0.5, X[i], o[EL_S13 + i]);
 }
 
-__global__ void __launch_bounds__(BEAM64_T) k_beam64(int mode, xk_mesh m, BeamConst64 sec, const double* __restrict__ ref,
-                                                     const int32_t* __restrict__ order, int k0, int k1,
-                                                     const int32_t* __restrict__ blk, const uint8_t* __restrict__ first,
-                                                     const double* __restrict__ u, double* __restrict__ f_int,
-                                                     double* __restrict__ Kv, int vec, long long n_threads) {
+__global__ void __launch_bounds__(BEAM64_T) k_beam64(int mode, xk_mesh m, xk_section sec,
+                                                     const double* __restrict__ ref, const int32_t* __restrict__ order,
+                                                     int k0, int k1, const int32_t* __restrict__ blk,
+                                                     const uint8_t* __restrict__ first, const double* __restrict__ u,
+                                                     double* __restrict__ f_int, double* __restrict__ Kv, int vec,
+                                                     long long n_threads) {
   __shared__ double slots[BEAM64_T * EL_STRIDE64];
   const long long t = (long long)blockIdx.x * BEAM64_T + threadIdx.x;
   if (t >= n_threads) return;  // n_threads is a multiple of 32 in the ordered mode
@@ -1194,19 +1297,6 @@ extern "C" xk_status xk_beam_reference(const xk_mesh* m, const double* v_ref, do
   return XK_OK;
 }
 
-static BeamConst64 beam_const64(const xk_section& s) {
-  BeamConst64 c;
-  c.ea = s.E * s.A;
-  c.gj = s.G * s.J;
-  c.eiy = s.E * s.Iy;
-  c.eiz = s.E * s.Iz;
-  c.py = 12.0 * c.eiy / (s.kappa_y * s.G * s.A);
-  c.pz = 12.0 * c.eiz / (s.kappa_z * s.G * s.A);
-  c.sy = s.scf > 0.0 ? s.scf * s.A / (12.0 * s.Iy) : 0.0;
-  c.sz = s.scf > 0.0 ? s.scf * s.A / (12.0 * s.Iz) : 0.0;
-  return c;
-}
-
 extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, const double* elem_ref,
                                       const xk_beam_plan* plan, const double* u, int precision, double* f_int,
                                       void* K_vals, xk_stream s) {
@@ -1214,12 +1304,11 @@ extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, c
   if (precision != XK_FP64 && precision != XK_MIXED) return xk_set_error(XK_ERR_ARG, "xk_beam_assemble: precision");
   if (!f_int && !K_vals) return XK_OK;
   cudaStream_t st = (cudaStream_t)s;
-  const BeamConst64 bc = beam_const64(*sec);
   const int vec = ((uintptr_t)K_vals & 15) == 0;
   if (precision == XK_FP64 && plan->node_diag && plan->chain_ordered) {  // one launch, one writer per block
     if (m->n_elems == 0) return XK_OK;
     const long long threads = 32 * ((long long)m->n_elems / 31 + 1);
-    k_beam64<<<xk_blocks(threads, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_ORDERED, *m, bc, elem_ref, nullptr, 0, 0, plan->blk,
+    k_beam64<<<xk_blocks(threads, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_ORDERED, *m, *sec, elem_ref, nullptr, 0, 0, plan->blk,
                                                                plan->first, u, f_int, (double*)K_vals, vec, threads);
     XK_CHECK_LAUNCH();
     return XK_OK;
@@ -1228,7 +1317,7 @@ extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, c
     int k0 = plan->color_ptr_host[c], k1 = plan->color_ptr_host[c + 1];
     if (k1 <= k0) continue;
     if (precision == XK_FP64)
-      k_beam64<<<xk_blocks(k1 - k0, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_COLOUR, *m, bc, elem_ref, plan->elem_order, k0, k1,
+      k_beam64<<<xk_blocks(k1 - k0, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_COLOUR, *m, *sec, elem_ref, plan->elem_order, k0, k1,
                                                                  plan->blk, plan->first, u, f_int, (double*)K_vals, vec,
                                                                  k1 - k0);
     else

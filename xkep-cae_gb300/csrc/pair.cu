@@ -360,20 +360,18 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
 //
 // What bounds them is the FP64 pipe, about two operations per clock and SM on this GPU, not memory: every
 // double divide and square root costs some ten of them, and a dot product with separately rounded terms
-// five instead of three.  The detection needs the reference's operation order (its active sets are compared
-// bit for bit) and keeps the exact routine; the per-iteration narrowphase needs double precision only, so it
-// is written for the fewest FP64 operations: fused multiply-adds, one reciprocal or reciprocal square root
-// per normalisation (two Newton-Raphson steps from the approximate PTX instruction), range tests on the high
-// word in the integer pipe, and the frame transported as R p = c p + v x p + v (v.p) / (1 + c).  Pairs outside
-// the ordinary case (near-parallel, degenerate, without a unit frame, NaN) take the exact routine.
+// five instead of three.  A pair that carries no force needs double precision only, so its narrowphase is
+// written for the fewest FP64 operations: fused multiply-adds, one reciprocal or reciprocal square root per
+// normalisation (two Newton-Raphson steps from the approximate PTX instruction), range tests on the high word
+// in the integer pipe, and the frame transported as R p = c p + v x p + v (v.p) / (1 + c).  A contributing
+// pair keeps the reference's operation order up to its normal, with cheaper correctly rounded divides; its
+// frame and friction are fused too.  Pairs outside the ordinary case (near-parallel, degenerate, without a
+// unit frame, NaN) take the exact routine.
 // Measured at the 1027-wire strand (2.46M other pairs, 0.75M contributing ones), exact routine for every
-// pair against this one: other pairs 1757 -> 652 us, contributing pairs 936 -> 393 us (132 and 262 FP64
-// operations a pair at the pipe's measured 1.64 per clock and SM).
+// pair against this: other pairs 1757 -> 652 us (132 FP64 operations a pair at the pipe's measured 1.64 per
+// clock and SM), contributing pairs 936 -> 599 us (393 us if these were fused throughout).
 // ===========================================================================
 
-XK_D bool above_one64(double x) { return __double_as_longlong(x) > 0x3ff0000000000000LL; }
-XK_D bool outside01(double x) { return __double2hiint(x) < 0 || above_one64(x); }
-XK_D double clamp01_64(double x) { return __double2hiint(x) < 0 ? 0.0 : (above_one64(x) ? 1.0 : x); }
 XK_D double fdot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
 XK_D void fcross3(const double* a, const double* b, double* c) {
   c[0] = fma(a[1], b[2], -(a[2] * b[1]));
@@ -381,10 +379,9 @@ XK_D void fcross3(const double* a, const double* b, double* c) {
   c[2] = fma(a[0], b[1], -(a[1] * b[0]));
 }
 
-// Closest point, gap and transported frame of one pair at positions x; rs: the radius sum; pn, pt1: the
-// previous frame.  False (nothing written) outside the ordinary case.
-XK_D bool narrow64(const double (*x)[3], double rs, const double* pn, const double* pt1, double& s, double& t,
-                   double& gap, double* n, double* t1, double* t2) {
+// Closest point, distance and unit normal of one pair at positions x, in fused operations.  False (nothing
+// written) outside the ordinary case.
+XK_D bool closest64(const double (*x)[3], double& s, double& t, double& dist, double* n) {
   double dA[3], dB[3], w[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -396,57 +393,59 @@ XK_D bool narrow64(const double (*x)[3], double rs, const double* pn, const doub
   const double ac = a * c, det = fma(-b, b, ac);
   // segments longer than 2^-14 and at an angle (det > 1e-3 ac): the absolute and relative tolerances of the
   // reference (1e-10) are far off
-  if (!(in_range64<-29, 300>(a) && in_range64<-29, 300>(c) && __double2hiint(fma(-1e-3, ac, det)) > 0)) return false;
+  if (!(in_range64<-29, 140>(a) && in_range64<-29, 140>(c) && __double2hiint(fma(-1e-3, ac, det)) > 0)) return false;
   const double idet = rcp64(det);
   const double su = fma(b, e, -(c * d)) * idet, tu = fma(a, e, -(b * d)) * idet;
-  double sc = clamp01_64(su), tc = clamp01_64(tu);
-  const bool s_out = outside01(su), t_out = outside01(tu);
+  double sc = clip01_64(su), tc = clip01_64(tu);
+  const bool s_out = outside01_64(su), t_out = outside01_64(tu);
   if (s_out || t_out) {
     const double ic = rcp64(c);
-    if (s_out) tc = clamp01_64(fma(b, sc, e) * ic);
+    if (s_out) tc = clip01_64(fma(b, sc, e) * ic);
     if (t_out) {
-      sc = clamp01_64(fma(b, tc, -d) * rcp64(a));
-      tc = clamp01_64(fma(b, sc, e) * ic);
+      sc = clip01_64(fma(b, tc, -d) * rcp64(a));
+      tc = clip01_64(fma(b, sc, e) * ic);
     }
   }
   double v[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) v[i] = fma(-tc, dB[i], fma(sc, dA[i], w[i]));
   const double d2 = fdot3(v, v);
-  const double pp = fdot3(pt1, pt1), qq = fdot3(pn, pn);
-  if (!(in_range64<-190, 300>(d2) && near_one64(qq) && in_range64<-60, 60>(pp))) return false;
+  if (!in_range64<-190, 300>(d2)) return false;
   const double iv = rsqrt64(d2);
-  double dist = d2 * iv;
+  dist = d2 * iv;
   dist = fma(fma(-dist, dist, d2), 0.5 * iv, dist);
-  double nn[3], no[3], tr[3], vx[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) n[i] = v[i] * iv;
+  s = sc;
+  t = tc;
+  return true;
+}
+
+// The frame at unit normal n transported from the previous one (pn, pt1).  False (nothing written) unless the
+// previous normal is a unit vector within 120 degrees of n and the tangent is one to speak of.
+XK_D bool frame64(const double* n, const double* pn, const double* pt1, double* t1, double* t2) {
+  const double pp = fdot3(pt1, pt1), qq = fdot3(pn, pn);
+  if (!(near_one64(qq) && in_range64<-60, 60>(pp))) return false;
+  double no[3], v[3], vx[3], tr[3];
   const double iq = fma(-0.5, qq, 1.5);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    nn[i] = v[i] * iv;
-    no[i] = pn[i] * iq;
-  }
-  fcross3(no, nn, v);
-  const double cv = fdot3(no, nn);
+  for (int i = 0; i < 3; ++i) no[i] = pn[i] * iq;
+  fcross3(no, n, v);
+  const double cv = fdot3(no, n);
   if (!(__double2hiint(cv + 0.5) > 0)) return false;
   fcross3(v, pt1, vx);
   const double f = fdot3(v, pt1) * rcp64(1.0 + cv);
 #pragma unroll
   for (int i = 0; i < 3; ++i) tr[i] = fma(f, v[i], fma(cv, pt1[i], vx[i]));
-  const double dn = fdot3(tr, nn);
+  const double dn = fdot3(tr, n);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) tr[i] = fma(-dn, nn[i], tr[i]);
+  for (int i = 0; i < 3; ++i) tr[i] = fma(-dn, n[i], tr[i]);
   const double rr = fdot3(tr, tr);
   if (!in_range64<-60, 60>(rr)) return false;
   const double ir = near_one64(rr) ? fma(-0.5, rr, 1.5) : rsqrt64(rr);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    n[i] = nn[i];
-    t1[i] = tr[i] * ir;
-  }
+  for (int i = 0; i < 3; ++i) t1[i] = tr[i] * ir;
   fcross3(n, t1, t2);
-  s = sc;
-  t = tc;
-  gap = dist - rs;
   return true;
 }
 
@@ -456,18 +455,35 @@ __noinline__ __device__ void narrow64_exact(const xk_mesh& m, const xk_pairs& p,
 }
 
 // Narrowphase of pair i (nodes nd, radius sum rs: the cores' on coated wires), written to the table.
+// EXACT: the closest point, gap and normal in the reference's operation order (contributing pairs: the
+// forces and the tangent they give are then the same bits however this kernel is scheduled; an iterative
+// solve of the tangent amplifies a rounding to 1e-8 of its solution); the frame is fused either way.
+template <bool EXACT>
 XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const int* nd, double rs,
                         const double* __restrict__ u, double& s, double& t, double& gap, double* n, double* t1,
                         double* t2) {
   const long long cap = p.cap;
-  double x[4][3], pt1[3], pn[3];
+  double x[4][3], pt1[3], pn[3], dist;
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) x[k][c] = m.X[3LL * nd[k] + c] + u[6LL * nd[k] + c];
+    for (int c = 0; c < 3; ++c) x[k][c] = xadd(m.X[3LL * nd[k] + c], u[6LL * nd[k] + c]);
   load3(p.t1, cap, i, pt1);
   load3(p.normal, cap, i, pn);
-  if (narrow64(x, rs, pn, pt1, s, t, gap, n, t1, t2)) {
+  bool ok;
+  if (EXACT) {
+    double nrm[3];
+    ok = closest_exact_fast(x, s, t, dist, nrm);
+    if (ok) {  // the frame's own normalisation (frame_exact)
+      const Divisor64 q = divisor64(sqrt64(xdot_es(nrm, nrm)));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) n[c] = div64(nrm[c], q);
+    }
+  } else {
+    ok = closest64(x, s, t, dist, n);
+  }
+  if (ok && frame64(n, pn, pt1, t1, t2)) {
+    gap = xsub(dist, rs);
     p.s[i] = s;
     p.t[i] = t;
     p.gap[i] = gap;
@@ -488,7 +504,7 @@ XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const int* n
 
 XK_D double narrow_radii(const xk_mesh& m, int ea, int eb) {
   const double* r = m.core_radii ? m.core_radii : m.radii;
-  return r[ea] + r[eb];
+  return xadd(r[ea], r[eb]);
 }
 
 constexpr int PAIR64_T = 128;
@@ -502,12 +518,12 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_other64(const __grid_constant
   const int ea = p.ea[i], eb = p.eb[i];
   const PairNodes pn = pair_nodes(m, ea, eb);
   double s, t, gap, n[3], t1[3], t2[3];
-  pair_narrow64(m, p, i, pn.n, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  pair_narrow64<false>(m, p, i, pn.n, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
 }
 
 // Contributing pairs, all four stages, combined records.  The frame is orthonormal (just formed), so the
 // geometric friction term q0 n t1^T + q1 t2 n^T - q1 [t1]x^T is n (q0 t1 + q1 t2)^T, since
-// [t1]x = n t2^T - t2 n^T, and the record's B = n (x) ((wm + wg) n + vf / dist) - wg I - T D T^T.
+// [t1]x = n t2^T - t2 n^T, and B = B_n - T D T^T + n vf^T / dist.
 template <bool COAT>
 __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constant__ xk_mesh m,
                                                             const __grid_constant__ xk_pairs p,
@@ -528,10 +544,10 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
   uint8_t status = p.status[i];
   double p_n = p.p_n[i];
   double s, t, gap, n[3], t1[3], t2[3];
-  pair_narrow64(m, p, i, nd, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  pair_narrow64<true>(m, p, i, nd, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
   double v[3] = {0.0, 0.0, 0.0};
   // normal force
-  const double xpen = -cp.k_pen * gap;
+  const double xpen = cp.k_pen * (-gap);
   if (status != ST_INACTIVE) {
     p_n = huber(xpen, dh);
     p.p_n[i] = p_n;
@@ -611,19 +627,25 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
   if (status != ST_INACTIVE) {
     const double dist = (gap + m.radii[ea]) + m.radii[eb];
     const double hd = huber_deriv(xpen, dh);
-    const bool nrm = !(hd < 1e-30 && p_n < 1e-30);
-    const double idist = in_range64<-45, 300>(dist) ? rcp64(dist) : (dist > 1e-15 ? 1.0 / dist : 0.0);
-    const double wg = nrm ? p_n * idist : 0.0, wn = nrm ? fma(hd, cp.k_pen, wg) : 0.0;
-    double w[3];
+    if (!(hd < 1e-30 && p_n < 1e-30)) {  // B_n, term by term as k_pair_member rounds it
+      const double wm = hd * cp.k_pen, wg = dist > 1e-15 ? div64(p_n, dist) : 0.0;
 #pragma unroll
-    for (int b = 0; b < 3; ++b) w[b] = fma(idist, vf[b], wn * n[b]);
+      for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+        for (int b = a; b < 3; ++b) {
+          const double nn = n[a] * n[b];
+          B[3 * a + b] = B[3 * b + a] = fma(wm, nn, -(wg * ((a == b ? 1.0 : 0.0) - nn)));
+        }
+    }
+    if (fric) {
+      const double idist = in_range64<-45, 300>(dist) ? rcp64(dist) : (dist >= 1e-15 ? 1.0 / dist : 0.0);
 #pragma unroll
-      for (int b = 0; b < 3; ++b) B[3 * a + b] = fma(n[a], w[b], -fma(t1[a], e[b], t2[a] * g[b]));
-    B[0] -= wg;
-    B[4] -= wg;
-    B[8] -= wg;
+      for (int b = 0; b < 3; ++b) {
+        const double w = idist * vf[b];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) B[3 * a + b] += fma(n[a], w, -fma(t1[a], e[b], t2[a] * g[b]));
+      }
+    }
   }
   if (COAT)
     coating_epilogue<double, double>(cp, p.coat_cc_prev, p.coat_z_t, p.coat_qtn, p.coat_diss, p.coat_stick, i, cap,
@@ -644,7 +666,7 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
 }
 
 // CTA size of the FP64 pair kernels: the FP64 pipe of every SM is what they need, so a small table is cut
-// into CTAs of one or two warps that reach all SMs (6,500 contributing pairs: 26 CTAs of 256 took 57 us, the same work in 204 of 32 takes 15 us).
+// into CTAs of one or two warps that reach all SMs (6,500 contributing pairs: 26 CTAs of 256 took 57 us, in 204 of 32, with the work above, 21 us).
 int pair64_block(long long n) {
   const long long sms = xk_sm_count();
   return n >= 4 * sms * PAIR64_T ? PAIR64_T : (n >= 2 * sms * 64 ? 64 : 32);

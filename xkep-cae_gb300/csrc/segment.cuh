@@ -41,3 +41,48 @@ XK_D void closest_exact(const double* xA0, const double* xA1, const double* xB0,
   if (dist < 1e-30) { normal[0] = 0.0; normal[1] = 0.0; normal[2] = 1.0; }
 }
 
+// Sign and range tests of doubles on their bits, in the integer pipe (the FP64 pipe also compares).
+XK_D bool below0_64(double x) { return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ULL; }
+XK_D bool above1_64(double x) { return __double_as_longlong(x) > 0x3ff0000000000000LL; }
+XK_D bool outside01_64(double x) { return below0_64(x) || above1_64(x); }
+XK_D double clip01_64(double x) { return below0_64(x) ? 0.0 : (above1_64(x) ? 1.0 : x); }
+
+// The same closest point for the ordinary case (both segments longer than 2^-14, det > 1e-3 ac, finite): the
+// operations of closest_exact in their order, each rounded on its own, so the same bits; the divides share
+// their reciprocals and are skipped where the unclamped parameters stand.  False outside that case.
+XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double& dist, double* normal) {
+  double dA[3], dB[3], w0[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dA[i] = xsub(x[1][i], x[0][i]);
+    dB[i] = xsub(x[3][i], x[2][i]);
+    w0[i] = xsub(x[0][i], x[2][i]);
+  }
+  const double a = xdot_es(dA, dA), b = xdot_es(dA, dB), c = xdot_es(dB, dB);
+  const double d = xdot_es(dA, w0), e = xdot_es(dB, w0);
+  const double ac = xmul(a, c), det = xsub(ac, xmul(b, b));
+  if (!(in_range64<-29, 140>(a) && in_range64<-29, 140>(c) && __double2hiint(fma(-1e-3, ac, det)) > 0)) return false;
+  const Divisor64 qd = divisor64(det);
+  const double su = div64(xsub(xmul(b, e), xmul(c, d)), qd), tu = div64(xsub(xmul(a, e), xmul(b, d)), qd);
+  s = clip01_64(su);
+  t = clip01_64(tu);
+  const bool s_cl = outside01_64(su), t_cl = outside01_64(tu);
+  if (s_cl || t_cl) {
+    const Divisor64 qc = divisor64(c);
+    if (s_cl) t = clip01_64(div64(xadd(xmul(b, s), e), qc));
+    if (t_cl) {
+      s = clip01_64(div64(xsub(xmul(b, t), d), a));
+      t = clip01_64(div64(xadd(xmul(b, s), e), qc));
+    }
+  }
+  double diff[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) diff[i] = xsub(xadd(x[0][i], xmul(s, dA[i])), xadd(x[2][i], xmul(t, dB[i])));
+  const double d2 = xdot_es(diff, diff);
+  if (!in_range64<-190, 300>(d2)) return false;
+  dist = sqrt64(d2);
+  const Divisor64 q = divisor64(dist);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) normal[i] = div64(diff[i], q);
+  return true;
+}

@@ -131,6 +131,33 @@ XK_D bool near_one64(double x) {
   return (unsigned long long)(__double_as_longlong(x) - 0x3fefffffffe00000LL) < 0x600000ULL;
 }
 
+// The correctly rounded quotient and square root (the bits of the operators) on fewer FP64 operations, after
+// Markstein ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r the
+// reciprocal to the last place, q = RN(x r) leaves an exact remainder x - d q, and RN(q + rem r) is x / d;
+// the square root likewise from g = RN(x y) and its exact remainder.  A divisor's reciprocal serves several
+// quotients.  Operands outside the range where the remainders are exact take the operators, out of line.
+__noinline__ static __device__ double div64_plain(double x, double d) { return x / d; }
+__noinline__ static __device__ double sqrt64_plain(double x) { return sqrt(x); }
+struct Divisor64 {
+  double d, r;
+  bool ok;
+};
+XK_D bool mag_in64(double x) {  // |x| in [2^-300, 2^300)
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (723u << 20) < (600u << 20);
+}
+XK_D Divisor64 divisor64(double d) { return {d, rcp64(d), mag_in64(d)}; }
+XK_D double div64(double x, const Divisor64& q) {
+  if (!(q.ok && mag_in64(x))) return x == 0.0 && q.ok ? x : div64_plain(x, q.d);
+  const double y = x * q.r;
+  return fma(fma(-q.d, y, x), q.r, y);
+}
+XK_D double div64(double x, double d) { return div64(x, divisor64(d)); }
+XK_D double sqrt64(double x) {
+  if (!in_range64<-300, 300>(x)) return x == 0.0 ? x : sqrt64_plain(x);
+  const double y = rsqrt64(x), g = x * y;
+  return fma(fma(-g, g, x), 0.5 * y, g);
+}
+
 // Eight floats from a 32-byte aligned read-only address in one 256-bit load.
 XK_D void ldg8(const float* __restrict__ p, float* v) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
