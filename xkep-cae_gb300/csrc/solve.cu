@@ -349,6 +349,377 @@ struct SolveStream {
   }
 };
 
+
+// ---------------------------------------------------------------------------
+// Small systems: the whole iteration in one thread-block cluster.
+//
+// The iteration above is 13 dependent launches, about 57 us however small the system.  Here 16 CTAs on 16
+// SMs hold it together: the nodes are dealt out to the CTAs, a CTA keeps its rows of every vector in shared
+// memory, and what the others need (the preconditioned vectors, the products of the dot products) goes through
+// global memory between hardware cluster barriers.  A CTA's rows of the matrix are packed once into shared
+// memory, without the fixed columns, where they fit.  The convergence checks run on the device: a solve is one
+// launch per CL_SLICE iterations (so that no launch runs for long).  Every sum keeps the order of the launches above (a row's terms; 256
+// consecutive products by the same tree, then the chunk sums by it), so x, the iteration count and the residual
+// are the same bits.
+// What bounds an iteration is the chain of dependent FP64 operations (68 clocks each): the longest row of the
+// two products (some 120 terms for a core wire's node), then the sums' trees, three divides and the five
+// barriers.  No more warps than rows need: a warp issues one FP64 instruction in 64 clocks, so further ones
+// only repeat the scalar work (714 unknowns: 25 us an iteration with 16 warps, 21 us with four).  Writing the
+// exchanged vectors into the other CTAs' shared memory instead measured the same.
+// Line: CL_MAX_N unknowns.  us an iteration, launches against cluster (FP64 / float values): 714 unknowns 58 / 65
+// against 21 / 22; 2,058: 62 / 76 against 27 / 27; 3,762: 62 / 73 against 40 / 47; beyond it the rows no longer
+// fit shared memory and 16 SMs are too few: 5,550: 62 / 73 against 62 / 66, 7,326: 62 / 73 against 64 / 69.
+// ---------------------------------------------------------------------------
+constexpr int CL = 16, CL_SLICE = 512;
+constexpr int CL_MAX_N = 4032;  // 252 rows a CTA, and below 32 chunks of 256
+constexpr int CL_SMEM = 225 * 1024;
+constexpr int CL_B = 8;  // terms loaded ahead of their operations; packed rows are padded to a multiple
+
+XK_D void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// The tree of k_dot2 over 256 values (index t + w added to t for w = 128 ... 1) by one warp: y[k] of lane l is
+// value l + 32 k.  The sum is in lane 0.
+XK_D double warp_tree256(double* y) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) y[k] += y[k + 4];
+  y[0] += y[2];
+  y[1] += y[3];
+  double x = y[0] + y[1];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  return x;
+}
+
+struct ClusterSolve {
+  const double* b;
+  double* x;
+  const double* dinv;
+  double* work;  // 8 vectors, the chunk sums (not used here), the scalars
+  double rtol;
+  int start, it0, it1, max_iter, interval;
+};
+
+template <typename T, int CL_T>
+__global__ void __launch_bounds__(CL_T, 1) k_bicgstab_cluster(const __grid_constant__ xk_system A,
+                                                              const __grid_constant__ ClusterSolve a) {
+  constexpr int CL_WARPS = CL_T / 32;
+  extern __shared__ double sm[];
+  __shared__ double s_part[2][32], s_sum[2];
+  __shared__ int s_max[2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = blockIdx.x;
+  const int nn = A.n_nodes, n = 6 * nn;
+  const int npc = (nn + CL - 1) / CL;  // nodes per CTA
+  const int v0 = rank * npc < nn ? rank * npc : nn, nv = (v0 + npc < nn ? v0 + npc : nn) - v0;
+  const int R = 6 * nv, g0 = 6 * v0, RS = 6 * npc;
+  // this CTA's rows
+  double *r = sm, *rh = r + RS, *p = rh + RS, *v = p + RS, *sv = v + RS, *t = sv + RS, *x = t + RS, *y = x + RS;
+  double* dinv = y + RS;         // [6 RS]
+  double* full = dinv + 6 * RS;  // [n + 1] the vector that the rows are multiplied with, then a zero
+  uint8_t* fx = reinterpret_cast<uint8_t*>(full + n + 1);
+  double* const vals = full + n + 1 + (n + 7) / 8;
+  double* const W = a.work;
+  // exchanged through global memory; each is written again only after a barrier that its readers have passed
+  double *gy = W + 4LL * n, *gz = W + 6LL * n, *P0 = W + 5LL * n, *P1 = W + 7LL * n, *P2 = W + 3LL * n, *P3 = W;
+  double* const sc = W + 8LL * n + 2 * SV_BLOCKS;
+  const int chunks = (n + SV_T - 1) / SV_T;
+  int half = 1;  // half the power of two that holds the chunks
+  while (2 * half < chunks) half *= 2;
+  for (int i = tid; i < n; i += CL_T) fx[i] = A.fixed ? A.fixed[i] : 0;
+  for (int i = tid; i < 6 * R; i += CL_T) dinv[i] = a.dinv[6LL * g0 + i];
+  if (tid < 2) s_max[tid] = 0;
+  if (tid == 0) full[n] = 0.0;
+  __syncthreads();
+
+  // row i of this CTA: the translational rows first (they also carry K_c), so that a warp's rows are alike
+  const int nt = 3 * nv;
+  auto row_of = [&](int i) { return i < nt ? 6 * (i / 3) + i % 3 : 6 * ((i - nt) / 3) + 3 + (i - nt) % 3; };
+  // the terms of k_spmv's row in its order: f(value, column) for every column that is not fixed
+  auto walk = [&](int row, auto f) {
+    const int w = (g0 + row) / 6, d = (g0 + row) % 6;
+    const T* kb = (const T*)A.kb_vals;
+    for (int q = A.kb_low_ptr[w]; q < A.kb_low_ptr[w + 1]; ++q) {
+      const int bk = A.kb_low_blk[q], c = 6 * A.kb_blk_row[bk];
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        if (!fx[c + j]) f(kb[36LL * bk + d + 6 * j], c + j);
+    }
+    for (int bk = A.kb_row_ptr[w]; bk < A.kb_row_ptr[w + 1]; ++bk) {
+      const int c = 6 * A.kb_col[bk];
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        if (!fx[c + j]) f(kb[36LL * bk + 6 * d + j], c + j);
+    }
+    if (d < 3 && A.kc_vals) {
+      const T* kc = (const T*)A.kc_vals;
+      for (int q = A.kc_low_ptr[w]; q < A.kc_low_ptr[w + 1]; ++q) {
+        const int bk = A.kc_low_blk[q], c = 6 * A.kc_blk_row[bk];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (!fx[c + j]) f(kc[9LL * bk + 3 * d + j], c + j);
+      }
+      for (int bk = A.kc_row_ptr[w]; bk < A.kc_row_ptr[w + 1]; ++bk) {
+        const int c = 6 * A.kc_col[bk];
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          if (!fx[c + j]) f(kc[9LL * bk + 3 * d + j], c + j);
+      }
+    }
+  };
+  // Packed rows: a panel of the rotational rows and one of the translational rows, each padded to its longest
+  // row with zero times the zero past the vector; term e of a panel's row i at e * nt + i.  A panel that does not
+  // fit is read from the block matrices instead.
+  for (int i = tid; i < R; i += CL_T) {
+    int e = 0;
+    if (!fx[g0 + row_of(i)]) walk(row_of(i), [&](T, int) { ++e; });
+    atomicMax(&s_max[i < nt ? 1 : 0], e);
+  }
+  __syncthreads();
+  const long long room = (CL_SMEM - (reinterpret_cast<char*>(vals) - reinterpret_cast<char*>(sm))) / 10 - 8;
+  const int len_r = (s_max[0] + CL_B - 1) / CL_B * CL_B, len_t = (s_max[1] + CL_B - 1) / CL_B * CL_B;
+  const bool pack_r = (long long)len_r * nt <= room, pack_t = pack_r && (long long)(len_r + len_t) * nt <= room;
+  uint16_t* const cols = reinterpret_cast<uint16_t*>(vals + (pack_r ? (long long)(len_r + (pack_t ? len_t : 0)) * nt : 0));
+  for (int i = tid; i < R; i += CL_T) {
+    const bool tr = i < nt;
+    if (tr ? !pack_t : !pack_r) continue;
+    const int at = tr ? len_r * nt + i : i - nt, len = tr ? len_t : len_r;
+    int e = 0;
+    if (!fx[g0 + row_of(i)])
+      walk(row_of(i), [&](T val, int c) {
+        vals[at + e * nt] = (double)val;
+        cols[at + e * nt] = (uint16_t)c;
+        ++e;
+      });
+    for (; e < len; ++e) {
+      vals[at + e * nt] = 0.0;
+      cols[at + e * nt] = (uint16_t)n;
+    }
+  }
+  __syncthreads();
+
+  auto matvec = [&](int i, int row) {
+    if (fx[g0 + row]) return full[g0 + row];
+    double acc = 0.0;
+    const bool tr = i < nt;
+    if (tr ? pack_t : pack_r) {
+      const double* z = vals + (tr ? len_r * nt + i : i - nt);
+      const uint16_t* c = cols + (z - vals);
+      const int len = tr ? len_t : len_r;
+      double z0[CL_B], w0[CL_B];
+      if (len > 0) {
+#pragma unroll
+        for (int j = 0; j < CL_B; ++j) {
+          z0[j] = z[j * nt];
+          w0[j] = full[c[j * nt]];
+        }
+      }
+      for (int e = CL_B; e <= len; e += CL_B) {  // the next terms are on their way while these are added
+        double z1[CL_B], w1[CL_B];
+        z += CL_B * nt;
+        c += CL_B * nt;
+        if (e < len) {
+#pragma unroll
+          for (int j = 0; j < CL_B; ++j) {
+            z1[j] = z[j * nt];
+            w1[j] = full[c[j * nt]];
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < CL_B; ++j) acc = fma(z0[j], w0[j], acc);
+#pragma unroll
+        for (int j = 0; j < CL_B; ++j) {
+          z0[j] = z1[j];
+          w0[j] = w1[j];
+        }
+      }
+    } else {
+      walk(row, [&](T val, int col) { acc = fma((double)val, full[col], acc); });
+    }
+    return acc;
+  };
+  auto precondition = [&](const double* src, int row) {  // k_apply_block_jacobi
+    const double* D = dinv + 6 * row;
+    const double* s = src + 6 * (row / 6);
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) acc = fma(D[j], s[j], acc);
+    return acc;
+  };
+  auto fetch = [&](const double* src) {
+    for (int i = tid; i < n; i += CL_T) full[i] = __ldcg(src + i);
+    __syncthreads();
+  };
+  // the sums of one or two exchanged product vectors, in every CTA the same bits
+  auto sums = [&](const double* Pa, const double* Pb, double& sa, double& sb) {
+    const int k = Pb ? 2 : 1;
+    for (int c = warp; c < chunks * k; c += CL_WARPS) {
+      const double* P = c < chunks ? Pa : Pb;
+      const int q = c < chunks ? c : c - chunks;
+      double z[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int i = SV_T * q + lane + 32 * j;
+        z[j] = i < n ? __ldcg(P + i) : 0.0;
+      }
+      const double s = warp_tree256(z);
+      if (lane == 0) s_part[c < chunks ? 0 : 1][q] = s;
+    }
+    __syncthreads();
+    if (warp < k) {  // the tree of sum_parts without its zeros
+      double s = lane < chunks ? s_part[warp][lane] : 0.0;
+      for (int o = half; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) s_sum[warp] = s;
+    }
+    __syncthreads();
+    sa = s_sum[0];
+    if (Pb) sb = s_sum[1];
+  };
+
+  double rho, alpha, omega, rho_next, bb, rr = 0.0, unused;
+  if (a.start) {
+    for (int i = tid; i < n; i += CL_T) full[i] = a.x[i];
+    __syncthreads();
+    for (int i = tid; i < R; i += CL_T) {
+      const int row = row_of(i), g = g0 + row;
+      const double ri = a.b[g] - matvec(i, row);
+      r[row] = ri;
+      rh[row] = ri;
+      p[row] = 0.0;
+      v[row] = 0.0;
+      x[row] = full[g];
+      P0[g] = ri * ri;
+      P1[g] = a.b[g] * a.b[g];
+    }
+    cluster_sync();
+    sums(P0, P1, rho_next, bb);
+    bb = bb > 0.0 ? bb : 1.0;
+    rho = alpha = omega = 1.0;
+  } else {
+    rho = sc[0];
+    alpha = sc[1];
+    omega = sc[2];
+    rho_next = sc[3];
+    bb = sc[4];
+    for (int row = tid; row < R; row += CL_T) {
+      const int g = g0 + row;
+      r[row] = W[g];
+      rh[row] = W[1LL * n + g];
+      p[row] = W[2LL * n + g];
+      v[row] = W[3LL * n + g];
+      x[row] = a.x[g];
+    }
+  }
+  cluster_sync();  // the state and the first products have been read by all
+  double ao = div64(alpha, omega);
+  int it = a.it0;
+  while (it < a.it1) {
+    const int k = a.max_iter - it < a.interval ? a.max_iter - it : a.interval;
+    for (int q = 0; q < k; ++q) {
+      const double beta = (rho != 0.0 && omega != 0.0) ? div64(rho_next, rho) * ao : 0.0;
+      rho = rho_next;
+      for (int row = tid; row < R; row += CL_T) p[row] = r[row] + beta * (p[row] - omega * v[row]);
+      __syncthreads();
+      for (int row = tid; row < R; row += CL_T) gy[g0 + row] = y[row] = precondition(p, row);
+      cluster_sync();
+      fetch(gy);
+      for (int i = tid; i < R; i += CL_T) {
+        const int row = row_of(i);
+        const double z = matvec(i, row);
+        v[row] = z;
+        P0[g0 + row] = rh[row] * z;
+      }
+      cluster_sync();
+      double d0, d1 = 0.0;
+      sums(P0, nullptr, d0, unused);
+      alpha = d0 != 0.0 ? div64(rho, d0) : 0.0;
+      for (int row = tid; row < R; row += CL_T) {
+        x[row] = fma(alpha, y[row], x[row]);
+        sv[row] = fma(-alpha, v[row], r[row]);
+      }
+      __syncthreads();
+      for (int row = tid; row < R; row += CL_T) gz[g0 + row] = y[row] = precondition(sv, row);
+      cluster_sync();
+      fetch(gz);
+      for (int i = tid; i < R; i += CL_T) {
+        const int row = row_of(i);
+        const double z = matvec(i, row);
+        t[row] = z;
+        P0[g0 + row] = z * sv[row];
+        P1[g0 + row] = z * z;
+      }
+      cluster_sync();
+      sums(P0, P1, d0, d1);
+      omega = d1 != 0.0 ? div64(d0, d1) : 0.0;
+      const bool check = q == k - 1;
+      for (int row = tid; row < R; row += CL_T) {
+        x[row] = fma(omega, y[row], x[row]);
+        const double ri = fma(-omega, t[row], sv[row]);
+        r[row] = ri;
+        P2[g0 + row] = rh[row] * ri;
+        if (check) P3[g0 + row] = ri * ri;
+      }
+      cluster_sync();
+      ao = div64(alpha, omega);
+      sums(P2, check ? P3 : nullptr, rho_next, rr);
+    }
+    it += k;
+    if (!(sqrt(rr / bb) > a.rtol)) break;  // converged (or a NaN): the same in every CTA
+  }
+  cluster_sync();  // the last sums have been read by all before the state goes out
+  for (int row = tid; row < R; row += CL_T) {
+    const int g = g0 + row;
+    W[g] = r[row];
+    W[1LL * n + g] = rh[row];
+    W[2LL * n + g] = p[row];
+    W[3LL * n + g] = v[row];
+    a.x[g] = x[row];
+  }
+  if (rank == 0 && tid == 0) {
+    sc[0] = rho;
+    sc[1] = alpha;
+    sc[2] = omega;
+    sc[3] = rho_next;
+    sc[4] = bb;
+    sc[5] = rr;
+    sc[6] = (double)it;
+  }
+}
+
+// One slice of a solve; false where a cluster of this size cannot be launched here.
+template <typename T, int CL_T>
+bool cluster_slice(const xk_system& A, const ClusterSolve& a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CL);
+  cfg.blockDim = dim3(CL_T);
+  cfg.dynamicSmemBytes = CL_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CL;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int resident = 0;
+  const auto kernel = k_bicgstab_cluster<T, CL_T>;
+  if ((a.start &&
+       (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&resident, kernel, &cfg) != cudaSuccess || resident < 1)) ||
+      cudaLaunchKernelEx(&cfg, kernel, A, a) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
+// a thread per row
+template <typename T>
+bool cluster_slice_any(const xk_system& A, const ClusterSolve& a, cudaStream_t st) {
+  const int rows = 6 * ((A.n_nodes + CL - 1) / CL);
+  return rows <= 128 ? cluster_slice<T, 128>(A, a, st) : cluster_slice<T, 256>(A, a, st);
+}
+
 }  // namespace
 
 extern "C" xk_status xk_bicgstab(const xk_system* A, const double* b, double* x, const double* dinv, double* work,
@@ -373,6 +744,27 @@ extern "C" xk_status xk_bicgstab(const xk_system* A, const double* b, double* x,
   double* part = t + n;          // [2 * SV_BLOCKS]
   double* sc = part + 2 * SV_BLOCKS;  // [S_N]
   const int nb = xk_blocks(n, SV_T);
+  const int interval = check_every < max_iter ? check_every : (max_iter > 0 ? max_iter : 1);
+  if (n <= CL_MAX_N && max_iter > 0) {  // one launch per slice of whole check intervals
+    ClusterSolve a{b, x, dinv, work, rtol, 1, 0, 0, max_iter, interval};
+    const int slice = interval * (interval < CL_SLICE ? CL_SLICE / interval : 1);
+    while (true) {
+      a.it1 = max_iter - a.it0 < slice ? max_iter : a.it0 + slice;
+      if (!(A->precision == XK_FP64 ? cluster_slice_any<double>(*A, a, st) : cluster_slice_any<float>(*A, a, st))) {
+        if (a.start) break;  // no such cluster here: the launches below
+        return xk_set_error(XK_ERR_CUDA, "xk_bicgstab: cluster launch failed");
+      }
+      double h[7];
+      XK_CUDA(cudaMemcpyAsync(h, sc, sizeof(h), cudaMemcpyDeviceToHost, st));
+      XK_CUDA(cudaStreamSynchronize(st));
+      a.it0 = (int)h[6];
+      a.start = 0;
+      const double res_c = sqrt(h[5] / h[4]);
+      if (iters) *iters = a.it0;
+      if (rel_res) *rel_res = res_c;
+      if (a.it0 >= max_iter || !(res_c > rtol)) return XK_OK;
+    }
+  }
   // ||b||^2 and r = b - A x
   dot2(n, b, b, nullptr, nullptr, part, st);
   k_scalars<0><<<1, SV_T, 0, st>>>(part, sc);
@@ -392,7 +784,6 @@ extern "C" xk_status xk_bicgstab(const xk_system* A, const double* b, double* x,
   XK_CUDA(cudaEventCreateWithFlags(&ss.ev, cudaEventDisableTiming));
   XK_CUDA(cudaEventRecord(ss.ev, st));
   XK_CUDA(cudaStreamWaitEvent(ss.cs, ss.ev, 0));
-  const int interval = check_every < max_iter ? check_every : (max_iter > 0 ? max_iter : 1);
   auto chunk = [&](int k, cudaStream_t cs) {
     for (int q = 0; q < k; ++q) bicgstab_iteration(*A, n, nb, dinv, x, r, rh, p, v, y, sv, z, t, part, sc, cs);
     residual_sq(n, r, part, sc, cs);
