@@ -9,7 +9,7 @@
 // mma.sync m16n8k16 (BF16 -> FP32), where a warp takes 16 candidates and each
 // layer's accumulator fragments are re-packed in registers as the next layer's
 // A operand.  Training runs
-// one sample per thread in FP32 on BF16-rounded operands, which is the same
+// in FP32 register tiles on BF16-rounded operands, which is the same
 // arithmetic up to the order of the float sums.
 #include <cuda_bf16.h>
 
@@ -502,178 +502,352 @@ __global__ void __launch_bounds__(TC_T) k_mlp_forward_tc(const uint16_t* __restr
   }
 }
 
-// ------------------------------------------------------------------ training (one sample per thread)
-
-constexpr int TR_T = 128;
-
+// ------------------------------------------------------------------ training
+//
 // Activations and deltas are stored plane-major: value q of sample i at [q * n + i].
-// The outer loops over units run at run time and the 64-wide dot products are
-// unrolled; a layer's input vector is read back from its (just written) plane
-// into registers, so no register array is indexed at run time.
-__global__ void __launch_bounds__(TR_T) k_mlp_train_fwd(const float* __restrict__ theta,
-                                                        const float* __restrict__ feat, long long n,
-                                                        float* __restrict__ act, float* __restrict__ logit) {
-  __shared__ float W[NP];
-  for (int i = threadIdx.x; i < NP; i += blockDim.x) W[i] = bf16r(theta[i]);
-  __syncthreads();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float x[MF];
+// The layers' products (n x 64 by 64 x 64, FP32 on BF16-rounded weights and activations) run as register tiles:
+// a CTA of 128 threads takes 128 samples, each thread eight samples by eight outputs from operands in shared
+// memory, 64 multiply-adds for sixteen loaded values.  One sample per thread, as before, loads a weight for
+// every multiply-add, and what bounds that is the 128 bytes per clock that shared memory returns to the
+// registers.  Every sum keeps its order (k ascending from zero), so activations, logits and deltas are the same
+// bits.  Tensor cores are no way here: another order of the sums rounds one activation in 20,000 to the other
+// bfloat16 neighbour, which moves the logits by more than float rounding.
+// Measured at 201,347 samples, one sample per thread against this: forward 161 -> 113 us, backward
+// 423 -> 159 us, weight gradients 963 -> 142 us (94,000 of 234,000 clocks of the forward are its multiply-adds).
+
+constexpr int TR_T = 128;   // threads, and samples of a tile
+constexpr int TR_LD = 132;  // row stride of a tile [value][sample]: rows 4 banks apart, 16-byte aligned
+struct TrainTile {
+  float v[MH][TR_LD];
+};
+
+// Weight matrix in shared memory for tile_mul: the eight outputs og + 8 j of thread group og (whose results then go
+// to rows one apart) stand at columns 4 og ... 4 og + 3 and 32 + 4 og ..., so that a warp's two 16-byte loads
+// meet every bank once.
+XK_D int tile_col(int out) { return 32 * (out >> 5) + 4 * (out & 7) + ((out >> 3) & 3); }
+
+// acc[i][j] = sum_k A[k][8 sg + i] B[k][og + 8 j], k ascending
+template <int K>
+XK_D void tile_mul(const float (*A)[TR_LD], const float (*B)[MH], int sg, int og, float (*acc)[8]) {
 #pragma unroll
-  for (int k = 0; k < MF; ++k) x[k] = bf16r(feat[MF * i + k]);
-#pragma unroll 1
-  for (int j = 0; j < MH; ++j) {
-    float z = 0.f;
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int k = 0; k < MF; ++k) z += W[O_W1 + j * MF + k] * x[k];
-    act[(long long)j * n + i] = bf16r(fmaxf(z + W[O_B1 + j], 0.f));
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    const float4 a0 = *reinterpret_cast<const float4*>(&A[k][8 * sg]);
+    const float4 a1 = *reinterpret_cast<const float4*>(&A[k][8 * sg + 4]);
+    const float4 b0 = *reinterpret_cast<const float4*>(&B[k][4 * og]);
+    const float4 b1 = *reinterpret_cast<const float4*>(&B[k][32 + 4 * og]);
+    const float x[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    const float w[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(w[j], x[i], acc[i][j]);
   }
-  float a[MH];
-#pragma unroll 1
-  for (int layer = 0; layer < 2; ++layer) {
-    const int ow = layer == 0 ? O_W2 : O_W3, ob = layer == 0 ? O_B2 : O_B3;
-#pragma unroll
-    for (int k = 0; k < MH; ++k) a[k] = act[(long long)(layer * MH + k) * n + i];
-#pragma unroll 1
-    for (int j = 0; j < MH; ++j) {
-      float z = 0.f;
-#pragma unroll
-      for (int k = 0; k < MH; ++k) z += W[ow + j * MH + k] * a[k];
-      act[(long long)((layer + 1) * MH + j) * n + i] = bf16r(fmaxf(z + W[ob + j], 0.f));
-    }
-  }
-  float s = 0.f;
-#pragma unroll
-  for (int k = 0; k < MH; ++k) s += act[(long long)(2 * MH + k) * n + i] * W[O_W4 + k];
-  logit[i] = s + W[O_B4];
 }
 
-__global__ void __launch_bounds__(TR_T) k_mlp_train_bwd(const float* __restrict__ theta, const float* __restrict__ act,
-                                                        const float* __restrict__ logit, const float* __restrict__ y,
-                                                        const float* __restrict__ w, long long n,
-                                                        float* __restrict__ dvec, float* __restrict__ gout,
-                                                        double* __restrict__ loss_part) {
-  __shared__ float W[NP];
-  __shared__ double red[TR_T];
-  for (int i = threadIdx.x; i < NP; i += blockDim.x) W[i] = bf16r(theta[i]);
-  __syncthreads();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double li = 0.0;
-  if (i < n) {
-    const double l = (double)logit[i], yi = (double)y[i], wi = (double)w[i];
-    const double sp = l > 0.0 ? l + log1p(exp(-l)) : log1p(exp(l));
-    li = wi * (sp - yi * l) / (double)n;
-    const float g = (float)(wi * (1.0 / (1.0 + exp(-l)) - yi) / (double)n);
-    gout[i] = g;
-#pragma unroll 1
-    for (int k = 0; k < MH; ++k)
-      dvec[(long long)(2 * MH + k) * n + i] = act[(long long)(2 * MH + k) * n + i] > 0.f ? g * W[O_W4 + k] : 0.f;
-    // d2 = (W3^T d3) masked, then d1 = (W2^T d2) masked
-    float d[MH];
-#pragma unroll 1
-    for (int layer = 1; layer >= 0; --layer) {
-      const int ow = layer == 1 ? O_W3 : O_W2;
+struct TrainFwdSmem {
+  float w1[MF][MH], w2[MH][MH], w3[MH][MH];
+  float b1[MH], b2[MH], b3[MH], w4[MH];
+  TrainTile a;
+};
+
+__global__ void __launch_bounds__(TR_T, 3) k_mlp_train_fwd(const float* __restrict__ theta,
+                                                           const float* __restrict__ feat, long long n,
+                                                           float* __restrict__ act, float* __restrict__ logit) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  TrainFwdSmem& sm = *reinterpret_cast<TrainFwdSmem*>(raw);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < MH * MF; i += TR_T) sm.w1[i % MF][tile_col(i / MF)] = bf16r(theta[O_W1 + i]);
+  for (int i = tid; i < MH * MH; i += TR_T) {
+    sm.w2[i % MH][tile_col(i / MH)] = bf16r(theta[O_W2 + i]);
+    sm.w3[i % MH][tile_col(i / MH)] = bf16r(theta[O_W3 + i]);
+  }
+  if (tid < MH) {
+    sm.b1[tid] = bf16r(theta[O_B1 + tid]);
+    sm.b2[tid] = bf16r(theta[O_B2 + tid]);
+    sm.b3[tid] = bf16r(theta[O_B3 + tid]);
+    sm.w4[tid] = bf16r(theta[O_W4 + tid]);
+  }
+  const float b4 = bf16r(theta[O_B4]);
+  const int og = tid & 7, sg = tid >> 3;  // outputs og + 8 j, samples 8 sg + i
+  for (long long s0 = (long long)blockIdx.x * TR_T; s0 < n; s0 += (long long)gridDim.x * TR_T) {
+    const int ns = n - s0 < TR_T ? (int)(n - s0) : TR_T;
+    __syncthreads();  // the weights are in place; the last tile has been read
 #pragma unroll
-      for (int j = 0; j < MH; ++j) d[j] = dvec[(long long)((layer + 1) * MH + j) * n + i];
+    for (int k = 0; k < MF; ++k) sm.a.v[k][tid] = tid < ns ? bf16r(feat[MF * (s0 + tid) + k]) : 0.f;
+    __syncthreads();
 #pragma unroll 1
+    for (int layer = 0; layer < 3; ++layer) {
+      float acc[8][8];
+      if (layer == 0) tile_mul<MF>(sm.a.v, sm.w1, sg, og, acc);
+      else tile_mul<MH>(sm.a.v, layer == 1 ? sm.w2 : sm.w3, sg, og, acc);
+      const float* b = layer == 0 ? sm.b1 : (layer == 1 ? sm.b2 : sm.b3);
+      __syncthreads();  // every thread has read the layer's inputs
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float bj = b[og + 8 * j];
+        float z[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = bf16r(fmaxf(acc[i][j] + bj, 0.f));
+        float4* o = reinterpret_cast<float4*>(&sm.a.v[og + 8 * j][8 * sg]);
+        o[0] = make_float4(z[0], z[1], z[2], z[3]);
+        o[1] = make_float4(z[4], z[5], z[6], z[7]);
+      }
+      __syncthreads();
+      if (tid < ns) {
+#pragma unroll 8
+        for (int j = 0; j < MH; ++j) act[(long long)(layer * MH + j) * n + s0 + tid] = sm.a.v[j][tid];
+      }
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < MH; ++k) s += sm.a.v[k][tid] * sm.w4[k];
+    if (tid < ns) logit[s0 + tid] = s + b4;
+  }
+}
+
+struct TrainBwdSmem {
+  float w2[MH][MH], w3[MH][MH];  // [j][k]: the rows that delta_j is multiplied with
+  float w4[MH];
+  double red[TR_T];
+  TrainTile d;
+};
+
+// Loss part of the tile, delta of the output (g) and the deltas of the three hidden layers.  The loss and the
+// sigmoid are taken in double from one exponential: with e = exp(-|l|), softplus(l) = max(l, 0) + log1p(e) and
+// sigmoid(l) = 1 / (1 + e) or e / (1 + e).
+__global__ void __launch_bounds__(TR_T, 3) k_mlp_train_bwd(const float* __restrict__ theta,
+                                                           const float* __restrict__ act,
+                                                           const float* __restrict__ logit,
+                                                           const float* __restrict__ y, const float* __restrict__ w,
+                                                           long long n, float* __restrict__ dvec,
+                                                           float* __restrict__ gout, double* __restrict__ loss_part) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  TrainBwdSmem& sm = *reinterpret_cast<TrainBwdSmem*>(raw);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < MH * MH; i += TR_T) {
+    sm.w2[i / MH][tile_col(i % MH)] = bf16r(theta[O_W2 + i]);
+    sm.w3[i / MH][tile_col(i % MH)] = bf16r(theta[O_W3 + i]);
+  }
+  if (tid < MH) sm.w4[tid] = bf16r(theta[O_W4 + tid]);
+  const int og = tid & 7, sg = tid >> 3;
+  const Divisor64 dn = divisor64((double)n);
+  for (long long t = blockIdx.x; t * TR_T < n; t += gridDim.x) {
+    const long long s0 = t * TR_T, i = s0 + tid;
+    const bool live = i < n;
+    // which of this sample's activations are positive, as bits: 32 loads in flight a thread, all of them before
+    // the tile's arithmetic (a load between the sums waited out its latency: 475 us)
+    uint32_t pos[NA / 32];
+#pragma unroll
+    for (int q = 0; q < NA / 32; ++q) {
+      pos[q] = 0u;
+      if (live) {
+        float v[32];
+#pragma unroll
+        for (int b = 0; b < 32; ++b) v[b] = act[(long long)(32 * q + b) * n + i];
+#pragma unroll
+        for (int b = 0; b < 32; ++b) pos[q] |= (v[b] > 0.f ? 1u : 0u) << b;
+      }
+    }
+    float g = 0.f;
+    double li = 0.0;
+    if (live) {
+      const double l = (double)logit[i], yi = (double)y[i], wi = (double)w[i];
+      const double e = exp(-fabs(l)), sig = (l >= 0.0 ? 1.0 : e) * rcp64(1.0 + e);
+      li = div64(wi * ((l > 0.0 ? l : 0.0) + log1p(e) - yi * l), dn);
+      g = (float)div64(wi * (sig - yi), dn);
+      gout[i] = g;
+    }
+    __syncthreads();  // the weights are in place; the last tile has been read
+    sm.red[tid] = li;
+#pragma unroll
+    for (int k = 0; k < MH; ++k) {
+      const float v = (pos[4 + k / 32] >> (k % 32)) & 1u ? g * sm.w4[k] : 0.f;
+      if (live) dvec[(long long)(2 * MH + k) * n + i] = v;
+      sm.d.v[k][tid] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int layer = 1; layer >= 0; --layer) {  // d2 = (W3^T d3) masked, then d1 = (W2^T d2) masked
+      float acc[8][8];
+      tile_mul<MH>(sm.d.v, layer == 1 ? sm.w3 : sm.w2, sg, og, acc);
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float4* o = reinterpret_cast<float4*>(&sm.d.v[og + 8 * j][8 * sg]);
+        o[0] = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+        o[1] = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
+      }
+      __syncthreads();
+#pragma unroll
       for (int k = 0; k < MH; ++k) {
-        float z = 0.f;
-#pragma unroll
-        for (int j = 0; j < MH; ++j) z += W[ow + j * MH + k] * d[j];
-        const long long q = (long long)(layer * MH + k) * n + i;
-        dvec[q] = act[q] > 0.f ? z : 0.f;
+        const float v = (pos[2 * layer + k / 32] >> (k % 32)) & 1u ? sm.d.v[k][tid] : 0.f;
+        if (live) dvec[(long long)(layer * MH + k) * n + i] = v;
+        if (layer == 1) sm.d.v[k][tid] = v;
       }
+      __syncthreads();
     }
-  }
-  red[threadIdx.x] = li;
-  __syncthreads();
-  for (int s = TR_T / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) loss_part[blockIdx.x] = red[0];
-}
-
-// Weight gradients: each block sums its chunk of samples for every parameter
-// (fixed order); a second kernel adds the block partials in block order.
-constexpr int WG_T = 256, WG_CHUNK = 1024, WG_SUB = 16, WG_SLOTS = (NP + WG_T - 1) / WG_T;
-
-__global__ void __launch_bounds__(WG_T) k_mlp_wgrad(const float* __restrict__ feat, const float* __restrict__ act,
-                                                    const float* __restrict__ dvec, const float* __restrict__ g,
-                                                    long long n, float* __restrict__ partial) {
-  __shared__ float Ds[WG_SUB][NA + 1];      // d1 d2 d3 | g
-  __shared__ float As[WG_SUB][MF + NA + 1];  // x0 a1 a2 a3 | 1
-  int drow[WG_SLOTS], acol[WG_SLOTS];
-  float acc[WG_SLOTS];
-#pragma unroll
-  for (int q = 0; q < WG_SLOTS; ++q) {
-    const int p = threadIdx.x + WG_T * q;
-    int dr = 0, ac = MF + NA;
-    if (p < O_B1) { dr = (p - O_W1) / MF; ac = (p - O_W1) % MF; }
-    else if (p < O_W2) { dr = p - O_B1; }
-    else if (p < O_B2) { dr = MH + (p - O_W2) / MH; ac = MF + (p - O_W2) % MH; }
-    else if (p < O_W3) { dr = MH + (p - O_B2); }
-    else if (p < O_B3) { dr = 2 * MH + (p - O_W3) / MH; ac = MF + MH + (p - O_W3) % MH; }
-    else if (p < O_W4) { dr = 2 * MH + (p - O_B3); }
-    else if (p < O_B4) { dr = NA; ac = MF + 2 * MH + (p - O_W4); }
-    else { dr = NA; }
-    drow[q] = dr;
-    acol[q] = ac;
-    acc[q] = 0.f;
-  }
-  const long long c0 = (long long)blockIdx.x * WG_CHUNK;
-  const long long c1 = (c0 + WG_CHUNK < n) ? c0 + WG_CHUNK : n;
-  for (long long s0 = c0; s0 < c1; s0 += WG_SUB) {
-    const int ns = (int)((c1 - s0) < WG_SUB ? (c1 - s0) : WG_SUB);
-    for (int e = threadIdx.x; e < WG_SUB * (NA + 1); e += WG_T) {
-      const int s = e % WG_SUB, q = e / WG_SUB;
-      float v = 0.f;
-      if (s < ns) v = q < NA ? dvec[(long long)q * n + s0 + s] : g[s0 + s];
-      Ds[s][q] = v;
+    for (int h = TR_T / 2; h > 0; h >>= 1) {
+      if (tid < h) sm.red[tid] += sm.red[tid + h];
+      __syncthreads();
     }
-    for (int e = threadIdx.x; e < WG_SUB * (MF + NA + 1); e += WG_T) {
-      const int s = e % WG_SUB, q = e / WG_SUB;
-      float v = 0.f;
-      if (s < ns) {
-        if (q < MF) v = bf16r(feat[MF * (s0 + s) + q]);
-        else if (q < MF + NA) v = act[(long long)(q - MF) * n + s0 + s];
-        else v = 1.f;
-      }
-      As[s][q] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < WG_SLOTS; ++q) {
-      if (threadIdx.x + WG_T * q < NP) {
-        float a = acc[q];
-#pragma unroll
-        for (int s = 0; s < WG_SUB; ++s) a += Ds[s][drow[q]] * As[s][acol[q]];
-        acc[q] = a;
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < WG_SLOTS; ++q) {
-    const int p = threadIdx.x + WG_T * q;
-    if (p < NP) partial[(long long)blockIdx.x * NP + p] = acc[q];
+    if (tid == 0) loss_part[t] = sm.red[0];
   }
 }
 
-__global__ void k_sum_partials(const float* __restrict__ partial, int nb, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= NP) return;
-  float s = 0.f;
-  for (int b = 0; b < nb; ++b) s += partial[(long long)b * NP + p];
-  grad[p] = s;
+// Weight gradients: a CTA sums a chunk of samples for every parameter in sample order, two warps with the 64 x 64
+// products d2 a1^T and two with d3 a2^T as 8 x 8 tiles a thread (four samples at a time from [value][sample] rows
+// in shared memory), then its share of the small ones; a second kernel adds the chunks' sums in a fixed order.
+// The chunk follows from n alone: the samples dealt out to WG_CTAS CTAs (three per SM of 152), in whole tiles.
+// Chunks of 1024 whatever n left a few thousand samples to one or two CTAs (1,200 samples: 600 us).
+constexpr int WG_T = 128, WG_S = 32, WG_LD = 36, WG_CTAS = 456;
+static_assert(NA % 64 == 0 && WG_T == 128, "row loads: 16 rows a warp and round");
+constexpr int WG_A = MF + NA;  // rows x0 a1 a2 a3
+struct WgradSmem {
+  float d[NA][WG_LD];  // d1 d2 d3
+  float a[WG_A][WG_LD];
+  float g[WG_LD];
+};
+long long wgrad_chunk(long long n) {
+  const long long per = (n + WG_CTAS - 1) / WG_CTAS;
+  return (per + WG_S - 1) / WG_S * WG_S;
 }
 
-__global__ void k_sum_loss(const double* __restrict__ part, int nb, float* __restrict__ loss) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+__global__ void __launch_bounds__(WG_T, 3) k_mlp_wgrad(const float* __restrict__ feat, const float* __restrict__ act,
+                                                       const float* __restrict__ dvec, const float* __restrict__ g,
+                                                       long long n, long long chunk, float* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  WgradSmem& sm = *reinterpret_cast<WgradSmem*>(raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int half = warp >> 1;                      // 0: d2 a1^T, 1: d3 a2^T
+  const int tr = (tid & 63) >> 3, tc = tid & 7;    // this thread's rows tr + 8 i and columns tc + 8 j
+  const float(*D)[WG_LD] = sm.d + MH * (1 + half);
+  const float(*A)[WG_LD] = sm.a + MF + MH * half;
+  float acc[8][8], w1[4] = {0.f, 0.f, 0.f, 0.f}, b0 = 0.f, b1 = 0.f, w4 = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  const int r1 = tid >> 1, c1 = 4 * (tid & 1);     // this thread's part of d1 x0^T: row r1, columns c1 ... c1 + 3
+  const long long c0 = (long long)blockIdx.x * chunk, ce = c0 + chunk < n ? c0 + chunk : n;
+  for (long long s0 = c0; s0 < ce; s0 += WG_S) {
+    const bool in = s0 + lane < ce;
+    __syncthreads();
+#pragma unroll
+    for (int q0 = warp; q0 < NA; q0 += 16 * (WG_T / 32)) {  // 32 loads in flight a thread
+      float vd[16], va[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const long long at = (long long)(q0 + 4 * q) * n + s0 + lane;
+        vd[q] = in ? dvec[at] : 0.f;
+        va[q] = in ? act[at] : 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        sm.d[q0 + 4 * q][lane] = vd[q];
+        sm.a[MF + q0 + 4 * q][lane] = va[q];
+      }
+    }
+#pragma unroll
+    for (int e = tid; e < WG_S * MF; e += WG_T) {
+      const int q = e % MF, s = e / MF;
+      sm.a[q][s] = s0 + s < ce ? bf16r(feat[MF * (s0 + s) + q]) : 0.f;
+    }
+    if (warp == 0) sm.g[lane] = in ? g[s0 + lane] : 0.f;
+    __syncthreads();
+    // samples past the chunk add zero times zero
+#pragma unroll 1
+    for (int s = 0; s < WG_S; s += 4) {
+      float4 x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = *reinterpret_cast<const float4*>(&A[tc + 8 * j][s]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 d = *reinterpret_cast<const float4*>(&D[tr + 8 * i][s]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          acc[i][j] = fmaf(d.w, x[j].w, fmaf(d.z, x[j].z, fmaf(d.y, x[j].y, fmaf(d.x, x[j].x, acc[i][j]))));
+      }
+      const float4 d1 = *reinterpret_cast<const float4*>(&sm.d[r1][s]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(&sm.a[c1 + j][s]);
+        w1[j] = fmaf(d1.w, v.w, fmaf(d1.z, v.z, fmaf(d1.y, v.y, fmaf(d1.x, v.x, w1[j]))));
+      }
+      const float4 e0 = *reinterpret_cast<const float4*>(&sm.d[tid][s]);
+      b0 = (((b0 + e0.x) + e0.y) + e0.z) + e0.w;
+      const float4 gs = *reinterpret_cast<const float4*>(&sm.g[s]);
+      if (tid < MH) {  // bias row 128 + tid, and w4
+        const float4 e1 = *reinterpret_cast<const float4*>(&sm.d[WG_T + tid][s]);
+        b1 = (((b1 + e1.x) + e1.y) + e1.z) + e1.w;
+        const float4 v = *reinterpret_cast<const float4*>(&sm.a[MF + 2 * MH + tid][s]);
+        w4 = fmaf(gs.w, v.w, fmaf(gs.z, v.z, fmaf(gs.y, v.y, fmaf(gs.x, v.x, w4))));
+      } else if (tid == MH) {
+        b1 = (((b1 + gs.x) + gs.y) + gs.z) + gs.w;  // b4
+      }
+    }
+  }
+  float* o = partial + (long long)blockIdx.x * NP;
+  float* m = o + (half == 0 ? O_W2 : O_W3);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[(tr + 8 * i) * MH + tc + 8 * j] = acc[i][j];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[O_W1 + r1 * MF + c1 + j] = w1[j];
+  o[tid < MH ? O_B1 + tid : O_B2 + tid - MH] = b0;
+  if (tid < MH) {
+    o[O_B3 + tid] = b1;
+    o[O_W4 + tid] = w4;
+  } else if (tid == MH) {
+    o[O_B4] = b1;
+  }
+}
+
+// grad[p] = the sum of the chunks' partials: SP_G groups of consecutive chunks, each in order, then the groups in
+// order.  One more block adds the tiles' loss parts in a fixed tree.
+constexpr int SP_P = 32, SP_G = 8;
+__global__ void __launch_bounds__(SP_P * SP_G) k_sum_partials(const float* __restrict__ partial, int nb,
+                                                              float* __restrict__ grad,
+                                                              const double* __restrict__ loss_part, long long nl,
+                                                              float* __restrict__ loss) {
+  __shared__ float part[SP_G][SP_P];
+  __shared__ double red[SP_P * SP_G];
+  const int tid = threadIdx.x, col = tid % SP_P, grp = tid / SP_P;
+  if (blockIdx.x == gridDim.x - 1) {
     double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += part[b];
-    *loss = (float)s;
+    for (long long b = tid; b < nl; b += SP_P * SP_G) s += loss_part[b];
+    red[tid] = s;
+    __syncthreads();
+    for (int h = SP_P * SP_G / 2; h > 0; h >>= 1) {
+      if (tid < h) red[tid] += red[tid + h];
+      __syncthreads();
+    }
+    if (tid == 0) *loss = (float)red[0];
+    return;
   }
+  const int p = blockIdx.x * SP_P + col;
+  const int per = (nb + SP_G - 1) / SP_G, b0 = grp * per, b1 = b0 + per < nb ? b0 + per : nb;
+  float s = 0.f;
+  if (p < NP) {
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) s += partial[(long long)b * NP + p];
+  }
+  part[grp][col] = s;
+  __syncthreads();
+  if (grp == 0 && p < NP) {
+    for (int q = 1; q < SP_G; ++q) s += part[q][col];
+    grad[p] = s;
+  }
+}
+
+// a persistent grid of tiles: as many CTAs as the SMs hold, at most one per tile
+int train_grid(long long n, int per_sm) {
+  const long long tiles = (n + TR_T - 1) / TR_T, cap = (long long)per_sm * xk_sm_count();
+  return (int)(tiles < cap ? tiles : cap);
 }
 
 // Adam with the float32 roundings of the oracle's NumPy expressions (no contraction).
@@ -832,7 +1006,8 @@ extern "C" xk_status xk_mlp_train_forward(const float* theta, const float* feat,
   if (!theta || n < 0 || (n > 0 && (!feat || !act || !logit)))
     return xk_set_error(XK_ERR_ARG, "xk_mlp_train_forward: bad arguments");
   if (n == 0) return XK_OK;
-  k_mlp_train_fwd<<<xk_blocks(n, TR_T), TR_T, 0, (cudaStream_t)s>>>(theta, feat, n, act, logit);
+  XK_CUDA(cudaFuncSetAttribute(k_mlp_train_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainFwdSmem)));
+  k_mlp_train_fwd<<<train_grid(n, 3), TR_T, sizeof(TrainFwdSmem), (cudaStream_t)s>>>(theta, feat, n, act, logit);
   XK_CHECK_LAUNCH();
   return XK_OK;
 }
@@ -843,20 +1018,21 @@ extern "C" xk_status xk_mlp_backward(const float* theta, const float* feat, cons
   if (!theta || !grad || !loss || n <= 0 || !feat || !act || !logit || !y || !w || !dvec || !g)
     return xk_set_error(XK_ERR_ARG, "xk_mlp_backward: bad arguments");
   cudaStream_t st = (cudaStream_t)s;
-  const int nb_t = xk_blocks(n, TR_T);
-  const int nb_w = (int)((n + WG_CHUNK - 1) / WG_CHUNK);
+  const long long tiles = (n + TR_T - 1) / TR_T, chunk = wgrad_chunk(n);
+  const int nb_w = (int)((n + chunk - 1) / chunk);
+  XK_CUDA(cudaFuncSetAttribute(k_mlp_train_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainBwdSmem)));
+  XK_CUDA(cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WgradSmem)));
   double* lpart = nullptr;
   float* part = nullptr;
-  XK_CUDA(cudaMallocAsync((void**)&lpart, sizeof(double) * nb_t, st));
+  XK_CUDA(cudaMallocAsync((void**)&lpart, sizeof(double) * tiles, st));
   cudaError_t e = cudaMallocAsync((void**)&part, sizeof(float) * (size_t)nb_w * NP, st);
   if (e != cudaSuccess) {
     cudaFreeAsync(lpart, st);
     return xk_set_cuda_error(e, __FILE__, __LINE__);
   }
-  k_mlp_train_bwd<<<nb_t, TR_T, 0, st>>>(theta, act, logit, y, w, n, dvec, g, lpart);
-  k_sum_loss<<<1, 32, 0, st>>>(lpart, nb_t, loss);
-  k_mlp_wgrad<<<nb_w, WG_T, 0, st>>>(feat, act, dvec, g, n, part);
-  k_sum_partials<<<(NP + 255) / 256, 256, 0, st>>>(part, nb_w, grad);
+  k_mlp_train_bwd<<<train_grid(n, 3), TR_T, sizeof(TrainBwdSmem), st>>>(theta, act, logit, y, w, n, dvec, g, lpart);
+  k_mlp_wgrad<<<nb_w, WG_T, sizeof(WgradSmem), st>>>(feat, act, dvec, g, n, chunk, part);
+  k_sum_partials<<<(NP + SP_P - 1) / SP_P + 1, SP_P * SP_G, 0, st>>>(part, nb_w, grad, lpart, tiles, loss);
   e = cudaGetLastError();
   cudaFreeAsync(lpart, st);
   cudaFreeAsync(part, st);
