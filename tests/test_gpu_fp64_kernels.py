@@ -103,6 +103,34 @@ def test_pair_kernels_against_the_oracle(n, delta, aligned):
         assert sparse_rel_err(K, K_ref) < 1e-8
 
 
+@pytest.mark.parametrize("n", [1, 33, 700])
+def test_exact_narrowphase_gives_the_oracle_bits(n):
+    """Every branch of the exact routine (ordinary, near-parallel, degenerate; frames fresh, transported, from
+    normals of any length, turned far) and the unit-vector forms of its divides, value for value."""
+    X, conn = _pairs(n, n + 5)
+    rng = np.random.default_rng(n)
+    nd = 6 * len(X)
+    radii = np.full(2 * n, 0.2)
+    mesh = DeviceMesh(X, conn, radii)
+    table = oc.new_pairs(np.stack([2 * np.arange(n), 2 * np.arange(n) + 1], 1), conn, radii)
+    dt = DevicePairTable(mesh.device)
+    cp = L.ContactParams(1.0, 0.5, 0.1, 0.0, 0.05, 0.1, 1, 0.0, 0.0, 0.0, 0.5, 0.0)
+    u = np.zeros(nd)
+    for step in range(4):
+        if step == 2:
+            for k in range(n):  # other lengths, no tangent, a normal turned round
+                table["normal"][k] *= (1.0, 1.0 + 2.0**-50, 1.5, -1.0)[k % 4]
+                table["t1"][k] *= (1.0, 0.0, 1.0 - 2.0**-40)[k % 3]
+        dt.from_host(table)
+        ud = torch.as_tensor(u, device="cuda")
+        L.call("xk_narrowphase", C.byref(mesh.c), C.byref(dt.c), ptr(ud), C.byref(cp), 1, stream_handle())
+        table = oc.update_geometry(table, oc.deformed_coords(X, u), g_on=0.05, g_off=0.1)
+        h = dt.to_host()
+        for k in ("s", "t", "gap", "normal", "t1", "t2", "status"):
+            assert np.array_equal(h[k], table[k]), (step, k)
+        u = u + 10.0 ** (-6 + 2 * step) * rng.normal(size=nd)
+
+
 @pytest.mark.parametrize("wires", [(1,), (30,), (31,), (32, 1), (62, 31), (5, 58, 3), "chain", "branched"])
 @pytest.mark.parametrize("scf", [None, 8.0])
 def test_beam_against_the_oracle(wires, scf):

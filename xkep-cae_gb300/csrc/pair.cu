@@ -36,36 +36,63 @@ XK_D void deformed(const xk_mesh& m, const double* u, int node, double* x) {
   x[2] = xadd(m.X[3LL * node + 2], u[6LL * node + 2]);
 }
 
-// _build_contact_frame_batch (geometry/_compute.py:154-261) for one pair, reference op order.
+// Correctly rounded square root of the square of a vector that is a unit vector up to rounding: with x = 1 + d
+// units of the last place, sqrt(x) = 1 + d/2 - O(d^2 2^-53) rounds to 1 + floor(d/2) units, on either side of one.
+XK_D double sqrt_unit64(double x) {
+  const long long one = 0x3ff0000000000000LL, d = __double_as_longlong(x) - one;
+  if ((unsigned long long)(d + 0x100000) < 0x200000ULL) return __longlong_as_double(one + (d >> 1));
+  return sqrt64(x);
+}
+
+// v / d by components, each correctly rounded, on one reciprocal; for d = 1 + e, |e| < 2^-49, as v - v e (the
+// quotient's further terms are below 2^-98 of it)
+XK_D void div3(const double* v, double d, double* out) {
+  if ((unsigned long long)(__double_as_longlong(d) - 0x3feffffffffffff0LL) < 0x18ULL) {
+    const double e = d - 1.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[i] = fma(-v[i], e, v[i]);
+    return;
+  }
+  const Divisor64 q = divisor64(d);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) out[i] = div64(v[i], q);
+}
+
+// x > c for a norm x, 2^LO > c: decided on the high word wherever x is at least 2^LO
+template <int LO>
+XK_D bool above64(double x, double c) { return in_range64<LO, 300>(x) || x > c; }
+
+// _build_contact_frame_batch (geometry/_compute.py:154-261) for one pair, reference op order; the divides
+// and square roots give the operators' bits (div64, sqrt64).
 XK_D void frame_exact(const double* nrm, const double* pt1, const double* pn, double* n, double* t1, double* t2) {
-  double nn = xsqrt(xdot_es(nrm, nrm));
-  if (!(nn >= 1e-30)) nn = (nn != nn) ? nn : 1e-30;
-  for (int i = 0; i < 3; ++i) n[i] = xdiv(nrm[i], nn);
-  const bool has_t1 = xsqrt(xdot_es(pt1, pt1)) > 1e-10;
-  const double pnn = xsqrt(xdot_es(pn, pn));
-  const bool has_n = pnn > 1e-10;
+  double nn = sqrt_unit64(xdot_es(nrm, nrm));
+  if (!in_range64<-99, 300>(nn) && !(nn >= 1e-30)) nn = (nn != nn) ? nn : 1e-30;
+  div3(nrm, nn, n);
+  const bool has_t1 = above64<-33>(sqrt_unit64(xdot_es(pt1, pt1)), 1e-10);
+  const double pnn = sqrt_unit64(xdot_es(pn, pn));
+  const bool has_n = above64<-33>(pnn, 1e-10);
   bool done = false;
   if (has_t1 && has_n) {
-    double so = (pnn >= 1e-30) ? pnn : 1e-30;
-    double no[3] = {xdiv(pn[0], so), xdiv(pn[1], so), xdiv(pn[2], so)};
-    double v[3];
+    const double so = pnn;  // above 1e-10 here
+    double no[3], v[3];
+    div3(pn, so, no);
     xcross(no, n, v);
-    const double sv = xsqrt(xdot_es(v, v));
+    const double sv = sqrt64(xdot_es(v, v));
     const double cv = xdot_es(no, n);
     double tr[3] = {pt1[0], pt1[1], pt1[2]};
-    if (sv >= 1e-12) {
+    if (above64<-39>(sv, 1e-12) || sv == 1e-12) {
       double vx[3], vvx[3];
       xcross(v, pt1, vx);
       xcross(v, vx, vvx);
-      const double f = xdiv(xsub(1.0, cv), xmul(sv, sv));
+      const double f = div64(xsub(1.0, cv), xmul(sv, sv));
       for (int i = 0; i < 3; ++i) tr[i] = xadd(xadd(pt1[i], vx[i]), xmul(f, vvx[i]));
     }
     const double dn = xdot_es(tr, n);
     double raw[3];
     for (int i = 0; i < 3; ++i) raw[i] = xsub(tr[i], xmul(dn, n[i]));
-    const double nr = xsqrt(xdot_es(raw, raw));
-    if (nr > 1e-10) {
-      for (int i = 0; i < 3; ++i) t1[i] = xdiv(raw[i], nr);
+    const double nr = sqrt_unit64(xdot_es(raw, raw));
+    if (above64<-33>(nr, 1e-10)) {
+      div3(raw, nr, t1);
       xcross(n, t1, t2);
       done = true;
     }
@@ -74,9 +101,9 @@ XK_D void frame_exact(const double* nrm, const double* pt1, const double* pn, do
     const double dn = xdot_es(pt1, n);
     double raw[3];
     for (int i = 0; i < 3; ++i) raw[i] = xsub(pt1[i], xmul(dn, n[i]));
-    const double nr = xsqrt(xdot_es(raw, raw));
-    if (nr > 1e-10) {
-      for (int i = 0; i < 3; ++i) t1[i] = xdiv(raw[i], nr);
+    const double nr = sqrt_unit64(xdot_es(raw, raw));
+    if (above64<-33>(nr, 1e-10)) {
+      div3(raw, nr, t1);
       xcross(n, t1, t2);
       done = true;
     }
@@ -88,9 +115,9 @@ XK_D void frame_exact(const double* nrm, const double* pt1, const double* pn, do
     const double dn = xdot_es(ref, n);
     double raw[3];
     for (int i = 0; i < 3; ++i) raw[i] = xsub(ref[i], xmul(dn, n[i]));
-    double nr = xsqrt(xdot_es(raw, raw));
+    double nr = sqrt_unit64(xdot_es(raw, raw));
     if (!(nr >= 1e-30)) nr = (nr != nr) ? nr : 1e-30;
-    for (int i = 0; i < 3; ++i) t1[i] = xdiv(raw[i], nr);
+    div3(raw, nr, t1);
     xcross(n, t1, t2);
   }
 }
@@ -206,14 +233,29 @@ XK_D double coat_compression(const xk_mesh& m, int ea, int eb, double gap) {
   return fmax(0.0, xsub(coat_total_of(m, ea, eb), gap));
 }
 
+__noinline__ __device__ void closest_exact_call(const double* y, double* o) {
+  double diff[3];
+  closest_exact(y, y + 3, y + 6, y + 9, o[0], o[1], o[2], o + 3, diff);
+}
+
 XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __restrict__ u, double g_on,
                            double g_off, int allow_deact, int update_active, int i) {
   const long long cap = p.cap;
   PairNodes nd = pair_nodes(m, p.ea[i], p.eb[i]);
   double x[4][3];
   for (int k = 0; k < 4; ++k) deformed(m, u, nd.n[k], x[k]);
-  double s, t, dist, nrm[3], diff[3];
-  closest_exact(x[0], x[1], x[2], x[3], s, t, dist, nrm, diff);
+  double s, t, dist, nrm[3];
+  if (!closest_exact_fast(x, s, t, dist, nrm)) {
+    // near-parallel or degenerate: every branch of the routine, out of line on its own copies, so that they
+    // neither hold registers here nor send this path's arrays to memory
+    double y[12], o[6];
+    for (int k = 0; k < 12; ++k) y[k] = x[k / 3][k % 3];
+    closest_exact_call(y, o);
+    s = o[0];
+    t = o[1];
+    dist = o[2];
+    for (int k = 0; k < 3; ++k) nrm[k] = o[3 + k];
+  }
   const bool coat = m.core_radii != nullptr;
   const double gap = coat ? xsub(dist, xadd(m.core_radii[p.ea[i]], m.core_radii[p.eb[i]]))
                           : xsub(dist, xadd(m.radii[p.ea[i]], m.radii[p.eb[i]]));
@@ -240,6 +282,8 @@ XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __
   }
 }
 
+// Bounded by the FP64 pipe: 328 operations a pair with div64 / sqrt64 in place of the operators (430 before),
+// 255 with the unit-vector forms in the frame.  632,000 pairs: 518 -> 331 us.
 __global__ void k_narrow_exact(xk_mesh m, xk_pairs p, const double* __restrict__ u, double g_on, double g_off,
                                int allow_deact, int update_active) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -369,7 +413,7 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
 // unit frame, NaN) take the exact routine.
 // Measured at the 1027-wire strand (2.46M other pairs, 0.75M contributing ones), exact routine for every
 // pair against this: other pairs 1757 -> 652 us (132 FP64 operations a pair at the pipe's measured 1.64 per
-// clock and SM), contributing pairs 936 -> 599 us (393 us if these were fused throughout).
+// clock and SM), contributing pairs 936 -> 572 us (393 us if these were fused throughout).
 // ===========================================================================
 
 XK_D double fdot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
@@ -475,9 +519,7 @@ XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const int* n
     double nrm[3];
     ok = closest_exact_fast(x, s, t, dist, nrm);
     if (ok) {  // the frame's own normalisation (frame_exact)
-      const Divisor64 q = divisor64(sqrt64(xdot_es(nrm, nrm)));
-#pragma unroll
-      for (int c = 0; c < 3; ++c) n[c] = div64(nrm[c], q);
+      div3(nrm, sqrt_unit64(xdot_es(nrm, nrm)), n);
     }
   } else {
     ok = closest64(x, s, t, dist, n);
