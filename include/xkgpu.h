@@ -678,6 +678,12 @@ xk_status xk_constraint_jacobian_noalloc(const xk_mesh* m, const xk_pairs* p, in
                                          double* vals, int32_t* pair_index, int64_t cap, int64_t* n_rows,
                                          xk_stream s);
 
+/* The detection entry points take their scratch from a memory pool of the
+ * library's own on the current device, which keeps up to 256 MiB between calls.
+ * This gives back what it holds beyond keep_bytes and does not use; calls in
+ * progress on any stream are not affected. */
+xk_status xk_scratch_trim(int64_t keep_bytes);
+
 /* Fixed-order FP64 sum of squares of x[0..n) into *out (device). */
 xk_status xk_norm2(const double* x, int64_t n, double* out, xk_stream s);
 

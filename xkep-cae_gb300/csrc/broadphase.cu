@@ -614,30 +614,6 @@ __global__ void k_merge_old(xk_pairs old, const int32_t* __restrict__ cand, cons
   out.status[pos] = 0;  // INACTIVE
 }
 
-struct Scratch {
-  cudaStream_t s;
-  void* p[24];
-  int n = 0;
-  template <typename T>
-  xk_status get(T** out, long long count) {
-    if (n >= (int)(sizeof(p) / sizeof(p[0]))) return xk_set_error(XK_ERR_OVERFLOW, "scratch table full");
-    if (count < 1) count = 1;
-    cudaError_t e = cudaMallocAsync((void**)out, sizeof(T) * count, s);
-    if (e != cudaSuccess) return xk_set_cuda_error(e, __FILE__, __LINE__);
-    p[n++] = *out;
-    return XK_OK;
-  }
-  ~Scratch() {
-    for (int i = 0; i < n; ++i) cudaFreeAsync(p[i], s);
-  }
-};
-
-#define XK_TRY(x)                  \
-  do {                             \
-    xk_status r__ = (x);           \
-    if (r__ != XK_OK) return r__;  \
-  } while (0)
-
 }  // namespace
 
 // slot-list length of the walk: grows to the longest list seen (a power of two), kept for later calls
@@ -653,7 +629,11 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   const long long ne = m->n_elems;
   if (ne < 2) return XK_OK;
   if (ne > 0x7fffffffLL) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: more than 2^31 segments");
-  Scratch S{st};
+  const long long cap_cells = ne * 8 > 4096 ? ne * 8 : 4096;
+  int slot_cap = g_slot_cap.load();
+  XkScratch S(st);
+  if ((double)ne * slot_cap * 8.0 <= 64.0e9)  // one allocation for the usual case: boxes, cells, lists, scans
+    XK_TRY(S.reserve((size_t)ne * (48 + 32 + 32 + 8 + 12 + 8 + 8 * (size_t)slot_cap) + (size_t)cap_cells * 9 + (1 << 16)));
   double* box;
   float4* boxf;
   double4_32a* mid;
@@ -674,7 +654,6 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   XK_CUDA(cudaMemcpyAsync(ext, init, sizeof(init), cudaMemcpyHostToDevice, st));
   k_aabb<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, u, bp->margin, box, boxf, mid, ext, ext_sum);
   // the grid has at most cap_cells cells, so the cell arrays are sized without reading it back
-  const long long cap_cells = ne * 8 > 4096 ? ne * 8 : 4096;
   k_grid<<<1, 1, 0, st>>>(ext, ext_sum, ne, cap_cells, bp->cell_size, grid);
   XK_CHECK_LAUNCH();
   int32_t *segs, *cstart, *cfill, *cnt, *cnt2, *off2, *ecell;
@@ -689,7 +668,7 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   XK_CUDA(cudaMemsetAsync(cfill, 0, sizeof(int32_t) * (cap_cells + 1), st));
   k_cell_count<<<xk_blocks(ne, 256), 256, 0, st>>>(box, ne, grid, ecell, cfill);
   XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(cfill, cstart, cap_cells + 1, nullptr, st));
+  XK_TRY(xk_exclusive_scan_i32(cfill, cstart, cap_cells + 1, nullptr, st, &S));
   XK_CUDA(cudaMemsetAsync(cfill, 0, sizeof(int32_t) * (cap_cells + 1), st));
   k_cell_scatter<<<xk_blocks(ne, 256), 256, 0, st>>>(ne, ecell, cstart, cfill, segs);
   k_cell_sort<<<xk_blocks(cap_cells, 256), 256, 0, st>>>(cap_cells, cstart, segs);
@@ -702,7 +681,6 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   XK_TRY(S.get(&tot, 2));
   const int warp_blocks = xk_blocks(ne * 32, BP_T);
   const int excl_layer = (bp->exclude_same_layer && m->layer) ? 1 : 0;
-  int slot_cap = g_slot_cap.load();
   for (int attempt = 0;; ++attempt) {
     if ((double)ne * slot_cap * 8.0 > 64.0e9)
       return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: candidate lists too long for the slot buffers");
@@ -714,7 +692,7 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
     k_sweep<<<warp_blocks, BP_T, 0, st>>>(*m, box, boxf, grid, segs, cstart, bp->exclude_shared, excl_layer,
                                           slot_cap, slot, cnt, rsum, raw_dev, max_cnt);
     XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt, off2, ne, tot, st));  // tot[0]: candidates before the prescreen
+    XK_TRY(xk_exclusive_scan_i32(cnt, off2, ne, tot, st, &S));  // tot[0]: candidates before the prescreen
     const double* ex = nullptr;
     if (bp->midpoint_prescreening) {
       if (!(bp->prescreening_margin > 0.0)) k_radsum_partial<<<RED_BLOCKS, RED_T, 0, st>>>(rsum, ne, part);
@@ -724,7 +702,7 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
     }
     k_slots_rank<<<warp_blocks, BP_T, 0, st>>>(*m, mid, slot, cnt, slot_cap, ex, srt, cnt2);
     XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt2, off2, ne, tot + 1, st));
+    XK_TRY(xk_exclusive_scan_i32(cnt2, off2, ne, tot + 1, st, &S));
     k_slots_emit<<<warp_blocks, BP_T, 0, st>>>(ne, srt, cnt, slot_cap, off2, cap, out_pairs);
     XK_CHECK_LAUNCH();
     int64_t h[2];
@@ -759,10 +737,11 @@ static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t
   if ((long long)out->cap < (long long)old->n + n_cands)
     return xk_set_error(XK_ERR_CAPACITY, "xk_pairs_merge: out->cap < old->n + n_cands");
   cudaStream_t st = (cudaStream_t)s;
-  Scratch S{st};
+  XkScratch S(st);
   int32_t *r, *R, *ostart, *cstart;
   int64_t* tot;
   const long long ne = m->n_elems;
+  XK_TRY(S.reserve(8 * ((size_t)old->n + 1) + 8 * ((size_t)ne + 2) + (size_t)old->n / 64 + 4096));
   XK_TRY(S.get(&r, (long long)old->n + 1));
   XK_TRY(S.get(&R, (long long)old->n + 1));
   XK_TRY(S.get(&ostart, ne + 2));
@@ -776,7 +755,7 @@ static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t
   else
     k_merge_flags<false><<<xk_blocks((long long)old->n + 1, 256), 256, 0, st>>>(*old, cands, cstart, n_cands, r);
   XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(r, R, (long long)old->n + 1, tot, st));
+  XK_TRY(xk_exclusive_scan_i32(r, R, (long long)old->n + 1, tot, st, &S));
   if (n_cands > 0) k_merge_new<<<xk_blocks(n_cands, 256), 256, 0, st>>>(*old, ostart, cands, n_cands, R, *out);
   if (old->n > 0) k_merge_old<<<xk_blocks(old->n, 256), 256, 0, st>>>(*old, cands, cstart, n_cands, r, R, *out);
   XK_CHECK_LAUNCH();

@@ -1120,30 +1120,6 @@ __global__ void __launch_bounds__(32 * GT_WARPS) k_gather_tangent(long long nnzb
   for (int i = lane; i < 9 * nblk; i += 32) K[9 * b0 + i] = A[i];
 }
 
-struct Scratch {
-  cudaStream_t s;
-  void* p[24];
-  int n = 0;
-  template <typename T>
-  xk_status get(T** out, long long count) {
-    if (n >= (int)(sizeof(p) / sizeof(p[0]))) return xk_set_error(XK_ERR_OVERFLOW, "scratch table full");
-    if (count < 1) count = 1;
-    cudaError_t e = cudaMallocAsync((void**)out, sizeof(T) * count, s);
-    if (e != cudaSuccess) return xk_set_cuda_error(e, __FILE__, __LINE__);
-    p[n++] = *out;
-    return XK_OK;
-  }
-  ~Scratch() {
-    for (int i = 0; i < n; ++i) cudaFreeAsync(p[i], s);
-  }
-};
-
-#define XK_TRY(x)                 \
-  do {                            \
-    xk_status r__ = (x);          \
-    if (r__ != XK_OK) return r__; \
-  } while (0)
-
 xk_status fetch_i64(const int64_t* dev, int64_t* host, int n, cudaStream_t st) {
   XK_CUDA(cudaMemcpyAsync(host, dev, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st));
   XK_CUDA(cudaStreamSynchronize(st));
@@ -1160,9 +1136,13 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
   const int nn = m->n_nodes;
   const long long np = p->n;
   pat->n_nodes = nn;
-  Scratch S{st};
+  XkScratch S(st);
   int32_t *flag, *mpos, *cnt, *fill, *err;
   int64_t* tot;
+  const long long nmx = m->n_elems > nn ? m->n_elems : nn;
+  XK_TRY(S.reserve(8 * ((size_t)np + 1) + 8 * ((size_t)nn + 1) + 8 * ((size_t)nmx + 1) +
+                   12 * ((size_t)pat->cap_blocks + 1) + ((size_t)np + 4 * (size_t)nmx + (size_t)pat->cap_blocks) / 64 +
+                   (1 << 14)));
   XK_TRY(S.get(&flag, np + 1));
   XK_TRY(S.get(&mpos, np + 1));
   XK_TRY(S.get(&cnt, nn + 1));
@@ -1172,7 +1152,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
   // members and others
   k_flags<<<xk_blocks(np + 1, 256), 256, 0, st>>>(*p, flag);
   XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(flag, mpos, np + 1, tot, st));
+  XK_TRY(xk_exclusive_scan_i32(flag, mpos, np + 1, tot, st, &S));
   int64_t h[4] = {0, 0, 0, 0};
   XK_TRY(fetch_i64(tot, h, 1, st));
   const long long nm = h[0];
@@ -1186,7 +1166,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
   XK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (nn + 1), st));
   if (nm > 0) k_inc_count<<<xk_blocks(nm, 256), 256, 0, st>>>(pat->member_nodes, (int)nm, cnt);
   XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(cnt, pat->inc_ptr, nn + 1, nullptr, st));
+  XK_TRY(xk_exclusive_scan_i32(cnt, pat->inc_ptr, nn + 1, nullptr, st, &S));
   XK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (nn + 1), st));
   if (nm > 0) k_inc_fill<<<xk_blocks(nm, 256), 256, 0, st>>>(pat->member_nodes, (int)nm, pat->inc_ptr, fill, pat->inc);
   k_segment_sort<<<xk_blocks(32LL * nn, SEG_T), SEG_T, 0, st>>>(pat->inc_ptr, nn, pat->inc);
@@ -1197,7 +1177,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
                                                    nullptr, nullptr, err);
   XK_CHECK_LAUNCH();
   XK_CUDA(cudaMemsetAsync(cnt + nn, 0, sizeof(int32_t), st));
-  XK_TRY(xk_exclusive_scan_i32(cnt, pat->row_ptr, nn + 1, tot + 1, st));
+  XK_TRY(xk_exclusive_scan_i32(cnt, pat->row_ptr, nn + 1, tot + 1, st, &S));
   int32_t herr = 0;
   XK_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   XK_TRY(fetch_i64(tot, h, 2, st));
@@ -1217,7 +1197,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
   if (nm > 0) k_contrib<0><<<xk_blocks(nm, 128), 128, 0, st>>>(pat->member_nodes, (int)nm, pat->row_ptr, pat->col,
                                                                 bcnt, nullptr, nullptr, err);
   XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(bcnt, pat->blk_ptr, nb + 1, tot + 2, st));
+  XK_TRY(xk_exclusive_scan_i32(bcnt, pat->blk_ptr, nb + 1, tot + 2, st, &S));
   XK_CUDA(cudaMemsetAsync(bfill, 0, sizeof(int32_t) * (nb + 1), st));
   if (nm > 0) k_contrib<1><<<xk_blocks(nm, 128), 128, 0, st>>>(pat->member_nodes, (int)nm, pat->row_ptr, pat->col,
                                                                 bfill, pat->blk_ptr, pat->contrib, err);
@@ -1236,7 +1216,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
     XK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (nn + 1), st));
     if (nb > 0) k_lower_index<0><<<xk_blocks(nb, 256), 256, 0, st>>>(nb, pat->blk_row, pat->col, cnt, nullptr, nullptr);
     XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt, pat->low_ptr, nn + 1, tot + 3, st));
+    XK_TRY(xk_exclusive_scan_i32(cnt, pat->low_ptr, nn + 1, tot + 3, st, &S));
     XK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (nn + 1), st));
     if (nb > 0)
       k_lower_index<1><<<xk_blocks(nb, 256), 256, 0, st>>>(nb, pat->blk_row, pat->col, fill, pat->low_ptr,
@@ -1261,7 +1241,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
       XK_CUDA(cudaMemsetAsync(ecnt, 0, sizeof(int32_t) * (nn + 1), st));
       if (ne > 0) k_node_elem_count<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, ecnt);
       XK_CHECK_LAUNCH();
-      XK_TRY(xk_exclusive_scan_i32(ecnt, pat->node_elem_ptr, nn + 1, nullptr, st));
+      XK_TRY(xk_exclusive_scan_i32(ecnt, pat->node_elem_ptr, nn + 1, nullptr, st, &S));
       XK_CUDA(cudaMemsetAsync(efill, 0, sizeof(int32_t) * (nn + 1), st));
       if (ne > 0)
         k_node_elem_fill<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, pat->node_elem_ptr, efill,
@@ -1274,7 +1254,7 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
     XK_CUDA(cudaMemsetAsync(ecnt, 0, sizeof(int32_t) * (ne + 1), st));
     if (nm > 0) k_elem_inc_count<<<xk_blocks(nm, 256), 256, 0, st>>>(*p, pat->members, (int)nm, ecnt);
     XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(ecnt, pat->elem_ptr, ne + 1, nullptr, st));
+    XK_TRY(xk_exclusive_scan_i32(ecnt, pat->elem_ptr, ne + 1, nullptr, st, &S));
     XK_CUDA(cudaMemsetAsync(efill, 0, sizeof(int32_t) * (ne + 1), st));
     if (nm > 0)
       k_elem_inc_fill<<<xk_blocks(nm, 256), 256, 0, st>>>(*p, pat->members, (int)nm, pat->elem_ptr, efill,

@@ -2,8 +2,6 @@
 // the factorised pair tangent.  One thread per pair; contributing pairs and
 // the rest run as two launches over the per-increment lists so that warps do
 // not diverge between the two kinds of work.
-#include <cuda.h>
-
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -1572,7 +1570,7 @@ extern "C" xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, cons
     return XK_OK;
   }
   int32_t* list = nullptr;
-  XK_CUDA(cudaMallocAsync((void**)&list, sizeof(int32_t) * ((size_t)p->n + 1), st));
+  XK_TRY(xk_scratch_alloc((void**)&list, sizeof(int32_t) * ((size_t)p->n + 1), st));
   xk_status r = XK_OK;
   cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int32_t), st);
   if (e == cudaSuccess) {
@@ -1773,32 +1771,6 @@ static_assert(JNA_MAX_PAIRS % 2 == 0, "flags are packed two per word");
 
 static __device__ __align__(256) int64_t g_jna_scratch[JNA_WORDS];
 
-// Id of the calling thread's current context (CUDA 12's cuCtxGetId, reached
-// through the runtime's driver entry points so that the library needs no
-// libcuda at link time); false when there is no current context yet or the
-// driver does not offer the calls.
-using PfnCtxGetCurrent = CUresult (*)(CUcontext*);
-using PfnCtxGetId = CUresult (*)(CUcontext, unsigned long long*);
-bool current_context_id(unsigned long long* id) {
-  static PfnCtxGetCurrent get_current = nullptr;
-  static PfnCtxGetId get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaDriverEntryPointQueryResult q;
-    void* f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<PfnCtxGetCurrent>(f);
-    f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<PfnCtxGetId>(f);
-  });
-  CUcontext c = nullptr;
-  if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || !c) return false;
-  return get_id(c, id) == CUDA_SUCCESS;
-}
-
 // Address of the scratch array in the current context.  The look-up loads this
 // module's device globals into the context, so the first call in a context is
 // the set-up call; make it before any work that must not see one.  The address
@@ -1817,7 +1789,7 @@ xk_status jna_scratch(int64_t** out) {
   XK_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return xk_set_error(XK_ERR_ARG, "device ordinal out of range");
   unsigned long long cid = 0;
-  bool have = current_context_id(&cid);
+  bool have = xk_context_id(&cid);
   if (have) {
     std::lock_guard<std::mutex> lock(g_jna_mutex);
     if (g_jna_cache[dev].ptr && g_jna_cache[dev].ctx == cid) {
@@ -1827,7 +1799,7 @@ xk_status jna_scratch(int64_t** out) {
   }
   int64_t* p = nullptr;
   XK_CUDA(cudaGetSymbolAddress((void**)&p, g_jna_scratch));
-  if (!have) have = current_context_id(&cid);  // the look-up made the primary context current
+  if (!have) have = xk_context_id(&cid);  // the look-up made the primary context current
   if (have) {
     std::lock_guard<std::mutex> lock(g_jna_mutex);
     g_jna_cache[dev].ctx = cid;

@@ -1,7 +1,10 @@
-// Error state, device-wide scans, radix sort and FP64 reductions.
+// Error state, scratch pool, device-wide scans and FP64 reductions.
+#include <cuda.h>
+
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "xk_common.cuh"
 
@@ -33,6 +36,102 @@ int xk_sm_count() {
   if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
   cache[dev].store(n, std::memory_order_relaxed);
   return n;
+}
+
+// --------------------------------------------------------------------------- scratch
+
+// Id of the calling thread's current context (CUDA 12's cuCtxGetId, reached
+// through the runtime's driver entry points so that the library needs no
+// libcuda at link time); false when there is no current context yet or the
+// driver does not offer the calls.
+namespace {
+using PfnCtxGetCurrent = CUresult (*)(CUcontext*);
+using PfnCtxGetId = CUresult (*)(CUcontext, unsigned long long*);
+}  // namespace
+
+bool xk_context_id(unsigned long long* id) {
+  static PfnCtxGetCurrent get_current = nullptr;
+  static PfnCtxGetId get_id = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaDriverEntryPointQueryResult q;
+    void* f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_current = reinterpret_cast<PfnCtxGetCurrent>(f);
+    f = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<PfnCtxGetId>(f);
+  });
+  CUcontext c = nullptr;
+  if (!get_current || !get_id || get_current(&c) != CUDA_SUCCESS || !c) return false;
+  return get_id(c, id) == CUDA_SUCCESS;
+}
+
+// The pool of each device, with the context it was made in: a context made later on the device (after
+// cudaDeviceReset) gets its own.
+namespace {
+struct ScratchPool {
+  unsigned long long ctx = 0;
+  cudaMemPool_t pool = nullptr;
+};
+std::mutex g_pool_mutex;
+ScratchPool g_pool[64];
+
+// Making and trimming a pool are no stream operations: a capture that another thread has under way must not
+// forbid them, nor end by them.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// the current device's pool, made on first use; null if there is none to be had
+cudaMemPool_t scratch_pool(bool make) {
+  int dev = 0;
+  unsigned long long id = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !xk_context_id(&id)) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  ScratchPool& g = g_pool[dev];
+  if (g.pool && g.ctx == id) return g.pool;
+  if (!make) return nullptr;
+  RelaxedCapture relaxed;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = XK_SCRATCH_KEEP;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    if (pool) cudaMemPoolDestroy(pool);
+    cudaGetLastError();
+    return nullptr;
+  }
+  g.pool = pool;
+  g.ctx = id;
+  return pool;
+}
+}  // namespace
+
+xk_status xk_scratch_alloc(void** out, size_t bytes, cudaStream_t s) {
+  if (bytes < 1) bytes = 1;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  XK_CUDA(cudaStreamIsCapturing(s, &cap));
+  cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool(true) : nullptr;
+  XK_CUDA(pool ? cudaMallocFromPoolAsync(out, bytes, pool, s) : cudaMallocAsync(out, bytes, s));
+  return XK_OK;
+}
+
+extern "C" xk_status xk_scratch_trim(int64_t keep_bytes) {
+  if (keep_bytes < 0) return xk_set_error(XK_ERR_ARG, "xk_scratch_trim: keep_bytes");
+  if (cudaMemPool_t pool = scratch_pool(false)) {
+    RelaxedCapture relaxed;
+    XK_CUDA(cudaMemPoolTrimTo(pool, (size_t)keep_bytes));
+  }
+  return XK_OK;
 }
 
 // --------------------------------------------------------------------------- scan
@@ -255,7 +354,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_onepass(const TI* __restrict__ 
 }
 
 template <typename TI, typename TO>
-xk_status scan_impl(const TI* in, TO* out, long long n, int64_t* total_dev, cudaStream_t s) {
+xk_status scan_impl(const TI* in, TO* out, long long n, int64_t* total_dev, cudaStream_t s, XkScratch* S) {
   if (n <= 0) {
     if (total_dev) XK_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(int64_t), s));
     return XK_OK;
@@ -264,7 +363,8 @@ xk_status scan_impl(const TI* in, TO* out, long long n, int64_t* total_dev, cuda
   // one allocation: aggregates, inclusive prefixes, then the flags and the ticket (zeroed)
   char* buf = nullptr;
   const size_t words = sizeof(int64_t) * 2 * nb, tail = sizeof(int) * (nb + 1);
-  XK_CUDA(cudaMallocAsync((void**)&buf, words + tail, s));
+  XkScratch own(s);
+  XK_TRY((S ? S : &own)->get(&buf, (long long)(words + tail)));
   int64_t* agg = reinterpret_cast<int64_t*>(buf);
   int* flag = reinterpret_cast<int*>(buf + words);
   cudaError_t e = cudaMemsetAsync(flag, 0, tail, s);
@@ -273,19 +373,14 @@ xk_status scan_impl(const TI* in, TO* out, long long n, int64_t* total_dev, cuda
                                                            reinterpret_cast<unsigned*>(flag + nb));
     e = cudaGetLastError();
   }
-  cudaFreeAsync(buf, s);
   if (e != cudaSuccess) return xk_set_cuda_error(e, __FILE__, __LINE__);
   return XK_OK;
 }
 }  // namespace
 
 xk_status xk_exclusive_scan_i32(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
-                                cudaStream_t s) {
-  return scan_impl<int32_t, int32_t>(in, out, n, total_dev, s);
-}
-xk_status xk_exclusive_scan_i64(const int64_t* in, int64_t* out, long long n, int64_t* total_dev,
-                                cudaStream_t s) {
-  return scan_impl<int64_t, int64_t>(in, out, n, total_dev, s);
+                                cudaStream_t s, XkScratch* S) {
+  return scan_impl<int32_t, int32_t>(in, out, n, total_dev, s, S);
 }
 
 long long xk_scan_tiles(long long n) { return n <= 0 ? 0 : (n + SCAN_TILE - 1) / SCAN_TILE; }
@@ -302,99 +397,6 @@ xk_status xk_exclusive_scan_i32_scratch(const int32_t* in, int32_t* out, long lo
   k_scan_bsums<<<1, SCAN_T, 0, s>>>(bsum, nb, total_dev);
   k_tile_scan<int32_t, int32_t><<<(unsigned)nb, SCAN_T, 0, s>>>(in, out, n, bsum);
   XK_CHECK_LAUNCH();
-  return XK_OK;
-}
-
-// --------------------------------------------------------------------------- radix sort
-
-namespace {
-constexpr int RS_T = 256;
-constexpr int RS_I = 8;
-constexpr int RS_TILE = RS_T * RS_I;
-
-__global__ void k_rs_hist(const uint64_t* __restrict__ keys, long long n, int shift,
-                          int32_t* __restrict__ hist, int nblocks) {
-  __shared__ int cnt[256];
-  cnt[threadIdx.x] = 0;
-  __syncthreads();
-  long long t0 = (long long)blockIdx.x * RS_TILE;
-  for (int i = 0; i < RS_I; ++i) {
-    long long idx = t0 + (long long)i * RS_T + threadIdx.x;
-    if (idx < n) atomicAdd(&cnt[(keys[idx] >> shift) & 255u], 1);
-  }
-  __syncthreads();
-  hist[(long long)threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
-}
-
-__global__ void k_rs_scatter(const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin,
-                             uint64_t* __restrict__ kout, int32_t* __restrict__ vout, long long n,
-                             int shift, const int32_t* __restrict__ off, int nblocks) {
-  __shared__ int run[256];
-  run[threadIdx.x] = off[(long long)threadIdx.x * nblocks + blockIdx.x];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  long long t0 = (long long)blockIdx.x * RS_TILE;
-  for (int i = 0; i < RS_I; ++i) {
-    long long idx = t0 + (long long)i * RS_T + threadIdx.x;
-    bool valid = idx < n;
-    uint64_t k = valid ? kin[idx] : 0ull;
-    int32_t v = valid ? vin[idx] : 0;
-    int d = valid ? (int)((k >> shift) & 255u) : 256;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    int rank = __popc(peers & lt);
-    int cntw = __popc(peers);
-    int leader = __ffs(peers) - 1;
-    for (int w = 0; w < RS_T / 32; ++w) {
-      __syncthreads();
-      if (warp == w) {
-        int base = (lane == leader && valid) ? run[d] : 0;
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (valid) {
-          long long dst = (long long)base + rank;
-          kout[dst] = k;
-          vout[dst] = v;
-        }
-        if (lane == leader && valid) run[d] = base + cntw;
-      }
-    }
-    __syncthreads();
-  }
-}
-}  // namespace
-
-xk_status xk_radix_sort_u64(uint64_t* keys, int32_t* vals, long long n, int bits, cudaStream_t s) {
-  if (n <= 1) return XK_OK;
-  int passes = (bits + 7) / 8;
-  if (passes <= 0) return XK_OK;
-  int nb = (int)((n + RS_TILE - 1) / RS_TILE);
-  uint64_t* k2 = nullptr;
-  int32_t *v2 = nullptr, *hist = nullptr;
-  XK_CUDA(cudaMallocAsync((void**)&k2, sizeof(uint64_t) * n, s));
-  XK_CUDA(cudaMallocAsync((void**)&v2, sizeof(int32_t) * n, s));
-  XK_CUDA(cudaMallocAsync((void**)&hist, sizeof(int32_t) * 256 * (long long)nb, s));
-  uint64_t *ka = keys, *kb = k2;
-  int32_t *va = vals, *vb = v2;
-  xk_status st = XK_OK;
-  for (int p = 0; p < passes && st == XK_OK; ++p) {
-    int shift = 8 * p;
-    k_rs_hist<<<nb, RS_T, 0, s>>>(ka, n, shift, hist, nb);
-    st = xk_exclusive_scan_i32(hist, hist, 256LL * nb, nullptr, s);
-    if (st != XK_OK) break;
-    k_rs_scatter<<<nb, RS_T, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb);
-    uint64_t* tk = ka; ka = kb; kb = tk;
-    int32_t* tv = va; va = vb; vb = tv;
-  }
-  cudaError_t e = cudaGetLastError();
-  if (st == XK_OK && e == cudaSuccess && ka != keys) {
-    e = cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(vals, va, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s);
-  }
-  cudaFreeAsync(k2, s);
-  cudaFreeAsync(v2, s);
-  cudaFreeAsync(hist, s);
-  if (st != XK_OK) return st;
-  if (e != cudaSuccess) return xk_set_cuda_error(e, __FILE__, __LINE__);
   return XK_OK;
 }
 

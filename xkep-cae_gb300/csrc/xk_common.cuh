@@ -193,16 +193,65 @@ xk_status xk_set_error(xk_status code, const char* msg);
 // SM count of the current device, read once per device ordinal (1 when it cannot be read).
 int xk_sm_count();
 
-// Device-wide exclusive scans (scan.cu).  Scratch is allocated stream-ordered.
+// Id of the calling thread's current context; false when there is none yet.
+bool xk_context_id(unsigned long long* id);
+
+// Stream-ordered scratch (freed with cudaFreeAsync) from a memory pool of this library's own, one per device: the
+// default pool gives freed memory back to the system at every synchronisation, and a detection has five of them,
+// each followed by allocations that map it again.  The pool holds on to at most XK_SCRATCH_KEEP bytes between
+// calls; xk_scratch_trim gives those back too.  While s is being captured the default pool is used.
+constexpr size_t XK_SCRATCH_KEEP = 256u << 20;
+xk_status xk_scratch_alloc(void** out, size_t bytes, cudaStream_t s);
+
+// The scratch of one call: get() carves aligned pieces from the block that reserve() allocated, or allocates
+// what does not fit; everything is freed with the object, in stream order.
+struct XkScratch {
+  cudaStream_t s;
+  void* p[24];
+  int n = 0;
+  char* base = nullptr;
+  size_t size = 0, used = 0;
+  explicit XkScratch(cudaStream_t st) : s(st) {}
+  XkScratch(const XkScratch&) = delete;
+  static size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+  xk_status take(void** out, size_t bytes) {
+    if (n >= (int)(sizeof(p) / sizeof(p[0]))) return xk_set_error(XK_ERR_OVERFLOW, "scratch table full");
+    const xk_status r = xk_scratch_alloc(out, bytes, s);
+    if (r == XK_OK) p[n++] = *out;
+    return r;
+  }
+  xk_status reserve(size_t bytes) {
+    size = padded(bytes);
+    used = 0;
+    return take((void**)&base, size);
+  }
+  template <typename T>
+  xk_status get(T** out, long long count) {
+    const size_t bytes = padded(sizeof(T) * (size_t)(count < 1 ? 1 : count));
+    if (used + bytes <= size) {
+      *out = reinterpret_cast<T*>(base + used);
+      used += bytes;
+      return XK_OK;
+    }
+    return take((void**)out, bytes);
+  }
+  ~XkScratch() {
+    for (int i = 0; i < n; ++i) cudaFreeAsync(p[i], s);
+  }
+};
+
+#define XK_TRY(x)                 \
+  do {                            \
+    xk_status r__ = (x);          \
+    if (r__ != XK_OK) return r__; \
+  } while (0)
+
+// Device-wide exclusive scan (util.cu), its scratch from S or of its own.
 xk_status xk_exclusive_scan_i32(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
-                                cudaStream_t s);
-xk_status xk_exclusive_scan_i64(const int64_t* in, int64_t* out, long long n, int64_t* total_dev,
-                                cudaStream_t s);
+                                cudaStream_t s, XkScratch* S = nullptr);
 // Number of block sums the scans use for n elements, and the int32 scan with a
 // caller-provided block-sum array of bsum_cap words (same kernels, same result;
 // allocates nothing).
 long long xk_scan_tiles(long long n);
 xk_status xk_exclusive_scan_i32_scratch(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
                                         int64_t* bsum, long long bsum_cap, cudaStream_t s);
-// Stable LSD radix sort of 64-bit keys with 32-bit values; `bits` low key bits are sorted.
-xk_status xk_radix_sort_u64(uint64_t* keys, int32_t* vals, long long n, int bits, cudaStream_t s);

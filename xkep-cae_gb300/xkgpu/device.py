@@ -7,6 +7,8 @@ xkgpu kernels behind the C ABI.
 from __future__ import annotations
 
 import ctypes as C
+import threading
+import weakref
 from dataclasses import dataclass
 
 import numpy as np
@@ -42,6 +44,25 @@ def as_dev(x, dtype, device) -> torch.Tensor:
 
 # ----------------------------------------------------------------------------- mesh
 
+_meshes: dict[int, int] = {}  # meshes alive per device
+_meshes_lock = threading.Lock()
+
+
+def _mesh_gone(index: int) -> None:
+    with _meshes_lock:
+        _meshes[index] -= 1
+        last = _meshes[index] == 0
+    if last:  # the detection's scratch goes back to the system with the last mesh of the device
+        with torch.cuda.device(index):
+            L.call("xk_scratch_trim", 0)
+
+
+def _count_mesh(mesh: "DeviceMesh") -> None:
+    index = mesh.device.index if mesh.device.index is not None else torch.cuda.current_device()
+    with _meshes_lock:
+        _meshes[index] = _meshes.get(index, 0) + 1
+    weakref.finalize(mesh, _mesh_gone, index).atexit = False
+
 
 class DeviceMesh:
     """Reference coordinates, connectivity, radii and layer ids on the device."""
@@ -69,6 +90,7 @@ class DeviceMesh:
             np.broadcast_to(np.asarray(core_radii, dtype=np.float64), (self.n_elems,)).copy(), torch.float64,
             self.device)
         self.conn_host = conn
+        _count_mesh(self)
         self.refresh()
 
     def refresh(self):
