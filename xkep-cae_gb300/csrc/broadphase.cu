@@ -6,9 +6,10 @@
 // binned once, by the cell of its box's lower corner (counting sort by cell, each cell's entries then
 // in ascending order).
 // A box j can overlap box i only if its lower corner lies in [lo_i - E, hi_i]
-// per axis, E the largest extent of any box on that axis, so a warp per
-// segment i walks the cells of that range (32 cells a batch) and tests every
-// entry j > i (found in each cell by a binary search): screened on float boxes rounded outward, tested on the exact
+// per axis, E the largest extent of any box on that axis.  Cells are numbered with
+// the axis of the largest extent running fastest, so the range is a few rows of
+// cells whose entries are contiguous; a warp per segment i walks those rows and tests every
+// entry j > i: screened on float boxes rounded outward, tested on the exact
 // double AABBs, filtered, compacted with ballot/popc into a fixed-size slot list
 // of the segment.  Each pair is found once, from its lower-numbered segment, in
 // a single walk: a second kernel sorts each slot list and applies the midpoint
@@ -16,6 +17,11 @@
 // kept pairs out in (i, j) order.  A slot list that overflows is detected at the
 // end and the walk is repeated with longer lists.  Filters follow
 // DetectCandidatesProcess (_manager_process.py:200-217,260-286).
+//
+// FP64 operations are what these kernels must not spend (1.6 per clock and SM): cell numbers and ranges are
+// computed once per segment by its own thread, not by every lane of the warp that walks it (96 operations a
+// lane there: most of the walk's 558 us at 98,592 segments, 189 us now); the radius sums of the margin are skipped
+// where every radius is the same; the prescreen decides in float from split midpoints (slot ranking 96 -> 58 us).
 #include <atomic>
 #include <cstdio>
 
@@ -26,11 +32,25 @@ namespace {
 constexpr int BP_T = 128;  // 4 warps per block, one warp per segment
 
 struct Grid {
-  double origin[3];
-  double cell;
-  int dims[3];
-  int pad;
-  double emax[3];  // largest box extent on each axis
+  double origin[3], inv[3];  // lower corner, 1 / cell size
+  double emax[3];            // largest box extent on each axis
+  int dims[3], stride[3];    // cells per axis; stride 1 on axis f
+  int f;
+  int uniform;               // every radius is `radius`
+  double radius;
+};
+
+// Words shared by the broadphase kernels, all zero at the start.
+struct Words {
+  unsigned long long lo_max[3];   // max of the inverted lower corners, order-preserving (the min, inverted)
+  unsigned long long hi_max[3];   // max of the upper corners
+  unsigned long long ext_max[3];  // max of the extents (bits of doubles >= 0)
+  unsigned long long r_lo, r_hi;  // radii: max of the inverted and of the plain ones
+  double ext_sum[3];              // sums of the extents (they set the cell size: any order will do)
+  double margin;                  // of the prescreen
+  unsigned int ticket, ticket2;
+  // read back by the host
+  long long raw, pre, longest, kept;
 };
 
 XK_D unsigned long long enc_min(double x) {  // order-preserving map of doubles to u64
@@ -42,23 +62,74 @@ XK_D double dec_min(unsigned long long k) {
   return __longlong_as_double((long long)b);
 }
 
+// A segment's midpoint in float hi / lo parts with its half length and radius: the prescreen's float form.
+struct __align__(32) MidF {
+  float hi[3], half, lo[3], r;
+};
+
+// cells of cell_size, or (cell_size <= 0) of these fractions of the mean extent on each axis: short on the
+// axis that runs fastest, where a row's length costs nothing, and on the others so that a segment's rows are
+// some 25 (one batch of the walk's lanes); coarsened while there would be more than cap_cells cells
+constexpr float CELL_FAST = 0.125f, CELL_OTHER = 0.5f;
+XK_D void make_grid(const Words& w, long long ne, long long cap_cells, double cell_size, Grid* g) {
+  // The walk is right for any cell size and count (cell coordinates are clamped and grow with the position), so
+  // these are taken in float: one thread does this, and an FP64 divide takes it a microsecond.
+  float span[3], cell[3], e[3];
+  for (int c = 0; c < 3; ++c) {
+    const double lo = dec_min(~w.lo_max[c]), hi = dec_min(w.hi_max[c]);
+    g->origin[c] = lo;
+    g->emax[c] = __longlong_as_double((long long)w.ext_max[c]);
+    e[c] = xk_d2f(g->emax[c]);
+    span[c] = xk_d2f(hi - lo);
+  }
+  const int f = (e[2] >= e[0] && e[2] >= e[1]) ? 2 : (e[1] >= e[0] ? 1 : 0);
+  const int a = f == 0 ? 1 : 0, b = f == 2 ? 1 : 2;
+  float n[3];
+  for (int c = 0; c < 3; ++c) {
+    cell[c] = cell_size > 0.0 ? xk_d2f(cell_size) : (c == f ? CELL_FAST : CELL_OTHER) * (xk_d2f(w.ext_sum[c]) / (float)ne);
+    cell[c] = fmaxf(cell[c], span[c] * 9.5367432e-7f);  // at most 2^20 cells on an axis
+    n[c] = span[c] > 0.f ? span[c] / cell[c] : 0.f;
+    if (!(n[c] >= 0.f && n[c] <= 2097152.f)) n[c] = 0.f;  // extents that are not finite: one cell
+  }
+  for (int it = 0; it < 400 && (n[0] + 1.f) * (n[1] + 1.f) * (n[2] + 1.f) > 0.999f * (float)cap_cells; ++it)
+    for (int c = 0; c < 3; ++c) n[c] *= 0.8f;
+  for (int c = 0; c < 3; ++c) {
+    g->dims[c] = (int)n[c] + 1;
+    g->inv[c] = n[c] > 0.f ? xk_f2d(n[c] / span[c]) : 0.0;
+  }
+  g->f = f;
+  g->stride[f] = 1;
+  g->stride[a] = g->dims[f];
+  g->stride[b] = g->dims[f] * g->dims[a];
+  g->uniform = w.r_hi == ~w.r_lo;
+  g->radius = dec_min(w.r_hi);
+}
+
 // box: the FP64 boxes, six doubles per segment (lower corner, upper corner); boxf: the same boxes in
 // float, rounded outward (lower corner down, upper corner up), as two float4 per segment (32 bytes): a
 // conservative screen for the sweep, which then tests the FP64 boxes.  mid: per segment its midpoint and
 // half length in the operation order of the midpoint prescreen (_manager_process.py:265-272), so that
-// the prescreen of a pair reads these 32 bytes of each segment and gives the same values.
-__global__ void k_aabb(xk_mesh m, const double* __restrict__ u, double margin, double* __restrict__ box,
-                       float4* __restrict__ boxf, double4_32a* __restrict__ mid, unsigned long long* __restrict__ ext,
-                       double* __restrict__ ext_sum) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long lmin[3] = {~0ull, ~0ull, ~0ull}, lmax[3] = {0ull, 0ull, 0ull}, lax[3] = {0ull, 0ull, 0ull};
-  double msum = 0.0;
+// the prescreen of a pair reads these 32 bytes of each segment and gives the same values; midf: the same in
+// float parts.  The extremes and sums go over the block, then by one atomic each into w; the last block forms
+// the grid.
+constexpr int AABB_T = 256, AABB_W = AABB_T / 32;
+__global__ void __launch_bounds__(AABB_T) k_aabb(xk_mesh m, const double* __restrict__ u, double margin,
+                                                 double* __restrict__ box, float4* __restrict__ boxf,
+                                                 double4_32a* __restrict__ mid, MidF* __restrict__ midf,
+                                                 Words* __restrict__ w, long long cap_cells, double cell_size,
+                                                 Grid* __restrict__ grid) {
+  __shared__ unsigned long long s_max[11][AABB_W];
+  __shared__ double s_sum[3][AABB_W];
+  __shared__ bool s_last;
+  const int e = blockIdx.x * AABB_T + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long mx[11] = {};  // as Words: inverted lower corners, upper corners, extents, radii
+  double sum[3] = {0.0, 0.0, 0.0};
   if (e < m.n_elems) {
-    int a = m.conn[2 * e], b = m.conn[2 * e + 1];
-    const double ex = xadd(m.radii[e], margin);
-    double mx = 0.0;
+    const int a = m.conn[2 * e], b = m.conn[2 * e + 1];
+    const double rad = m.radii[e], ex = xadd(rad, margin);
     float lf[3], hf[3];
     double ma[3], da[3];
+    MidF mf;
     for (int c = 0; c < 3; ++c) {
       double x0 = u ? xadd(m.X[3LL * a + c], u[6LL * a + c]) : m.X[3LL * a + c];
       double x1 = u ? xadd(m.X[3LL * b + c], u[6LL * b + c]) : m.X[3LL * b + c];
@@ -70,12 +141,15 @@ __global__ void k_aabb(xk_mesh m, const double* __restrict__ u, double margin, d
       box[6LL * e + 3 + c] = hi;
       lf[c] = __double2float_rd(lo);
       hf[c] = __double2float_ru(hi);
-      lmin[c] = enc_min(lo);
-      lmax[c] = enc_min(hi);
-      const double extc = hi - lo;  // >= 0: the bit patterns order as the values
-      lax[c] = (unsigned long long)__double_as_longlong(extc);
-      mx = fmax(mx, extc);
+      mf.hi[c] = xk_d2f(ma[c]);
+      mf.lo[c] = xk_d2f(ma[c] - xk_f2d(mf.hi[c]));
+      mx[c] = ~enc_min(lo);
+      mx[3 + c] = enc_min(hi);
+      sum[c] = fmax(hi - lo, 0.0);  // >= 0 (a negative margin may turn a box round): the bits order as the values
+      mx[6 + c] = (unsigned long long)__double_as_longlong(sum[c]);
     }
+    mx[9] = ~enc_min(rad);
+    mx[10] = enc_min(rad);
     // the spare fourth word carries the element's layer (-1 without layers), read by the walk's filter
     boxf[2LL * e] = make_float4(lf[0], lf[1], lf[2], __int_as_float(m.layer ? m.layer[e] : -1));
     boxf[2LL * e + 1] = make_float4(hf[0], hf[1], hf[2], 0.f);
@@ -85,104 +159,106 @@ __global__ void k_aabb(xk_mesh m, const double* __restrict__ u, double margin, d
     me.z = ma[2];
     me.w = xmul(0.5, xsqrt(xdot_seq(da, da)));
     mid[e] = me;
-    msum = mx;
+    mf.half = xk_d2f(me.w);
+    mf.r = xk_d2f(rad);
+    midf[e] = mf;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    for (int c = 0; c < 3; ++c) {
-      unsigned long long y = __shfl_down_sync(0xffffffffu, lmin[c], o);
-      lmin[c] = y < lmin[c] ? y : lmin[c];
-      y = __shfl_down_sync(0xffffffffu, lmax[c], o);
-      lmax[c] = y > lmax[c] ? y : lmax[c];
-      y = __shfl_down_sync(0xffffffffu, lax[c], o);
-      lax[c] = y > lax[c] ? y : lax[c];
+#pragma unroll
+  for (int k = 0; k < 11; ++k) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long y = __shfl_down_sync(0xffffffffu, mx[k], o);
+      mx[k] = y > mx[k] ? y : mx[k];
     }
-    msum += __shfl_down_sync(0xffffffffu, msum, o);
+    if (lane == 0) s_max[k][warp] = mx[k];
   }
-  if ((threadIdx.x & 31) == 0) {
-    for (int c = 0; c < 3; ++c) {
-      atomicMin(&ext[1 + c], lmin[c]);
-      atomicMax(&ext[4 + c], lmax[c]);
-      atomicMax(&ext[9 + c], lax[c]);
-    }
-    atomicAdd(ext_sum, msum);  // the cell size only sets the work, not the result: any order will do
-  }
-}
-// the grid over the boxes' bounding box: cells of cell_size, or (cell_size <= 0) of AUTO_CELL times the
-// mean of each box's largest extent; coarsened while it would have more than cap_cells cells
-constexpr double AUTO_CELL = 0.5;
-__global__ void k_grid(const unsigned long long* __restrict__ ext, const double* __restrict__ ext_sum, long long ne,
-                       long long cap_cells, double cell_size, Grid* g) {
-  double mx = *ext_sum / (double)ne;
-  double lo[3], hi[3];
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
-    lo[c] = dec_min(ext[1 + c]);
-    hi[c] = dec_min(ext[4 + c]);
+    for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_down_sync(0xffffffffu, sum[c], o);
+    if (lane == 0) s_sum[c][warp] = sum[c];
   }
-  double cell = cell_size > 0.0 ? cell_size : AUTO_CELL * mx * (1.0 + 1e-6) + 1e-300;
-  long long tot;
-  int dims[3];
-  for (int it = 0; it < 200; ++it) {
-    tot = 1;
-    for (int c = 0; c < 3; ++c) {
-      double n = floor((hi[c] - lo[c]) / cell) + 1.0;
-      if (n > 2097151.0) n = 2097151.0;
-      dims[c] = (int)n;
-      tot *= dims[c];
-    }
-    if (tot <= cap_cells) break;
-    cell *= 1.25;
+  __syncthreads();
+  if (threadIdx.x < 11) {
+    unsigned long long v = s_max[threadIdx.x][0];
+    for (int q = 1; q < AABB_W; ++q) v = s_max[threadIdx.x][q] > v ? s_max[threadIdx.x][q] : v;
+    atomicMax(reinterpret_cast<unsigned long long*>(w) + threadIdx.x, v);
+  } else if (threadIdx.x >= 32 && threadIdx.x < 35) {
+    const int c = threadIdx.x - 32;
+    double v = 0.0;
+    for (int q = 0; q < AABB_W; ++q) v += s_sum[c][q];
+    atomicAdd(&w->ext_sum[c], v);
   }
-  for (int c = 0; c < 3; ++c) {
-    g->origin[c] = lo[c];
-    g->dims[c] = dims[c];
-  }
-  g->cell = cell;
-  for (int c = 0; c < 3; ++c) g->emax[c] = __longlong_as_double((long long)ext[9 + c]);
-}
-
-XK_D void cell_of(const Grid& g, double lo0, double lo1, double lo2, int* c) {
-  const double l[3] = {lo0, lo1, lo2};
-  for (int k = 0; k < 3; ++k) {
-    double f = floor((l[k] - g.origin[k]) / g.cell);
-    int ci = (int)f;
-    c[k] = ci < 0 ? 0 : (ci >= g.dims[k] ? g.dims[k] - 1 : ci);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&w->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (s_last && threadIdx.x == 0) {
+    __threadfence();
+    const volatile unsigned long long* v = reinterpret_cast<const volatile unsigned long long*>(w);
+    Words c;
+    unsigned long long* d = reinterpret_cast<unsigned long long*>(&c);
+    for (int k = 0; k < 14; ++k) d[k] = v[k];
+    make_grid(c, m.n_elems, cap_cells, cell_size, grid);
   }
 }
 
-// per-cell counts of the segments binned by the cell of their box's lower corner
+XK_D int cell_coord(const Grid& g, int c, double x) {
+  const int ci = (int)floor((x - g.origin[c]) * g.inv[c]);
+  return ci < 0 ? 0 : (ci >= g.dims[c] ? g.dims[c] - 1 : ci);
+}
+
+// Per segment: its cell (of its box's lower corner) with the cells' counts, and its range of the walk, the
+// cells of [lo - E, hi] (widened by a relative 1e-12 against rounding): first cell, steps along the fast
+// axis, rows along the other two.
 __global__ void k_cell_count(const double* __restrict__ box, long long ne, const Grid* __restrict__ gp,
-                             int32_t* __restrict__ ecell, int32_t* __restrict__ ccnt) {
+                             int32_t* __restrict__ ecell, int32_t* __restrict__ ccnt, int4* __restrict__ range) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const Grid g = *gp;
-  int c[3];
-  cell_of(g, box[6 * e], box[6 * e + 1], box[6 * e + 2], c);
-  const int lin = (int)(((long long)c[2] * g.dims[1] + c[1]) * g.dims[0] + c[0]);
+  int lin = 0, base = 0, n[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double lo = box[6 * e + c], hi = box[6 * e + 3 + c];
+    lin += cell_coord(g, c, lo) * g.stride[c];
+    const int c0 = cell_coord(g, c, xsub(xsub(lo, g.emax[c]), 1e-12 * (fabs(lo) + g.emax[c])));
+    n[c] = cell_coord(g, c, hi) - c0;
+    base += c0 * g.stride[c];
+  }
   ecell[e] = lin;
   atomicAdd(&ccnt[lin], 1);
+  const int a = g.f == 0 ? 1 : 0, b = g.f == 2 ? 1 : 2;
+  const bool any = n[0] >= 0 && n[1] >= 0 && n[2] >= 0;  // a box turned round may have none
+  range[e] = any ? make_int4(base, n[g.f] + 1, n[a] + 1, n[b] + 1) : make_int4(0, 0, 0, 0);
 }
 
-// counting sort of the segments by cell, then each cell's entries in ascending order (a thread per cell;
-// cells of more than CELL_SORTED entries are left as they are)
+// counting sort of the segments by cell (the counts run down to zero)
 __global__ void k_cell_scatter(long long ne, const int32_t* __restrict__ ecell, const int32_t* __restrict__ cstart,
-                               int32_t* __restrict__ cfill, int32_t* __restrict__ segs) {
+                               int32_t* __restrict__ ccnt, int32_t* __restrict__ segs) {
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= ne) return;
   const int c = ecell[e];
-  segs[cstart[c] + atomicAdd(&cfill[c], 1)] = (int32_t)e;
+  segs[cstart[c] + atomicSub(&ccnt[c], 1) - 1] = (int32_t)e;
 }
-constexpr int CELL_SORTED = 64;  // cells with more entries stay unsorted (insertion sort by one thread)
-__global__ void k_cell_sort(long long ncell, const int32_t* __restrict__ cstart, int32_t* __restrict__ segs) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  const int lo = cstart[c], hi = cstart[c + 1];
-  if (hi - lo > CELL_SORTED) return;
-  for (int x = lo + 1; x < hi; ++x) {
-    const int key = segs[x];
-    int y = x - 1;
-    while (y >= lo && segs[y] > key) { segs[y + 1] = segs[y]; --y; }
-    segs[y + 1] = key;
+
+// The float boxes in the order of the cells, each cell's in ascending order of the segments (each thread finds
+// its entry's rank among the cell's; cells of more than CELL_SORTED entries keep the order of the scatter), so
+// that a row of cells is read as one run.  The last word of a box is its segment.
+constexpr int CELL_SORTED = 64;
+__global__ void k_cell_boxes(long long ne, const int32_t* __restrict__ segs, const int32_t* __restrict__ ecell,
+                             const int32_t* __restrict__ cstart, const float4* __restrict__ boxf,
+                             float4* __restrict__ sorted) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= ne) return;
+  const int e = segs[x], c = ecell[e], lo = cstart[c], hi = cstart[c + 1];
+  long long at = x;
+  if (hi - lo <= CELL_SORTED) {
+    at = lo;
+    for (int y = lo; y < hi; ++y) at += segs[y] < e;
   }
+  const float4 l = boxf[2LL * e];
+  float4 h = boxf[2LL * e + 1];
+  h.w = __int_as_float(e);
+  sorted[2 * at] = l;
+  sorted[2 * at + 1] = h;
 }
 
 // the neighbouring floats above and below x (finite x): the outward-rounded float bounds lf <= lo, hf >= hi
@@ -197,75 +273,62 @@ XK_D float dn1(float x) {
   return __int_as_float(x == 0.f ? (int)0x80000001 : (x > 0.f ? b - 1 : b + 1));
 }
 
-// the FP64 boxes of i (registers) and j (six doubles at box + 6 j, 16-byte aligned) overlap, closed
-XK_D bool overlap(const double (&bi)[6], const double* __restrict__ box, int j) {
+// the FP64 boxes of i and j (six doubles at box + 6 k, 16-byte aligned) overlap, closed
+XK_D bool overlap(const double* __restrict__ box, int i, int j) {
+  const double2* bi = reinterpret_cast<const double2*>(box + 6LL * i);
   const double2* bj = reinterpret_cast<const double2*>(box + 6LL * j);
-  const double2 p = __ldg(bj), q = __ldg(bj + 1), r = __ldg(bj + 2);  // lo x,y | lo z, hi x | hi y,z
-  return bi[0] <= q.y && p.x <= bi[3] && bi[1] <= r.x && p.y <= bi[4] && bi[2] <= r.y && q.x <= bi[5];
+  const double2 a = __ldg(bi), b = __ldg(bi + 1), c = __ldg(bi + 2);  // lo x,y | lo z, hi x | hi y,z
+  const double2 p = __ldg(bj), q = __ldg(bj + 1), r = __ldg(bj + 2);
+  return a.x <= q.y && p.x <= b.y && a.y <= r.x && p.y <= c.x && b.x <= r.y && q.x <= c.y;
 }
 
-// A warp per segment i.  The cells that can hold the lower corner of a box overlapping box i, those
-// of [lo_i - E, hi_i] (E per axis the largest extent of any box, widened by a relative 1e-12 against
-// rounding), are taken 32 at a time: lane l reads cell l's entry range, a warp scan lays the ranges
-// out as one list, and the warp walks it 32 entries at a time, each lane finding its entry's cell
-// by a binary search over the offsets held in the lanes.  An entry j > i is screened on the
-// outward-rounded float boxes (which can never reject an FP64 overlap), tested on the FP64 boxes,
-// then the shared-node and same-layer filters apply and hits are compacted with ballot/popc into
-// segment i's slot list (the first `cap` of them; cnt[i] counts them all).  Also per segment: the sum
-// of r_i + r_j over its kept candidates (each lane sums its own entries in walk order, then a fixed
-// butterfly: rsum[i], for the prescreen margin), the raw overlap count and the longest list.
-__global__ void __launch_bounds__(BP_T, 7) k_sweep(xk_mesh m, const double* __restrict__ box,
-                                                const float4* __restrict__ boxf, const Grid* __restrict__ gp,
-                                                const int32_t* __restrict__ segs, const int32_t* __restrict__ cstart,
-                                                int excl_shared, int excl_layer, int cap, int32_t* __restrict__ slot,
-                                                int32_t* __restrict__ cnt, double* __restrict__ rsum,
-                                                unsigned long long* __restrict__ raw_total,
-                                                int32_t* __restrict__ max_cnt) {
+// A warp per segment i.  The rows of its range are taken 32 at a time: lane l reads row l's entry range (its
+// cells are consecutive), a warp scan lays the ranges of the rows that have entries out as one list, and the
+// warp walks it 64 entries at a time: the rows that begin in a window of 32 entries are a bit mask, so a lane
+// finds its entry's row by a population count.  An entry
+// j > i is screened on the outward-rounded float boxes (which can never reject an FP64 overlap), tested on
+// the FP64 boxes where those are not certain, then the shared-node and same-layer filters apply and hits are
+// compacted with ballot/popc into segment i's slot list (the first `cap` of them; cnt[i] counts them all,
+// raw[i] the overlaps).  Unless all radii are equal, also the sum of r_i + r_j over its kept candidates (each
+// lane sums its own entries in walk order, then a fixed butterfly: rsum[i], for the prescreen margin).
+// UNIFORM: all radii equal, no radius sums (predicated off they would still issue on the FP64 pipe).
+template <bool UNIFORM>
+XK_D void sweep(const xk_mesh& m, const double* __restrict__ box,
+                                                   const float4* __restrict__ boxf, const float4* __restrict__ sorted,
+                                                   const Grid* __restrict__ gp, const int4* __restrict__ range,
+                                                   const int32_t* __restrict__ cstart, int excl_shared,
+                                                   int excl_layer, int cap, int32_t* __restrict__ slot,
+                                                   int32_t* __restrict__ cnt, int32_t* __restrict__ raw,
+                                                   double* __restrict__ rsum, int* offs) {
   const long long ne = m.n_elems;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= ne) return;
-  const Grid g = *gp;
   const int i = (int)w;
-  double bi[6];
-  for (int c = 0; c < 6; ++c) bi[c] = box[6LL * i + c];
-  int c0[3], c1[3];
-  {
-    double lw[3];
-    for (int c = 0; c < 3; ++c) lw[c] = xsub(xsub(bi[c], g.emax[c]), 1e-12 * (fabs(bi[c]) + g.emax[c]));
-    cell_of(g, lw[0], lw[1], lw[2], c0);
-    cell_of(g, bi[3], bi[4], bi[5], c1);
-  }
-  const int sx = c1[0] - c0[0] + 1, sy = c1[1] - c0[1] + 1, sz = c1[2] - c0[2] + 1;
-  const int ncell = sx * sy * sz;
-  const int ia = m.conn[2 * i], ib = m.conn[2 * i + 1];
+  const int4 rg = range[i];
+  const int f = gp->f, sa = gp->stride[f == 0 ? 1 : 0], sb = gp->stride[f == 2 ? 1 : 2];
+  const int rows = rg.z * rg.w;
+  const int2* conn2 = reinterpret_cast<const int2*>(m.conn);
+  const int2 ci = __ldg(conn2 + i);
   const int li = (excl_layer && m.layer) ? m.layer[i] : -1;
   const float4 il = boxf[2LL * i], ih = boxf[2LL * i + 1];
-  const float iux = up1(il.x), iuy = up1(il.y), iuz = up1(il.z);  // box i shrunk to within its FP64 bounds
-  const float idx_ = dn1(ih.x), idy = dn1(ih.y), idz = dn1(ih.z);
-  const double ri = m.radii[i];
+  // an outward float overlap is an FP64 overlap when the boxes shrunk by one float step each still overlap
+  // (a <= dn1(b) is up1(a) <= b: both steps are taken on box i); only the rare pair between the two takes the
+  // FP64 boxes
+  const float ux = up1(up1(il.x)), uy = up1(up1(il.y)), uz = up1(up1(il.z));
+  const float vx = dn1(dn1(ih.x)), vy = dn1(dn1(ih.y)), vz = dn1(dn1(ih.z));
   int32_t* const my = slot + (long long)i * cap;
-  int n_raw = 0, n_keep = 0;
+  const unsigned below = (1u << lane) - 1u;
+  int n_raw = 0, n_keep = 0;  // n_raw: this lane's overlaps
   double rs = 0.0;
-  for (int cb = 0; cb < ncell; cb += 32) {
-    // this lane's cell of the batch and its entry range
+  for (int rb = 0; rb < rows; rb += 32) {
+    // this lane's row of the batch and its entry range
     int s0 = 0, n0 = 0;
-    const int q0 = cb + lane;
-    if (q0 < ncell) {
-      const int x = c0[0] + q0 % sx, y = c0[1] + (q0 / sx) % sy, z = c0[2] + q0 / (sx * sy);
-      const int lin = (int)(((long long)z * g.dims[1] + y) * g.dims[0] + x);
-      s0 = cstart[lin];
-      const int e0 = cstart[lin + 1];
-      // a cell of at most CELL_SORTED entries holds them in ascending order: only those past i can pair
-      // with it (each pair is taken from its lower-numbered segment); a larger one is walked whole
-      int lo = s0, hi = e0;
-      if (e0 - s0 <= CELL_SORTED)
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (segs[mid] <= i) lo = mid + 1; else hi = mid;
-        }
-      s0 = lo;
-      n0 = e0 - lo;
+    const int q0 = rb + lane;
+    if (q0 < rows) {
+      const int c = rg.x + (q0 % rg.z) * sa + (q0 / rg.z) * sb;
+      s0 = cstart[c];
+      n0 = cstart[c + rg.y] - s0;
     }
     int incl = n0;
 #pragma unroll
@@ -275,99 +338,152 @@ __global__ void __launch_bounds__(BP_T, 7) k_sweep(xk_mesh m, const double* __re
     }
     const int pre = incl - n0;
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int nq = (ncell - cb) < 32 ? (ncell - cb) : 32;
-    // two entries per lane and pass (f and f + 32), their loads issued together: half the dependent
-    // round trips of one entry per lane; each lane still meets its entries in increasing f
-    auto entry = [&](int f) {  // the segment at list position f of the batch, or -1
-      int q = 0;  // the last cell q of the batch with pre_q <= f (cells without entries share their successor's offset)
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int cand = q + step;
-        const int pc = __shfl_sync(0xffffffffu, pre, cand < nq ? cand : nq - 1);
-        if (cand < nq && pc <= f) q = cand;
-      }
-      const int sq = __shfl_sync(0xffffffffu, s0, q);
-      const int pq = __shfl_sync(0xffffffffu, pre, q);
-      return f < total ? segs[sq + (f - pq)] : -1;
+    // offs[r]: the offset from list position to sorted position of the r-th row that has entries
+    const unsigned some = __ballot_sync(0xffffffffu, n0 > 0);
+    __syncwarp();
+    if (n0 > 0) offs[__popc(some & below)] = s0 - pre;
+    __syncwarp();
+    int before = -1;  // rows begun before the window, less one
+    auto entry = [&](int f0) {  // sorted position of this lane's entry of the window at f0 (any past the list)
+      const unsigned d = (unsigned)(pre - f0);
+      const unsigned begun = __reduce_or_sync(0xffffffffu, n0 > 0 && d < 32u ? 1u << d : 0u);
+      const int r = before + __popc(begun & (below | (1u << lane)));
+      before += __popc(begun);
+      return offs[r & 31] + f0 + lane;
     };
-    const int2* conn2 = reinterpret_cast<const int2*>(m.conn);
-    // an outward float overlap is an FP64 overlap when the boxes shrunk by one float step still overlap;
-    // only the rare pair between the two takes the FP64 boxes
-    auto hit_of = [&](int j, const float4& jl, const float4& jh) {
+    auto hit_of = [&](const float4& jl, const float4& jh) {
       if (!(il.x <= jh.x && jl.x <= ih.x && il.y <= jh.y && jl.y <= ih.y && il.z <= jh.z && jl.z <= ih.z))
         return false;
-      const bool sure = iux <= dn1(jh.x) && up1(jl.x) <= idx_ && iuy <= dn1(jh.y) && up1(jl.y) <= idy &&
-                        iuz <= dn1(jh.z) && up1(jl.z) <= idz;
-      return sure || overlap(bi, box, j);
+      const bool sure = ux <= jh.x && jl.x <= vx && uy <= jh.y && jl.y <= vy && uz <= jh.z && jl.z <= vz;
+      return sure || overlap(box, i, __float_as_int(jh.w));
     };
+    auto keep = [&](bool hit, const float4& jl, const float4& jh) {
+      if (!hit || (li >= 0 && __float_as_int(jl.w) == li)) return false;
+      if (!excl_shared) return true;
+      const int2 cj = __ldg(conn2 + __float_as_int(jh.w));
+      return !(ci.x == cj.x || ci.x == cj.y || ci.y == cj.x || ci.y == cj.y);
+    };
+    auto put = [&](bool kept, int j) {
+      const unsigned bal = __ballot_sync(0xffffffffu, kept);
+      if (kept) {
+        if (!UNIFORM) rs = xadd(rs, xadd(m.radii[i], m.radii[j]));  // this lane's entries, in walk order
+        const int at = n_keep + __popc(bal & below);
+        if (at < cap) my[at] = j;
+      }
+      n_keep += __popc(bal);
+    };
+    // two entries per lane and pass, their loads issued together; each lane meets its entries in increasing order
     for (int f0 = 0; f0 < total; f0 += 64) {
-      const int jA = entry(f0 + lane), jB = entry(f0 + 32 + lane);
-      const bool nearA = jA > i, nearB = jB > i;
-      float4 al = make_float4(0.f, 0.f, 0.f, 0.f), ah = al, bl = al, bh = al;
-      int2 ca = make_int2(-1, -1), cb2 = ca;
-      if (nearA) { al = __ldg(boxf + 2LL * jA); ah = __ldg(boxf + 2LL * jA + 1); ca = __ldg(conn2 + jA); }
-      if (nearB) { bl = __ldg(boxf + 2LL * jB); bh = __ldg(boxf + 2LL * jB + 1); cb2 = __ldg(conn2 + jB); }
-      const bool hitA = nearA && hit_of(jA, al, ah), hitB = nearB && hit_of(jB, bl, bh);
-      bool keptA = hitA, keptB = hitB;
-      if (excl_shared) {
-        if (ia == ca.x || ia == ca.y || ib == ca.x || ib == ca.y) keptA = false;
-        if (ia == cb2.x || ia == cb2.y || ib == cb2.x || ib == cb2.y) keptB = false;
-      }
-      if (li >= 0) {
-        if (__float_as_int(al.w) == li) keptA = false;
-        if (__float_as_int(bl.w) == li) keptB = false;
-      }
-      n_raw += __popc(__ballot_sync(0xffffffffu, hitA)) + __popc(__ballot_sync(0xffffffffu, hitB));
-      const unsigned balA = __ballot_sync(0xffffffffu, keptA), balB = __ballot_sync(0xffffffffu, keptB);
-      const unsigned below = (1u << lane) - 1u;
-      if (keptA) {
-        rs = xadd(rs, xadd(ri, m.radii[jA]));  // this lane's entries, in walk order
-        const int at = n_keep + __popc(balA & below);
-        if (at < cap) my[at] = jA;
-      }
-      n_keep += __popc(balA);
-      if (keptB) {
-        rs = xadd(rs, xadd(ri, m.radii[jB]));
-        const int at = n_keep + __popc(balB & below);
-        if (at < cap) my[at] = jB;
-      }
-      n_keep += __popc(balB);
+      const int pA = entry(f0), pB = entry(f0 + 32);
+      const bool inA = f0 + lane < total, inB = f0 + 32 + lane < total;
+      float4 al, ah, bl, bh;
+      al = bl = make_float4(0.f, 0.f, 0.f, 0.f);
+      ah = bh = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+      if (inA) { al = __ldg(sorted + 2LL * pA); ah = __ldg(sorted + 2LL * pA + 1); }
+      if (inB) { bl = __ldg(sorted + 2LL * pB); bh = __ldg(sorted + 2LL * pB + 1); }
+      const int jA = __float_as_int(ah.w), jB = __float_as_int(bh.w);
+      const bool hitA = jA > i && hit_of(al, ah), hitB = jB > i && hit_of(bl, bh);
+      n_raw += (int)hitA + (int)hitB;
+      const bool keptA = keep(hitA, al, ah), keptB = keep(hitB, bl, bh);
+      put(keptA, jA);
+      put(keptB, jB);
     }
   }
+  n_raw = __reduce_add_sync(0xffffffffu, n_raw);
+  if (!UNIFORM) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);  // fixed butterfly order
+    for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);  // fixed butterfly order
+  }
   if (lane == 0) {
     cnt[i] = n_keep;
-    rsum[i] = rs;
-    atomicAdd(raw_total, (unsigned long long)n_raw);
-    atomicMax(max_cnt, n_keep);
+    raw[i] = n_raw;
+    if (!UNIFORM) rsum[i] = rs;
   }
 }
 
-constexpr int RED_BLOCKS = 304, RED_T = 256;
+__global__ void __launch_bounds__(BP_T, 8) k_sweep(xk_mesh m, const double* __restrict__ box,
+                                                   const float4* __restrict__ boxf, const float4* __restrict__ sorted,
+                                                   const Grid* __restrict__ gp, const int4* __restrict__ range,
+                                                   const int32_t* __restrict__ cstart, int excl_shared,
+                                                   int excl_layer, int cap, int32_t* __restrict__ slot,
+                                                   int32_t* __restrict__ cnt, int32_t* __restrict__ raw,
+                                                   double* __restrict__ rsum) {
+  __shared__ int s_off[BP_T / 32][32];
+  int* const offs = s_off[threadIdx.x >> 5];
+  if (gp->uniform)
+    sweep<true>(m, box, boxf, sorted, gp, range, cstart, excl_shared, excl_layer, cap, slot, cnt, raw, rsum, offs);
+  else
+    sweep<false>(m, box, boxf, sorted, gp, range, cstart, excl_shared, excl_layer, cap, slot, cnt, raw, rsum, offs);
+}
 
-// prescreen margin: mean(r_a + r_b) / 2 over the candidates after the shared-node and same-layer
-// filters (_manager_process.py:275-279), from the per-segment sums, in a fixed order
-__global__ void k_radsum_partial(const double* __restrict__ rsum, long long ne, double* __restrict__ part) {
+// Totals over the segments (overlaps, candidates before the prescreen, the longest slot list) and the
+// prescreen margin: mean(r_a + r_b) / 2 over the candidates after the shared-node and same-layer filters
+// (_manager_process.py:275-279) from the per-segment sums, in a fixed order (a tree in every block, the last
+// block over the blocks), or the common radius.
+constexpr int RED_BLOCKS = 152, RED_T = 256;
+__global__ void __launch_bounds__(RED_T) k_totals(const int32_t* __restrict__ cnt, const int32_t* __restrict__ raw,
+                                                  const double* __restrict__ rsum, long long ne,
+                                                  const Grid* __restrict__ gp, double fixed, double* __restrict__ part,
+                                                  Words* __restrict__ w) {
   __shared__ double sm[RED_T];
+  __shared__ bool s_last;
+  const bool sums = !(fixed > 0.0) && !gp->uniform;
   double acc = 0.0;
-  for (long long k = (long long)blockIdx.x * RED_T + threadIdx.x; k < ne; k += (long long)RED_BLOCKS * RED_T)
-    acc += rsum[k];
-  sm[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = RED_T / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-    __syncthreads();
+  long long c = 0, r = 0;
+  int mx = 0;
+  for (long long k = (long long)blockIdx.x * RED_T + threadIdx.x; k < ne; k += (long long)RED_BLOCKS * RED_T) {
+    const int v = cnt[k];
+    c += v;
+    r += raw[k];
+    mx = v > mx ? v : mx;
+    if (sums) acc += rsum[k];
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
-}
-
-__global__ void k_margin(const double* __restrict__ part, const int64_t* __restrict__ n, double fixed,
-                         double* __restrict__ out) {
-  if (fixed > 0.0) { *out = fixed; return; }
-  double s = 0.0;
-  for (int b = 0; b < RED_BLOCKS; ++b) s += part[b];
-  *out = *n > 0 ? xmul(xdiv(s, (double)*n), 0.5) : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    c += __shfl_down_sync(0xffffffffu, c, o);
+    r += __shfl_down_sync(0xffffffffu, r, o);
+    const int y = __shfl_down_sync(0xffffffffu, mx, o);
+    mx = y > mx ? y : mx;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(reinterpret_cast<unsigned long long*>(&w->pre), (unsigned long long)c);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&w->raw), (unsigned long long)r);
+    atomicMax(reinterpret_cast<unsigned long long*>(&w->longest), (unsigned long long)mx);
+  }
+  auto tree = [&](double v) {
+    sm[threadIdx.x] = v;
+    __syncthreads();
+    for (int h = RED_T / 2; h > 0; h >>= 1) {
+      if (threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
+      __syncthreads();
+    }
+    return sm[0];
+  };
+  if (sums) {
+    const double v = tree(acc);
+    if (threadIdx.x == 0) part[blockIdx.x] = v;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&w->ticket2, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double margin = fixed;
+  if (!(fixed > 0.0)) {
+    const long long n = *(volatile long long*)&w->pre;
+    if (sums) {
+      __syncthreads();
+      const double v = tree(threadIdx.x < RED_BLOCKS ? __ldcg(part + threadIdx.x) : 0.0);
+      margin = n > 0 ? xmul(xdiv(v, (double)n), 0.5) : 0.0;
+    } else {
+      margin = n > 0 ? xmul(xadd(gp->radius, gp->radius), 0.5) : 0.0;
+    }
+  }
+  if (threadIdx.x == 0) {
+    w->margin = margin;
+    w->ticket2 = 0u;  // the walk may be repeated
+  }
 }
 
 // Midpoint prescreen of DetectCandidatesProcess (_manager_process.py:260-286) for the pair (i, j), from
@@ -381,25 +497,28 @@ XK_D bool midpoint_keep(const double4_32a a, const double4_32a b, double ra, dou
   return mp <= xadd(xadd(ra, rb), extra);
 }
 
-// The same decision with a float screen first: the separation |m_i - m_j| in float (from the exact double
-// differences) against the threshold r_i + r_j + extra + h_i + h_j decides every pair farther than a
-// relative 1e-5 from it (float rounding of the separation stays below 1e-6 relative); the rest take the
-// exact routine, so the decision is the exact one.
-XK_D bool midpoint_keep_fast(const double4_32a a, const double4_32a b, double ra, double rb, double extra) {
-  const float dx = (float)xsub(a.x, b.x), dy = (float)xsub(a.y, b.y), dz = (float)xsub(a.z, b.z);
-  const float md = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-  const float thr = (float)(ra + rb + extra + a.w + b.w);
-  if (md < __fmul_rn(thr, 0.99999f)) return true;
-  if (md > __fmul_rn(thr, 1.00001f)) return false;
-  return midpoint_keep(a, b, ra, rb, extra);
+// The same decision with a float screen first: the separation |m_i - m_j| from the split midpoints against the
+// threshold r_i + r_j + extra + h_i + h_j in float decides every pair farther than a relative 1e-5 from it
+// (the roundings of both stay below 1e-6 relative); the rest, and what is not finite, take the exact routine,
+// so the decision is the exact one.
+XK_D bool midpoint_keep_fast(const MidF& a, const MidF& b, float extra, const double4_32a* __restrict__ mid, int i,
+                             int j, const double* __restrict__ radii, double extra64) {
+  const float dx = (a.hi[0] - b.hi[0]) + (a.lo[0] - b.lo[0]), dy = (a.hi[1] - b.hi[1]) + (a.lo[1] - b.lo[1]),
+              dz = (a.hi[2] - b.hi[2]) + (a.lo[2] - b.lo[2]);
+  const float md = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+  const float thr = ((a.r + b.r) + extra) + (a.half + b.half);
+  if (md < thr * 0.99999f) return true;
+  if (md > thr * 1.00001f) return false;
+  return midpoint_keep(mid[i], mid[j], radii[i], radii[j], extra64);
 }
 
 // A warp per segment: its slot list sorted by j (a rank sort; the j are distinct), the prescreen
-// applied (extra null: none), written to srt as j (kept) or ~j (dropped); cnt2[i] = kept count.
+// applied (if wanted), written to srt as j (kept) or ~j (dropped); cnt2[i] = kept count.
 __global__ void __launch_bounds__(BP_T) k_slots_rank(xk_mesh m, const double4_32a* __restrict__ mid,
-                                                     const int32_t* __restrict__ slot, const int32_t* __restrict__ cnt,
-                                                     int cap, const double* __restrict__ extra,
-                                                     int32_t* __restrict__ srt, int32_t* __restrict__ cnt2) {
+                                                     const MidF* __restrict__ midf, const int32_t* __restrict__ slot,
+                                                     const int32_t* __restrict__ cnt, int cap, int prescreen,
+                                                     const Words* __restrict__ words, int32_t* __restrict__ srt,
+                                                     int32_t* __restrict__ cnt2) {
   const long long ne = m.n_elems;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -408,13 +527,19 @@ __global__ void __launch_bounds__(BP_T) k_slots_rank(xk_mesh m, const double4_32
   const int n = cnt[i] < cap ? cnt[i] : cap;
   const int32_t* const my = slot + (long long)i * cap;
   int32_t* const out = srt + (long long)i * cap;
-  const double4_32a mi = mid[i];
-  const double ri = m.radii[i];
-  const double ex = extra ? *extra : 0.0;
+  const MidF mi = midf[i];
+  const double ex = words->margin;
+  const float exf = xk_d2f(ex);
+  auto keep = [&](int j) {
+    return !prescreen || midpoint_keep_fast(mi, midf[j], exf, mid, i, j, m.radii, ex);
+  };
   int kept = 0;
   if (n <= 64) {  // two entries per lane, ranked by shuffle-broadcast comparisons
     const int v0 = lane < n ? my[lane] : 0x7fffffff;
     const int v1 = lane + 32 < n ? my[lane + 32] : 0x7fffffff;
+    bool k0 = false, k1 = false;
+    if (lane < n) k0 = keep(v0);
+    if (lane + 32 < n) k1 = keep(v1);
     int r0 = 0, r1 = 0;
     const int n0 = n < 32 ? n : 32;
     for (int k = 0; k < n0; ++k) {
@@ -427,21 +552,14 @@ __global__ void __launch_bounds__(BP_T) k_slots_rank(xk_mesh m, const double4_32
       r0 += x < v0;
       r1 += x < v1;
     }
-    if (lane < n) {
-      const bool k = !extra || midpoint_keep_fast(mi, mid[v0], ri, m.radii[v0], ex);
-      out[r0] = k ? v0 : ~v0;
-      kept += k;
-    }
-    if (lane + 32 < n) {
-      const bool k = !extra || midpoint_keep_fast(mi, mid[v1], ri, m.radii[v1], ex);
-      out[r1] = k ? v1 : ~v1;
-      kept += k;
-    }
+    if (lane < n) out[r0] = k0 ? v0 : ~v0;
+    if (lane + 32 < n) out[r1] = k1 ? v1 : ~v1;
+    kept = k0 + k1;
   } else for (int l = lane; l < n; l += 32) {
     const int v = my[l];
     int r = 0;
     for (int q = 0; q < n; ++q) r += my[q] < v;
-    const bool k = !extra || midpoint_keep_fast(mi, mid[v], ri, m.radii[v], ex);
+    const bool k = keep(v);
     out[r] = k ? v : ~v;
     kept += k;
   }
@@ -629,56 +747,53 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   const long long ne = m->n_elems;
   if (ne < 2) return XK_OK;
   if (ne > 0x7fffffffLL) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: more than 2^31 segments");
+  // the grid has at most cap_cells cells, so the cell arrays are sized without reading it back
   const long long cap_cells = ne * 8 > 4096 ? ne * 8 : 4096;
   int slot_cap = g_slot_cap.load();
   XkScratch S(st);
   if ((double)ne * slot_cap * 8.0 <= 64.0e9)  // one allocation for the usual case: boxes, cells, lists, scans
-    XK_TRY(S.reserve((size_t)ne * (48 + 32 + 32 + 8 + 12 + 8 + 8 * (size_t)slot_cap) + (size_t)cap_cells * 9 + (1 << 16)));
-  double* box;
-  float4* boxf;
+    XK_TRY(S.reserve((size_t)ne * (48 + 32 + 32 + 32 + 32 + 16 + 8 + 16 + 8 + 8 * (size_t)slot_cap) +
+                     (size_t)cap_cells * 9 + (1 << 16)));
+  Words* words;
+  int32_t *ccnt, *segs, *cstart, *cnt, *raw, *cnt2, *off2, *ecell;
+  double *box, *rsum, *part;
+  float4 *boxf, *sorted;
   double4_32a* mid;
-  unsigned long long* ext;
+  MidF* midf;
+  int4* range;
   Grid* grid;
+  // the words and the cell counts start at zero: they stand together
+  char* zero;
+  const size_t words_bytes = XkScratch::padded(sizeof(Words)), zero_bytes = words_bytes + sizeof(int32_t) * (cap_cells + 1);
+  XK_TRY(S.get(&zero, (long long)zero_bytes));
+  words = reinterpret_cast<Words*>(zero);
+  ccnt = reinterpret_cast<int32_t*>(zero + words_bytes);
   XK_TRY(S.get(&box, 6 * ne));
   XK_TRY(S.get(&boxf, 2 * ne));
+  XK_TRY(S.get(&sorted, 2 * ne));
   XK_TRY(S.get(&mid, ne));
-  XK_TRY(S.get(&ext, 16));
+  XK_TRY(S.get(&midf, ne));
+  XK_TRY(S.get(&range, ne));
   XK_TRY(S.get(&grid, 1));
-  // words: 0 unused, 1-3 lowest lower corner, 4-6 highest upper corner, 7 raw count, 8 the sum of the
-  // box extents (a double, +0.0), 9-11 the largest extent on each axis, 12 the longest slot list
-  double* ext_sum = reinterpret_cast<double*>(ext + 8);
-  unsigned long long* raw_dev = ext + 7;
-  int32_t* max_cnt = reinterpret_cast<int32_t*>(ext + 12);
-  unsigned long long init[16] = {0ull, ~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull,
-                                 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-  XK_CUDA(cudaMemcpyAsync(ext, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  k_aabb<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, u, bp->margin, box, boxf, mid, ext, ext_sum);
-  // the grid has at most cap_cells cells, so the cell arrays are sized without reading it back
-  k_grid<<<1, 1, 0, st>>>(ext, ext_sum, ne, cap_cells, bp->cell_size, grid);
-  XK_CHECK_LAUNCH();
-  int32_t *segs, *cstart, *cfill, *cnt, *cnt2, *off2, *ecell;
   XK_TRY(S.get(&ecell, ne));
   XK_TRY(S.get(&segs, ne));
   XK_TRY(S.get(&cstart, cap_cells + 1));
-  XK_TRY(S.get(&cfill, cap_cells + 1));
   XK_TRY(S.get(&cnt, ne + 1));
+  XK_TRY(S.get(&raw, ne + 1));
   XK_TRY(S.get(&cnt2, ne + 1));
   XK_TRY(S.get(&off2, ne + 1));
-  // segments sorted by the cell of their lower corner
-  XK_CUDA(cudaMemsetAsync(cfill, 0, sizeof(int32_t) * (cap_cells + 1), st));
-  k_cell_count<<<xk_blocks(ne, 256), 256, 0, st>>>(box, ne, grid, ecell, cfill);
-  XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(cfill, cstart, cap_cells + 1, nullptr, st, &S));
-  XK_CUDA(cudaMemsetAsync(cfill, 0, sizeof(int32_t) * (cap_cells + 1), st));
-  k_cell_scatter<<<xk_blocks(ne, 256), 256, 0, st>>>(ne, ecell, cstart, cfill, segs);
-  k_cell_sort<<<xk_blocks(cap_cells, 256), 256, 0, st>>>(cap_cells, cstart, segs);
-  XK_CHECK_LAUNCH();
-  double *rsum, *part, *extra;
-  int64_t* tot;
   XK_TRY(S.get(&rsum, ne));
   XK_TRY(S.get(&part, RED_BLOCKS));
-  XK_TRY(S.get(&extra, 1));
-  XK_TRY(S.get(&tot, 2));
+  XK_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, st));
+  k_aabb<<<xk_blocks(ne, AABB_T), AABB_T, 0, st>>>(*m, u, bp->margin, box, boxf, mid, midf, words, cap_cells,
+                                                   bp->cell_size, grid);
+  // segments sorted by the cell of their lower corner
+  k_cell_count<<<xk_blocks(ne, 256), 256, 0, st>>>(box, ne, grid, ecell, ccnt, range);
+  XK_CHECK_LAUNCH();
+  XK_TRY(xk_exclusive_scan_i32(ccnt, cstart, cap_cells + 1, nullptr, st, &S));
+  k_cell_scatter<<<xk_blocks(ne, 256), 256, 0, st>>>(ne, ecell, cstart, ccnt, segs);
+  k_cell_boxes<<<xk_blocks(ne, 256), 256, 0, st>>>(ne, segs, ecell, cstart, boxf, sorted);
+  XK_CHECK_LAUNCH();
   const int warp_blocks = xk_blocks(ne * 32, BP_T);
   const int excl_layer = (bp->exclude_same_layer && m->layer) ? 1 : 0;
   for (int attempt = 0;; ++attempt) {
@@ -687,31 +802,20 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
     int32_t *slot, *srt;
     XK_TRY(S.get(&slot, ne * slot_cap));
     XK_TRY(S.get(&srt, ne * slot_cap));
-    XK_CUDA(cudaMemsetAsync(ext + 7, 0, sizeof(unsigned long long), st));
-    XK_CUDA(cudaMemsetAsync(ext + 12, 0, sizeof(unsigned long long), st));
-    k_sweep<<<warp_blocks, BP_T, 0, st>>>(*m, box, boxf, grid, segs, cstart, bp->exclude_shared, excl_layer,
-                                          slot_cap, slot, cnt, rsum, raw_dev, max_cnt);
+    if (attempt > 0) XK_CUDA(cudaMemsetAsync(&words->raw, 0, 4 * sizeof(long long), st));
+    k_sweep<<<warp_blocks, BP_T, 0, st>>>(*m, box, boxf, sorted, grid, range, cstart, bp->exclude_shared, excl_layer,
+                                          slot_cap, slot, cnt, raw, rsum);
+    k_totals<<<RED_BLOCKS, RED_T, 0, st>>>(cnt, raw, rsum, ne, grid, bp->prescreening_margin, part, words);
+    k_slots_rank<<<warp_blocks, BP_T, 0, st>>>(*m, mid, midf, slot, cnt, slot_cap, bp->midpoint_prescreening ? 1 : 0,
+                                               words, srt, cnt2);
     XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt, off2, ne, tot, st, &S));  // tot[0]: candidates before the prescreen
-    const double* ex = nullptr;
-    if (bp->midpoint_prescreening) {
-      if (!(bp->prescreening_margin > 0.0)) k_radsum_partial<<<RED_BLOCKS, RED_T, 0, st>>>(rsum, ne, part);
-      k_margin<<<1, 1, 0, st>>>(part, tot, bp->prescreening_margin, extra);
-      XK_CHECK_LAUNCH();
-      ex = extra;
-    }
-    k_slots_rank<<<warp_blocks, BP_T, 0, st>>>(*m, mid, slot, cnt, slot_cap, ex, srt, cnt2);
-    XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt2, off2, ne, tot + 1, st, &S));
+    XK_TRY(xk_exclusive_scan_i32(cnt2, off2, ne, reinterpret_cast<int64_t*>(&words->kept), st, &S));
     k_slots_emit<<<warp_blocks, BP_T, 0, st>>>(ne, srt, cnt, slot_cap, off2, cap, out_pairs);
     XK_CHECK_LAUNCH();
-    int64_t h[2];
-    unsigned long long hw[2] = {0ull, 0ull};
-    XK_CUDA(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, st));
-    XK_CUDA(cudaMemcpyAsync(hw, ext + 7, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    XK_CUDA(cudaMemcpyAsync(hw + 1, ext + 12, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    long long h[4];  // raw, pre, longest, kept
+    XK_CUDA(cudaMemcpyAsync(h, &words->raw, sizeof(h), cudaMemcpyDeviceToHost, st));
     XK_CUDA(cudaStreamSynchronize(st));
-    const int longest = (int)(uint32_t)hw[1];
+    const int longest = (int)h[2];
     if (longest > slot_cap) {  // some lists were cut short: walk again with lists long enough for all
       if (attempt > 0) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: slot lists overflowed twice");
       int c = slot_cap;
@@ -722,11 +826,11 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
       }
       continue;
     }
-    if (h[1] > 0x7fffffffLL) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: more than 2^31 candidates");
-    if (n_raw) *n_raw = (int64_t)hw[0];
-    if (n_prefilter) *n_prefilter = h[0];
-    *n_out = h[1];
-    if (h[1] > cap) return xk_set_error(XK_ERR_CAPACITY, "xk_broadphase: output capacity too small");
+    if (h[3] > 0x7fffffffLL) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: more than 2^31 candidates");
+    if (n_raw) *n_raw = h[0];
+    if (n_prefilter) *n_prefilter = h[1];
+    *n_out = h[3];
+    if (h[3] > cap) return xk_set_error(XK_ERR_CAPACITY, "xk_broadphase: output capacity too small");
     return XK_OK;
   }
 }
