@@ -15,21 +15,11 @@
 // friction acts).  So the pattern holds the blocks with row <= column only
 // ("upper" blocks), each computed once, and a lower index lists, per node w,
 // the stored blocks (v, w) with v < w, for readers that need whole rows.
-#include "xk_common.cuh"
+#include "scan.cuh"
 
 xk_status xk_sumsq_into(const double* x, long long n, double* out, cudaStream_t s);
 
 namespace {
-
-constexpr int MAX_COLS = 256;  // distinct column nodes per pattern row
-
-XK_D void pair_nodes4(const xk_mesh& m, const xk_pairs& p, int i, int* nd) {
-  const int ea = p.ea[i], eb = p.eb[i];
-  nd[0] = m.conn[2 * ea];
-  nd[1] = m.conn[2 * ea + 1];
-  nd[2] = m.conn[2 * eb];
-  nd[3] = m.conn[2 * eb + 1];
-}
 
 template <typename T>
 XK_D T shape_c(T s, T t, int k) {
@@ -43,69 +33,168 @@ XK_D T shape_c(T s, T t, int k) {
 
 // A pair contributes in the increment when it is not INACTIVE or still carries a normal force; with
 // coated wires every pair does, since the reference evaluates the coating force of every pair.
-XK_D bool is_member(const xk_pairs& p, int i) {
+XK_D bool is_member(const xk_pairs& p, long long i) {
   return (p.status[i] != 0) || (p.p_n[i] > 0.0) || (p.coat_cc != nullptr);
 }
 
-__global__ void k_flags(xk_pairs p, int32_t* __restrict__ flag) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < p.n) flag[i] = is_member(p, i) ? 1 : 0;
-  else if (i == p.n) flag[i] = 0;
-}
+// ---------------------------------------------------------------------------------------------------------------
+// Contact pattern.  Seven launches whose sizes are bounded by the host's (pairs, nodes, elements), so that the
+// host waits once, at the end: a kernel that needs the number of members or blocks reads it on the device, and one
+// that would run past a capacity writes nothing.
+//   members      scan over the pairs: members, their nodes, the other pairs, members per element
+//   elements     scans over the elements (elem_ptr) and the nodes (inc_ptr = its elements' members)
+//   sides        member sides of each element, in the order the atomics give
+//   k_pat_cols   per node: incidences sorted, distinct neighbours sorted, contributions counted;
+//                per element: member sides sorted
+//   rows         scans over the nodes (row_ptr with the first contribution; low_ptr)
+//   k_pat_rows   per node: columns, contributor lists, term lists and lower index of its row
+// The incidences of a node are sorted, so a row that places its contributions in that order emits every block's
+// list sorted: no list is sorted after it is filled, and none is filled through atomics.  Before, lists were
+// counted, scanned, filled and sorted one after another (30 launches, three waits).  GB300, a detection from the
+// same state: 37 wires 630 -> 434 us, 397 wires 1190 -> 957, 1027 wires 2330 -> 2065.
+// ---------------------------------------------------------------------------------------------------------------
 
-__global__ void k_split_lists(xk_mesh m, xk_pairs p, const int32_t* __restrict__ mpos, int32_t* __restrict__ members,
-                              int32_t* __restrict__ mnodes, int32_t* __restrict__ others) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= p.n) return;
-  const int k = mpos[i];
-  if (is_member(p, i)) {
-    members[k] = i;
-    int nd[4];
-    pair_nodes4(m, p, i, nd);
-    for (int q = 0; q < 4; ++q) mnodes[4LL * k + q] = nd[q];
-  } else {
-    others[i - k] = i;
-  }
-}
+struct Totals {
+  int64_t members, blocks, contribs, low;
+};
 
-__global__ void k_inc_count(const int32_t* __restrict__ mnodes, int nm, int32_t* __restrict__ cnt) {
-  int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  for (int k = 0; k < 4; ++k) atomicAdd(&cnt[mnodes[4LL * mi + k]], 1);
-}
-
-__global__ void k_inc_fill(const int32_t* __restrict__ mnodes, int nm, const int32_t* __restrict__ ptr,
-                           int32_t* __restrict__ fill, int32_t* __restrict__ inc) {
-  int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  for (int k = 0; k < 4; ++k) {
-    const int v = mnodes[4LL * mi + k];
-    inc[ptr[v] + atomicAdd(&fill[v], 1)] = (mi << 2) | k;
-  }
-}
-
-// Sort every segment [ptr[v], ptr[v+1]) ascending, so that sums run in a fixed order whatever the
-// order of the atomic fill.  A warp per segment: up to 64 entries (the entries of a segment are
-// distinct) sit in two registers per lane and each finds its rank by comparing against all others
-// broadcast by shuffles, then the warp writes them to their ranks; a longer segment is sorted by
-// insertion by one lane.
-constexpr int SEG_T = 128;
-XK_D void warp_sort_segment(int lo, int hi, int32_t* __restrict__ a, int lane) {
-  const int n = hi - lo;
-  if (n <= 1) return;
-  if (n > 64) {
-    if (lane == 0) {
-      for (int x = lo + 1; x < hi; ++x) {
-        const int key = a[x];
-        int y = x - 1;
-        while (y >= lo && a[y] > key) { a[y + 1] = a[y]; --y; }
-        a[y + 1] = key;
-      }
+struct MemberScan {
+  xk_mesh m;
+  xk_pairs p;
+  long long cap;  // members that fit
+  long long cap_others;
+  int32_t *members, *mnodes, *others, *ecnt;
+  Totals* tot;
+  bool wide;  // status, p_n and mnodes aligned for vector access
+  XK_D long long size(int) const { return p.n; }
+  XK_D int64_t one(int, long long i) const { return is_member(p, i) ? 1 : 0; }
+  XK_D void eight(int, long long i, int64_t* v) const {
+    if (!wide) {
+#pragma unroll
+      for (int k = 0; k < SCAN_I; ++k) v[k] = one(0, i + k);
+      return;
     }
-    return;
+    const uint2 st = *reinterpret_cast<const uint2*>(p.status + i);
+    double pn[SCAN_I];
+#pragma unroll
+    for (int k = 0; k < SCAN_I; k += 2) {
+      const double2 x = *reinterpret_cast<const double2*>(p.p_n + i + k);
+      pn[k] = x.x;
+      pn[k + 1] = x.y;
+    }
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k)
+      v[k] = ((((k < 4 ? st.x : st.y) >> (8 * (k & 3))) & 0xffu) != 0 || pn[k] > 0.0 || p.coat_cc != nullptr) ? 1 : 0;
   }
-  const int v0 = lane < n ? a[lo + lane] : 0x7fffffff;
-  const int v1 = lane + 32 < n ? a[lo + lane + 32] : 0x7fffffff;
+  XK_D void store(int, long long i, int n, int64_t prefix, const int64_t* v) const {
+    int ea[SCAN_I], eb[SCAN_I];
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k)
+      if (k < n && v[k]) {
+        ea[k] = p.ea[i + k];
+        eb[k] = p.eb[i + k];
+      }
+    int4 nd[SCAN_I];
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k)
+      if (k < n && v[k])
+        nd[k] = make_int4(m.conn[2 * ea[k]], m.conn[2 * ea[k] + 1], m.conn[2 * eb[k]], m.conn[2 * eb[k] + 1]);
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k) {
+      if (k >= n) continue;
+      if (!v[k]) {
+        const long long o = i + k - prefix;
+        if (o < cap_others) others[o] = (int32_t)(i + k);
+        continue;
+      }
+      if (prefix < cap) {
+        members[prefix] = (int32_t)(i + k);
+        int32_t* q = mnodes + 4 * prefix;
+        if (wide) {
+          *reinterpret_cast<int4*>(q) = nd[k];
+        } else {
+          q[0] = nd[k].x; q[1] = nd[k].y; q[2] = nd[k].z; q[3] = nd[k].w;
+        }
+        atomicAdd(ecnt + ea[k], 1);
+        atomicAdd(ecnt + eb[k], 1);
+      }
+      ++prefix;
+    }
+  }
+  XK_D void total(int, int64_t s) const { tot->members = s; }
+};
+
+// elem_ptr (channel 0) and inc_ptr (channel 1): a node's incidences are its elements' members
+struct ElemScan {
+  int nn, ne;
+  const int32_t *ecnt, *neptr;
+  const int2* nelem;
+  int32_t *eptr, *iptr;
+  XK_D long long size(int c) const { return (c == 0 ? ne : nn) + 1; }
+  XK_D int64_t one(int c, long long i) const {
+    if (c == 0) return i < ne ? ecnt[i] : 0;
+    int64_t s = 0;
+    if (i < nn)
+      for (int y = neptr[i]; y < neptr[i + 1]; ++y) s += ecnt[nelem[y].x >> 1];
+    return s;
+  }
+  XK_D void eight(int c, long long i, int64_t* v) const {
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k) v[k] = one(c, i + k);
+  }
+  XK_D void store(int c, long long i, int n, int64_t prefix, const int64_t* v) const {
+    int32_t* out = c == 0 ? eptr : iptr;
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k) {
+      if (k < n) out[i + k] = (int32_t)prefix;
+      prefix += v[k];
+    }
+  }
+  XK_D void total(int, int64_t) const {}
+};
+
+// row_ptr and the rows' first contributions (channel 0, both counts in one word), low_ptr (channel 1)
+struct RowScan {
+  int nn;
+  const int32_t *rcnt, *ccnt, *lcnt;
+  int32_t *rptr, *cbase, *lptr;  // lptr nullable
+  Totals* tot;
+  XK_D long long size(int) const { return nn + 1; }
+  XK_D int64_t one(int c, long long i) const {
+    if (i >= nn) return 0;
+    return c == 0 ? ((int64_t)ccnt[i] << 32) + rcnt[i] : lcnt[i];
+  }
+  XK_D void eight(int c, long long i, int64_t* v) const {
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k) v[k] = one(c, i + k);
+  }
+  XK_D void store(int c, long long i, int n, int64_t prefix, const int64_t* v) const {
+#pragma unroll
+    for (int k = 0; k < SCAN_I; ++k) {
+      if (k < n) {
+        if (c == 0) {
+          rptr[i + k] = (int32_t)prefix;
+          cbase[i + k] = (int32_t)(prefix >> 32);
+        } else if (lptr) {
+          lptr[i + k] = (int32_t)prefix;
+        }
+      }
+      prefix += v[k];
+    }
+  }
+  XK_D void total(int c, int64_t s) const {
+    if (c == 0) {
+      tot->blocks = s & 0xffffffffLL;
+      tot->contribs = s >> 32;
+    } else {
+      tot->low = s;
+    }
+  }
+};
+
+// Ascending sort of a warp's n <= 64 distinct values, two per lane: each finds its rank by comparing against all
+// others broadcast by shuffles and goes to that place.
+XK_D void warp_rank_sort(int v0, int v1, int n, int32_t* out, int lane) {
   int r0 = 0, r1 = 0;
   const int n0 = n < 32 ? n : 32;
   for (int k = 0; k < n0; ++k) {
@@ -118,166 +207,15 @@ XK_D void warp_sort_segment(int lo, int hi, int32_t* __restrict__ a, int lane) {
     r0 += x < v0;
     r1 += x < v1;
   }
-  __syncwarp();
-  if (lane < n) a[lo + r0] = v0;
-  if (lane + 32 < n) a[lo + r1] = v1;
+  if (lane < n) out[r0] = v0;
+  if (lane + 32 < n) out[r1] = v1;
 }
 
-__global__ void __launch_bounds__(SEG_T) k_segment_sort(const int32_t* __restrict__ ptr, long long nseg,
-                                                        int32_t* __restrict__ a) {
-  const long long v = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (v >= nseg) return;
-  warp_sort_segment(ptr[v], ptr[v + 1], a, threadIdx.x & 31);
-}
-
-// The same sort for many short segments (the contributor lists of the blocks, a few entries each, where a
-// warp per segment spends its time on warps): a thread per segment sorts one of at most SEG_SHORT entries
-// by insertion in place and lists a longer one (a diagonal block, one entry per member at the node) for
-// k_segment_sort_listed, whose persistent warps take the listed segments in turn.
-constexpr int SEG_SHORT = 12;
-__global__ void k_segment_sort_short(const int32_t* __restrict__ ptr, long long nseg, int32_t* __restrict__ a,
-                                     int32_t* __restrict__ longs, int32_t* __restrict__ n_longs) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nseg) return;
-  const int lo = ptr[v], hi = ptr[v + 1];
-  if (hi - lo > SEG_SHORT) {
-    longs[atomicAdd(n_longs, 1)] = (int)v;
-    return;
-  }
-  for (int x = lo + 1; x < hi; ++x) {
-    const int key = a[x];
-    int y = x - 1;
-    while (y >= lo && a[y] > key) { a[y + 1] = a[y]; --y; }
-    a[y + 1] = key;
-  }
-}
-
-__global__ void __launch_bounds__(SEG_T) k_segment_sort_listed(const int32_t* __restrict__ ptr,
-                                                               int32_t* __restrict__ a,
-                                                               const int32_t* __restrict__ longs,
-                                                               const int32_t* __restrict__ n_longs) {
-  const int n = *n_longs;
-  const int lane = threadIdx.x & 31;
-  const long long nw = (long long)gridDim.x * (SEG_T / 32);
-  for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += nw) {
-    const int v = longs[w];
-    warp_sort_segment(ptr[v], ptr[v + 1], a, lane);
-  }
-}
-
-// The distinct column nodes c >= v of row v, in ascending order, from its member incidences (the four nodes
-// of every member touching v).  A warp per node: the candidates >= v (4 per incidence, at most RC_CAP) go
-// into a per-warp open-addressing hash set in shared memory (twice the candidates' power of two, linear
-// probing, atomicCAS among the warp's lanes), which drops the repeats; the distinct values are gathered
-// by a ballot scan of the set and ranked: by shuffles when at most 64 (two per lane), else by a bitonic
-// sort in shared memory.  MODE 0 counts them (rcnt[v]); MODE 1 writes them at rptr[v] (col, and v in
-// brow).  A node with more than RC_CAP candidates takes the serial path of one lane (insertion into a
-// sorted local buffer of MAX_COLS distinct columns; err bit 1 if that overflows).
-constexpr int RC_WARPS = 4, RC_CAP = 512, RC_TAB = 2 * RC_CAP;
-XK_D int row_cols_serial(const int32_t* __restrict__ mnodes, const int32_t* __restrict__ inc, int x0, int x1, int v,
-                         int* buf, int32_t* __restrict__ err) {
-  int n = 0;
-  for (int x = x0; x < x1; ++x) {
-    const long long mi = inc[x] >> 2;
-    for (int k = 0; k < 4; ++k) {
-      const int c = mnodes[4 * mi + k];
-      if (c < v) continue;
-      int y = n - 1;
-      while (y >= 0 && buf[y] > c) --y;
-      if (y >= 0 && buf[y] == c) continue;
-      if (n >= MAX_COLS) { atomicOr(err, 1); continue; }
-      for (int z = n - 1; z > y; --z) buf[z + 1] = buf[z];
-      buf[y + 1] = c;
-      ++n;
-    }
-  }
-  return n;
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(32 * RC_WARPS) k_row_cols(const int32_t* __restrict__ mnodes,
-                                                            const int32_t* __restrict__ ptr,
-                                                            const int32_t* __restrict__ inc, int n_nodes,
-                                                            int32_t* __restrict__ rcnt,
-                                                            const int32_t* __restrict__ rptr,
-                                                            int32_t* __restrict__ col, int32_t* __restrict__ brow,
-                                                            int32_t* __restrict__ err) {
-  __shared__ int stab[RC_WARPS][RC_TAB];
-  __shared__ int slist[RC_WARPS][RC_CAP];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int v = blockIdx.x * RC_WARPS + wid;
-  if (v >= n_nodes) return;
-  const int x0 = ptr[v], x1 = ptr[v + 1];
-  const int nc = 4 * (x1 - x0);
-  if (nc > RC_CAP) {
-    if (lane == 0) {
-      int buf[MAX_COLS];
-      const int n = row_cols_serial(mnodes, inc, x0, x1, v, buf, err);
-      if (MODE == 0) {
-        rcnt[v] = n;
-      } else {
-        for (int k = 0; k < n; ++k) {
-          col[rptr[v] + k] = buf[k];
-          brow[rptr[v] + k] = v;
-        }
-      }
-    }
-    return;
-  }
-  constexpr int EMPTY = -1;
-  int* t = stab[wid];
-  int* l = slist[wid];
-  int ts = 64;
-  while (ts < 2 * nc) ts <<= 1;  // a power of two, at least twice the candidates
-  for (int i = lane; i < ts; i += 32) t[i] = EMPTY;
-  __syncwarp();
-  for (int i = lane; i < nc; i += 32) {
-    const int c = mnodes[4LL * (inc[x0 + (i >> 2)] >> 2) + (i & 3)];
-    if (c < v) continue;
-    unsigned h = ((unsigned)c * 2654435761u) & (unsigned)(ts - 1);
-    while (true) {
-      const int o = atomicCAS(&t[h], EMPTY, c);
-      if (o == EMPTY || o == c) break;
-      h = (h + 1) & (unsigned)(ts - 1);
-    }
-  }
-  __syncwarp();
-  int nd = 0;
-  const unsigned below = (1u << lane) - 1u;
-  for (int i0 = 0; i0 < ts; i0 += 32) {
-    const int x = t[i0 + lane];
-    const unsigned bal = __ballot_sync(0xffffffffu, x != EMPTY);
-    if (x != EMPTY) l[nd + __popc(bal & below)] = x;
-    nd += __popc(bal);
-  }
-  __syncwarp();
-  if (MODE == 0) {
-    if (lane == 0) rcnt[v] = nd;
-    return;
-  }
-  const int o = rptr[v];
-  if (nd <= 64) {  // ranks by shuffle-broadcast comparisons (the values are distinct)
-    const int v0 = lane < nd ? l[lane] : 0x7fffffff;
-    const int v1 = lane + 32 < nd ? l[lane + 32] : 0x7fffffff;
-    int r0 = 0, r1 = 0;
-    const int n0 = nd < 32 ? nd : 32;
-    for (int k = 0; k < n0; ++k) {
-      const int x = __shfl_sync(0xffffffffu, v0, k);
-      r0 += x < v0;
-      r1 += x < v1;
-    }
-    for (int k = 0; k < nd - 32; ++k) {
-      const int x = __shfl_sync(0xffffffffu, v1, k);
-      r0 += x < v0;
-      r1 += x < v1;
-    }
-    if (lane < nd) { col[o + r0] = v0; brow[o + r0] = v; }
-    if (lane + 32 < nd) { col[o + r1] = v1; brow[o + r1] = v; }
-    return;
-  }
+// Bitonic sort of l[0, n) in shared memory; l has room for the next power of two.
+XK_D void warp_bitonic_sort(int* l, int n, int lane) {
   int N = 32;
-  while (N < nd) N <<= 1;
-  for (int i = nd + lane; i < N; i += 32) l[i] = 0x7fffffff;
+  while (N < n) N <<= 1;
+  for (int i = n + lane; i < N; i += 32) l[i] = 0x7fffffff;
   __syncwarp();
   for (int k = 2; k <= N; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1) {
@@ -293,56 +231,360 @@ __global__ void __launch_bounds__(32 * RC_WARPS) k_row_cols(const int32_t* __res
       }
       __syncwarp();
     }
-  for (int i = lane; i < nd; i += 32) {
-    col[o + i] = l[i];
-    brow[o + i] = v;
+}
+
+// The n values of l (shared memory, n <= RC_CAP) in ascending order to out.
+constexpr int RC_WARPS = 4, RC_CAP = 512, RC_TAB = 2 * RC_CAP;
+XK_D void warp_sort_shared(int* l, int n, int32_t* out, int lane) {
+  if (n <= 64) {
+    warp_rank_sort(lane < n ? l[lane] : 0x7fffffff, lane + 32 < n ? l[lane + 32] : 0x7fffffff, n, out, lane);
+    return;
+  }
+  warp_bitonic_sort(l, n, lane);
+  for (int i = lane; i < n; i += 32) out[i] = l[i];
+}
+
+XK_D void serial_insertion_sort(int32_t* a, int n) {
+  for (int x = 1; x < n; ++x) {
+    const int key = a[x];
+    int y = x - 1;
+    while (y >= 0 && a[y] > key) { a[y + 1] = a[y]; --y; }
+    a[y + 1] = key;
   }
 }
 
-// Lower index: per node w, the stored blocks (v, w) with v < w in the order of v (MODE 0 counts).
-template <int MODE>
-__global__ void k_lower_index(long long nb, const int32_t* __restrict__ brow, const int32_t* __restrict__ col,
-                              int32_t* __restrict__ cnt, const int32_t* __restrict__ lptr, int32_t* __restrict__ lblk) {
-  const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int w = col[b];
-  if (brow[b] == w) return;
-  if (MODE == 0) atomicAdd(&cnt[w], 1);
-  else lblk[lptr[w] + atomicAdd(&cnt[w], 1)] = (int)b;
+// The member sides of the elements, in the order the atomics give (ecnt counts down to zero).
+__global__ void k_pat_sides(xk_pairs p, const int32_t* __restrict__ members, const Totals* __restrict__ tot,
+                            long long cap, const int32_t* __restrict__ eptr, int32_t* __restrict__ ecnt,
+                            int32_t* __restrict__ raw) {
+  const long long mi = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long nm = tot->members;
+  if (nm > cap || mi >= nm) return;
+  const int i = members[mi];
+  const int ea = p.ea[i], eb = p.eb[i];
+  raw[eptr[ea] + atomicSub(&ecnt[ea], 1) - 1] = (int)(mi << 1);
+  raw[eptr[eb] + atomicSub(&ecnt[eb], 1) - 1] = (int)(mi << 1) | 1;
 }
 
-XK_D int find_block(const int32_t* __restrict__ rptr, const int32_t* __restrict__ col, int row, int c) {
-  int lo = rptr[row], hi = rptr[row + 1];
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (col[mid] < c) lo = mid + 1; else hi = mid;
+// A warp per node, then a warp per element.  A node's incidences are its elements' member sides; its neighbours (the
+// nodes of every member touching it) are its own elements' nodes and each incidence's partner nodes, so one 8-byte
+// load per incidence and one insertion per partner node into an open-addressing hash set in shared memory (twice
+// the candidates' power of two, linear probing, atomicCAS among the warp's lanes) find them.  The sorted neighbours
+// stay in list + 4 inc_ptr[v] for k_pat_rows.  A node with more than RC_CAP candidates takes the serial path of one
+// lane; as in the reference's sizes a row there holds at most MAX_COLS columns (err otherwise).
+constexpr int MAX_COLS = 256;
+struct PatternArgs {
+  int nn, ne;
+  long long cap, cap_blocks;
+  Totals* tot;
+  const int32_t *mnodes, *neptr, *eptr, *iptr, *raw;
+  const int2* nelem;
+  int32_t *inc, *einc;  // einc nullable
+  int32_t *list, *rcnt, *ccnt, *lcnt, *err;
+  // k_pat_rows
+  const int32_t *rptr, *cbase, *lptr;
+  int32_t *col, *brow, *bptr, *contrib, *lblk, *bcodes, *serr;  // lblk, bcodes nullable
+};
+
+__global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constant__ PatternArgs g) {
+  __shared__ int stab[RC_WARPS][RC_TAB];
+  __shared__ int slist[RC_WARPS][RC_CAP];
+  if (g.tot->members > g.cap) return;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  int* l = slist[wid];
+  const long long w = (long long)blockIdx.x * RC_WARPS + wid;
+  if (w >= g.nn) {  // an element
+    const long long e = w - g.nn;
+    if (e >= g.ne || !g.einc) return;
+    const int o = g.eptr[e], n = g.eptr[e + 1] - o;
+    if (n <= RC_CAP) {
+      for (int i = lane; i < n; i += 32) l[i] = g.raw[o + i];
+      __syncwarp();
+      warp_sort_shared(l, n, g.einc + o, lane);
+    } else if (lane == 0) {
+      for (int i = 0; i < n; ++i) g.einc[o + i] = g.raw[o + i];
+      serial_insertion_sort(g.einc + o, n);
+    }
+    return;
+  }
+  const int v = (int)w;
+  const int x0 = g.iptr[v], n = g.iptr[v + 1] - x0;
+  if (n == 0) {
+    if (lane == 0) g.rcnt[v] = g.ccnt[v] = g.lcnt[v] = 0;
+    return;
+  }
+  const int y0 = g.neptr[v], y1 = g.neptr[v + 1];
+  int32_t* inc = g.inc + x0;
+  int32_t* out = g.list + 4LL * x0;
+  if (4 * n > RC_CAP) {
+    if (lane != 0) return;
+    int q = 0;
+    for (int y = y0; y < y1; ++y) {
+      const int e = g.nelem[y].x >> 1, p = g.nelem[y].x & 1;
+      for (int x = g.eptr[e]; x < g.eptr[e + 1]; ++x)
+        inc[q++] = ((g.raw[x] >> 1) << 2) | ((g.raw[x] & 1) << 1) | p;
+    }
+    serial_insertion_sort(inc, n);
+    int nd = 0, nc = 0, low = 0;
+    for (int x = 0; x < n; ++x)
+      for (int k = 0; k < 4; ++k) {
+        const int c = g.mnodes[4LL * (inc[x] >> 2) + k];
+        nc += c >= v;
+        int y = nd - 1;
+        while (y >= 0 && out[y] > c) --y;
+        if (y >= 0 && out[y] == c) continue;
+        for (int z = nd - 1; z > y; --z) out[z + 1] = out[z];
+        out[y + 1] = c;
+        ++nd;
+        low += c < v;
+      }
+    if (nd - low > MAX_COLS) atomicOr(g.err, 1);
+    g.rcnt[v] = nd - low;
+    g.ccnt[v] = nc;
+    g.lcnt[v] = low;
+    return;
+  }
+  // incidences: the elements' segments one after the other, then sorted
+  int q = 0;
+  for (int y = y0; y < y1; ++y) {
+    const int2 en = g.nelem[y];
+    const int o = g.eptr[en.x >> 1], m = g.eptr[(en.x >> 1) + 1] - o;
+    for (int i = lane; i < m; i += 32) {
+      const int x = g.raw[o + i];
+      l[q + i] = ((x >> 1) << 2) | ((x & 1) << 1) | (en.x & 1);
+    }
+    q += m;
+  }
+  int* t = stab[wid];
+  constexpr int EMPTY = -1;
+  int ts = 64;
+  while (ts < 4 * n + 4 * (y1 - y0) && ts < RC_TAB) ts <<= 1;
+  for (int i = lane; i < ts; i += 32) t[i] = EMPTY;
+  __syncwarp();
+  auto insert = [&](int c) {
+    unsigned h = ((unsigned)c * 2654435761u) & (unsigned)(ts - 1);
+    while (true) {
+      const int o = atomicCAS(&t[h], EMPTY, c);
+      if (o == EMPTY || o == c) break;
+      h = (h + 1) & (unsigned)(ts - 1);
+    }
+  };
+  int nc = 0;  // contributions to the row: candidates >= v
+  for (int i = lane; i < n; i += 32) {
+    const int x = l[i];
+    const int32_t* nd = g.mnodes + 4LL * (x >> 2) + ((x & 2) ? 0 : 2);
+    const int a = nd[0], b = nd[1];
+    nc += (a >= v) + (b >= v);
+    insert(a);
+    insert(b);
+  }
+  for (int y = y0 + lane; y < y1; y += 32) {
+    const int2 en = g.nelem[y];
+    const int m = g.eptr[(en.x >> 1) + 1] - g.eptr[en.x >> 1];
+    nc += m * (1 + (en.y >= v));
+    if (m > 0) insert(en.y);
+  }
+  if (lane == 0) insert(v);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nc += __shfl_xor_sync(0xffffffffu, nc, o);
+  __syncwarp();
+  warp_sort_shared(l, n, inc, lane);
+  __syncwarp();
+  int nd = 0, low = 0;
+  for (int i0 = 0; i0 < ts; i0 += 32) {
+    const int x = t[i0 + lane];
+    const unsigned bal = __ballot_sync(0xffffffffu, x != EMPTY);
+    if (x != EMPTY) l[nd + __popc(bal & below)] = x;
+    nd += __popc(bal);
+    low += __popc(__ballot_sync(0xffffffffu, x != EMPTY && x < v));
+  }
+  __syncwarp();
+  warp_sort_shared(l, nd, out, lane);
+  if (lane == 0) {
+    g.rcnt[v] = nd - low;
+    g.ccnt[v] = nc;
+    g.lcnt[v] = low;
+  }
+}
+
+// First place in a[0, n) not below c.
+XK_D int lower_bound(const int32_t* a, int n, int c) {
+  int lo = 0;
+  while (lo < n) {
+    const int mid = (lo + n) >> 1;
+    if (a[mid] < c) lo = mid + 1; else n = mid;
   }
   return lo;
 }
 
-// MODE 0: count contributions per block; MODE 1: fill (member << 4 | k << 2 | l).
-template <int MODE>
-__global__ void k_contrib(const int32_t* __restrict__ mnodes, int nm, const int32_t* __restrict__ rptr,
-                          const int32_t* __restrict__ col, int32_t* __restrict__ cnt,
-                          const int32_t* __restrict__ bptr, int32_t* __restrict__ contrib, int32_t* __restrict__ err) {
-  int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  int nd[4];
-  for (int q = 0; q < 4; ++q) nd[q] = mnodes[4LL * mi + q];
-  for (int k = 0; k < 4; ++k)
-    for (int l = 0; l < 4; ++l) {
-      if (nd[k] > nd[l]) continue;  // a lower block: the same values as its stored mirror
-      const int b = find_block(rptr, col, nd[k], nd[l]);
-      if (b >= rptr[nd[k] + 1] || col[b] != nd[l]) {  // cannot happen for a consistent pattern
-        atomicOr(err, 2);
-        continue;
-      }
-      if (MODE == 0) {
-        atomicAdd(&cnt[b], 1);
-      } else {
-        contrib[bptr[b] + atomicAdd(&cnt[b], 1)] = (mi << 4) | (k << 2) | l;
+// Inline term lists of the blocks (variant "sides"): a block's same-side terms are element sums.
+constexpr int SIDE_FLAG = (int)0x80000000;
+// An element's three sums S^00, S^01, S^11, each as 16 values: the 9 of the
+// sum, then 1, 1 in the places of a record's s, t and padding, so that a term
+// loads the same values from an element sum as from a combined record (both
+// 64-byte aligned) and the weight c_1 c_1 = s s of an element-sum term is 1.
+constexpr int SUM_STRIDE = 16;
+constexpr int ELEM_SUMS = 3 * SUM_STRIDE;
+
+// The terms of block (v, c), ascending: the sums of v's elements (diagonal: S^pp of each; a neighbour on an element:
+// S^01), empty places, then room for the block's n_cross cross codes.  False when more than four (the variant is
+// then off).
+XK_D bool side_terms(const PatternArgs& g, int v, int c, int n_cross, int* terms) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) terms[k] = -1;
+  int n = 0;
+  auto add = [&](int code) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {  // into its place (no array index at run time)
+      if (k > n) continue;
+      if (k == n || code < terms[k]) {
+        const int t = terms[k];
+        terms[k] = code;
+        code = t;
       }
     }
+    ++n;
+  };
+  for (int y = g.neptr[v]; y < g.neptr[v + 1]; ++y) {
+    const int2 en = g.nelem[y];
+    const int base = ELEM_SUMS * (en.x >> 1);
+    if (c == v) add(SIDE_FLAG | (base + ((en.x & 1) ? 2 * SUM_STRIDE : 0)));
+    if (c == en.y) add(SIDE_FLAG | (base + SUM_STRIDE));
+  }
+  if (n + n_cross <= 4) return true;
+  atomicOr(g.serr, 1);
+  return false;
+}
+
+// A warp per node: its row's columns, each block's contributor and term lists, its lower index.  Contributions are
+// taken in the incidences' order, 32 at a time, and each goes behind the ones before it in its block (match over
+// the warp, a running position per block in shared memory), so the lists come out sorted.
+constexpr int PR_WARPS = 4;
+__global__ void __launch_bounds__(32 * PR_WARPS) k_pat_rows(const __grid_constant__ PatternArgs g) {
+  __shared__ int s_col[PR_WARPS][RC_CAP];
+  __shared__ int s_pos[PR_WARPS][RC_CAP];    // next contribution of a block
+  __shared__ int s_cross[PR_WARPS][RC_CAP];  // next cross term
+  __shared__ short s_rank[PR_WARPS][RC_CAP];
+  if (g.tot->members > g.cap || g.tot->blocks > g.cap_blocks) return;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int v = blockIdx.x * PR_WARPS + wid;
+  if (v >= g.nn) return;
+  const int o = g.rptr[v], nup = g.rptr[v + 1] - o;
+  if (v == g.nn - 1 && lane == 0) g.bptr[o + nup] = g.cbase[g.nn];
+  const int x0 = g.iptr[v], nc = 4 * (g.iptr[v + 1] - x0);
+  if (nc == 0) return;
+  const int low = g.lcnt[v], cb = g.cbase[v];
+  const int32_t* list = g.list + 4LL * x0;
+  if (g.lblk) {
+    const int lo = g.lptr[v];
+    for (int i = lane; i < low; i += 32) {
+      const int c = list[i];
+      const int rc = g.rptr[c];
+      g.lblk[lo + i] = rc + lower_bound(g.list + 4LL * g.iptr[c] + g.lcnt[c], g.rptr[c + 1] - rc, v);
+    }
+  }
+  list += low;
+  const int32_t* inc = g.inc + x0;
+  if (nc > RC_CAP) {  // a block at a time, its contributions collected from all candidates
+    int at = cb;
+    for (int r = 0; r < nup; ++r) {
+      const int c = list[r];
+      const int b = o + r;
+      if (lane == 0) {
+        g.col[b] = c;
+        g.brow[b] = v;
+        g.bptr[b] = at;
+      }
+      int n_cross = 0;
+      for (int i0 = 0; i0 < nc; i0 += 32) {
+        const int i = i0 + lane;
+        const int x = i < nc ? inc[i >> 2] : 0;
+        const bool hit = i < nc && g.mnodes[4LL * (x >> 2) + (i & 3)] == c;
+        const bool cross = hit && ((x >> 1) & 1) != ((i & 3) >> 1);
+        const unsigned bh = __ballot_sync(0xffffffffu, hit), bc = __ballot_sync(0xffffffffu, cross);
+        if (hit) g.contrib[at + __popc(bh & below)] = (x << 2) | (i & 3);
+        const int k = n_cross + __popc(bc & below);
+        if (cross && k < 4) s_cross[wid][k] = (x << 2) | (i & 3);
+        at += __popc(bh);
+        n_cross += __popc(bc);
+      }
+      __syncwarp();
+      if (g.bcodes && lane == 0) {
+        int terms[4];
+        if (side_terms(g, v, c, n_cross, terms))
+          for (int k = 0; k < n_cross; ++k) terms[4 - n_cross + k] = s_cross[wid][k];
+        *reinterpret_cast<int4*>(g.bcodes + 4LL * b) = make_int4(terms[0], terms[1], terms[2], terms[3]);
+      }
+      __syncwarp();
+    }
+    return;
+  }
+  int* sc = s_col[wid];
+  int* sp = s_pos[wid];
+  int* sx = s_cross[wid];
+  short* rk = s_rank[wid];
+  for (int r = lane; r < nup; r += 32) {
+    sc[r] = list[r];
+    sp[r] = 0;
+  }
+  __syncwarp();
+  for (int i = lane; i < nc; i += 32) {  // counts per block: all contributions, cross ones in the upper half
+    const int x = inc[i >> 2];
+    const int c = g.mnodes[4LL * (x >> 2) + (i & 3)];
+    const int r = c >= v ? lower_bound(sc, nup, c) : -1;
+    rk[i] = (short)r;
+    if (r >= 0) atomicAdd(&sp[r], ((x >> 1) & 1) != ((i & 3) >> 1) ? 0x10001 : 1);
+  }
+  __syncwarp();
+  int at = cb;
+  for (int r0 = 0; r0 < nup; r0 += 32) {
+    const int r = r0 + lane;
+    const int c = r < nup ? sp[r] : 0;
+    int x = c & 0xffff;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (r < nup) {
+      const int b = o + r, n_cross = c >> 16;
+      const int first = at + x - (c & 0xffff);
+      g.col[b] = sc[r];
+      g.brow[b] = v;
+      g.bptr[b] = first;
+      sp[r] = first;
+      if (g.bcodes) {
+        int terms[4];
+        sx[r] = side_terms(g, v, sc[r], n_cross, terms) ? 4 - n_cross : 4;
+        *reinterpret_cast<int4*>(g.bcodes + 4LL * b) = make_int4(terms[0], terms[1], terms[2], terms[3]);
+      }
+    }
+    at += __shfl_sync(0xffffffffu, x, 31);
+  }
+  __syncwarp();
+  for (int i0 = 0; i0 < nc; i0 += 32) {
+    const int i = i0 + lane;
+    const int r = i < nc ? rk[i] : -1;
+    const int x = i < nc ? inc[i >> 2] : 0;
+    const int code = (x << 2) | (i & 3);
+    const bool cross = r >= 0 && ((x >> 1) & 1) != ((i & 3) >> 1);
+    const unsigned same = __match_any_sync(0xffffffffu, r);
+    const unsigned crosses = __ballot_sync(0xffffffffu, cross) & same;
+    int k = 4;
+    if (r >= 0) {
+      g.contrib[sp[r] + __popc(same & below)] = code;
+      if (cross && g.bcodes) k = sx[r] + __popc(crosses & below);
+    }
+    if (k < 4) g.bcodes[4LL * (o + r) + k] = code;
+    __syncwarp();
+    if (r >= 0 && (same & below) == 0) {  // the first of its block moves the block on
+      sp[r] += __popc(same);
+      if (g.bcodes) sx[r] += __popc(crosses);
+    }
+    __syncwarp();
+  }
 }
 
 // Mesh node -> (element, local index, other node) lists, and member sides per element.
@@ -373,25 +615,6 @@ __global__ void k_segment_sort_pairs(const int32_t* __restrict__ ptr, long long 
     while (y >= lo && a[y].x > key.x) { a[y + 1] = a[y]; --y; }
     a[y + 1] = key;
   }
-}
-
-__global__ void k_elem_inc_count(xk_pairs p, const int32_t* __restrict__ members, int nm, int32_t* __restrict__ cnt) {
-  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  const int i = members[mi];
-  atomicAdd(&cnt[p.ea[i]], 1);
-  atomicAdd(&cnt[p.eb[i]], 1);
-}
-
-__global__ void k_elem_inc_fill(xk_pairs p, const int32_t* __restrict__ members, int nm,
-                                const int32_t* __restrict__ ptr, int32_t* __restrict__ fill,
-                                int32_t* __restrict__ inc) {
-  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  const int i = members[mi];
-  const int ea = p.ea[i], eb = p.eb[i];
-  inc[ptr[ea] + atomicAdd(&fill[ea], 1)] = mi << 1;
-  inc[ptr[eb] + atomicAdd(&fill[eb], 1)] = (mi << 1) | 1;
 }
 
 // One member record (16 values for combined records) through vector loads.
@@ -476,75 +699,6 @@ XK_D void add_contrib(const T* __restrict__ rec, int code, T* acc) {
   const T w = shape_c<T>(r[ST], r[ST + 1], k) * shape_c<T>(r[ST], r[ST + 1], l);
 #pragma unroll
   for (int q = 0; q < 9; ++q) acc[q] += w * r[BCOL + q];
-}
-
-// Inline term lists of the blocks (variant "sides").  k_side_codes writes the
-// same-side terms of every block (diagonal: S^pp of each element of the row
-// node; neighbour on an element: S^01) and the count; k_cross_codes appends
-// the cross codes of every member; k_sort_codes sorts each block's four slots.
-constexpr int SIDE_FLAG = (int)0x80000000;
-// An element's three sums S^00, S^01, S^11, each as 16 values: the 9 of the
-// sum, then 1, 1 in the places of a record's s, t and padding, so that a term
-// loads the same values from an element sum as from a combined record (both
-// 64-byte aligned) and the weight c_1 c_1 = s s of an element-sum term is 1.
-constexpr int SUM_STRIDE = 16;
-constexpr int ELEM_SUMS = 3 * SUM_STRIDE;
-
-__global__ void k_side_codes(long long nb, const int32_t* __restrict__ brow, const int32_t* __restrict__ col,
-                             const int32_t* __restrict__ neptr, const int2* __restrict__ ne,
-                             int32_t* __restrict__ codes, int32_t* __restrict__ cnt, int32_t* __restrict__ err) {
-  const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int i = brow[b], j = col[b];
-  int n = 0;
-  for (int y = neptr[i]; y < neptr[i + 1]; ++y) {
-    const int2 en = ne[y];
-    const int base = ELEM_SUMS * (en.x >> 1);
-    if (j == i) {
-      if (n < 4) codes[4 * b + n] = SIDE_FLAG | (base + ((en.x & 1) ? 2 * SUM_STRIDE : 0));
-      ++n;
-    }
-    if (j == en.y) {
-      if (n < 4) codes[4 * b + n] = SIDE_FLAG | (base + SUM_STRIDE);
-      ++n;
-    }
-  }
-  if (n > 4) atomicOr(err, 1);
-  cnt[b] = n;
-}
-
-__global__ void k_cross_codes(const int32_t* __restrict__ mnodes, int nm, const int32_t* __restrict__ rptr,
-                              const int32_t* __restrict__ col, int32_t* __restrict__ cnt,
-                              int32_t* __restrict__ codes, int32_t* __restrict__ err) {
-  const int mi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mi >= nm) return;
-  int nd[4];
-  for (int q = 0; q < 4; ++q) nd[q] = mnodes[4LL * mi + q];
-  for (int k = 0; k < 4; ++k)
-    for (int l = 0; l < 4; ++l) {
-      if ((k >> 1) == (l >> 1) || nd[k] > nd[l]) continue;
-      const int b = find_block(rptr, col, nd[k], nd[l]);
-      if (b >= rptr[nd[k] + 1] || col[b] != nd[l]) {
-        atomicOr(err, 2);
-        continue;
-      }
-      const int slot = atomicAdd(&cnt[b], 1);
-      if (slot < 4) codes[4LL * b + slot] = (mi << 4) | (k << 2) | l;
-      else atomicOr(err, 1);
-    }
-}
-
-__global__ void k_sort_codes(long long nb, int4* __restrict__ codes) {
-  const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  int4 c = codes[b];
-  int v[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-  for (int x = 1; x < 4; ++x)
-#pragma unroll
-    for (int y = x; y > 0; --y)
-      if (v[y - 1] > v[y]) { const int t = v[y]; v[y] = v[y - 1]; v[y - 1] = t; }
-  codes[b] = make_int4(v[0], v[1], v[2], v[3]);
 }
 
 // Variant "sides", step 1: S_e^00, S_e^01, S_e^11 (9 values each) of every
@@ -1120,12 +1274,6 @@ __global__ void __launch_bounds__(32 * GT_WARPS) k_gather_tangent(long long nnzb
   for (int i = lane; i < 9 * nblk; i += 32) K[9 * b0 + i] = A[i];
 }
 
-xk_status fetch_i64(const int64_t* dev, int64_t* host, int n, cudaStream_t st) {
-  XK_CUDA(cudaMemcpyAsync(host, dev, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st));
-  XK_CUDA(cudaStreamSynchronize(st));
-  return XK_OK;
-}
-
 }  // namespace
 
 extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* p, xk_contact_pattern* pat,
@@ -1133,158 +1281,123 @@ extern "C" xk_status xk_contact_pattern_build(const xk_mesh* m, const xk_pairs* 
   if (!m || !p || !pat) return xk_set_error(XK_ERR_ARG, "xk_contact_pattern_build: null argument");
   if (!pat->inc_ptr || !pat->row_ptr) return xk_set_error(XK_ERR_ARG, "xk_contact_pattern_build: row arrays missing");
   cudaStream_t st = (cudaStream_t)s;
-  const int nn = m->n_nodes;
+  const int nn = m->n_nodes, ne = m->n_elems;
   const long long np = p->n;
   pat->n_nodes = nn;
-  XkScratch S(st);
-  int32_t *flag, *mpos, *cnt, *fill, *err;
-  int64_t* tot;
-  const long long nmx = m->n_elems > nn ? m->n_elems : nn;
-  XK_TRY(S.reserve(8 * ((size_t)np + 1) + 8 * ((size_t)nn + 1) + 8 * ((size_t)nmx + 1) +
-                   12 * ((size_t)pat->cap_blocks + 1) + ((size_t)np + 4 * (size_t)nmx + (size_t)pat->cap_blocks) / 64 +
-                   (1 << 14)));
-  XK_TRY(S.get(&flag, np + 1));
-  XK_TRY(S.get(&mpos, np + 1));
-  XK_TRY(S.get(&cnt, nn + 1));
-  XK_TRY(S.get(&fill, nn + 1));
-  XK_TRY(S.get(&err, 1));
-  XK_TRY(S.get(&tot, 4));
-  // members and others
-  k_flags<<<xk_blocks(np + 1, 256), 256, 0, st>>>(*p, flag);
-  XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(flag, mpos, np + 1, tot, st, &S));
-  int64_t h[4] = {0, 0, 0, 0};
-  XK_TRY(fetch_i64(tot, h, 1, st));
-  const long long nm = h[0];
-  pat->n_members = (int32_t)nm;
-  pat->n_others = (int32_t)(np - nm);
-  if (nm > pat->cap_members || np - nm > pat->cap_others)
-    return xk_set_error(XK_ERR_CAPACITY, "xk_contact_pattern_build: member / other-pair capacity too small");
-  if (np > 0) k_split_lists<<<xk_blocks(np, 256), 256, 0, st>>>(*m, *p, mpos, pat->members, pat->member_nodes,
-                                                                 pat->others);
-  // node incidence of the members
-  XK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (nn + 1), st));
-  if (nm > 0) k_inc_count<<<xk_blocks(nm, 256), 256, 0, st>>>(pat->member_nodes, (int)nm, cnt);
-  XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(cnt, pat->inc_ptr, nn + 1, nullptr, st, &S));
-  XK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (nn + 1), st));
-  if (nm > 0) k_inc_fill<<<xk_blocks(nm, 256), 256, 0, st>>>(pat->member_nodes, (int)nm, pat->inc_ptr, fill, pat->inc);
-  k_segment_sort<<<xk_blocks(32LL * nn, SEG_T), SEG_T, 0, st>>>(pat->inc_ptr, nn, pat->inc);
-  // block pattern rows
-  XK_CUDA(cudaMemsetAsync(err, 0, sizeof(int32_t), st));
-  if (nn > 0)
-    k_row_cols<0><<<(unsigned)((nn + RC_WARPS - 1) / RC_WARPS), 32 * RC_WARPS, 0, st>>>(pat->member_nodes, pat->inc_ptr, pat->inc, nn, cnt, nullptr,
-                                                   nullptr, nullptr, err);
-  XK_CHECK_LAUNCH();
-  XK_CUDA(cudaMemsetAsync(cnt + nn, 0, sizeof(int32_t), st));
-  XK_TRY(xk_exclusive_scan_i32(cnt, pat->row_ptr, nn + 1, tot + 1, st, &S));
-  int32_t herr = 0;
-  XK_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  XK_TRY(fetch_i64(tot, h, 2, st));
-  if (herr) return xk_set_error(XK_ERR_OVERFLOW, "xk_contact_pattern_build: a node touches more than 256 contact nodes");
-  const long long nb = h[1];
-  pat->nnzb = nb;
-  if (nb > pat->cap_blocks) return xk_set_error(XK_ERR_CAPACITY, "xk_contact_pattern_build: block capacity too small");
-  if (nn > 0)
-    k_row_cols<1><<<(unsigned)((nn + RC_WARPS - 1) / RC_WARPS), 32 * RC_WARPS, 0, st>>>(pat->member_nodes, pat->inc_ptr, pat->inc, nn, nullptr,
-                                                   pat->row_ptr, pat->col, pat->blk_row, err);
-  XK_CHECK_LAUNCH();
-  // contributor lists of the blocks
-  int32_t *bcnt, *bfill;
-  XK_TRY(S.get(&bcnt, nb + 1));
-  XK_TRY(S.get(&bfill, nb + 1));
-  XK_CUDA(cudaMemsetAsync(bcnt, 0, sizeof(int32_t) * (nb + 1), st));
-  if (nm > 0) k_contrib<0><<<xk_blocks(nm, 128), 128, 0, st>>>(pat->member_nodes, (int)nm, pat->row_ptr, pat->col,
-                                                                bcnt, nullptr, nullptr, err);
-  XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(bcnt, pat->blk_ptr, nb + 1, tot + 2, st, &S));
-  XK_CUDA(cudaMemsetAsync(bfill, 0, sizeof(int32_t) * (nb + 1), st));
-  if (nm > 0) k_contrib<1><<<xk_blocks(nm, 128), 128, 0, st>>>(pat->member_nodes, (int)nm, pat->row_ptr, pat->col,
-                                                                bfill, pat->blk_ptr, pat->contrib, err);
-  if (nb > 0) {
-    int32_t *longs, *n_longs;
-    XK_TRY(S.get(&longs, nb));
-    XK_TRY(S.get(&n_longs, 1));
-    XK_CUDA(cudaMemsetAsync(n_longs, 0, sizeof(int32_t), st));
-    k_segment_sort_short<<<xk_blocks(nb, 256), 256, 0, st>>>(pat->blk_ptr, nb, pat->contrib, longs, n_longs);
-    k_segment_sort_listed<<<xk_sm_count() * 8, SEG_T, 0, st>>>(pat->blk_ptr, pat->contrib, longs, n_longs);
-  }
-  XK_CHECK_LAUNCH();
-  // lower index of the stored blocks
-  pat->nnzb_full = nb;
-  if (pat->low_ptr && pat->low_blk) {
-    XK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (nn + 1), st));
-    if (nb > 0) k_lower_index<0><<<xk_blocks(nb, 256), 256, 0, st>>>(nb, pat->blk_row, pat->col, cnt, nullptr, nullptr);
-    XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(cnt, pat->low_ptr, nn + 1, tot + 3, st, &S));
-    XK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (nn + 1), st));
-    if (nb > 0)
-      k_lower_index<1><<<xk_blocks(nb, 256), 256, 0, st>>>(nb, pat->blk_row, pat->col, fill, pat->low_ptr,
-                                                           pat->low_blk);
-    k_segment_sort<<<xk_blocks(32LL * nn, SEG_T), SEG_T, 0, st>>>(pat->low_ptr, nn, pat->low_blk);
-    XK_CHECK_LAUNCH();
-  }
-  // the contribution and lower-index totals are read with the final synchronisation
-  // element-side form (gather variant XK_GATHER_SIDES)
-  const bool sides = pat->node_elem_ptr && pat->node_elem && pat->elem_ptr && pat->elem_inc && pat->bcodes;
-  int32_t herr2 = 0;
-  const int ne = m->n_elems;
   pat->n_elems = ne;
   pat->sides_ok = 0;
-  if (sides) {
-    int32_t *ecnt, *efill, *serr;
-    XK_TRY(S.get(&ecnt, (long long)(ne > nn ? ne : nn) + 1));
-    XK_TRY(S.get(&efill, (long long)(ne > nn ? ne : nn) + 1));
-    XK_TRY(S.get(&serr, 1));
-    // mesh node -> elements (mesh topology: built once per pattern and mesh)
-    if (!pat->node_elem_ready) {
-      XK_CUDA(cudaMemsetAsync(ecnt, 0, sizeof(int32_t) * (nn + 1), st));
-      if (ne > 0) k_node_elem_count<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, ecnt);
-      XK_CHECK_LAUNCH();
-      XK_TRY(xk_exclusive_scan_i32(ecnt, pat->node_elem_ptr, nn + 1, nullptr, st, &S));
-      XK_CUDA(cudaMemsetAsync(efill, 0, sizeof(int32_t) * (nn + 1), st));
-      if (ne > 0)
-        k_node_elem_fill<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, pat->node_elem_ptr, efill,
-                                                             reinterpret_cast<int2*>(pat->node_elem));
-      k_segment_sort_pairs<<<xk_blocks(nn, 128), 128, 0, st>>>(pat->node_elem_ptr, nn,
-                                                               reinterpret_cast<int2*>(pat->node_elem));
-      XK_CHECK_LAUNCH();
-    }
-    // element -> member sides
-    XK_CUDA(cudaMemsetAsync(ecnt, 0, sizeof(int32_t) * (ne + 1), st));
-    if (nm > 0) k_elem_inc_count<<<xk_blocks(nm, 256), 256, 0, st>>>(*p, pat->members, (int)nm, ecnt);
-    XK_CHECK_LAUNCH();
-    XK_TRY(xk_exclusive_scan_i32(ecnt, pat->elem_ptr, ne + 1, nullptr, st, &S));
-    XK_CUDA(cudaMemsetAsync(efill, 0, sizeof(int32_t) * (ne + 1), st));
-    if (nm > 0)
-      k_elem_inc_fill<<<xk_blocks(nm, 256), 256, 0, st>>>(*p, pat->members, (int)nm, pat->elem_ptr, efill,
-                                                          pat->elem_inc);
-    if (ne > 0) k_segment_sort<<<xk_blocks(32LL * ne, SEG_T), SEG_T, 0, st>>>(pat->elem_ptr, ne, pat->elem_inc);
-    XK_CHECK_LAUNCH();
-    // inline term lists; a flag in serr (more than four terms somewhere) only disables the variant
-    XK_CUDA(cudaMemsetAsync(serr, 0, sizeof(int32_t), st));
-    XK_CUDA(cudaMemsetAsync(pat->bcodes, 0xff, sizeof(int32_t) * 4 * (nb > 0 ? nb : 1), st));
-    if (nb > 0)
-      k_side_codes<<<xk_blocks(nb, 256), 256, 0, st>>>(nb, pat->blk_row, pat->col, pat->node_elem_ptr,
-                                                       reinterpret_cast<const int2*>(pat->node_elem), pat->bcodes,
-                                                       bcnt, serr);
-    if (nm > 0)
-      k_cross_codes<<<xk_blocks(nm, 128), 128, 0, st>>>(pat->member_nodes, (int)nm, pat->row_ptr, pat->col, bcnt,
-                                                        pat->bcodes, serr);
-    if (nb > 0) k_sort_codes<<<xk_blocks(nb, 256), 256, 0, st>>>(nb, reinterpret_cast<int4*>(pat->bcodes));
-    XK_CHECK_LAUNCH();
-    XK_CUDA(cudaMemcpyAsync(&herr2, serr, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  const bool sides = pat->node_elem_ptr && pat->node_elem && pat->elem_ptr && pat->elem_inc && pat->bcodes;
+  const bool lower = pat->low_ptr && pat->low_blk;
+  const long long nmx = np < pat->cap_members ? np : pat->cap_members;  // members this build can hold
+  const long long longest = (ne > nn ? ne : nn) + 1;
+  // one piece that starts at zero: the counts and the scans' words
+  const long long w_mem = scan_words(np, 1), w_el = scan_words(longest, 2), w_row = scan_words(nn + 1, 2);
+  const long long n_sums = scan_sums(np, 1) + scan_sums(longest, 2) + scan_sums(nn + 1, 2);
+  const size_t zero = sizeof(Totals) + sizeof(int32_t) * (size_t)(2 + w_mem + w_el + w_row + ne + 1);
+  XkScratch S(st);
+  XK_TRY(S.reserve(zero + 4 * ((size_t)(sides ? 0 : 2 * (nn + 1) + 4 * (size_t)ne + ne + 1) + 18 * (size_t)nmx +
+                               4 * ((size_t)nn + 1) + 2 * (size_t)n_sums) + (1 << 14)));
+  char* z;
+  int64_t* sums;
+  PatternArgs g = {};
+  XK_TRY(S.get(&z, (long long)zero));
+  XK_TRY(S.get(&sums, n_sums));
+  int32_t *raw, *cbase;
+  XK_TRY(S.get(&raw, 2 * nmx));
+  XK_TRY(S.get(&g.list, 16 * nmx));
+  XK_TRY(S.get(&g.rcnt, nn));
+  XK_TRY(S.get(&g.ccnt, nn));
+  XK_TRY(S.get(&g.lcnt, nn));
+  XK_TRY(S.get(&cbase, nn + 1));
+  int32_t *neptr = pat->node_elem_ptr, *nelem = pat->node_elem, *eptr = pat->elem_ptr;
+  if (!sides) {  // the mesh topology of this call only
+    XK_TRY(S.get(&neptr, nn + 1));
+    XK_TRY(S.get(&nelem, 4 * (long long)ne));
+    XK_TRY(S.get(&eptr, ne + 1));
   }
-  XK_CUDA(cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  XK_CUDA(cudaMemcpyAsync(h + 2, tot + 2, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  XK_CUDA(cudaMemsetAsync(z, 0, zero, st));
+  Totals* tot = reinterpret_cast<Totals*>(z);
+  int32_t* err = reinterpret_cast<int32_t*>(z + sizeof(Totals));  // err, then serr
+  int* words = err + 2;
+  int32_t* ecnt = words + w_mem + w_el + w_row;
+  // mesh node -> elements (mesh topology: built once per pattern and mesh)
+  if (!sides || !pat->node_elem_ready) {
+    int32_t *cnt, *fill;
+    XK_TRY(S.get(&cnt, nn + 1));
+    XK_TRY(S.get(&fill, nn + 1));
+    XK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (nn + 1), st));
+    XK_CUDA(cudaMemsetAsync(fill, 0, sizeof(int32_t) * (nn + 1), st));
+    if (ne > 0) k_node_elem_count<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, cnt);
+    XK_CHECK_LAUNCH();
+    XK_TRY(xk_exclusive_scan_i32(cnt, neptr, nn + 1, nullptr, st, &S));
+    if (ne > 0) k_node_elem_fill<<<xk_blocks(ne, 256), 256, 0, st>>>(*m, neptr, fill, reinterpret_cast<int2*>(nelem));
+    k_segment_sort_pairs<<<xk_blocks(nn, 128), 128, 0, st>>>(neptr, nn, reinterpret_cast<int2*>(nelem));
+    XK_CHECK_LAUNCH();
+  }
+  const int2* node_elem = reinterpret_cast<const int2*>(nelem);
+  // members and others
+  if (np > 0) {
+    auto on = [](const void* q, uintptr_t bytes) { return ((uintptr_t)q & (bytes - 1)) == 0; };
+    const MemberScan op = {*m, *p, pat->cap_members, pat->cap_others, pat->members, pat->member_nodes, pat->others,
+                           ecnt, tot, on(p->status, 8) && on(p->p_n, 16) && on(pat->member_nodes, 16)};
+    XK_TRY(scan_launch(op, np, 1, sums, words, st));
+  }
+  // member sides per element, incidences per node
+  XK_TRY(scan_launch(ElemScan{nn, ne, ecnt, neptr, node_elem, eptr, pat->inc_ptr}, longest, 2,
+                     sums + scan_sums(np, 1), words + w_mem, st));
+  if (nmx > 0) k_pat_sides<<<xk_blocks(nmx, 256), 256, 0, st>>>(*p, pat->members, tot, pat->cap_members, eptr, ecnt, raw);
+  XK_CHECK_LAUNCH();
+  g.nn = nn;
+  g.ne = ne;
+  g.cap = pat->cap_members;
+  g.cap_blocks = pat->cap_blocks;
+  g.tot = tot;
+  g.mnodes = pat->member_nodes;
+  g.neptr = neptr;
+  g.eptr = eptr;
+  g.iptr = pat->inc_ptr;
+  g.raw = raw;
+  g.nelem = node_elem;
+  g.inc = pat->inc;
+  g.einc = sides ? pat->elem_inc : nullptr;
+  g.err = err;
+  g.serr = err + 1;
+  g.rptr = pat->row_ptr;
+  g.cbase = cbase;
+  g.lptr = lower ? pat->low_ptr : nullptr;
+  g.col = pat->col;
+  g.brow = pat->blk_row;
+  g.bptr = pat->blk_ptr;
+  g.contrib = pat->contrib;
+  g.lblk = lower ? pat->low_blk : nullptr;
+  g.bcodes = sides ? pat->bcodes : nullptr;
+  const long long warps = (long long)nn + (sides ? ne : 0);
+  if (warps > 0) k_pat_cols<<<xk_blocks(warps, RC_WARPS), 32 * RC_WARPS, 0, st>>>(g);
+  XK_CHECK_LAUNCH();
+  // rows
+  XK_TRY(scan_launch(RowScan{nn, g.rcnt, g.ccnt, g.lcnt, pat->row_ptr, cbase, lower ? pat->low_ptr : nullptr, tot},
+                     nn + 1, 2, sums + scan_sums(np, 1) + scan_sums(longest, 2), words + w_mem + w_el, st));
+  if (nn > 0) k_pat_rows<<<xk_blocks(nn, PR_WARPS), 32 * PR_WARPS, 0, st>>>(g);
+  else XK_CUDA(cudaMemsetAsync(pat->blk_ptr, 0, sizeof(int32_t), st));
+  XK_CHECK_LAUNCH();
+  struct {
+    Totals t;
+    int32_t err, serr;
+  } h;
+  XK_CUDA(cudaMemcpyAsync(&h, z, sizeof(h), cudaMemcpyDeviceToHost, st));
   XK_CUDA(cudaStreamSynchronize(st));
-  pat->n_contrib = h[2];
-  if (pat->low_ptr && pat->low_blk) pat->nnzb_full = nb + h[3];
-  if (sides) {
-    pat->sides_ok = herr2 ? 0 : 1;
-    pat->node_elem_ready = 1;
-  }
-  if (herr) return xk_set_error(XK_ERR_OVERFLOW, "xk_contact_pattern_build: inconsistent block pattern");
+  pat->n_members = (int32_t)h.t.members;
+  pat->n_others = (int32_t)(np - h.t.members);
+  if (sides) pat->node_elem_ready = 1;
+  if (h.t.members > pat->cap_members || np - h.t.members > pat->cap_others)
+    return xk_set_error(XK_ERR_CAPACITY, "xk_contact_pattern_build: member / other-pair capacity too small");
+  if (h.err) return xk_set_error(XK_ERR_OVERFLOW, "xk_contact_pattern_build: a node touches more than 256 contact nodes");
+  pat->nnzb = h.t.blocks;
+  if (h.t.blocks > pat->cap_blocks)
+    return xk_set_error(XK_ERR_CAPACITY, "xk_contact_pattern_build: block capacity too small");
+  pat->n_contrib = h.t.contribs;
+  pat->nnzb_full = h.t.blocks + (lower ? h.t.low : 0);
+  pat->sides_ok = sides && !h.serr ? 1 : 0;
   return XK_OK;
 }
 
