@@ -51,7 +51,7 @@ XK_D bool is_member(const xk_pairs& p, long long i) {
 // The incidences of a node are sorted, so a row that places its contributions in that order emits every block's
 // list sorted: no list is sorted after it is filled, and none is filled through atomics.  Before, lists were
 // counted, scanned, filled and sorted one after another (30 launches, three waits).  GB300, a detection from the
-// same state: 37 wires 630 -> 434 us, 397 wires 1190 -> 957, 1027 wires 2330 -> 2065.
+// same state: 37 wires 630 -> 434 us, 397 wires 1190 -> 885, 1027 wires 2330 -> 1752.
 // ---------------------------------------------------------------------------------------------------------------
 
 struct Totals {
@@ -192,56 +192,52 @@ struct RowScan {
   }
 };
 
-// Ascending sort of a warp's n <= 64 distinct values, two per lane: each finds its rank by comparing against all
-// others broadcast by shuffles and goes to that place.
-XK_D void warp_rank_sort(int v0, int v1, int n, int32_t* out, int lane) {
-  int r0 = 0, r1 = 0;
-  const int n0 = n < 32 ? n : 32;
-  for (int k = 0; k < n0; ++k) {
-    const int x = __shfl_sync(0xffffffffu, v0, k);
-    r0 += x < v0;
-    r1 += x < v1;
-  }
-  for (int k = 0; k < n - 32; ++k) {
-    const int x = __shfl_sync(0xffffffffu, v1, k);
-    r0 += x < v0;
-    r1 += x < v1;
-  }
-  if (lane < n) out[r0] = v0;
-  if (lane + 32 < n) out[r1] = v1;
-}
-
-// Bitonic sort of l[0, n) in shared memory; l has room for the next power of two.
-XK_D void warp_bitonic_sort(int* l, int n, int lane) {
-  int N = 32;
-  while (N < n) N <<= 1;
-  for (int i = n + lane; i < N; i += 32) l[i] = 0x7fffffff;
-  __syncwarp();
-  for (int k = 2; k <= N; k <<= 1)
+// Bitonic sort of 32 K values, value 32 r + lane in v[r]: partners less than 32 apart by shuffle, the others in
+// the lane's own registers.
+template <int K>
+XK_D void warp_sort_regs(int (&v)[K], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * K; k <<= 1)
+#pragma unroll
     for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < N; i += 32) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const int p = l[i], q = l[ixj];
-          if (((i & k) == 0) == (p > q)) {
-            l[i] = q;
-            l[ixj] = p;
-          }
+      if (j >= 32) {
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+          if (r & (j >> 5)) continue;
+          const int q = r | (j >> 5), x = min(v[r], v[q]), y = max(v[r], v[q]);
+          v[r] = (r & (k >> 5)) ? y : x;
+          v[q] = (r & (k >> 5)) ? x : y;
         }
+        continue;
       }
-      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        const int o = __shfl_xor_sync(0xffffffffu, v[r], j);
+        const bool up = k >= 32 ? (r & (k >> 5)) == 0 : (lane & k) == 0;
+        v[r] = up == ((lane & j) == 0) ? min(v[r], o) : max(v[r], o);
+      }
     }
 }
 
-// The n values of l (shared memory, n <= RC_CAP) in ascending order to out.
-constexpr int RC_WARPS = 4, RC_CAP = 512, RC_TAB = 2 * RC_CAP;
-XK_D void warp_sort_shared(int* l, int n, int32_t* out, int lane) {
-  if (n <= 64) {
-    warp_rank_sort(lane < n ? l[lane] : 0x7fffffff, lane + 32 < n ? l[lane + 32] : 0x7fffffff, n, out, lane);
-    return;
-  }
-  warp_bitonic_sort(l, n, lane);
-  for (int i = lane; i < n; i += 32) out[i] = l[i];
+template <int K>
+XK_D void warp_sort_k(const int* l, int n, int32_t* out, int lane) {
+  int v[K];
+#pragma unroll
+  for (int r = 0; r < K; ++r) v[r] = 32 * r + lane < n ? l[32 * r + lane] : 0x7fffffff;
+  __syncwarp();  // out may be l
+  warp_sort_regs<K>(v, lane);
+#pragma unroll
+  for (int r = 0; r < K; ++r)
+    if (32 * r + lane < n) out[32 * r + lane] = v[r];
+}
+
+// The n <= WS_CAP values of l (shared memory) in ascending order to out.
+constexpr int WS_CAP = 256;
+__device__ __noinline__ void warp_sort(const int* l, int n, int32_t* out, int lane) {
+  if (n <= 32) warp_sort_k<1>(l, n, out, lane);
+  else if (n <= 64) warp_sort_k<2>(l, n, out, lane);
+  else if (n <= 128) warp_sort_k<4>(l, n, out, lane);
+  else warp_sort_k<8>(l, n, out, lane);
 }
 
 XK_D void serial_insertion_sort(int32_t* a, int n) {
@@ -267,12 +263,14 @@ __global__ void k_pat_sides(xk_pairs p, const int32_t* __restrict__ members, con
 }
 
 // A warp per node, then a warp per element.  A node's incidences are its elements' member sides; its neighbours (the
-// nodes of every member touching it) are its own elements' nodes and each incidence's partner nodes, so one 8-byte
-// load per incidence and one insertion per partner node into an open-addressing hash set in shared memory (twice
-// the candidates' power of two, linear probing, atomicCAS among the warp's lanes) find them.  The sorted neighbours
-// stay in list + 4 inc_ptr[v] for k_pat_rows.  A node with more than RC_CAP candidates takes the serial path of one
-// lane; as in the reference's sizes a row there holds at most MAX_COLS columns (err otherwise).
-constexpr int MAX_COLS = 256;
+// nodes of every member touching it) are its own elements' nodes and each incidence's partner nodes: up to WS_CAP
+// such candidates are sorted in the warp's registers and stand next to their repeats.  The sorted neighbours stay in
+// list + 4 inc_ptr[v] for k_pat_rows.  A node with more takes the serial path of one lane; one with more than
+// MAX_INC incidences holds at most MAX_COLS columns in its row (err otherwise).
+// Bound by the instructions issued.  A hash set in shared memory, its ranking by n comparisons per value and the
+// same ranking of the incidences took 1500 instructions a warp and 348 us at 99.6k nodes with 30 incidences and 55
+// neighbours each; the register sorts take 107 us.
+constexpr int RC_WARPS = 4, MAX_INC = 128, MAX_COLS = 256;
 struct PatternArgs {
   int nn, ne;
   long long cap, cap_blocks;
@@ -287,21 +285,22 @@ struct PatternArgs {
 };
 
 __global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constant__ PatternArgs g) {
-  __shared__ int stab[RC_WARPS][RC_TAB];
-  __shared__ int slist[RC_WARPS][RC_CAP];
+  __shared__ int s_inc[RC_WARPS][MAX_INC];
+  __shared__ int s_cand[RC_WARPS][WS_CAP];
   if (g.tot->members > g.cap) return;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  int* l = slist[wid];
+  int* l = s_inc[wid];
+  int* cand = s_cand[wid];
   const long long w = (long long)blockIdx.x * RC_WARPS + wid;
   if (w >= g.nn) {  // an element
     const long long e = w - g.nn;
     if (e >= g.ne || !g.einc) return;
     const int o = g.eptr[e], n = g.eptr[e + 1] - o;
-    if (n <= RC_CAP) {
-      for (int i = lane; i < n; i += 32) l[i] = g.raw[o + i];
+    if (n <= WS_CAP) {
+      for (int i = lane; i < n; i += 32) cand[i] = g.raw[o + i];
       __syncwarp();
-      warp_sort_shared(l, n, g.einc + o, lane);
+      warp_sort(cand, n, g.einc + o, lane);
     } else if (lane == 0) {
       for (int i = 0; i < n; ++i) g.einc[o + i] = g.raw[o + i];
       serial_insertion_sort(g.einc + o, n);
@@ -317,7 +316,7 @@ __global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constan
   const int y0 = g.neptr[v], y1 = g.neptr[v + 1];
   int32_t* inc = g.inc + x0;
   int32_t* out = g.list + 4LL * x0;
-  if (4 * n > RC_CAP) {
+  if (n > MAX_INC || 2 * n + (y1 - y0) + 1 > WS_CAP) {
     if (lane != 0) return;
     int q = 0;
     for (int y = y0; y < y1; ++y) {
@@ -339,7 +338,7 @@ __global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constan
         ++nd;
         low += c < v;
       }
-    if (nd - low > MAX_COLS) atomicOr(g.err, 1);
+    if (n > MAX_INC && nd - low > MAX_COLS) atomicOr(g.err, 1);
     g.rcnt[v] = nd - low;
     g.ccnt[v] = nc;
     g.lcnt[v] = low;
@@ -356,51 +355,40 @@ __global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constan
     }
     q += m;
   }
-  int* t = stab[wid];
-  constexpr int EMPTY = -1;
-  int ts = 64;
-  while (ts < 4 * n + 4 * (y1 - y0) && ts < RC_TAB) ts <<= 1;
-  for (int i = lane; i < ts; i += 32) t[i] = EMPTY;
   __syncwarp();
-  auto insert = [&](int c) {
-    unsigned h = ((unsigned)c * 2654435761u) & (unsigned)(ts - 1);
-    while (true) {
-      const int o = atomicCAS(&t[h], EMPTY, c);
-      if (o == EMPTY || o == c) break;
-      h = (h + 1) & (unsigned)(ts - 1);
-    }
-  };
-  int nc = 0;  // contributions to the row: candidates >= v
+  int nc = 0;  // contributions to the row: the members' nodes >= v
   for (int i = lane; i < n; i += 32) {
     const int x = l[i];
     const int32_t* nd = g.mnodes + 4LL * (x >> 2) + ((x & 2) ? 0 : 2);
     const int a = nd[0], b = nd[1];
     nc += (a >= v) + (b >= v);
-    insert(a);
-    insert(b);
+    cand[2 * i] = a;
+    cand[2 * i + 1] = b;
   }
   for (int y = y0 + lane; y < y1; y += 32) {
     const int2 en = g.nelem[y];
     const int m = g.eptr[(en.x >> 1) + 1] - g.eptr[en.x >> 1];
     nc += m * (1 + (en.y >= v));
-    if (m > 0) insert(en.y);
+    cand[2 * n + y - y0] = m > 0 ? en.y : v;
   }
-  if (lane == 0) insert(v);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) nc += __shfl_xor_sync(0xffffffffu, nc, o);
+  q = 2 * n + (y1 - y0);
+  if (lane == 0) cand[q] = v;
+  ++q;
+  nc = __reduce_add_sync(0xffffffffu, nc);
   __syncwarp();
-  warp_sort_shared(l, n, inc, lane);
+  warp_sort(l, n, inc, lane);
+  warp_sort(cand, q, cand, lane);
   __syncwarp();
   int nd = 0, low = 0;
-  for (int i0 = 0; i0 < ts; i0 += 32) {
-    const int x = t[i0 + lane];
-    const unsigned bal = __ballot_sync(0xffffffffu, x != EMPTY);
-    if (x != EMPTY) l[nd + __popc(bal & below)] = x;
+  for (int i0 = 0; i0 < q; i0 += 32) {
+    const int i = i0 + lane;
+    const int x = i < q ? cand[i] : 0;
+    const bool first = i < q && (i == 0 || cand[i - 1] != x);
+    const unsigned bal = __ballot_sync(0xffffffffu, first);
+    if (first) out[nd + __popc(bal & below)] = x;
     nd += __popc(bal);
-    low += __popc(__ballot_sync(0xffffffffu, x != EMPTY && x < v));
+    low += __popc(__ballot_sync(0xffffffffu, first && x < v));
   }
-  __syncwarp();
-  warp_sort_shared(l, nd, out, lane);
   if (lane == 0) {
     g.rcnt[v] = nd - low;
     g.ccnt[v] = nc;
@@ -408,12 +396,26 @@ __global__ void __launch_bounds__(32 * RC_WARPS) k_pat_cols(const __grid_constan
   }
 }
 
-// First place in a[0, n) not below c.
-XK_D int lower_bound(const int32_t* a, int n, int c) {
+// First place in a[0, n) not below c, three probes in flight at a time: a step is one latency of the list's memory.
+XK_D int lower_bound4(const int32_t* a, int n, int c) {
   int lo = 0;
-  while (lo < n) {
-    const int mid = (lo + n) >> 1;
-    if (a[mid] < c) lo = mid + 1; else n = mid;
+  while (n > 0) {
+    const int h = n >> 1, q = h >> 1, t = h + 1 + ((n - h - 1) >> 1);  // q <= h < t; t == n at the end of a short range
+    const int x = a[lo + q], y = a[lo + h], z = a[lo + (t < n ? t : h)];
+    if (y < c) {
+      if (t < n && z < c) {
+        lo += t + 1;
+        n -= t + 1;
+      } else {
+        lo += h + 1;
+        n = t - h - 1;
+      }
+    } else if (x < c) {
+      lo += q + 1;
+      n = h - q - 1;
+    } else {
+      n = q;
+    }
   }
   return lo;
 }
@@ -427,70 +429,69 @@ constexpr int SIDE_FLAG = (int)0x80000000;
 constexpr int SUM_STRIDE = 16;
 constexpr int ELEM_SUMS = 3 * SUM_STRIDE;
 
-// The terms of block (v, c), ascending: the sums of v's elements (diagonal: S^pp of each; a neighbour on an element:
-// S^01), empty places, then room for the block's n_cross cross codes.  False when more than four (the variant is
-// then off).
-XK_D bool side_terms(const PatternArgs& g, int v, int c, int n_cross, int* terms) {
+// code into its place among the n terms of a block (ascending; past four it only counts).
+XK_D void add_term(int (&terms)[4], int& n, int code) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) terms[k] = -1;
-  int n = 0;
-  auto add = [&](int code) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {  // into its place (no array index at run time)
-      if (k > n) continue;
-      if (k == n || code < terms[k]) {
-        const int t = terms[k];
-        terms[k] = code;
-        code = t;
-      }
+  for (int k = 0; k < 4; ++k) {  // no array index at run time
+    if (k <= n && (k == n || code < terms[k])) {
+      const int t = terms[k];
+      terms[k] = code;
+      code = t;
     }
-    ++n;
-  };
-  for (int y = g.neptr[v]; y < g.neptr[v + 1]; ++y) {
-    const int2 en = g.nelem[y];
-    const int base = ELEM_SUMS * (en.x >> 1);
-    if (c == v) add(SIDE_FLAG | (base + ((en.x & 1) ? 2 * SUM_STRIDE : 0)));
-    if (c == en.y) add(SIDE_FLAG | (base + SUM_STRIDE));
   }
-  if (n + n_cross <= 4) return true;
-  atomicOr(g.serr, 1);
-  return false;
+  ++n;
+}
+
+// The same-side terms of block (v, c) from one of v's elements: its S^pp on the diagonal, S^01 to its other node.
+XK_D void side_terms(int2 en, int v, int c, int (&terms)[4], int& n) {
+  const int base = SIDE_FLAG | (ELEM_SUMS * (en.x >> 1));
+  const bool other = c == en.y;
+  if (c == v) {
+    add_term(terms, n, base + ((en.x & 1) ? 2 * SUM_STRIDE : 0));
+    if (other) add_term(terms, n, base + SUM_STRIDE);
+  } else if (other) {
+    add_term(terms, n, base + SUM_STRIDE);
+  }
 }
 
 // A warp per node: its row's columns, each block's contributor and term lists, its lower index.  Contributions are
 // taken in the incidences' order, 32 at a time, and each goes behind the ones before it in its block (match over
 // the warp, a running position per block in shared memory), so the lists come out sorted.
-constexpr int PR_WARPS = 4;
-__global__ void __launch_bounds__(32 * PR_WARPS) k_pat_rows(const __grid_constant__ PatternArgs g) {
-  __shared__ int s_col[PR_WARPS][RC_CAP];
-  __shared__ int s_pos[PR_WARPS][RC_CAP];    // next contribution of a block
-  __shared__ int s_cross[PR_WARPS][RC_CAP];  // next cross term
-  __shared__ short s_rank[PR_WARPS][RC_CAP];
-  if (g.tot->members > g.cap || g.tot->blocks > g.cap_blocks) return;
+// Bound by latency: a warp's chain of dependent loads.  So the first 32 incidences, neighbours and elements are asked
+// for together, then what hangs on them, before anything is searched; the lower index searches with three probes in
+// flight.  282 -> 214 us at 99.6k nodes with 28 blocks a row, against the same kernel without that order and with a
+// search per contribution.  A mask of the incidences per block in place of the match took more instructions: 242 us.
+constexpr int PR_WARPS = 4, PR_CAP = 512;  // contributions of a row (4 per incidence), columns padded to a power of two
+__global__ void __launch_bounds__(32 * PR_WARPS, 8) k_pat_rows(const __grid_constant__ PatternArgs g) {
+  __shared__ int s_col[PR_WARPS][PR_CAP];
+  __shared__ int s_pos[PR_WARPS][PR_CAP];            // next contribution of a block
+  __shared__ int s_inc[PR_WARPS][PR_CAP / 4];
+  __shared__ signed char s_cross[PR_WARPS][PR_CAP];  // next cross term
+  __shared__ __align__(8) short s_rank[PR_WARPS][PR_CAP];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int v = blockIdx.x * PR_WARPS + wid;
-  if (v >= g.nn) return;
+  if (g.tot->members > g.cap || g.tot->blocks > g.cap_blocks || v >= g.nn) return;
   const int o = g.rptr[v], nup = g.rptr[v + 1] - o;
+  const int x0 = g.iptr[v], n = g.iptr[v + 1] - x0;
+  const int low = g.lcnt[v], cb = g.cbase[v], lo = g.lblk ? g.lptr[v] : 0;
+  const int y0 = g.neptr[v], ny = g.neptr[v + 1] - y0;
   if (v == g.nn - 1 && lane == 0) g.bptr[o + nup] = g.cbase[g.nn];
-  const int x0 = g.iptr[v], nc = 4 * (g.iptr[v + 1] - x0);
-  if (nc == 0) return;
-  const int low = g.lcnt[v], cb = g.cbase[v];
+  if (n == 0) return;
+  const int nc = 4 * n;
   const int32_t* list = g.list + 4LL * x0;
-  if (g.lblk) {
-    const int lo = g.lptr[v];
-    for (int i = lane; i < low; i += 32) {
-      const int c = list[i];
-      const int rc = g.rptr[c];
-      g.lblk[lo + i] = rc + lower_bound(g.list + 4LL * g.iptr[c] + g.lcnt[c], g.rptr[c + 1] - rc, v);
-    }
-  }
-  list += low;
   const int32_t* inc = g.inc + x0;
-  if (nc > RC_CAP) {  // a block at a time, its contributions collected from all candidates
+  const bool fast = nc <= PR_CAP && nup < PR_CAP;
+  // the first of each, then the lower neighbours' rows
+  int x = lane < n ? inc[lane] : 0;
+  int lc = lane < low ? list[lane] : 0;
+  const int up = lane < nup ? list[low + lane] : 0x7fffffff;
+  int2 en = lane < ny ? g.nelem[y0 + lane] : make_int2(0, -1);
+  const int l0 = g.rptr[lc], l1 = g.rptr[lc + 1], li = g.iptr[lc], ll = g.lcnt[lc];
+  if (!fast) {  // a block at a time, its contributions collected from all candidates
     int at = cb;
     for (int r = 0; r < nup; ++r) {
-      const int c = list[r];
+      const int c = list[low + r];
       const int b = o + r;
       if (lane == 0) {
         g.col[b] = c;
@@ -500,90 +501,128 @@ __global__ void __launch_bounds__(32 * PR_WARPS) k_pat_rows(const __grid_constan
       int n_cross = 0;
       for (int i0 = 0; i0 < nc; i0 += 32) {
         const int i = i0 + lane;
-        const int x = i < nc ? inc[i >> 2] : 0;
-        const bool hit = i < nc && g.mnodes[4LL * (x >> 2) + (i & 3)] == c;
-        const bool cross = hit && ((x >> 1) & 1) != ((i & 3) >> 1);
+        const int y = i < nc ? inc[i >> 2] : 0;
+        const bool hit = i < nc && g.mnodes[4LL * (y >> 2) + (i & 3)] == c;
+        const bool cross = hit && ((y >> 1) & 1) != ((i & 3) >> 1);
         const unsigned bh = __ballot_sync(0xffffffffu, hit), bc = __ballot_sync(0xffffffffu, cross);
-        if (hit) g.contrib[at + __popc(bh & below)] = (x << 2) | (i & 3);
+        if (hit) g.contrib[at + __popc(bh & below)] = (y << 2) | (i & 3);
         const int k = n_cross + __popc(bc & below);
-        if (cross && k < 4) s_cross[wid][k] = (x << 2) | (i & 3);
+        if (cross && k < 4) s_col[wid][k] = (y << 2) | (i & 3);
         at += __popc(bh);
         n_cross += __popc(bc);
       }
       __syncwarp();
       if (g.bcodes && lane == 0) {
-        int terms[4];
-        if (side_terms(g, v, c, n_cross, terms))
-          for (int k = 0; k < n_cross; ++k) terms[4 - n_cross + k] = s_cross[wid][k];
+        int terms[4] = {-1, -1, -1, -1}, nt = 0;
+        for (int y = 0; y < ny; ++y) side_terms(g.nelem[y0 + y], v, c, terms, nt);
+        if (nt + n_cross > 4) atomicOr(g.serr, 1);
+        else
+          for (int k = 0; k < n_cross; ++k) terms[4 - n_cross + k] = s_col[wid][k];
         *reinterpret_cast<int4*>(g.bcodes + 4LL * b) = make_int4(terms[0], terms[1], terms[2], terms[3]);
       }
       __syncwarp();
     }
-    return;
-  }
-  int* sc = s_col[wid];
-  int* sp = s_pos[wid];
-  int* sx = s_cross[wid];
-  short* rk = s_rank[wid];
-  for (int r = lane; r < nup; r += 32) {
-    sc[r] = list[r];
-    sp[r] = 0;
-  }
-  __syncwarp();
-  for (int i = lane; i < nc; i += 32) {  // counts per block: all contributions, cross ones in the upper half
-    const int x = inc[i >> 2];
-    const int c = g.mnodes[4LL * (x >> 2) + (i & 3)];
-    const int r = c >= v ? lower_bound(sc, nup, c) : -1;
-    rk[i] = (short)r;
-    if (r >= 0) atomicAdd(&sp[r], ((x >> 1) & 1) != ((i & 3) >> 1) ? 0x10001 : 1);
-  }
-  __syncwarp();
-  int at = cb;
-  for (int r0 = 0; r0 < nup; r0 += 32) {
-    const int r = r0 + lane;
-    const int c = r < nup ? sp[r] : 0;
-    int x = c & 0xffff;
+  } else {
+    int* sc = s_col[wid];
+    int* sp = s_pos[wid];
+    int* sn = s_inc[wid];
+    signed char* sx = s_cross[wid];
+    short* rk = s_rank[wid];
+    int top = 1;
+    while (top <= nup) top <<= 1;  // the columns, padded to a power of two above their number
+    for (int r = lane; r < top; r += 32) {
+      sc[r] = r < 32 ? up : (r < nup ? list[low + r] : 0x7fffffff);
+      sp[r] = 0;
+    }
+    __syncwarp();
+    // the block of each contribution and the counts per block, cross ones in the upper half; v is column 0
+    for (int j = lane; j < n; j += 32) {
+      if (j >= 32) x = inc[j];
+      sn[j] = x;
+      const int k = x & 3;
+      const int32_t* nd = g.mnodes + 4LL * (x >> 2);
+      const int c[3] = {nd[k ^ 1], nd[(k & 2) ^ 2], nd[(k & 2) ^ 3]};
+      int r[3] = {0, 0, 0};
+      for (int st = top >> 1; st > 0; st >>= 1)
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, d);
-      if (lane >= d) x += y;
-    }
-    if (r < nup) {
-      const int b = o + r, n_cross = c >> 16;
-      const int first = at + x - (c & 0xffff);
-      g.col[b] = sc[r];
-      g.brow[b] = v;
-      g.bptr[b] = first;
-      sp[r] = first;
-      if (g.bcodes) {
-        int terms[4];
-        sx[r] = side_terms(g, v, sc[r], n_cross, terms) ? 4 - n_cross : 4;
-        *reinterpret_cast<int4*>(g.bcodes + 4LL * b) = make_int4(terms[0], terms[1], terms[2], terms[3]);
+        for (int q = 0; q < 3; ++q)
+          if (sc[r[q] + st - 1] < c[q]) r[q] += st;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (c[q] < v) r[q] = -1;
+        else atomicAdd(&sp[r[q]], q > 0 ? 0x10001 : 1);
       }
+      // in the order of the local nodes
+      const int own0 = (k & 1) ? r[0] : 0, own1 = (k & 1) ? 0 : r[0];
+      const bool a = (k & 2) == 0;
+      *reinterpret_cast<short4*>(rk + 4 * j) =
+          make_short4(a ? own0 : r[1], a ? own1 : r[2], a ? r[1] : own0, a ? r[2] : own1);
     }
-    at += __shfl_sync(0xffffffffu, x, 31);
+    if (lane == 0) atomicAdd(&sp[0], n);
+    __syncwarp();
+    int at = cb;
+    for (int r0 = 0; r0 < nup; r0 += 32) {
+      const int r = r0 + lane;
+      const int c = r < nup ? sp[r] : 0, w = r < nup ? sc[r] : -1;
+      int f = c & 0xffff;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, f, d);
+        if (lane >= d) f += y;
+      }
+      const int b = o + r;
+      if (g.bcodes) {
+        int terms[4] = {-1, -1, -1, -1}, nt = 0;
+        for (int y = 0; y < ny; ++y) {
+          const int2 ey = y < 32 ? make_int2(__shfl_sync(0xffffffffu, en.x, y & 31), __shfl_sync(0xffffffffu, en.y, y & 31))
+                                 : g.nelem[y0 + y];
+          side_terms(ey, v, w, terms, nt);
+        }
+        if (r < nup) {
+          const int n_cross = c >> 16;
+          if (nt + n_cross > 4) atomicOr(g.serr, 1);
+          sx[r] = nt + n_cross > 4 ? 4 : 4 - n_cross;
+          *reinterpret_cast<int4*>(g.bcodes + 4LL * b) = make_int4(terms[0], terms[1], terms[2], terms[3]);
+        }
+      }
+      if (r < nup) {
+        const int first = at + f - (c & 0xffff);
+        g.col[b] = w;
+        g.brow[b] = v;
+        g.bptr[b] = first;
+        sp[r] = first;
+      }
+      at += __shfl_sync(0xffffffffu, f, 31);
+    }
+    __syncwarp();
+    for (int i0 = 0; i0 < nc; i0 += 32) {
+      const int i = i0 + lane;
+      const int r = i < nc ? rk[i] : -1;
+      const int y = i < nc ? sn[i >> 2] : 0;
+      const int code = (y << 2) | (i & 3);
+      const bool cross = r >= 0 && ((y >> 1) & 1) != ((i & 3) >> 1);
+      const unsigned same = __match_any_sync(0xffffffffu, r);
+      const unsigned crosses = __ballot_sync(0xffffffffu, cross) & same;
+      int k = 4;
+      if (r >= 0) {
+        g.contrib[sp[r] + __popc(same & below)] = code;
+        if (cross && g.bcodes) k = sx[r] + __popc(crosses & below);
+      }
+      if (k < 4) g.bcodes[4LL * (o + r) + k] = code;
+      __syncwarp();
+      if (r >= 0 && (same & below) == 0) {  // the first of its block moves the block on
+        sp[r] += __popc(same);
+        if (g.bcodes) sx[r] += __popc(crosses);
+      }
+      __syncwarp();
+    }
   }
-  __syncwarp();
-  for (int i0 = 0; i0 < nc; i0 += 32) {
-    const int i = i0 + lane;
-    const int r = i < nc ? rk[i] : -1;
-    const int x = i < nc ? inc[i >> 2] : 0;
-    const int code = (x << 2) | (i & 3);
-    const bool cross = r >= 0 && ((x >> 1) & 1) != ((i & 3) >> 1);
-    const unsigned same = __match_any_sync(0xffffffffu, r);
-    const unsigned crosses = __ballot_sync(0xffffffffu, cross) & same;
-    int k = 4;
-    if (r >= 0) {
-      g.contrib[sp[r] + __popc(same & below)] = code;
-      if (cross && g.bcodes) k = sx[r] + __popc(crosses & below);
-    }
-    if (k < 4) g.bcodes[4LL * (o + r) + k] = code;
-    __syncwarp();
-    if (r >= 0 && (same & below) == 0) {  // the first of its block moves the block on
-      sp[r] += __popc(same);
-      if (g.bcodes) sx[r] += __popc(crosses);
-    }
-    __syncwarp();
+  if (!g.lblk) return;
+  if (lane < low) g.lblk[lo + lane] = l0 + lower_bound4(g.list + 4LL * li + ll, l1 - l0, v);
+  for (int i = lane + 32; i < low; i += 32) {
+    lc = list[i];
+    const int rc = g.rptr[lc];
+    g.lblk[lo + i] = rc + lower_bound4(g.list + 4LL * g.iptr[lc] + g.lcnt[lc], g.rptr[lc + 1] - rc, v);
   }
 }
 
