@@ -245,22 +245,31 @@ __global__ void __launch_bounds__(32 * FW_WARPS) k_mlp_forward_mma(const uint16_
   }
 }
 
-// ------------------------------------------------------------------ inference (tcgen05, TMEM accumulators)
+// ------------------------------------------------------------------ inference (tcgen05, TMEM operands and accumulators)
 //
-// One CTA of 128 threads per tile of 128 candidates, persistent over tiles.
-// Operands live in shared memory in the canonical K-major layout without
-// swizzle: 8-row x 16-byte core matrices (row r of a core at +16 r), cores
-// adjacent along K LBO = 128 B apart, 8-row groups SBO apart.  Thread 0 issues
-// tcgen05.mma (kind::f16, BF16 in, FP32 accumulate, M 128, N 64, K 16 per
-// instruction) into a 64-column TMEM accumulator and commits to an mbarrier;
-// the four warps read their 32 lanes (rows) back with tcgen05.ld, add the bias,
-// apply ReLU, round to BF16 and write the next layer's operand tile.
-// Every wait is bounded: on expiry the kernel sets *err, skips the remaining
-// work, and still frees its TMEM.
+// One CTA per SM, persistent over tiles of 128 candidates, five tiles in flight: 128 threads (four warps, a
+// thread per candidate) run one tile's three layers, each group of four warps with its own 64-column TMEM
+// accumulator, 32-column TMEM operand, mbarrier and named barrier.  A layer is tcgen05.mma (kind::f16, BF16 in,
+// FP32 accumulate, M 128, N 64, K 16 per instruction) with the activations as the A operand in TMEM (a lane per
+// candidate, two BF16 values per column) and the weights in shared memory in the canonical K-major layout without
+// swizzle: 8-row x 16-byte core matrices (row r of a core at +16 r), cores adjacent along K LBO = 128 B
+// apart, 8-row groups SBO apart.  A group's first thread issues the MMAs and commits to the mbarrier; the
+// four warps read their 32 lanes back with tcgen05.ld, apply ReLU, round to BF16 and store the next operand
+// with tcgen05.st.  The next tile's first layer runs while this tile's output sums are taken.
+// What bounds it is latency: a tile is three dependent rounds.  Activations that go through TMEM need neither
+// shared-memory stores, nor the proxy fence, nor the tensor core's reads of A from shared memory (which at
+// N 64 take longer than the MMA itself), and one barrier a round is left of two.
+// Measured at 3,197,900 candidates: operands staged in shared memory, five CTAs an SM 124 us, this 85.5 us (656
+// TFLOP/s; of 164k clocks the tensor pipe is busy 35 %, the issue slots 52 %, the ALU 50 %: 96 conversions and
+// 64 unpackings a candidate).  The logits are the same bits.
+// Every wait is bounded: on expiry the kernel sets *err, skips the group's remaining work, and still frees its
+// TMEM.
 
-constexpr int TC_T = 128;
-constexpr int TC_PER_SM = 5;
-constexpr uint32_t TC_COLS = 64;
+constexpr int TC_SLOTS = 5;
+constexpr int TC_T = 128 * TC_SLOTS;
+// columns: the accumulators, then the operands, then the constant operand of the biases
+constexpr uint32_t TC_COLS = 512, TC_A = 64 * TC_SLOTS, TC_ONES = TC_A + 32 * TC_SLOTS;
+static_assert(TC_ONES + 8 <= TC_COLS, "TMEM columns");
 // instruction descriptor: D f32 (bit 4), A bf16 (bits 7-9 = 1), B bf16 (bits 10-12 = 1),
 // K-major A and B (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28
 constexpr uint32_t TC_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
@@ -275,13 +284,14 @@ XK_D uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-XK_D void tc_mma(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+XK_D void tc_mma(uint32_t dtmem, uint32_t atmem, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
       :
-      : "r"(dtmem), "l"(adesc), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate));
+      : "r"(dtmem), "r"(atmem), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate)
+      : "memory");
 }
 
 XK_D void tc_commit(uint32_t mbar) {
@@ -312,15 +322,46 @@ XK_D void tc_ld16(uint32_t taddr, float* v) {
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+      : "r"(taddr)
+      : "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 8 or 16 consecutive 32-bit columns of this thread's TMEM lane
+XK_D void tc_st8(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+XK_D void tc_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(
+          taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+
 XK_D void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+XK_D void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 XK_D void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 XK_D void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 XK_D void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
+// a barrier of the 128 threads of one group; the disjunction of their predicates, the same in all of them
+XK_D bool group_or(int id, bool pred) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %2, 0;\n\t"
+      "barrier.cta.red.or.aligned.pred q, %1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(any)
+      : "r"(id), "r"((uint32_t)pred)
+      : "memory");
+  return any != 0;
+}
 
 // byte offset of element (row, k) (16-bit elements) in a K-major no-swizzle tile with K columns
 XK_D uint32_t core_off(int row, int k, int K) {
@@ -329,22 +370,17 @@ XK_D uint32_t core_off(int row, int k, int K) {
 
 // The biases ride in the MMAs: layer 1's operand has a constant-one column
 // (k = 8) matched by b1 in W1's padding, and layers 2 and 3 add one K-16 MMA
-// of a constant tile (column 0 = 1) against a bias tile (column 0 = b).  The
+// of a constant operand (k = 0 is 1) against a bias tile (column 0 = b).  The
 // BF16 biases times 1 are exact in the FP32 accumulator.
 struct __align__(128) TcSmem {
-  // hidden operand (layers 2 and 3); its first 4 KB also hold the layer-1 operand
-  // (128 candidates x K 16: 8 features, 1, 7 zeros), read only before the hidden
-  // operand is first written for the tile
-  uint16_t a2[128 * 64];
-  uint16_t ones[128 * 16];  // 128 x K 16, column 0 = 1
-  uint16_t w1[64 * 16];     // [W1 | b1 | 0] as N 64 x K 16
+  uint16_t w1[64 * 16];  // [W1 | b1 | 0] as N 64 x K 16
   uint16_t w2[64 * 64];
   uint16_t w3[64 * 64];
-  uint16_t bb2[64 * 16];    // column 0 = b2
-  uint16_t bb3[64 * 16];    // column 0 = b3
+  uint16_t bb2[64 * 16];  // column 0 = b2
+  uint16_t bb3[64 * 16];  // column 0 = b3
   float w4[64];
   float b4;
-  uint64_t mbar;
+  uint64_t mbar[TC_SLOTS];
   uint32_t tmem;
 };
 
@@ -355,14 +391,14 @@ XK_D uint32_t pack_relu_bf16(float lo, float hi) {
   return d;
 }
 
-__global__ void __launch_bounds__(TC_T) k_mlp_forward_tc(const uint16_t* __restrict__ P,
-                                                         const float* __restrict__ feat, long long n,
-                                                         float* __restrict__ logit, int* __restrict__ err) {
+__global__ void __launch_bounds__(TC_T, 1) k_mlp_forward_tc(const uint16_t* __restrict__ P,
+                                                            const float* __restrict__ feat, long long n,
+                                                            float* __restrict__ logit, int* __restrict__ err) {
   __shared__ TcSmem sm;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int slot = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
   // weights in the operand layout (N rows = outputs, K = inputs), biases as float
   constexpr uint16_t BF16_ONE = 0x3F80;
-  for (int i = tid; i < 64 * 16; i += TC_T) {
+  for (int i = threadIdx.x; i < 64 * 16; i += TC_T) {
     const int nn = i >> 4, k = i & 15;
     const uint16_t v = k < MF ? P[O_W1 + nn * MF + k] : k == MF ? P[O_B1 + nn] : (uint16_t)0;
     const uint32_t o = core_off(nn, k, 16);
@@ -370,27 +406,22 @@ __global__ void __launch_bounds__(TC_T) k_mlp_forward_tc(const uint16_t* __restr
     *reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm.bb2) + o) = k == 0 ? P[O_B2 + nn] : (uint16_t)0;
     *reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm.bb3) + o) = k == 0 ? P[O_B3 + nn] : (uint16_t)0;
   }
-  for (int i = tid; i < 128 * 16; i += TC_T) {
-    const int r = i >> 4, k = i & 15;
-    *reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm.ones) + core_off(r, k, 16)) =
-        k == 0 ? BF16_ONE : (uint16_t)0;
-  }
   // W2, W3: one 16-byte core-matrix row (8 consecutive k of output nn) per copy; the
   // parameter offsets of both are multiples of 8 elements
   static_assert(O_W2 % 8 == 0 && O_W3 % 8 == 0, "16-byte weight rows");
-  for (int i = tid; i < 64 * 8; i += TC_T) {
+  for (int i = threadIdx.x; i < 64 * 8; i += TC_T) {
     const int nn = i >> 3, kc = i & 7;
     const uint32_t o = core_off(nn, 8 * kc, 64);
     *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.w2) + o) = *reinterpret_cast<const uint4*>(P + O_W2 + 8 * i);
     *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.w3) + o) = *reinterpret_cast<const uint4*>(P + O_W3 + 8 * i);
   }
-  if (tid < 64) sm.w4[tid] = bf16_at(P, O_W4 + tid);
+  if (threadIdx.x < 64) sm.w4[threadIdx.x] = bf16_at(P, O_W4 + threadIdx.x);
+  if (threadIdx.x == 0) sm.b4 = bf16_at(P, O_B4);
   if (tid == 0) {
-    sm.b4 = bf16_at(P, O_B4);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&sm.mbar)) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&sm.mbar[slot])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sm.tmem)),
                  "r"(TC_COLS)
                  : "memory");
@@ -401,105 +432,119 @@ __global__ void __launch_bounds__(TC_T) k_mlp_forward_tc(const uint16_t* __restr
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem;
-  const uint32_t mbar = smem_u32(&sm.mbar);
-  const uint32_t lane_base = tmem + ((uint32_t)(32 * warp) << 16);  // this warp's 32 TMEM lanes
-  uint32_t phase = 0;
-  bool ok = true;
-  const long long tiles = (n + 127) / 128;
-  // features of this thread's row of a tile (zero beyond n); the next tile's are loaded while
-  // the current tile runs its layers
-  auto load_row = [&](long long tile, float4& lo, float4& hi) {
-    const long long row = tile * 128 + tid;
-    if (tile < tiles && row < n) {
-      const float4* f4 = reinterpret_cast<const float4*>(feat + MF * row);
-      lo = __ldcs(f4);
-      hi = __ldcs(f4 + 1);
-    } else {
-      lo = hi = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  float4 x_lo, x_hi;
-  load_row(blockIdx.x, x_lo, x_hi);
-  for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-    const long long row = tile * 128 + tid;  // thread tid owns tile row tid (its TMEM lane)
-    {  // layer-1 operand: the features rounded to bf16, the one for b1, zeros
-      uint4 v0, v1;
-      v0.x = pack_bf16(x_lo.x, x_lo.y); v0.y = pack_bf16(x_lo.z, x_lo.w);
-      v0.z = pack_bf16(x_hi.x, x_hi.y); v0.w = pack_bf16(x_hi.z, x_hi.w);
-      v1.x = BF16_ONE;  // k = 8: the constant-one column that carries b1
-      v1.y = v1.z = v1.w = 0u;
-      *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.a2) + core_off(tid, 0, 16)) = v0;
-      *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.a2) + core_off(tid, 8, 16)) = v1;
-    }
-    load_row(tile + gridDim.x, x_lo, x_hi);
-    float out = 0.f;
-#pragma unroll 1
-    for (int layer = 0; layer < 3 && ok; ++layer) {
-      fence_async_smem();
-      tc_fence_before();
-      __syncthreads();
-      tc_fence_after();
-      if (tid == 0) {
-        if (layer == 0) {
-          tc_mma(tmem, tc_desc(smem_u32(sm.a2), 128, 256), tc_desc(smem_u32(sm.w1), 128, 256), 0u);
-        } else {
-          const uint16_t* w = layer == 1 ? sm.w2 : sm.w3;
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            tc_mma(tmem, tc_desc(smem_u32(sm.a2) + ks * 256, 128, 1024), tc_desc(smem_u32(w) + ks * 256, 128, 1024),
-                   ks > 0 ? 1u : 0u);
-          tc_mma(tmem, tc_desc(smem_u32(sm.ones), 128, 256), tc_desc(smem_u32(layer == 1 ? sm.bb2 : sm.bb3), 128, 256),
-                 1u);
-        }
-        tc_commit(mbar);
-      }
-      // the outcome of the wait is made uniform over the block before anyone acts on it
-      if (__syncthreads_or(tc_wait(mbar, phase) ? 0 : 1)) {
-        ok = false;
-        break;
-      }
-      phase ^= 1u;
-      tc_fence_after();
-      // the MMA that read the operand tile has completed, so the next operand is written in
-      // place; the next MMA is issued only after the barrier at the top of the layer loop,
-      // which every thread reaches after its tcgen05.ld has retired
-      float z[64];
-      tc_ld16(lane_base + 0, z);
-      tc_ld16(lane_base + 16, z + 16);
-      tc_ld16(lane_base + 32, z + 32);
-      tc_ld16(lane_base + 48, z + 48);
-      tc_wait_ld();
-      if (layer < 2) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint4 v;
-          v.x = pack_relu_bf16(z[8 * c + 0], z[8 * c + 1]);
-          v.y = pack_relu_bf16(z[8 * c + 2], z[8 * c + 3]);
-          v.z = pack_relu_bf16(z[8 * c + 4], z[8 * c + 5]);
-          v.w = pack_relu_bf16(z[8 * c + 6], z[8 * c + 7]);
-          *reinterpret_cast<uint4*>(reinterpret_cast<char*>(sm.a2) + core_off(tid, 8 * c, 64)) = v;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 64; j += 2) {
-          const uint32_t h = pack_relu_bf16(z[j], z[j + 1]);
-          out = fmaf(__uint_as_float(h << 16), sm.w4[j], out);
-          out = fmaf(__uint_as_float(h & 0xFFFF0000u), sm.w4[j + 1], out);
-        }
-      }
-      if (layer == 2) out += sm.b4;
-    }
-    if (ok && row < n) logit[row] = out;
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+  const uint32_t lanes = (uint32_t)(32 * warp) << 16;  // this warp's 32 TMEM lanes
+  if (slot == 0) {  // the constant operand: 1 at k = 0
+    const uint32_t v[8] = {BF16_ONE, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    tc_st8(tmem + lanes + TC_ONES, v);
+    tc_wait_st();
   }
-  if (!ok && tid == 0) atomicExch(err, 1);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC_COLS) : "memory");
+  tc_fence_after();
+  const uint32_t mbar = smem_u32(&sm.mbar[slot]);
+  const uint32_t acc = tmem + 64u * slot, opnd = tmem + TC_A + 32u * slot;
+  const long long tiles = (n + 127) / 128, stride = (long long)gridDim.x * TC_SLOTS;
+  long long tile = blockIdx.x + (long long)gridDim.x * slot;
+  // features of this thread's row of a tile (zero beyond n); the next tile's are loaded while
+  // the current tile runs its layers
+  float4 x_lo, x_hi;
+  auto load_row = [&](long long t) {
+    const long long row = t * 128 + tid;
+    x_lo = x_hi = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < tiles && row < n) {
+      const float4* f4 = reinterpret_cast<const float4*>(feat + MF * row);
+      x_lo = __ldcs(f4);
+      x_hi = __ldcs(f4 + 1);
+    }
+  };
+  auto stage = [&] {  // layer-1 operand: the features rounded to bf16, the one for b1, zeros
+    const uint32_t v[8] = {pack_bf16(x_lo.x, x_lo.y), pack_bf16(x_lo.z, x_lo.w), pack_bf16(x_hi.x, x_hi.y),
+                           pack_bf16(x_hi.z, x_hi.w), BF16_ONE, 0u, 0u, 0u};
+    tc_st8(opnd + lanes, v);
+    tc_wait_st();
+  };
+  uint32_t phase = 0;
+  bool bad = false;  // a wait of this thread has expired
+  // the group's operand is stored (and its accumulator read): its first thread issues a layer's MMAs.
+  // False, in all threads of the group, once a wait of any of them has expired.
+  auto issue = [&](int layer) {
+    tc_fence_before();
+    if (group_or(1 + slot, bad)) return false;
+    tc_fence_after();
+    if (tid == 0) {
+      if (layer == 0) {
+        tc_mma(acc, opnd, tc_desc(smem_u32(sm.w1), 128, 256), 0u);
+      } else {
+        const uint32_t w = smem_u32(layer == 1 ? sm.w2 : sm.w3);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) tc_mma(acc, opnd + 8u * ks, tc_desc(w + ks * 256, 128, 1024), ks > 0 ? 1u : 0u);
+        tc_mma(acc, tmem + TC_ONES, tc_desc(smem_u32(layer == 1 ? sm.bb2 : sm.bb3), 128, 256), 1u);
+      }
+      tc_commit(mbar);
+    }
+    __syncwarp();
+    return true;
+  };
+  float z[64];
+  auto fetch = [&] {  // wait for the layer and read this candidate's accumulator row
+    bad |= !tc_wait(mbar, phase);
+    phase ^= 1u;
+    __syncwarp();
+    tc_fence_after();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tc_ld16(acc + lanes + 16u * k, z + 16 * k);
+    tc_wait_ld();
+#pragma unroll
+    for (int k = 0; k < 64; ++k) asm volatile("" : "+f"(z[k]));  // nothing that uses a value moves before the wait
+  };
+  load_row(tile);
+  bool go = tile < tiles;  // the same in the whole group
+  if (go) {
+    stage();
+    load_row(tile + stride);
+    go = issue(0);
   }
+  while (go) {
+#pragma unroll 1
+    for (int layer = 1; layer < 3 && go; ++layer) {
+      fetch();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = pack_relu_bf16(z[32 * h + 2 * c], z[32 * h + 2 * c + 1]);
+        tc_st16(opnd + lanes + 16u * h, v);
+      }
+      tc_wait_st();
+      go = issue(layer);
+    }
+    if (!go) break;
+    fetch();
+    // the last layer's MMAs have read the operand and its accumulator is in registers: the next tile begins
+    const long long row = tile * 128 + tid;
+    tile += stride;
+    if (tile < tiles) {
+      stage();
+      load_row(tile + stride);
+      go = issue(0);
+    } else {
+      go = false;
+    }
+    float out = 0.f;
+#pragma unroll
+    for (int j = 0; j < 64; j += 2) {
+      const uint32_t h = pack_relu_bf16(z[j], z[j + 1]);
+      out = fmaf(__uint_as_float(h << 16), sm.w4[j], out);
+      out = fmaf(__uint_as_float(h & 0xFFFF0000u), sm.w4[j + 1], out);
+    }
+    if (!bad && row < n) logit[row] = out + sm.b4;
+  }
+  if (bad) atomicExch(err, 1);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC_COLS) : "memory");
 }
 
 // ------------------------------------------------------------------ training
@@ -989,13 +1034,10 @@ extern "C" xk_status xk_mlp_forward_tcgen05(const uint16_t* params_bf16, const f
   if ((reinterpret_cast<uintptr_t>(params_bf16) & 15) || (reinterpret_cast<uintptr_t>(feat) & 15))
     return xk_set_error(XK_ERR_ARG, "xk_mlp_forward_tcgen05: params and feat must be 16-byte aligned");
   if (n == 0) return XK_OK;
-  // persistent grid of TC_PER_SM CTAs per SM: each CTA runs its tiles' three layers back to back
-  // (MMA, completion wait, read-back), so several CTAs per SM overlap one's MMA with another's
-  // read-back; five measured best on 400k-8M samples (4 to 8 within 15%)
-  const int sms = xk_sm_count();
-  const long long resident = (long long)TC_PER_SM * sms;
+  // one CTA per SM (it takes all of the SM's TMEM); tiles go round the CTAs, then round their groups, so that
+  // few tiles spread over many SMs
   const long long tiles = (n + 127) / 128;
-  const int blocks = (int)(tiles < resident ? tiles : resident);
+  const int sms = xk_sm_count(), blocks = (int)(tiles < sms ? tiles : sms);
   k_mlp_forward_tc<<<blocks, TC_T, 0, (cudaStream_t)s>>>(params_bf16, feat, n, logit, err);
   XK_CHECK_LAUNCH();
   return XK_OK;
