@@ -31,6 +31,14 @@ XK_D T shape_c(T s, T t, int k) {
   }
 }
 
+// In double one subtraction, whatever the lanes' k (a switch issues one for every k that a warp has), and the
+// sign moved as a bit: the same values.
+template <>
+XK_D double shape_c<double>(double s, double t, int k) {
+  const double x = (k & 2) ? t : s, om = 1.0 - x, c = (k & 1) ? x : om;
+  return __hiloint2double(__double2hiint(c) ^ (int)((unsigned)(k & 2) << 30), __double2loint(c));
+}
+
 // A pair contributes in the increment when it is not INACTIVE or still carries a normal force; with
 // coated wires every pair does, since the reference evaluates the coating force of every pair.
 XK_D bool is_member(const xk_pairs& p, long long i) {
@@ -1075,18 +1083,63 @@ XK_D int4 sides_code(const int4* __restrict__ codes, long long nnzb, long long t
   return b < nnzb ? __ldcs(codes + b) : make_int4(-1, -1, -1, -1);
 }
 
+// The blocks of a tile in descending order of their numbers of terms (stable): thread t gets the codes of the
+// t-th in c; returns which block of the tile that is.  Most blocks have one term and some have up to four, so a
+// warp of consecutive blocks issues its slowest lane's three to four terms; the FP64 pipe, which bounds the
+// double gather, takes a full issue for every one.  Sorted, one warp of four has the long blocks.  Every block's
+// sum is its own thread's, in the order of its codes.
+// Measured at the 1027-wire strand (2.79M blocks, 3.3M terms): 251 us -> 175 us.  In float, where the loads bound it,
+// the blocks stay in order.
+struct TermOrder {
+  int4 code[GS_T];
+  int idx[GS_T];
+  int cnt[GS_T / 32][4];  // blocks of a warp with 4, 3, 2, 1 terms
+};
+XK_D int order_by_terms(int4& c, TermOrder& s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = (c.x != -1) + (c.y != -1) + (c.z != -1) + (c.w != -1);
+  const unsigned below = (1u << lane) - 1u;
+  int before = 0;  // blocks of this warp with more terms, or as many and a lower lane
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned m = __ballot_sync(0xffffffffu, n == 4 - k);
+    if (lane == k) s.cnt[warp][k] = __popc(m);
+    if (n == 4 - k) before = __popc(m & below);
+  }
+  const unsigned none = __ballot_sync(0xffffffffu, n == 0);
+  __syncthreads();
+  int rank = before;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int w = 0; w < GS_T / 32; ++w)
+      if (n < 4 - k || (n == 4 - k && w < warp)) rank += s.cnt[w][k];
+  if (n == 0) {  // after all others: the warps' empty blocks in turn
+    rank += __popc(none & below);
+    for (int w = 0; w < warp; ++w) rank += 32 - (s.cnt[w][0] + s.cnt[w][1] + s.cnt[w][2] + s.cnt[w][3]);
+  }
+  s.code[rank] = c;
+  s.idx[rank] = threadIdx.x;
+  __syncthreads();
+  c = s.code[threadIdx.x];
+  return s.idx[threadIdx.x];
+}
+
 template <typename T, int RS, int BCOL>
 __global__ void __launch_bounds__(GS_T, sizeof(T) == 4 ? 16 : 8) k_gather_tangent_sides(long long nnzb, const int4* __restrict__ codes,
                                                                const T* __restrict__ S, const T* __restrict__ rec,
                                                                T* __restrict__ K) {
   __shared__ __align__(16) T stage[GS_T * 9];
+  __shared__ TermOrder order;
   const long long ntiles = (nnzb + GS_T - 1) / GS_T;
   long long tile = blockIdx.x;
   int4 cn = tile < ntiles ? sides_code(codes, nnzb, tile) : make_int4(-1, -1, -1, -1);
   for (; tile < ntiles; tile += gridDim.x) {
     const long long b0 = tile * GS_T;
-    const int4 c = cn;
+    int4 c = cn;
+    int at = threadIdx.x;  // this thread's block of the tile
     if (tile + gridDim.x < ntiles) cn = sides_code(codes, nnzb, tile + gridDim.x);
+    if (sizeof(T) == 8) at = order_by_terms(c, order);
     T acc[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) acc[q] = T(0);
@@ -1103,7 +1156,7 @@ __global__ void __launch_bounds__(GS_T, sizeof(T) == 4 ? 16 : 8) k_gather_tangen
       add_term<T, RS, BCOL>(S, rec, c.w, acc);
     }
 #pragma unroll
-    for (int q = 0; q < 9; ++q) stage[threadIdx.x * 9 + q] = acc[q];
+    for (int q = 0; q < 9; ++q) stage[at * 9 + q] = acc[q];
     __syncthreads();
     const long long rem = nnzb - b0;
     const int nv = 9 * (int)(rem < GS_T ? rem : GS_T);
