@@ -441,6 +441,39 @@ xk_status xk_pairs_from32(const xk_pairs32* q, xk_pairs* p, xk_stream s);
 xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk_contact_params* cp, float* rec, int parts,
                          xk_stream s);
 
+/* What the pairs of a segment share in one iteration of the FP64 pair kernels, XK_SEG64_STRIDE doubles per
+ * element (seg64 32-byte aligned): X + u of its first node, the difference to its second node and the squared
+ * length (in two orders of the sum), and the same of u - u_ref (u_ref nullable: zero). */
+#define XK_SEG64_STRIDE 16
+xk_status xk_segments64(const xk_mesh* m, const double* u, const double* u_ref, double* seg64, xk_stream s);
+
+/* One Newton iteration's assembly as one call (ContactForceAssemblyProcess + TangentAssemblyProcess,
+ * _newton_steps.py:79-135,289-313): node records (mixed), pair kernels, beam, contact tangent, residual
+ * R = f_int + f_c - f_ext with R[fixed] = 0 and its squared norm.  The parts run on s and the three side
+ * streams (of the same device, not used by another call in progress), which s waits for at the end; under
+ * capture of s they become parallel branches.  FP64 uses pairs, elem_ref and seg64
+ * (nullable: workspace of XK_SEG64_STRIDE doubles per element), XK_MIXED uses pairs32, elem32 and node32.
+ * tangent 0: no K_beam, no K_c.  gather_variant as in xk_contact_gather_tangent. */
+typedef struct {
+  const xk_mesh* mesh;
+  const xk_section* section;
+  const xk_beam_plan* plan;
+  const xk_contact_pattern* pat;
+  const xk_contact_params* cp;
+  xk_pairs* pairs;
+  xk_pairs32* pairs32;
+  const double* elem_ref;
+  const float* elem32;
+  float* node32;
+  double* seg64;
+  void *rec, *K_c, *K_beam;
+  double *f_int, *R, *norm2;
+  xk_stream side[3];
+  int32_t precision, gather_variant, tangent, pad;
+} xk_assembly;
+xk_status xk_assemble(const xk_assembly* a, const double* u, const double* u_ref, const double* f_ext,
+                      const uint8_t* fixed, xk_stream s);
+
 /* Smooth (softplus) normal law for n gaps, element-wise:
  * _evaluate_smooth_normal_force_vectorized (contact/penalty/law_normal.py:129-149):
  * x = -g + lambda / k_pen, p_n = k_pen delta log(1 + exp(x / delta)),

@@ -421,17 +421,74 @@ XK_D void fcross3(const double* a, const double* b, double* c) {
   c[2] = fma(a[0], b[1], -(a[1] * b[0]));
 }
 
-// Closest point, distance and unit normal of one pair at positions x, in fused operations.  False (nothing
-// written) outside the ordinary case.
-XK_D bool closest64(const double (*x)[3], double& s, double& t, double& dist, double* n) {
-  double dA[3], dB[3], w[3];
+// What the pairs of a segment share, formed once per segment and iteration (k_seg64) instead of in every pair
+// (24 of the 132 FP64 operations of a pair without force, 46 of a contributing one): its first point X + u, the
+// difference to its second point and the squared length, in fused order (a) and in the reference's (ae); the
+// displacement since u_ref of its first point and the difference to that of its second one.  The pairs' values
+// keep their bits.  Measured at the 1027-wire strand: assembly 1785 -> 1558 us.
+struct Seg64 {
+  double x[3], a, d[3], ae;
+};
+constexpr int SEG64_STRIDE = XK_SEG64_STRIDE;
+static_assert(SEG64_STRIDE == 16, "four vectors of four doubles");
+XK_D void ldg4(const double* p, double* v) {  // p 32-byte aligned
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+XK_D Seg64 load_seg(const double* __restrict__ seg, int e) {
+  Seg64 r;
+  double v[8];
+  ldg4(seg + (long long)SEG64_STRIDE * e, v);
+  ldg4(seg + (long long)SEG64_STRIDE * e + 4, v + 4);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    dA[i] = x[1][i] - x[0][i];
-    dB[i] = x[3][i] - x[2][i];
-    w[i] = x[0][i] - x[2][i];
+    r.x[i] = v[i];
+    r.d[i] = v[4 + i];
   }
-  const double a = fdot3(dA, dA), b = fdot3(dA, dB), c = fdot3(dB, dB), d = fdot3(dA, w), e = fdot3(dB, w);
+  r.a = v[3];
+  r.ae = v[7];
+  return r;
+}
+// the same from the nodes' positions (the square in the order that is asked for only)
+template <bool EXACT>
+XK_D Seg64 seg_of(const xk_mesh& m, const double* __restrict__ u, int n0, int n1) {
+  Seg64 r;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r.x[i] = xadd(m.X[3LL * n0 + i], u[6LL * n0 + i]);
+    r.d[i] = xsub(xadd(m.X[3LL * n1 + i], u[6LL * n1 + i]), r.x[i]);
+  }
+  if (EXACT) r.ae = xdot_es(r.d, r.d); else r.a = fdot3(r.d, r.d);
+  return r;
+}
+
+__global__ void k_seg64(xk_mesh m, const double* __restrict__ u, const double* __restrict__ u_ref,
+                        double* __restrict__ seg) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m.n_elems) return;
+  const int n0 = m.conn[2LL * e], n1 = m.conn[2LL * e + 1];
+  const Seg64 r = seg_of<false>(m, u, n0, n1);
+  double o[16] = {r.x[0], r.x[1], r.x[2], r.a, r.d[0], r.d[1], r.d[2], xdot_es(r.d, r.d)};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const long long d0 = 6LL * n0 + c, d1 = 6LL * n1 + c;
+    const double du0 = u_ref ? u[d0] - u_ref[d0] : u[d0], du1 = u_ref ? u[d1] - u_ref[d1] : u[d1];
+    o[8 + c] = du0;
+    o[12 + c] = du1 - du0;
+  }
+  o[11] = o[15] = 0.0;
+  double2* w = reinterpret_cast<double2*>(seg + (long long)SEG64_STRIDE * e);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) w[k] = make_double2(o[2 * k], o[2 * k + 1]);
+}
+
+// Closest point, distance and unit normal of one pair of segments, in fused operations.  False (nothing
+// written) outside the ordinary case.
+XK_D bool closest64(const Seg64& A, const Seg64& B, double& s, double& t, double& dist, double* n) {
+  const double *dA = A.d, *dB = B.d;
+  double w[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) w[i] = A.x[i] - B.x[i];
+  const double a = A.a, b = fdot3(dA, dB), c = B.a, d = fdot3(dA, w), e = fdot3(dB, w);
   const double ac = a * c, det = fma(-b, b, ac);
   // segments longer than 2^-14 and at an angle (det > 1e-3 ac): the absolute and relative tolerances of the
   // reference (1e-10) are far off
@@ -496,31 +553,27 @@ __noinline__ __device__ void narrow64_exact(const xk_mesh& m, const xk_pairs& p,
   narrow_exact_one(m, p, u, 0.0, 0.0, 0, 0, i);
 }
 
-// Narrowphase of pair i (nodes nd, radius sum rs: the cores' on coated wires), written to the table.
+// Narrowphase of pair i (segments A and B, radius sum rs: the cores' on coated wires), written to the table.
 // EXACT: the closest point, gap and normal in the reference's operation order (contributing pairs: the
 // forces and the tangent they give are then the same bits however this kernel is scheduled; an iterative
 // solve of the tangent amplifies a rounding to 1e-8 of its solution); the frame is fused either way.
 template <bool EXACT>
-XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const int* nd, double rs,
+XK_D void pair_narrow64(const xk_mesh& m, const xk_pairs& p, int i, const Seg64& A, const Seg64& B, double rs,
                         const double* __restrict__ u, double& s, double& t, double& gap, double* n, double* t1,
                         double* t2) {
   const long long cap = p.cap;
-  double x[4][3], pt1[3], pn[3], dist;
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) x[k][c] = xadd(m.X[3LL * nd[k] + c], u[6LL * nd[k] + c]);
+  double pt1[3], pn[3], dist;
   load3(p.t1, cap, i, pt1);
   load3(p.normal, cap, i, pn);
   bool ok;
   if (EXACT) {
     double nrm[3];
-    ok = closest_exact_fast(x, s, t, dist, nrm);
+    ok = closest_exact_fast(A.x, A.d, A.ae, B.x, B.d, B.ae, s, t, dist, nrm);
     if (ok) {  // the frame's own normalisation (frame_exact)
       div3(nrm, sqrt_unit64(xdot_es(nrm, nrm)), n);
     }
   } else {
-    ok = closest64(x, s, t, dist, n);
+    ok = closest64(A, B, s, t, dist, n);
   }
   if (ok && frame64(n, pn, pt1, t1, t2)) {
     gap = xsub(dist, rs);
@@ -547,24 +600,35 @@ XK_D double narrow_radii(const xk_mesh& m, int ea, int eb) {
   return xadd(r[ea], r[eb]);
 }
 
+// SEG: the segments' records were formed (k_seg64); else from the nodes.
 constexpr int PAIR64_T = 128;
+template <bool SEG>
 __global__ void __launch_bounds__(PAIR64_T) k_pair_other64(const __grid_constant__ xk_mesh m,
                                                            const __grid_constant__ xk_pairs p,
                                                            const int32_t* __restrict__ others, int n_o,
-                                                           const double* __restrict__ u) {
+                                                           const double* __restrict__ u,
+                                                           const double* __restrict__ seg) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= n_o) return;
   const int i = others[o];
   const int ea = p.ea[i], eb = p.eb[i];
-  const PairNodes pn = pair_nodes(m, ea, eb);
+  Seg64 A, B;
+  if (SEG) {
+    A = load_seg(seg, ea);
+    B = load_seg(seg, eb);
+  } else {
+    const PairNodes pn = pair_nodes(m, ea, eb);
+    A = seg_of<false>(m, u, pn.n[0], pn.n[1]);
+    B = seg_of<false>(m, u, pn.n[2], pn.n[3]);
+  }
   double s, t, gap, n[3], t1[3], t2[3];
-  pair_narrow64<false>(m, p, i, pn.n, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  pair_narrow64<false>(m, p, i, A, B, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
 }
 
 // Contributing pairs, all four stages, combined records.  The frame is orthonormal (just formed), so the
 // geometric friction term q0 n t1^T + q1 t2 n^T - q1 [t1]x^T is n (q0 t1 + q1 t2)^T, since
 // [t1]x = n t2^T - t2 n^T, and B = B_n - T D T^T + n vf^T / dist.
-template <bool COAT>
+template <bool COAT, bool SEG>
 __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constant__ xk_mesh m,
                                                             const __grid_constant__ xk_pairs p,
                                                             const int32_t* __restrict__ members,
@@ -572,19 +636,32 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
                                                             const double* __restrict__ u,
                                                             const double* __restrict__ u_ref,
                                                             const __grid_constant__ xk_contact_params cp, double dh,
-                                                            int rec_vec, double* __restrict__ rec) {
+                                                            int rec_vec, const double* __restrict__ seg,
+                                                            double* __restrict__ rec) {
   const int mi = blockIdx.x * blockDim.x + threadIdx.x;
   if (mi >= n_m) return;
   const int i = members[mi];
   const long long cap = p.cap;
   int nd[4];
+  if (!SEG || COAT) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) nd[k] = mnodes[4LL * mi + k];
+    for (int k = 0; k < 4; ++k) nd[k] = mnodes[4LL * mi + k];
+  }
   const int ea = p.ea[i], eb = p.eb[i];
   uint8_t status = p.status[i];
   double p_n = p.p_n[i];
   double s, t, gap, n[3], t1[3], t2[3];
-  pair_narrow64<true>(m, p, i, nd, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  {
+    Seg64 A, B;
+    if (SEG) {
+      A = load_seg(seg, ea);
+      B = load_seg(seg, eb);
+    } else {
+      A = seg_of<true>(m, u, nd[0], nd[1]);
+      B = seg_of<true>(m, u, nd[2], nd[3]);
+    }
+    pair_narrow64<true>(m, p, i, A, B, narrow_radii(m, ea, eb), u, s, t, gap, n, t1, t2);
+  }
   double v[3] = {0.0, 0.0, 0.0};
   // normal force
   const double xpen = cp.k_pen * (-gap);
@@ -603,7 +680,7 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
   double vf[3] = {0.0, 0.0, 0.0};
   bool fric = false;
   double du[4][3];
-  if (fproc || COAT) {
+  if (COAT || (!SEG && fproc)) {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -613,6 +690,22 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
       }
   }
   if (fproc) {
+    double dA[8], dB[8];  // displacement since u_ref: first point, then (at 4) the second point's less that
+    if (SEG) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        ldg4(seg + (long long)SEG64_STRIDE * ea + 8 + 4 * k, dA + 4 * k);
+        ldg4(seg + (long long)SEG64_STRIDE * eb + 8 + 4 * k, dB + 4 * k);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        dA[c] = du[0][c];
+        dA[4 + c] = du[1][c] - du[0][c];
+        dB[c] = du[2][c];
+        dB[4 + c] = du[3][c] - du[2][c];
+      }
+    }
     double kt = p.k_t[i];
     if (p.k_pen[i] <= 0.0) {
       p.k_pen[i] = cp.k_pen;
@@ -621,8 +714,7 @@ __global__ void __launch_bounds__(PAIR64_T) k_pair_member64(const __grid_constan
     }
     double dr[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      dr[c] = fma(t, du[3][c] - du[2][c], du[2][c]) - fma(s, du[1][c] - du[0][c], du[0][c]);
+    for (int c = 0; c < 3; ++c) dr[c] = fma(t, dB[4 + c], dB[c]) - fma(s, dA[4 + c], dA[c]);
     const double d0 = fdot3(dr, t1), d1 = fdot3(dr, t2);
     const double q0 = fma(kt, d0, p.z_t[i]), q1 = fma(kt, d1, p.z_t[cap + i]);
     const double q2 = fma(q0, q0, q1 * q1);
@@ -1590,9 +1682,30 @@ extern "C" xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, cons
   return r;
 }
 
+extern "C" xk_status xk_segments64(const xk_mesh* m, const double* u, const double* u_ref, double* seg64, xk_stream s) {
+  if (!m || !u || (m->n_elems > 0 && !seg64)) return xk_set_error(XK_ERR_ARG, "xk_segments64: null argument");
+  if ((uintptr_t)seg64 & 31) return xk_set_error(XK_ERR_ARG, "xk_segments64: seg64 must be 32-byte aligned");
+  if (m->n_elems <= 0) return XK_OK;
+  // FP64 work of a few operations a segment: small CTAs reach all SMs
+  k_seg64<<<xk_blocks(m->n_elems, 64), 64, 0, (cudaStream_t)s>>>(*m, u, u_ref, seg64);
+  XK_CHECK_LAUNCH();
+  return XK_OK;
+}
+
+// xk_pair_step with the segments' records of this u and u_ref (or null): the FP64 engine's kernels read them
+xk_status xk_pair_step_seg(const xk_mesh* m, xk_pairs* p, const xk_contact_pattern* pat, const double* u,
+                           const double* u_ref, const xk_contact_params* cp, int stages, int precision, int out_mode,
+                           const double* seg64, void* rec, xk_stream s);
+
 extern "C" xk_status xk_pair_step(const xk_mesh* m, xk_pairs* p, const xk_contact_pattern* pat, const double* u,
                                   const double* u_ref, const xk_contact_params* cp, int stages, int precision,
                                   int out_mode, void* rec, xk_stream s) {
+  return xk_pair_step_seg(m, p, pat, u, u_ref, cp, stages, precision, out_mode, nullptr, rec, s);
+}
+
+xk_status xk_pair_step_seg(const xk_mesh* m, xk_pairs* p, const xk_contact_pattern* pat, const double* u,
+                           const double* u_ref, const xk_contact_params* cp, int stages, int precision, int out_mode,
+                           const double* seg64, void* rec, xk_stream s) {
   if (!m || !p || !pat || !cp) return xk_set_error(XK_ERR_ARG, "xk_pair_step: null argument");
   if (((stages & XK_STAGE_NARROW) || (stages & XK_STAGE_FRICTION)) && !u)
     return xk_set_error(XK_ERR_ARG, "xk_pair_step: u is required for the narrowphase and friction stages");
@@ -1607,7 +1720,11 @@ extern "C" xk_status xk_pair_step(const xk_mesh* m, xk_pairs* p, const xk_contac
   if ((stages & XK_STAGE_NARROW) && !(stages & XK_STAGE_NO_OTHERS) && pat->n_others > 0) {
     if (precision == XK_FP64) {
       const int bs = pair64_block(pat->n_others);
-      k_pair_other64<<<xk_blocks(pat->n_others, bs), bs, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
+      const int nb64 = xk_blocks(pat->n_others, bs);
+      if (seg64)
+        k_pair_other64<true><<<nb64, bs, 0, st>>>(*m, *p, pat->others, pat->n_others, u, seg64);
+      else
+        k_pair_other64<false><<<nb64, bs, 0, st>>>(*m, *p, pat->others, pat->n_others, u, nullptr);
     } else if (precision == XK_MIXED)
       k_pair_other<XK_MIXED><<<xk_blocks(pat->n_others, PAIR_T), PAIR_T, 0, st>>>(*m, *p, pat->others, pat->n_others, u);
     else
@@ -1623,12 +1740,15 @@ extern "C" xk_status xk_pair_step(const xk_mesh* m, xk_pairs* p, const xk_contac
     const double dh = cp->smoothing_delta > 0.0 ? cp->k_pen / cp->smoothing_delta : 0.0;
     const int bs = pair64_block(pat->n_members), nb64 = xk_blocks(pat->n_members, bs);
     const int rv = ((uintptr_t)rec & 31) == 0;
-    if (coat)
-      k_pair_member64<true><<<nb64, bs, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u, u_ref, *cp,
-                                                 dh, rv, (double*)rec);
-    else
-      k_pair_member64<false><<<nb64, bs, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u, u_ref,
-                                                  *cp, dh, rv, (double*)rec);
+#define XK_MEMBER64(CC, SS)                                                                                       \
+  k_pair_member64<CC, SS><<<nb64, bs, 0, st>>>(*m, *p, pat->members, pat->member_nodes, pat->n_members, u, u_ref, *cp, \
+                                               dh, rv, seg64, (double*)rec)
+    if (coat) {
+      if (seg64) XK_MEMBER64(true, true); else XK_MEMBER64(true, false);
+    } else {
+      if (seg64) XK_MEMBER64(false, true); else XK_MEMBER64(false, false);
+    }
+#undef XK_MEMBER64
     XK_CHECK_LAUNCH();
     return XK_OK;
   }

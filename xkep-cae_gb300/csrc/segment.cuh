@@ -50,16 +50,13 @@ XK_D double clip01_64(double x) { return below0_64(x) ? 0.0 : (above1_64(x) ? 1.
 // The same closest point for the ordinary case (both segments longer than 2^-14, det > 1e-3 ac, finite): the
 // operations of closest_exact in their order, each rounded on its own, so the same bits; the divides share
 // their reciprocals and are skipped where the unclamped parameters stand.  False outside that case.
-XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double& dist, double* normal) {
-  double dA[3], dB[3], w0[3];
+// From the segments' first points, their difference vectors and the squares of these (xdot_es).
+XK_D bool closest_exact_fast(const double* xA, const double* dA, double a, const double* xB, const double* dB, double c,
+                             double& s, double& t, double& dist, double* normal) {
+  double w0[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    dA[i] = xsub(x[1][i], x[0][i]);
-    dB[i] = xsub(x[3][i], x[2][i]);
-    w0[i] = xsub(x[0][i], x[2][i]);
-  }
-  const double a = xdot_es(dA, dA), b = xdot_es(dA, dB), c = xdot_es(dB, dB);
-  const double d = xdot_es(dA, w0), e = xdot_es(dB, w0);
+  for (int i = 0; i < 3; ++i) w0[i] = xsub(xA[i], xB[i]);
+  const double b = xdot_es(dA, dB), d = xdot_es(dA, w0), e = xdot_es(dB, w0);
   const double ac = xmul(a, c), det = xsub(ac, xmul(b, b));
   if (!(in_range64<-29, 140>(a) && in_range64<-29, 140>(c) && __double2hiint(fma(-1e-3, ac, det)) > 0)) return false;
   const Divisor64 qd = divisor64(det);
@@ -77,7 +74,7 @@ XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double&
   }
   double diff[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) diff[i] = xsub(xadd(x[0][i], xmul(s, dA[i])), xadd(x[2][i], xmul(t, dB[i])));
+  for (int i = 0; i < 3; ++i) diff[i] = xsub(xadd(xA[i], xmul(s, dA[i])), xadd(xB[i], xmul(t, dB[i])));
   const double d2 = xdot_es(diff, diff);
   if (!in_range64<-190, 300>(d2)) return false;
   dist = sqrt64(d2);
@@ -85,4 +82,13 @@ XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double&
 #pragma unroll
   for (int i = 0; i < 3; ++i) normal[i] = div64(diff[i], q);
   return true;
+}
+XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double& dist, double* normal) {
+  double dA[3], dB[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dA[i] = xsub(x[1][i], x[0][i]);
+    dB[i] = xsub(x[3][i], x[2][i]);
+  }
+  return closest_exact_fast(x[0], dA, xdot_es(dA, dA), x[2], dB, xdot_es(dB, dB), s, t, dist, normal);
 }

@@ -19,6 +19,7 @@ XK_STAGE_NO_OTHERS, XK_STAGE_NO_MEMBERS = 16, 32
 XK_PAIRS_OTHERS, XK_PAIRS_MEMBERS, XK_PAIRS_ALL = 1, 2, 3
 XK_OUT_COMBINED, XK_OUT_SPLIT = 0, 1
 XK_WHICH_COMBINED, XK_WHICH_NORMAL, XK_WHICH_FRICTION = 0, 1, 2
+SEG64_STRIDE = 16
 REC_STRIDE = {XK_OUT_COMBINED: 16, XK_OUT_SPLIT: 32}
 XK_GATHER_DEFAULT, XK_GATHER_LANES, XK_GATHER_CHUNKS, XK_GATHER_SIDES = 0, 1, 2, 3
 XK_GATHER_SIDES_SUMS, XK_GATHER_SIDES_BLOCKS = 4, 5
@@ -104,6 +105,14 @@ class ContactPattern(C.Structure):
                                               ("sides_per_sm", C.c_int32), ("node_elem_ready", C.c_int32)]
 
 
+
+class Assembly(C.Structure):
+    _fields_ = [(n, vp) for n in ("mesh", "section", "plan", "pat", "cp", "pairs", "pairs32", "elem_ref", "elem32",
+                                  "node32", "seg64", "rec", "K_c", "K_beam", "f_int", "R", "norm2", "side_others",
+                                  "side_beam", "side_tangent")] + [
+        (n, C.c_int32) for n in ("precision", "gather_variant", "tangent", "pad")]
+
+
 P = C.POINTER
 i64p = P(C.c_int64)
 
@@ -138,6 +147,8 @@ SIGNATURES = {
     "xk_beam_assemble32": [P(Mesh), P(Section), vp, P(BeamPlan), vp, vp, vp, vp],
     "xk_pairs_to32": [P(Mesh), P(Pairs), P(ContactPattern), P(Pairs32), vp],
     "xk_pairs_from32": [P(Pairs32), P(Pairs), vp],
+    "xk_segments64": [P(Mesh), vp, vp, vp, vp],
+    "xk_assemble": [P(Assembly), vp, vp, vp, vp, vp],
     "xk_pair_step32": [P(Pairs32), vp, P(ContactParams), vp, C.c_int, vp],
     "xk_genalpha_predict": [C.c_int64, vp, vp, vp, vp, vp, vp, vp, C.c_double, C.c_double, C.c_double, vp],
     "xk_genalpha_correct": [C.c_int64, vp, vp, vp, vp, vp, C.c_double, C.c_double, C.c_double, vp],

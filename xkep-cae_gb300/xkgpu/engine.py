@@ -116,6 +116,9 @@ class AssemblyEngine:
         self.rec = torch.zeros(L.REC_STRIDE[L.XK_OUT_COMBINED] * self.pattern.cap_members, dtype=self.t_dtype,
                                device=dev)
         self.K_c = torch.zeros(9 * max(self.pattern.cap_blocks, 1), dtype=self.t_dtype, device=dev)
+        self.seg64 = None  # the FP64 pair kernels' records per element
+        if self.precision == L.XK_FP64:
+            self.seg64 = torch.empty(L.SEG64_STRIDE * max(self.mesh.n_elems, 1), dtype=torch.float64, device=dev)
         self.graph = None
 
     def update_reference_frames(self, stream=None):
@@ -318,67 +321,19 @@ class AssemblyEngine:
         overlap.
         """
         main = stream if stream is not None else torch.cuda.current_stream()
-        s = stream_handle(main)
-        p = self.precision
-        pat = C.byref(self.pattern.c)
-        so, sb, st = self._side_streams()
-        if p == L.XK_MIXED:
+        if self.precision == L.XK_MIXED:
             if not self._state_in32:
-                self._to32(s)
+                self._to32(stream_handle(main))
             self.pairs32.c.block = self._pair_block  # the float table's struct is rebuilt when it grows
-            L.call("xk_nodes_prepare", C.byref(self.mesh.c), ptr(u), ptr(u_ref), ptr(self.node32), s)
-        so.wait_stream(main)
-        sb.wait_stream(main)
-        # other pairs' narrowphase
-        if p == L.XK_MIXED:
-            L.call("xk_pair_step32", C.byref(self.pairs32.c), ptr(self.node32), C.byref(self.cp), ptr(self.rec),
-                   L.XK_PAIRS_OTHERS, stream_handle(so))
-        else:
-            L.call("xk_pair_step", C.byref(self.mesh.c), C.byref(self.pairs.c), pat, ptr(u), ptr(u_ref),
-                   C.byref(self.cp), L.XK_STAGE_NARROW | L.XK_STAGE_NO_MEMBERS, p, L.XK_OUT_COMBINED,
-                   ptr(self.rec), stream_handle(so))
-        # beam elements
-        if p == L.XK_MIXED:
-            L.call("xk_beam_assemble32", C.byref(self.mesh.c), C.byref(self.beam.section), ptr(self.elem32),
-                   C.byref(self.beam.plan), ptr(self.node32), ptr(self.f_int), ptr(self.K_beam) if tangent else None,
-                   stream_handle(sb))
-        else:
-            self.beam.assemble(u, p, self.f_int, self.K_beam if tangent else None, sb)
-        # contributing pairs, then the contact tangent from their records
-        if p == L.XK_MIXED:
-            L.call("xk_pair_step32", C.byref(self.pairs32.c), ptr(self.node32), C.byref(self.cp), ptr(self.rec),
-                   L.XK_PAIRS_MEMBERS, s)
-        else:
-            L.call("xk_pair_step", C.byref(self.mesh.c), C.byref(self.pairs.c), pat, ptr(u), ptr(u_ref),
-                   C.byref(self.cp), L.XK_STAGE_ALL | L.XK_STAGE_NO_OTHERS, p, L.XK_OUT_COMBINED, ptr(self.rec), s)
-        gather = tangent and self.pattern.nnzb > 0
-        # the element-side schedules leave per-element force sums that the residual reads
-        elem_force = gather and self.gather_variant == L.XK_GATHER_SIDES
-        sums_done = None
-        if gather:
-            st.wait_stream(main)
-            if elem_force:  # element sums, then the blocks; the residual needs only the sums
-                L.call("xk_contact_gather_tangent", pat, ptr(self.rec), p, L.XK_OUT_COMBINED, L.XK_WHICH_COMBINED,
-                       L.XK_GATHER_SIDES_SUMS, ptr(self.K_c), stream_handle(st))
-                sums_done = torch.cuda.Event()
-                sums_done.record(st)
-                L.call("xk_contact_gather_tangent", pat, ptr(self.rec), p, L.XK_OUT_COMBINED, L.XK_WHICH_COMBINED,
-                       L.XK_GATHER_SIDES_BLOCKS, ptr(self.K_c), stream_handle(st))
-            else:
-                L.call("xk_contact_gather_tangent", pat, ptr(self.rec), p, L.XK_OUT_COMBINED, L.XK_WHICH_COMBINED,
-                       self.gather_variant, ptr(self.K_c), stream_handle(st))
-        # residual after the members (or the tangent gather's element sums) and the beam
-        main.wait_stream(sb)
-        if elem_force:
-            main.wait_event(sums_done)
-            L.call("xk_contact_gather_force_elem", pat, p, ptr(self.f_int), -1.0, ptr(f_ext), ptr(fixed),
-                   ptr(self.R), ptr(self.norm2), s)
-        else:
-            L.call("xk_contact_gather_force", pat, ptr(self.rec), p, L.XK_OUT_COMBINED, L.XK_WHICH_COMBINED,
-                   ptr(self.f_int), -1.0, ptr(f_ext), ptr(fixed), ptr(self.R), ptr(self.norm2), s)
-        main.wait_stream(so)
-        if gather:
-            main.wait_stream(st)
+        so, sb, st = (x.cuda_stream for x in self._side_streams())
+        at, beam = C.addressof, self.beam
+        data = torch.Tensor.data_ptr
+        a = L.Assembly(at(self.mesh.c), at(beam.section), at(beam.plan), at(self.pattern.c), at(self.cp),
+                       at(self.pairs.c), at(self.pairs32.c), data(beam.elem_ref), data(self.elem32), data(self.node32),
+                       None if self.seg64 is None else data(self.seg64), data(self.rec), data(self.K_c),
+                       data(self.K_beam), data(self.f_int), data(self.R), data(self.norm2), so, sb, st,
+                       self.precision, self.gather_variant, int(tangent), 0)
+        L.call("xk_assemble", C.byref(a), ptr(u), ptr(u_ref), ptr(f_ext), ptr(fixed), main.cuda_stream)
         return self.R
 
     def _side_streams(self):
