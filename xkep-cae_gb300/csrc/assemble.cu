@@ -12,6 +12,9 @@
 xk_status xk_pair_step_seg(const xk_mesh* m, xk_pairs* p, const xk_contact_pattern* pat, const double* u,
                            const double* u_ref, const xk_contact_params* cp, int stages, int precision, int out_mode,
                            const double* seg64, void* rec, xk_stream s);
+xk_status xk_contact_gather_force_norm(const xk_contact_pattern* pat, const void* rec, int precision,
+                                       const double* base, double scale, const double* f_ext, const uint8_t* fixed,
+                                       double* out, double* norm2, xk_stream s);
 
 namespace {
 
@@ -112,8 +115,7 @@ extern "C" xk_status xk_assemble(const xk_assembly* a, const double* u, const do
     XK_TRY(wait(st, ev->e[EV_SUMS]));
     XK_TRY(xk_contact_gather_force_elem(pat, a->precision, a->f_int, -1.0, f_ext, fixed, a->R, a->norm2, s));
   } else {
-    XK_TRY(xk_contact_gather_force(pat, a->rec, a->precision, XK_OUT_COMBINED, XK_WHICH_COMBINED, a->f_int, -1.0,
-                                   f_ext, fixed, a->R, a->norm2, s));
+    XK_TRY(xk_contact_gather_force_norm(pat, a->rec, a->precision, a->f_int, -1.0, f_ext, fixed, a->R, a->norm2, s));
   }
   if (n_o > 0) {
     XK_TRY(mark(ev->e[EV_OTHERS], so));

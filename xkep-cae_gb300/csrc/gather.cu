@@ -728,6 +728,136 @@ __global__ void k_gather_force(int n_nodes, const int32_t* __restrict__ ptr, con
   }
 }
 
+// The block sums of a residual kernel's squares go to `part`; the last block to finish (`count`, zero between
+// launches, finds it) adds them in block order into *norm2: a fixed order whatever the timing.  b: this
+// block's sum, in thread 0; T threads, all of which call it.
+template <int T>
+XK_D void norm2_of_blocks(double b, double* __restrict__ part, unsigned int* __restrict__ count,
+                          double* __restrict__ norm2) {
+  __shared__ double red[T / 32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = b;
+    __threadfence();
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += T) a += __ldcg(part + k);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  if (lane == 0) red[warp] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < T / 32; ++w) t += red[w];
+    *norm2 = t;
+    *count = 0u;  // ready for the next launch
+  }
+}
+// the counter of both residual kernels, the last word of norm_scratch: beyond the block sums of either
+unsigned int* norm_count(double* part, int n_nodes) {
+  return part ? reinterpret_cast<unsigned int*>(part + (6LL * n_nodes + 255) / 256) : nullptr;
+}
+
+XK_D double to_f64(float x) { return xk_f2d(x); }  // the conversion in integer arithmetic (the FP64 pipe is slow)
+XK_D double to_f64(double x) { return x; }
+
+// s, t and v of a combined record
+XK_D void load_stv(const float* __restrict__ r, float* o) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(r) + 2), b = __ldg(reinterpret_cast<const float4*>(r) + 3);
+  o[0] = a.y; o[1] = a.z; o[2] = a.w; o[3] = b.x; o[4] = b.y;
+}
+XK_D void load_stv(const double* __restrict__ r, double* o) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(r) + 4), b = __ldg(reinterpret_cast<const double2*>(r) + 5),
+                c = __ldg(reinterpret_cast<const double2*>(r) + 6);
+  o[0] = a.y; o[1] = b.x; o[2] = b.y; o[3] = c.x; o[4] = c.y;
+}
+
+// The assembly's form of k_gather_force: combined records, the squared norm fused.  The same sums in the same
+// order; what it saves is latency: a record's five values come by two (three in double) vector loads, two
+// incidences' loads are in flight together, and the norm takes no further launches.
+// GFN_NODES a CTA, so that the block sums fit norm_scratch.
+// Measured with both norm launches: 37-wire strand in double (4,773 nodes) 18 -> 11 us, its eager assembly 75 -> 67 us;
+// 64 small strands in float 26 -> 22 us, 93 -> 89 us.
+constexpr int GFN_NODES = 48, GFN_T = GFN_NODES * GF_LANES;
+static_assert(6 * GFN_NODES % 32 == 0, "whole warps of squares");
+template <typename T>
+__global__ void __launch_bounds__(GFN_T) k_gather_force_norm(int n_nodes, const int32_t* __restrict__ ptr,
+                                                             const int32_t* __restrict__ inc,
+                                                             const T* __restrict__ rec,
+                                                             const double* __restrict__ base, double scale,
+                                                             const double* __restrict__ f_ext,
+                                                             const uint8_t* __restrict__ fixed,
+                                                             double* __restrict__ out, double* __restrict__ part,
+                                                             unsigned int* __restrict__ count,
+                                                             double* __restrict__ norm2) {
+  static_assert(XK_REC_S == 9 && XK_REC_V == 11, "combined record layout");
+  __shared__ T s_acc[3 * GFN_NODES];
+  __shared__ double s_sq[6 * GFN_NODES];
+  const int local = threadIdx.x / GF_LANES, lane = threadIdx.x % GF_LANES, v0 = blockIdx.x * GFN_NODES;
+  const bool live = v0 + local < n_nodes;
+  // the DOFs of the CTA's nodes, one a thread, on their way while the records are gathered
+  const long long dof = 6LL * v0 + threadIdx.x;
+  const bool mine = threadIdx.x < 6 * GFN_NODES && dof < 6LL * n_nodes;
+  double r = 0.0, f = 0.0;
+  bool fix = false;
+  if (mine) {
+    if (base) r = base[dof];
+    if (f_ext) f = f_ext[dof];
+    if (fixed) fix = fixed[dof] != 0;
+  }
+  T acc[3] = {T(0), T(0), T(0)};
+  if (live && ptr) {
+    const int x0 = ptr[v0 + local], x1 = ptr[v0 + local + 1];
+    for (int x = x0 + lane; x < x1; x += 2 * GF_LANES) {
+      const bool two = x + GF_LANES < x1;
+      const int c0 = inc[x], c1 = two ? inc[x + GF_LANES] : c0;
+      T q[2][5];
+      load_stv(rec + (long long)(c0 >> 2) * XK_REC_STRIDE_COMBINED, q[0]);
+      if (two) load_stv(rec + (long long)(c1 >> 2) * XK_REC_STRIDE_COMBINED, q[1]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (j == 1 && !two) break;
+        const T c = shape_c<T>(q[j][0], q[j][1], (j == 0 ? c0 : c1) & 3);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[d] += c * q[j][2 + d];
+      }
+    }
+  }
+#pragma unroll
+  for (int o = GF_LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) acc[d] += __shfl_down_sync(0xffffffffu, acc[d], o, GF_LANES);
+  if (lane == 0)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s_acc[3 * local + d] = acc[d];
+  __syncthreads();
+  if (threadIdx.x < 6 * GFN_NODES) {
+    if (mine) {
+      const int d = threadIdx.x % 6;
+      if (d < 3) r += scale * to_f64(s_acc[3 * (threadIdx.x / 6) + d]);
+      if (f_ext) r -= f;
+      if (fix) r = 0.0;
+      out[dof] = r;
+    }
+    s_sq[threadIdx.x] = r * r;
+  }
+  if (!norm2) return;  // uniform over the launch
+  __syncthreads();
+  double b = 0.0;
+  if (threadIdx.x < 32) {  // the FP64 pipe takes a warp's addition for as long as a thread's: one warp adds
+#pragma unroll
+    for (int k = 0; k < 6 * GFN_NODES / 32; ++k) b += s_sq[threadIdx.x + 32 * k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  norm2_of_blocks<GFN_T>(b, part, count, norm2);
+}
+
 // Column of s (then t) in a record of RS values: combined records put B first.
 template <int RS>
 __host__ __device__ constexpr int rec_st() { return RS == XK_REC_STRIDE_COMBINED ? XK_REC_S : 0; }
@@ -926,9 +1056,6 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 7 : 4) k_elem_sums_rec(i
 // f_ext and out are 16-byte aligned and moved as double2.
 constexpr int GFE_T = 256;
 
-XK_D double to_f64(float x) { return xk_f2d(x); }  // the conversion in integer arithmetic (the FP64 pipe is slow)
-XK_D double to_f64(double x) { return x; }
-
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(GFE_T) k_gather_force_elem(int n_nodes, int ne, const int32_t* __restrict__ neptr,
                                                              const int2* __restrict__ nelem, const T* __restrict__ S,
@@ -938,8 +1065,6 @@ __global__ void __launch_bounds__(GFE_T) k_gather_force_elem(int n_nodes, int ne
                                                              double* __restrict__ out, double* __restrict__ part,
                                                              unsigned int* __restrict__ count,
                                                              double* __restrict__ norm2) {
-  __shared__ double red[GFE_T / 32];
-  __shared__ bool last;
   const int v = blockIdx.x * GFE_T + threadIdx.x;
   double sq = 0.0;
   if (v < n_nodes) {
@@ -999,33 +1124,15 @@ __global__ void __launch_bounds__(GFE_T) k_gather_force_elem(int n_nodes, int ne
     for (int c = 0; c < 6; ++c) sq = fma(r[c], r[c], sq);
   }
   if (!norm2) return;  // uniform over the launch
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ double red[GFE_T / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-  if (lane == 0) red[warp] = sq;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0.0;
+  double b = 0.0;
+  if (threadIdx.x == 0)
     for (int w = 0; w < GFE_T / 32; ++w) b += red[w];
-    part[blockIdx.x] = b;
-    __threadfence();
-    last = atomicAdd(count, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double a = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += GFE_T) a += __ldcg(part + b);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-  if (lane == 0) red[warp] = a;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < GFE_T / 32; ++w) t += red[w];
-    *norm2 = t;
-    *count = 0u;  // ready for the next launch
-  }
+  norm2_of_blocks<GFE_T>(b, part, count, norm2);
 }
 
 template <typename T>
@@ -1544,6 +1651,30 @@ extern "C" xk_status xk_contact_gather_force(const xk_contact_pattern* pat, cons
   return XK_OK;
 }
 
+// xk_contact_gather_force from combined records with the norm fused, for a caller that owns the pattern's
+// norm_scratch (calls that overlap on one pattern would race on it).
+xk_status xk_contact_gather_force_norm(const xk_contact_pattern* pat, const void* rec, int precision,
+                                       const double* base, double scale, const double* f_ext, const uint8_t* fixed,
+                                       double* out, double* norm2, xk_stream s) {
+  const int nn = pat->n_nodes;
+  if (nn <= 0 || !out || !pat->norm_scratch || ((uintptr_t)rec & 15) != 0)
+    return xk_contact_gather_force(pat, rec, precision, XK_OUT_COMBINED, XK_WHICH_COMBINED, base, scale, f_ext, fixed,
+                                   out, norm2, s);
+  const bool use = pat->n_members > 0 && rec;
+  const int32_t* ptr = use ? pat->inc_ptr : nullptr;
+  const int nb = xk_blocks((long long)GF_LANES * nn, GFN_T);
+  unsigned int* count = norm_count(pat->norm_scratch, nn);
+  cudaStream_t st = (cudaStream_t)s;
+  if (precision == XK_FP64)
+    k_gather_force_norm<double><<<nb, GFN_T, 0, st>>>(nn, ptr, pat->inc, (const double*)rec, base, scale, f_ext, fixed,
+                                                      out, pat->norm_scratch, count, norm2);
+  else
+    k_gather_force_norm<float><<<nb, GFN_T, 0, st>>>(nn, ptr, pat->inc, (const float*)rec, base, scale, f_ext, fixed,
+                                                     out, pat->norm_scratch, count, norm2);
+  XK_CHECK_LAUNCH();
+  return XK_OK;
+}
+
 extern "C" xk_status xk_contact_gather_force_elem(const xk_contact_pattern* pat, int precision, const double* base,
                                                   double scale, const double* f_ext, const uint8_t* fixed,
                                                   double* out, double* norm2, xk_stream s) {
@@ -1557,9 +1688,9 @@ extern "C" xk_status xk_contact_gather_force_elem(const xk_contact_pattern* pat,
     if (norm2) XK_CUDA(cudaMemsetAsync(norm2, 0, sizeof(double), (cudaStream_t)s));
     return XK_OK;
   }
-  const int nb = xk_blocks(nn, GFE_T);  // <= (6 n_nodes + 255) / 256, the partial sums of norm_scratch
+  const int nb = xk_blocks(nn, GFE_T);  // at most (6 n_nodes + 255) / 256 block sums fit norm_scratch
   double* part = pat->norm_scratch;
-  unsigned int* count = part ? reinterpret_cast<unsigned int*>(part + nb) : nullptr;
+  unsigned int* count = norm_count(part, nn);
   const int2* nelem = reinterpret_cast<const int2*>(pat->node_elem);
   const bool vec = ((uintptr_t)base & 15) == 0 && ((uintptr_t)f_ext & 15) == 0 && ((uintptr_t)out & 15) == 0;
   cudaStream_t st = (cudaStream_t)s;
