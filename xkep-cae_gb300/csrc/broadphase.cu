@@ -25,7 +25,7 @@
 #include <atomic>
 #include <cstdio>
 
-#include "xk_common.cuh"
+#include "merge.cuh"
 
 namespace {
 
@@ -596,18 +596,34 @@ __global__ void __launch_bounds__(BP_T) k_slots_emit(long long ne, const int32_t
 // ------------------------------------------------------------------------- merge
 
 
-// start[s] = the first row of a list sorted by (a, b) whose a >= s, s in [0, ne] (a binary search per s; the
-// rows' a values are read at stride S: 1 for a table, 2 for (a, b) rows)
+// The first row of a list sorted by a (read at stride S) whose a >= s: eight-way steps, whose seven loads wait
+// together (a binary search's twenty wait in turn).
 template <int S>
-__global__ void k_seg_start(const int32_t* __restrict__ a, long long n, long long ne, int32_t* __restrict__ start) {
-  long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s > ne) return;
-  long long lo = 0, hi = n;
-  while (lo < hi) {
-    long long mid = (lo + hi) >> 1;
-    if (a[S * mid] < s) lo = mid + 1; else hi = mid;
+XK_D int32_t row_start(const int32_t* __restrict__ a, long long n, long long s) {
+  long long lo = 0, hi = n;  // rows below lo are < s, rows from hi on are >= s
+  while (hi - lo > 8) {
+    const long long step = (hi - lo) >> 3;
+    int32_t v[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) v[k] = a[S * (lo + (k + 1) * step)];
+    int less = 0;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) less += v[k] < s;
+    if (less < 7) hi = lo + (less + 1) * step;
+    if (less > 0) lo += less * step + 1;
   }
-  start[s] = (int32_t)lo;
+  int less = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) less += lo + k < hi && a[S * (lo + k)] < s;
+  return (int32_t)(lo + less);
+}
+
+// Row ranges of the segments, s in [0, ne]: ostart of the table, cstart of the candidate rows.
+__global__ void k_seg_starts(const int32_t* __restrict__ old, long long no, const int32_t* __restrict__ cand,
+                             long long nc, long long ne, int32_t* __restrict__ ostart, int32_t* __restrict__ cstart) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x <= ne) ostart[x] = row_start<1>(old, no, x);
+  else if (x <= 2 * ne + 1) cstart[x - ne - 1] = row_start<2>(cand, nc, x - ne - 1);
 }
 
 // the first row in [lo, hi) of a list sorted by b within one a whose b >= key
@@ -619,117 +635,76 @@ XK_D long long lower_bound_b(const int32_t* __restrict__ b, int S, long long lo,
   return lo;
 }
 
-XK_D long long lower_bound_old(const xk_pairs& p, const int32_t* __restrict__ start, int a, int b) {
-  return lower_bound_b(p.eb, 1, start[a], start[a + 1], b);
-}
-XK_D long long lower_bound_cand(const int32_t* c, const int32_t* __restrict__ start, int a, int b) {
-  return lower_bound_b(c + 1, 2, start[a], start[a + 1], b);
-}
-
-XK_D void copy_state(const xk_pairs& a, long long i, xk_pairs& b, long long j) {
-  const long long ca = a.cap, cb = b.cap;
-  b.ea[j] = a.ea[i];
-  b.eb[j] = a.eb[i];
-  b.s[j] = a.s[i];
-  b.t[j] = a.t[i];
-  b.gap[j] = a.gap[i];
-  for (int c = 0; c < 3; ++c) {
-    b.normal[c * cb + j] = a.normal[c * ca + i];
-    b.t1[c * cb + j] = a.t1[c * ca + i];
-    b.t2[c * cb + j] = a.t2[c * ca + i];
-  }
-  b.lambda_n[j] = a.lambda_n[i];
-  b.k_pen[j] = a.k_pen[i];
-  b.k_t[j] = a.k_t[i];
-  b.p_n[j] = a.p_n[i];
-  b.z_t[j] = a.z_t[i];
-  b.z_t[cb + j] = a.z_t[ca + i];
-  b.q_trial_norm[j] = a.q_trial_norm[i];
-  b.dissipation[j] = a.dissipation[i];
-  b.status[j] = a.status[i];
-  b.stick[j] = a.stick[i];
-  if (b.coat_cc) {  // coated wires: the coating state travels with the pair (fresh if the source has none)
-    const bool has = a.coat_cc != nullptr;
-    b.coat_cc[j] = has ? a.coat_cc[i] : 0.0;
-    b.coat_cc_prev[j] = has ? a.coat_cc_prev[i] : 0.0;
-    b.coat_z_t[j] = has ? a.coat_z_t[i] : 0.0;
-    b.coat_z_t[cb + j] = has ? a.coat_z_t[ca + i] : 0.0;
-    b.coat_qtn[j] = has ? a.coat_qtn[i] : 0.0;
-    b.coat_diss[j] = has ? a.coat_diss[i] : 0.0;
-    b.coat_stick[j] = has ? a.coat_stick[i] : 1;
-  }
-}
-
-// r[o] = 1 for an old pair that stays as an old-only (INACTIVE) pair: not a candidate, and with DROP not
-// pristine either (status INACTIVE, p_n = k_pen = 0, z_t = 0)
+// A warp per segment: which of its old rows stay as old-only (INACTIVE) pairs (not a candidate, and with DROP not
+// pristine either: status INACTIVE, p_n = k_pen = 0, z_t = 0), one bit each, 32 rows a word; cnt = rows of the
+// merged segment.  The words of segment w stand from (ostart[w] >> 5) + w on: segments do not share one.
+XK_D long long stay_word(long long o0, long long w) { return (o0 >> 5) + w; }
 template <bool DROP>
-__global__ void k_merge_flags(xk_pairs old, const int32_t* __restrict__ cand, const int32_t* __restrict__ cstart,
-                              long long nc, int32_t* __restrict__ r) {
-  long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o > old.n) return;
-  if (o == old.n) { r[o] = 0; return; }
-  const int a = old.ea[o], b = old.eb[o];
-  long long l = lower_bound_cand(cand, cstart, a, b);
-  bool found = l < nc && cand[2 * l] == a && cand[2 * l + 1] == b;
-  bool stays = !found;
-  if (DROP && stays) {
-    const long long c = old.cap;
-    stays = old.status[o] != 0 || old.p_n[o] != 0.0 || old.k_pen[o] != 0.0 || old.z_t[o] != 0.0 ||
-            old.z_t[c + o] != 0.0;
+__global__ void __launch_bounds__(BP_T) k_merge_count(xk_pairs old, const int32_t* __restrict__ cand,
+                                                      const int32_t* __restrict__ ostart,
+                                                      const int32_t* __restrict__ cstart, long long ne,
+                                                      unsigned* __restrict__ stay, int32_t* __restrict__ cnt) {
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= ne) return;
+  const long long o0 = ostart[w], o1 = ostart[w + 1], c0 = cstart[w], c1 = cstart[w + 1];
+  int n = (int)(c1 - c0);
+  for (long long j = 0; o0 + 32 * j < o1; ++j) {
+    const long long o = o0 + 32 * j + lane;
+    bool stays = false;
+    if (o < o1) {
+      const int b = old.eb[o];
+      const long long l = lower_bound_b(cand + 1, 2, c0, c1, b);
+      stays = !(l < c1 && cand[2 * l + 1] == b);
+      if (DROP && stays)
+        stays = old.status[o] != 0 || old.p_n[o] != 0.0 || old.k_pen[o] != 0.0 || old.z_t[o] != 0.0 ||
+                old.z_t[old.cap + o] != 0.0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, stays);
+    if (lane == 0) stay[stay_word(o0, w) + j] = m;
+    n += __popc(m);
   }
-  r[o] = stays ? 1 : 0;
+  if (lane == 0) cnt[w] = n;
 }
 
-__global__ void k_merge_new(xk_pairs old, const int32_t* __restrict__ ostart, const int32_t* __restrict__ cand,
-                            long long nc, const int32_t* __restrict__ R, xk_pairs out) {
-  long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nc) return;
-  const int a = cand[2 * k], b = cand[2 * k + 1];
-  long long lo = lower_bound_old(old, ostart, a, b);
-  long long pos = k + R[lo];
-  if (lo < old.n && old.ea[lo] == a && old.eb[lo] == b) {
-    copy_state(old, lo, out, pos);
-    return;
+// A warp per segment: ea, eb and source of its merged rows in order of eb.  src: the old row it continues, or
+// MERGE_NEW, or MERGE_OLD - o for the old-only row o.
+__global__ void __launch_bounds__(BP_T) k_merge_order(xk_pairs old, const int32_t* __restrict__ cand,
+                                                      const int32_t* __restrict__ ostart,
+                                                      const int32_t* __restrict__ cstart, long long ne,
+                                                      const unsigned* __restrict__ stay,
+                                                      const int32_t* __restrict__ off, int32_t* __restrict__ ea,
+                                                      int32_t* __restrict__ eb, int32_t* __restrict__ src) {
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= ne) return;
+  const long long o0 = ostart[w], o1 = ostart[w + 1], c0 = cstart[w], c1 = cstart[w + 1], base = off[w];
+  const unsigned* const words = stay + stay_word(o0, w);
+  for (long long k = c0 + lane; k < c1; k += 32) {
+    const int b = cand[2 * k + 1];
+    const long long lo = lower_bound_b(old.eb, 1, o0, o1, b);
+    long long pos = base + (k - c0);
+    for (long long j = 0; 32 * j < lo - o0; ++j) {  // old-only rows before it
+      const long long below = lo - o0 - 32 * j;
+      pos += __popc(words[j] & (below >= 32 ? 0xffffffffu : (1u << below) - 1u));
+    }
+    ea[pos] = (int)w;
+    eb[pos] = b;
+    src[pos] = lo < o1 && old.eb[lo] == b ? (int32_t)lo : MERGE_NEW;
   }
-  const long long cb = out.cap;
-  out.ea[pos] = a;
-  out.eb[pos] = b;
-  out.s[pos] = 0.0;
-  out.t[pos] = 0.0;
-  out.gap[pos] = 0.0;
-  for (int c = 0; c < 3; ++c) {
-    out.normal[c * cb + pos] = 0.0;
-    out.t1[c * cb + pos] = 0.0;
-    out.t2[c * cb + pos] = 0.0;
+  int before = 0;
+  for (long long j = 0; o0 + 32 * j < o1; ++j) {
+    const unsigned m = words[j];
+    if ((m >> lane) & 1u) {
+      const long long o = o0 + 32 * j + lane;
+      const int b = old.eb[o];
+      const long long pos = base + before + __popc(m & ((1u << lane) - 1u)) + (lower_bound_b(cand + 1, 2, c0, c1, b) - c0);
+      ea[pos] = (int)w;
+      eb[pos] = b;
+      src[pos] = MERGE_OLD - (int32_t)o;
+    }
+    before += __popc(m);
   }
-  out.lambda_n[pos] = 0.0;
-  out.k_pen[pos] = 0.0;
-  out.k_t[pos] = 0.0;
-  out.p_n[pos] = 0.0;
-  out.z_t[pos] = 0.0;
-  out.z_t[cb + pos] = 0.0;
-  out.q_trial_norm[pos] = 0.0;
-  out.dissipation[pos] = 0.0;
-  out.status[pos] = 0;
-  out.stick[pos] = 1;
-  if (out.coat_cc) {
-    out.coat_cc[pos] = 0.0;
-    out.coat_cc_prev[pos] = 0.0;
-    out.coat_z_t[pos] = 0.0;
-    out.coat_z_t[cb + pos] = 0.0;
-    out.coat_qtn[pos] = 0.0;
-    out.coat_diss[pos] = 0.0;
-    out.coat_stick[pos] = 1;
-  }
-}
-
-__global__ void k_merge_old(xk_pairs old, const int32_t* __restrict__ cand, const int32_t* __restrict__ cstart,
-                            long long nc, const int32_t* __restrict__ r, const int32_t* __restrict__ R, xk_pairs out) {
-  long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= old.n || !r[o]) return;
-  long long pos = R[o] + lower_bound_cand(cand, cstart, old.ea[o], old.eb[o]);
-  copy_state(old, o, out, pos);
-  out.status[pos] = 0;  // INACTIVE
 }
 
 }  // namespace
@@ -835,38 +810,48 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   }
 }
 
+// The merged rows' order first (two lists of a few dozen rows per segment), then one kernel moves every row's state
+// (pair.cu), with the detection's narrowphase on the way where that is the screened one.
+// A thread per old row and one per candidate, as before, took two passes over the whole table, a scan of its rows
+// and, in a mixed detection, two more passes for the float state and the narrowphase.
+// Measured at the 1027-wire strand (3.2M rows), mixed: 580 us in eight launches -> 380 us in six.
 static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t* cands, int64_t n_cands,
-                            xk_pairs* out, xk_stream s, bool drop) {
+                            xk_pairs* out, xk_stream s, bool drop, const MergeScreen* screen = nullptr) {
   if (!m || !old || !out || (n_cands > 0 && !cands)) return xk_set_error(XK_ERR_ARG, "xk_pairs_merge: null argument");
   if ((long long)out->cap < (long long)old->n + n_cands)
     return xk_set_error(XK_ERR_CAPACITY, "xk_pairs_merge: out->cap < old->n + n_cands");
   cudaStream_t st = (cudaStream_t)s;
   XkScratch S(st);
-  int32_t *r, *R, *ostart, *cstart;
+  int32_t *cnt, *off, *ostart, *cstart, *src, *list = nullptr;
+  unsigned* stay;
   int64_t* tot;
-  const long long ne = m->n_elems;
-  XK_TRY(S.reserve(8 * ((size_t)old->n + 1) + 8 * ((size_t)ne + 2) + (size_t)old->n / 64 + 4096));
-  XK_TRY(S.get(&r, (long long)old->n + 1));
-  XK_TRY(S.get(&R, (long long)old->n + 1));
-  XK_TRY(S.get(&ostart, ne + 2));
-  XK_TRY(S.get(&cstart, ne + 2));
+  const long long ne = m->n_elems, most = (long long)old->n + n_cands, words = old->n / 32 + ne + 1;
+  XK_TRY(S.reserve(4 * (size_t)(4 * ne + most * (screen ? 2 : 1) + words) + 16 * (size_t)(ne / 512) + 16384));
+  XK_TRY(S.get(&cnt, ne + 1));
+  XK_TRY(S.get(&off, ne + 1));
+  XK_TRY(S.get(&ostart, ne + 1));
+  XK_TRY(S.get(&cstart, ne + 1));
+  XK_TRY(S.get(&src, most));
+  XK_TRY(S.get(&stay, words));
   XK_TRY(S.get(&tot, 1));
-  // per-segment row ranges of both sorted lists: each lookup searches only its segment's rows
-  k_seg_start<1><<<xk_blocks(ne + 1, 256), 256, 0, st>>>(old->ea, old->n, ne, ostart);
-  k_seg_start<2><<<xk_blocks(ne + 1, 256), 256, 0, st>>>(cands, n_cands, ne, cstart);
-  if (drop)
-    k_merge_flags<true><<<xk_blocks((long long)old->n + 1, 256), 256, 0, st>>>(*old, cands, cstart, n_cands, r);
-  else
-    k_merge_flags<false><<<xk_blocks((long long)old->n + 1, 256), 256, 0, st>>>(*old, cands, cstart, n_cands, r);
-  XK_CHECK_LAUNCH();
-  XK_TRY(xk_exclusive_scan_i32(r, R, (long long)old->n + 1, tot, st, &S));
-  if (n_cands > 0) k_merge_new<<<xk_blocks(n_cands, 256), 256, 0, st>>>(*old, ostart, cands, n_cands, R, *out);
-  if (old->n > 0) k_merge_old<<<xk_blocks(old->n, 256), 256, 0, st>>>(*old, cands, cstart, n_cands, r, R, *out);
-  XK_CHECK_LAUNCH();
+  if (screen) XK_TRY(S.get(&list, most + 1));
   int64_t h = 0;
-  XK_CUDA(cudaMemcpyAsync(&h, tot, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  XK_CUDA(cudaStreamSynchronize(st));
-  out->n = (int32_t)(n_cands + h);
+  if (ne > 0) {
+    const int warp_blocks = xk_blocks(ne * 32, BP_T);
+    k_seg_starts<<<xk_blocks(2 * ne + 2, 128), 128, 0, st>>>(old->ea, old->n, cands, n_cands, ne, ostart, cstart);
+    if (drop)
+      k_merge_count<true><<<warp_blocks, BP_T, 0, st>>>(*old, cands, ostart, cstart, ne, stay, cnt);
+    else
+      k_merge_count<false><<<warp_blocks, BP_T, 0, st>>>(*old, cands, ostart, cstart, ne, stay, cnt);
+    XK_CHECK_LAUNCH();
+    XK_TRY(xk_exclusive_scan_i32(cnt, off, ne, tot, st, &S));
+    k_merge_order<<<warp_blocks, BP_T, 0, st>>>(*old, cands, ostart, cstart, ne, stay, off, out->ea, out->eb, src);
+    XK_CHECK_LAUNCH();
+    XK_TRY(xk_merge_rows(m, old, src, tot, most, out, screen, list, st));
+    XK_CUDA(cudaMemcpyAsync(&h, tot, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    XK_CUDA(cudaStreamSynchronize(st));
+  }
+  out->n = (int32_t)h;
   return XK_OK;
 }
 
@@ -878,4 +863,18 @@ extern "C" xk_status xk_pairs_merge(const xk_mesh* m, const xk_pairs* old, const
 extern "C" xk_status xk_pairs_merge_pruned(const xk_mesh* m, const xk_pairs* old, const int32_t* cands,
                                            int64_t n_cands, xk_pairs* out, xk_stream s) {
   return merge_impl(m, old, cands, n_cands, out, s, true);
+}
+
+extern "C" xk_status xk_pairs_merge_screened(const xk_mesh* m, const xk_pairs* old, const xk_pairs32* old32,
+                                             const int32_t* cands, int64_t n_cands, xk_pairs* out, int drop,
+                                             const double* u, const float* node32, const xk_contact_params* cp,
+                                             int32_t* n_exact, xk_stream s) {
+  if (!u || !node32 || !cp || !n_exact) return xk_set_error(XK_ERR_ARG, "xk_pairs_merge_screened: null argument");
+  if (m && (m->core_radii || (out && out->coat_cc)))
+    return xk_set_error(XK_ERR_ARG, "xk_pairs_merge_screened: not for coated wires");
+  if (old32 && (drop || !old32->slot || !old || old32->n != old->n))
+    return xk_set_error(XK_ERR_ARG, "xk_pairs_merge_screened: the float table needs its slots and the table's rows, "
+                                    "and no pruning");
+  const MergeScreen q{old32, u, node32, cp, n_exact};
+  return merge_impl(m, old, cands, n_cands, out, s, drop != 0, &q);
 }

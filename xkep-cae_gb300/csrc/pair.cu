@@ -6,7 +6,7 @@
 #include <cmath>
 #include <mutex>
 
-#include "xk_common.cuh"
+#include "merge.cuh"
 #include "segment.cuh"
 
 namespace {
@@ -1325,13 +1325,10 @@ XK_D void store3f(float* base, long long stride, long long i, const float* v) {
 // the decisions are all in float (FP64 runs at 1/64 of the FP32 rate on this GPU); the bound is
 // rounded up and the band's ends rounded outward, so that a gap outside the band lies on the same side
 // of the thresholds as the exact one.
-__global__ void __launch_bounds__(PAIR_T) k_narrow_screen(xk_mesh m, xk_pairs p, const float* __restrict__ n32,
-                                                         float g_on_lo, float g_off_hi, int allow_deact,
-                                                         int32_t* __restrict__ list) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= p.n) return;
-  const long long cap = p.cap;
-  const int ea = p.ea[i], eb = p.eb[i];
+// One pair's screen: s, t, gap and frame in float (n and t1 hold the previous ones on entry).  True: to the exact
+// routine.  lo, hi: the band's ends.
+XK_D bool screen32(const xk_mesh& m, const float* __restrict__ n32, int ea, int eb, float g_on_lo, float g_off_hi,
+                   float* n, float* t1, float* t2, float& s, float& t, float& gap, float& lo, float& hi) {
   const PairNodes pn = pair_nodes(m, ea, eb);
   const int nd[4] = {pn.n[0], pn.n[1], pn.n[2], pn.n[3]};
   const double rs = xadd(m.radii[ea], m.radii[eb]);
@@ -1349,39 +1346,130 @@ __global__ void __launch_bounds__(PAIR_T) k_narrow_screen(xk_mesh m, xk_pairs p,
       scale = fmaxf(scale, fmaxf(fabsf(xh[1][c] - xh[0][c]), fmaxf(fabsf(xh[3][c] - xh[2][c]),
                                                                    fabsf(xh[0][c] - xh[2][c]))));
   }
-  float n[3], t1[3], t2[3], sf, tf, gf;
-  {
-    double v[3];
-    load3(p.normal, cap, i, v);
-    for (int c = 0; c < 3; ++c) n[c] = xk_d2f(v[c]);
-    load3(p.t1, cap, i, v);
-    for (int c = 0; c < 3; ++c) t1[c] = xk_d2f(v[c]);
-  }
-  const bool deferred = m.core_radii != nullptr || narrow32<false, true>(n32, nd, R, sf, tf, gf, n, t1, t2);
+  const bool deferred = m.core_radii != nullptr || narrow32<false, true>(n32, nd, R, s, t, gap, n, t1, t2);
   const float u24 = 5.9604645e-8f;  // 2^-24
   const float pe = 8.0e3f * u24 * scale;
   // eps = 2e-5 scale + pe^2 / (2 r_s), raised by 2^-20 of itself for its own roundings (the fast
   // division's 2 ulp and the float constants included)
   const float eps = (2e-5f * scale + __fdividef(pe * pe, 2.0f * rh)) * (1.0f + 9.5367432e-7f);
-  const float lo = __fsub_rd(g_on_lo, eps), hi = __fadd_ru(g_off_hi, eps);
-  if (deferred || (gf >= lo && gf <= hi)) {
-    list[1 + atomicAdd(list, 1)] = i;
-    return;
-  }
-  p.s[i] = xk_f2d(sf);
-  p.t[i] = xk_f2d(tf);
-  p.gap[i] = xk_f2d(gf);
+  lo = __fsub_rd(g_on_lo, eps);
+  hi = __fadd_ru(g_off_hi, eps);
+  return deferred || (gap >= lo && gap <= hi);
+}
+
+XK_D void store_screened(const xk_pairs& p, int i, float s, float t, float gap, const float* n, const float* t1,
+                         const float* t2) {
+  p.s[i] = xk_f2d(s);
+  p.t[i] = xk_f2d(t);
+  p.gap[i] = xk_f2d(gap);
   const double nn[3] = {xk_f2d(n[0]), xk_f2d(n[1]), xk_f2d(n[2])};
   const double tt1[3] = {xk_f2d(t1[0]), xk_f2d(t1[1]), xk_f2d(t1[2])};
   const double tt2[3] = {xk_f2d(t2[0]), xk_f2d(t2[1]), xk_f2d(t2[2])};
-  store3(p.normal, cap, i, nn);
-  store3(p.t1, cap, i, tt1);
-  store3(p.t2, cap, i, tt2);
-  const uint8_t st = p.status[i];  // gf is outside [lo, hi]: the exact gap is on the same side of both thresholds
-  if (st == ST_INACTIVE) {
-    if (gf < lo) p.status[i] = ST_ACTIVE;
-  } else if (allow_deact && gf > hi) {
-    p.status[i] = ST_INACTIVE;
+  store3(p.normal, p.cap, i, nn);
+  store3(p.t1, p.cap, i, tt1);
+  store3(p.t2, p.cap, i, tt2);
+}
+
+// gf outside [lo, hi]: the exact gap is on the same side of both thresholds
+XK_D uint8_t screened_status(uint8_t st, float gf, float lo, float hi, int allow_deact) {
+  if (st == ST_INACTIVE) return gf < lo ? ST_ACTIVE : st;
+  return allow_deact && gf > hi ? ST_INACTIVE : st;
+}
+
+__global__ void __launch_bounds__(PAIR_T) k_narrow_screen(xk_mesh m, xk_pairs p, const float* __restrict__ n32,
+                                                         float g_on_lo, float g_off_hi, int allow_deact,
+                                                         int32_t* __restrict__ list) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.n) return;
+  float n[3], t1[3], t2[3], s, t, gap, lo, hi;
+  {
+    double v[3];
+    load3(p.normal, p.cap, i, v);
+    for (int c = 0; c < 3; ++c) n[c] = xk_d2f(v[c]);
+    load3(p.t1, p.cap, i, v);
+    for (int c = 0; c < 3; ++c) t1[c] = xk_d2f(v[c]);
+  }
+  if (screen32(m, n32, p.ea[i], p.eb[i], g_on_lo, g_off_hi, n, t1, t2, s, t, gap, lo, hi)) {
+    list[1 + atomicAdd(list, 1)] = i;
+    return;
+  }
+  store_screened(p, i, s, t, gap, n, t1, t2);
+  const uint8_t st = p.status[i], now = screened_status(st, gap, lo, hi, allow_deact);
+  if (now != st) p.status[i] = now;
+}
+
+// The rows of a merge (merge.cuh): continued state, fresh state, or an old-only row (INACTIVE).  FROM32: the old
+// state is the float table's, read through its slots (as k_pairs_from32 would bring it to the double one first);
+// SCREEN: the narrowphase of the row on the way, from the old frame in registers, so that what it replaces is
+// neither written nor read again.  Memory bounds it: a row is 95 (double: 178) bytes in and 178 out.
+template <bool FROM32, bool SCREEN>
+__global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 6) k_merge_rows(
+    const __grid_constant__ xk_mesh m, const __grid_constant__ xk_pairs a, const __grid_constant__ xk_pairs32 q,
+    const int32_t* __restrict__ src, const int64_t* __restrict__ count, const __grid_constant__ xk_pairs out,
+    const float* __restrict__ n32, float g_on_lo, float g_off_hi, int allow_deact, int32_t* __restrict__ list) {
+  const long long n = *count, co = out.cap, ca = a.cap, cq = q.cap;
+  for (long long i = (long long)blockIdx.x * PAIR_T + threadIdx.x; i < n; i += (long long)gridDim.x * PAIR_T) {
+    const int code = src[i];
+    const bool fresh = code == MERGE_NEW, only = code <= MERGE_OLD;
+    const long long o = only ? MERGE_OLD - code : code;  // its old row
+    const long long j = FROM32 && !fresh ? q.slot[o] : 0;
+    // a value of the old state, in double or in float (the float table's values are the double one's)
+    auto get = [&](const double* d, const float* f, int c) {
+      return fresh ? 0.0 : (FROM32 ? xk_f2d(f[c * cq + j]) : d[c * ca + o]);
+    };
+    auto getf = [&](const double* d, const float* f, int c) {
+      return fresh ? 0.0f : (FROM32 ? f[c * cq + j] : xk_d2f(d[c * ca + o]));
+    };
+    uint8_t status = fresh || only ? ST_INACTIVE : (FROM32 ? q.status[j] : a.status[o]);
+    const uint8_t stick = fresh ? 1 : (FROM32 ? q.stick[j] : a.stick[o]);
+    out.lambda_n[i] = fresh ? 0.0 : a.lambda_n[o];  // not in the float table
+    out.k_pen[i] = get(a.k_pen, q.k_pen, 0);
+    out.k_t[i] = get(a.k_t, q.k_t, 0);
+    out.p_n[i] = get(a.p_n, q.p_n, 0);
+    out.z_t[i] = get(a.z_t, q.z_t, 0);
+    out.z_t[co + i] = get(a.z_t, q.z_t, 1);
+    out.q_trial_norm[i] = get(a.q_trial_norm, q.q_trial_norm, 0);
+    out.dissipation[i] = get(a.dissipation, q.dissipation, 0);
+    out.stick[i] = stick;
+    bool exact = false;
+    if (SCREEN) {
+      float nf[3], t1f[3], t2f[3], s, t, gap, lo, hi;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        nf[c] = getf(a.normal, q.normal, c);
+        t1f[c] = getf(a.t1, q.t1, c);
+      }
+      exact = screen32(m, n32, out.ea[i], out.eb[i], g_on_lo, g_off_hi, nf, t1f, t2f, s, t, gap, lo, hi);
+      if (!exact) {
+        store_screened(out, (int)i, s, t, gap, nf, t1f, t2f);
+        status = screened_status(status, gap, lo, hi, allow_deact);
+      } else {
+        list[1 + atomicAdd(list, 1)] = (int)i;
+      }
+    }
+    out.status[i] = status;
+    if (!SCREEN) {
+      out.s[i] = get(a.s, q.s, 0);
+      out.t[i] = get(a.t, q.t, 0);
+      out.gap[i] = get(a.gap, q.gap, 0);
+      for (int c = 0; c < 3; ++c) out.t2[c * co + i] = get(a.t2, q.t2, c);
+    }
+    if (!SCREEN || exact) {  // the exact routine reads the old frame here and writes the rest
+      for (int c = 0; c < 3; ++c) {
+        out.normal[c * co + i] = get(a.normal, q.normal, c);
+        out.t1[c * co + i] = get(a.t1, q.t1, c);
+      }
+    }
+    if (!SCREEN && out.coat_cc) {  // coated wires: the coating state travels with the pair (fresh if the source has none)
+      const bool has = !fresh && a.coat_cc != nullptr;
+      out.coat_cc[i] = has ? a.coat_cc[o] : 0.0;
+      out.coat_cc_prev[i] = has ? a.coat_cc_prev[o] : 0.0;
+      out.coat_z_t[i] = has ? a.coat_z_t[o] : 0.0;
+      out.coat_z_t[co + i] = has ? a.coat_z_t[ca + o] : 0.0;
+      out.coat_qtn[i] = has ? a.coat_qtn[o] : 0.0;
+      out.coat_diss[i] = has ? a.coat_diss[o] : 0.0;
+      out.coat_stick[i] = has ? a.coat_stick[o] : 1;
+    }
   }
 }
 
@@ -1653,6 +1741,43 @@ extern "C" xk_status xk_narrowphase(const xk_mesh* m, xk_pairs* p, const double*
   return XK_OK;
 }
 
+// the active-set thresholds rounded outward to float
+static void screen_band(const xk_contact_params& cp, float* on_lo, float* off_hi) {
+  *on_lo = (float)cp.g_on;
+  *off_hi = (float)cp.g_off;
+  if ((double)*on_lo > cp.g_on) *on_lo = std::nextafter(*on_lo, -INFINITY);
+  if ((double)*off_hi < cp.g_off) *off_hi = std::nextafter(*off_hi, INFINITY);
+}
+
+xk_status xk_merge_rows(const xk_mesh* m, const xk_pairs* old, const int32_t* src, const int64_t* n, long long most,
+                        xk_pairs* out, const MergeScreen* screen, int32_t* list, cudaStream_t st) {
+  if (screen) XK_CUDA(cudaMemsetAsync(list, 0, sizeof(int32_t), st));
+  if (most > 0) {
+    // the number of rows is on the device: a grid of at most eight rounds of the SMs strides over them
+    const long long cap = 64LL * xk_sm_count(), blocks = (most + PAIR_T - 1) / PAIR_T;
+    const int nb = (int)(blocks < cap ? blocks : cap);
+    const xk_pairs32 none = {};
+    float on_lo = 0.0f, off_hi = 0.0f;
+    if (!screen) {
+      k_merge_rows<false, false><<<nb, PAIR_T, 0, st>>>(*m, *old, none, src, n, *out, nullptr, on_lo, off_hi, 0, nullptr);
+    } else {
+      const xk_contact_params& cp = *screen->cp;
+      screen_band(cp, &on_lo, &off_hi);
+      if (screen->old32)
+        k_merge_rows<true, true><<<nb, PAIR_T, 0, st>>>(*m, *old, *screen->old32, src, n, *out, screen->node32, on_lo,
+                                                        off_hi, cp.allow_deactivation, list);
+      else
+        k_merge_rows<false, true><<<nb, PAIR_T, 0, st>>>(*m, *old, none, src, n, *out, screen->node32, on_lo, off_hi,
+                                                         cp.allow_deactivation, list);
+      k_narrow_exact_list<<<2 * xk_sm_count(), PAIR_T, 0, st>>>(*m, *out, screen->u, cp.g_on, cp.g_off,
+                                                                cp.allow_deactivation, list);
+    }
+    XK_CHECK_LAUNCH();
+  }
+  if (screen) XK_CUDA(cudaMemcpyAsync(screen->n_exact, list, sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+  return XK_OK;
+}
+
 extern "C" xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, const double* u, const float* node32,
                                              const xk_contact_params* cp, int32_t* n_exact, xk_stream s) {
   if (!m || !p || !u || !node32 || !cp) return xk_set_error(XK_ERR_ARG, "xk_narrowphase_screened: null argument");
@@ -1666,10 +1791,8 @@ extern "C" xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, cons
   xk_status r = XK_OK;
   cudaError_t e = cudaMemsetAsync(list, 0, sizeof(int32_t), st);
   if (e == cudaSuccess) {
-    // the thresholds rounded outward to float
-    float on_lo = (float)cp->g_on, off_hi = (float)cp->g_off;
-    if ((double)on_lo > cp->g_on) on_lo = std::nextafter(on_lo, -INFINITY);
-    if ((double)off_hi < cp->g_off) off_hi = std::nextafter(off_hi, INFINITY);
+    float on_lo, off_hi;
+    screen_band(*cp, &on_lo, &off_hi);
     k_narrow_screen<<<xk_blocks(p->n, PAIR_T), PAIR_T, 0, st>>>(*m, *p, node32, on_lo, off_hi,
                                                                cp->allow_deactivation, list);
     k_narrow_exact_list<<<2 * xk_sm_count(), PAIR_T, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation,

@@ -262,14 +262,17 @@ class AssemblyEngine:
         s = stream_handle(stream)
         self._phase_marks = []
         self._mark("start", stream)
-        self.sync_state(stream)
+        screened = self.precision == L.XK_MIXED and self.screened_detection and not self.coated
+        # the merge of a screened detection reads the float state itself
+        from32 = screened and self._state_in32 and self.pruner is None and self.pairs32.c.n == self.pairs.n
+        if not from32:
+            self.sync_state(stream)
         self._mark("table_back", stream)
         cands, nc = self.candidates(u, stream)
         self._mark("broadphase", stream)
         n_raw, n_pre = self._bp_counts
         n_all = nc
         self._merge_pruned = False
-        screened = self.precision == L.XK_MIXED and self.screened_detection and not self.coated
         if self.pruner is not None or screened:  # node records at u: pruning features, screened narrowphase
             L.call("xk_nodes_prepare", C.byref(self.mesh.c), ptr(u), ptr(u), ptr(self.node32), s)
         if self.pruner is not None:
@@ -279,15 +282,18 @@ class AssemblyEngine:
         need = self.pairs.n + nc
         if self._spare.cap < need:
             self._spare.reserve(int(need * 1.25) + 64, keep=False)
-        L.call("xk_pairs_merge_pruned" if self._merge_pruned else "xk_pairs_merge", C.byref(self.mesh.c),
-               C.byref(self.pairs.c), ptr(cands), nc, C.byref(self._spare.c), s)
+        if screened:  # the narrowphase is part of the merge's pass over the rows
+            L.call("xk_pairs_merge_screened", C.byref(self.mesh.c), C.byref(self.pairs.c),
+                   C.byref(self.pairs32.c) if from32 else None, ptr(cands), nc, C.byref(self._spare.c),
+                   int(self._merge_pruned), ptr(u), ptr(self.node32), C.byref(self.cp), ptr(self._n_exact), s)
+        else:
+            L.call("xk_pairs_merge_pruned" if self._merge_pruned else "xk_pairs_merge", C.byref(self.mesh.c),
+                   C.byref(self.pairs.c), ptr(cands), nc, C.byref(self._spare.c), s)
+        self._state_in32 = False
         self._spare.set_n(self._spare.c.n)
         self.pairs, self._spare = self._spare, self.pairs
         self._mark("merge", stream)
-        if screened:
-            L.call("xk_narrowphase_screened", C.byref(self.mesh.c), C.byref(self.pairs.c), ptr(u), ptr(self.node32),
-                   C.byref(self.cp), ptr(self._n_exact), s)
-        else:
+        if not screened:
             L.call("xk_narrowphase", C.byref(self.mesh.c), C.byref(self.pairs.c), ptr(u), C.byref(self.cp), 1, s)
         self._mark("narrowphase", stream)
         self.pattern.build(self.pairs, stream)
