@@ -13,7 +13,7 @@ if not torch.cuda.is_available():
 
 from xkgpu import _lib as L  # noqa: E402
 from xkgpu import workloads as W  # noqa: E402
-from xkgpu.device import DeviceMesh, DevicePairTable, ptr, stream_handle  # noqa: E402
+from xkgpu.device import DeviceMesh, DevicePairTable, DevicePairTable32, ptr, stream_handle  # noqa: E402
 from xkgpu.engine import AssemblyEngine  # noqa: E402
 
 COUNTS = [0, 0, 1, 31, 32, 33, 64, 65, 97, 2, 0, 130]
@@ -107,3 +107,53 @@ def test_screened_merge_is_merge_then_narrowphase(workload, from32):
     assert na == nb and a["ea"].size > 0
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n,kind", [(1, "all"), (255, "some"), (256, "none"), (257, "all"), (3000, "some"),
+                                    (70_000, "runs"), (140_001, "all")])
+def test_float_table_slots(n, kind):
+    """Slots of the float table: members first, both in ascending order; the state comes back to the same pairs."""
+    rng = np.random.default_rng(n)
+    ne = 600
+    k = rng.choice(ne * ne, n, replace=False)
+    k.sort()
+    d = {"ea": k // ne, "eb": k % ne, "stick": rng.random(n) < 0.5}
+    for f in FIELDS:
+        w = {"normal": 3, "t1": 3, "t2": 3, "z_t": 2}.get(f, 1)
+        d[f] = rng.normal(size=(n, w) if w > 1 else n).astype(np.float32).astype(np.float64)
+    mem = {"all": np.ones(n, bool), "none": np.zeros(n, bool), "some": rng.random(n) < 0.2,
+           "runs": (np.arange(n) // 700) % 3 == 1}[kind]
+    d["status"] = np.where(mem, 1, 0)
+    d["p_n"] = np.where(mem, np.abs(d["p_n"]), 0.0)
+    X = rng.normal(size=(ne + 1, 3))
+    mesh = DeviceMesh(X, np.stack([np.arange(ne), np.arange(1, ne + 1)], 1), np.full(ne, 0.1))
+    table = DevicePairTable(mesh.device, cap=n + 16)
+    table.from_host(d)
+    # the pattern's two lists, which are all that the float table takes from it
+    members = torch.as_tensor(np.flatnonzero(mem).astype(np.int32), device="cuda")
+    others = torch.as_tensor(np.flatnonzero(~mem).astype(np.int32), device="cuda")
+    pat = L.ContactPattern()
+    pat.n_nodes, pat.n_members, pat.n_others = ne + 1, members.numel(), others.numel()
+    pat.members, pat.others = ptr(members), ptr(others)
+    q = DevicePairTable32(mesh.device)
+    q.ensure(n)
+    s = stream_handle(None)
+    L.call("xk_pairs_to32", C.byref(mesh.c), C.byref(table.c), C.byref(pat), C.byref(q.c), s)
+    order = np.concatenate([np.flatnonzero(mem), np.flatnonzero(~mem)])
+    assert q.c.n == n and q.c.n_members == mem.sum()
+    assert np.array_equal(q.t["pair"][:n].cpu().numpy(), order)
+    assert np.array_equal(order[q.t["slot"][:n].cpu().numpy()], np.arange(n))
+    assert np.array_equal(q.t["gap"][:n].cpu().numpy(), d["gap"][order].astype(np.float32))
+    conn = mesh.conn.cpu().numpy().reshape(-1, 2)
+    nodes = np.concatenate([conn[d["ea"][order]], conn[d["eb"][order]]], 1)
+    assert np.array_equal(q.t["nodes"][: 4 * n].cpu().numpy().reshape(-1, 4), nodes)
+    back = DevicePairTable(mesh.device, cap=n + 16)
+    back.from_host({**d, **{f: np.zeros_like(d[f]) for f in FIELDS if f != "lambda_n"}})
+    L.call("xk_pairs_from32", C.byref(q.c), C.byref(back.c), s)
+    got = back.to_host()
+    for f in FIELDS:
+        if f == "t2":  # the others' is formed again from the normal and t1
+            assert np.array_equal(got[f][mem], d[f][mem])
+        else:
+            assert np.array_equal(got[f], d[f]), f
+    assert np.array_equal(got["status"], d["status"]) and np.array_equal(got["stick"], d["stick"])

@@ -626,19 +626,35 @@ __global__ void k_seg_starts(const int32_t* __restrict__ old, long long no, cons
   else if (x <= 2 * ne + 1) cstart[x - ne - 1] = row_start<2>(cand, nc, x - ne - 1);
 }
 
-// the first row in [lo, hi) of a list sorted by b within one a whose b >= key
-XK_D long long lower_bound_b(const int32_t* __restrict__ b, int S, long long lo, long long hi, int key) {
-  while (lo < hi) {
-    long long mid = (lo + hi) >> 1;
-    if (b[S * mid] < key) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 // A warp per segment: which of its old rows stay as old-only (INACTIVE) pairs (not a candidate, and with DROP not
 // pristine either: status INACTIVE, p_n = k_pen = 0, z_t = 0), one bit each, 32 rows a word; cnt = rows of the
 // merged segment.  The words of segment w stand from (ostart[w] >> 5) + w on: segments do not share one.
 XK_D long long stay_word(long long o0, long long w) { return (o0 >> 5) + w; }
+
+// A segment's list of b, in a warp's shared memory where it fits (a search there is a few dozen clocks a step, in
+// global memory a few hundred until its lines have come: k_merge_count 36 -> 30 us, k_merge_order 49 -> 40 us at the
+// 1027-wire strand).  rank(key): the entries below key.
+constexpr int SEG_LIST = 128;
+struct SegList {
+  const int32_t* g;  // entry k at g[S k]
+  const int* s;      // or at s[k]
+  int S, n;
+  XK_D int at(int k) const { return s ? s[k] : g[(long long)S * k]; }
+  XK_D int rank(int key) const {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (at(mid) < key) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  }
+};
+XK_D SegList seg_list(const int32_t* g, int S, int n, int* buf, int lane) {
+  SegList r{g, n <= SEG_LIST ? buf : nullptr, S, n};
+  if (r.s)
+    for (int k = lane; k < n; k += 32) buf[k] = g[(long long)S * k];
+  return r;
+}
 template <bool DROP>
 __global__ void __launch_bounds__(BP_T) k_merge_count(xk_pairs old, const int32_t* __restrict__ cand,
                                                       const int32_t* __restrict__ ostart,
@@ -647,15 +663,17 @@ __global__ void __launch_bounds__(BP_T) k_merge_count(xk_pairs old, const int32_
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= ne) return;
+  __shared__ int buf[BP_T / 32][SEG_LIST];
   const long long o0 = ostart[w], o1 = ostart[w + 1], c0 = cstart[w], c1 = cstart[w + 1];
   int n = (int)(c1 - c0);
+  const SegList cl = seg_list(cand + 2 * c0 + 1, 2, n, buf[threadIdx.x >> 5], lane);
+  __syncwarp();
   for (long long j = 0; o0 + 32 * j < o1; ++j) {
     const long long o = o0 + 32 * j + lane;
     bool stays = false;
     if (o < o1) {
-      const int b = old.eb[o];
-      const long long l = lower_bound_b(cand + 1, 2, c0, c1, b);
-      stays = !(l < c1 && cand[2 * l + 1] == b);
+      const int b = old.eb[o], l = cl.rank(b);
+      stays = !(l < cl.n && cl.at(l) == b);
       if (DROP && stays)
         stays = old.status[o] != 0 || old.p_n[o] != 0.0 || old.k_pen[o] != 0.0 || old.z_t[o] != 0.0 ||
                 old.z_t[old.cap + o] != 0.0;
@@ -680,28 +698,31 @@ __global__ void __launch_bounds__(BP_T) k_merge_order(xk_pairs old, const int32_
   if (w >= ne) return;
   const long long o0 = ostart[w], o1 = ostart[w + 1], c0 = cstart[w], c1 = cstart[w + 1], base = off[w];
   const unsigned* const words = stay + stay_word(o0, w);
-  for (long long k = c0 + lane; k < c1; k += 32) {
-    const int b = cand[2 * k + 1];
-    const long long lo = lower_bound_b(old.eb, 1, o0, o1, b);
-    long long pos = base + (k - c0);
-    for (long long j = 0; 32 * j < lo - o0; ++j) {  // old-only rows before it
-      const long long below = lo - o0 - 32 * j;
+  __shared__ int buf[BP_T / 32][2][SEG_LIST];
+  int(*const mine)[SEG_LIST] = buf[threadIdx.x >> 5];
+  const SegList cl = seg_list(cand + 2 * c0 + 1, 2, (int)(c1 - c0), mine[0], lane);
+  const SegList ol = seg_list(old.eb + o0, 1, (int)(o1 - o0), mine[1], lane);
+  __syncwarp();
+  for (int k = lane; k < cl.n; k += 32) {
+    const int b = cl.at(k), lo = ol.rank(b);
+    long long pos = base + k;
+    for (int j = 0; 32 * j < lo; ++j) {  // old-only rows before it
+      const int below = lo - 32 * j;
       pos += __popc(words[j] & (below >= 32 ? 0xffffffffu : (1u << below) - 1u));
     }
     ea[pos] = (int)w;
     eb[pos] = b;
-    src[pos] = lo < o1 && old.eb[lo] == b ? (int32_t)lo : MERGE_NEW;
+    src[pos] = lo < ol.n && ol.at(lo) == b ? (int32_t)(o0 + lo) : MERGE_NEW;
   }
   int before = 0;
-  for (long long j = 0; o0 + 32 * j < o1; ++j) {
+  for (int j = 0; 32 * j < ol.n; ++j) {
     const unsigned m = words[j];
     if ((m >> lane) & 1u) {
-      const long long o = o0 + 32 * j + lane;
-      const int b = old.eb[o];
-      const long long pos = base + before + __popc(m & ((1u << lane) - 1u)) + (lower_bound_b(cand + 1, 2, c0, c1, b) - c0);
+      const int b = ol.at(32 * j + lane);
+      const long long pos = base + before + __popc(m & ((1u << lane) - 1u)) + cl.rank(b);
       ea[pos] = (int)w;
       eb[pos] = b;
-      src[pos] = MERGE_OLD - (int32_t)o;
+      src[pos] = MERGE_OLD - (int32_t)(o0 + 32 * j + lane);
     }
     before += __popc(m);
   }
