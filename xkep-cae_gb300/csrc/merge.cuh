@@ -6,8 +6,7 @@
 // Sources of merged rows that do not continue an old row: a new pair, or MERGE_OLD - o: the old-only row o.
 constexpr int32_t MERGE_NEW = -1, MERGE_OLD = -2;
 
-// The screened detection narrowphase taken on the way, and where the old state is (old32: the float table, by its
-// slots; else the double one).
+// The old state's float table, which holds it, and the screened detection narrowphase taken on the way.
 struct MergeScreen {
   const xk_pairs32* old32;
   const double* u;

@@ -1464,12 +1464,24 @@ __global__ void __launch_bounds__(PAIR_T) k_narrow_screen(xk_mesh m, xk_pairs p,
   if (now != st) p.status[i] = now;
 }
 
-// The rows of a merge (merge.cuh): continued state, fresh state, or an old-only row (INACTIVE).  FROM32: the old
-// state is the float table's, read through its slots (as k_pairs_from32 would bring it to the double one first);
-// SCREEN: the narrowphase of the row on the way, from the old frame in registers, so that what it replaces is
-// neither written nor read again.  Memory bounds it: a row is 95 (double: 178) bytes in and 178 out.
-template <bool FROM32, bool SCREEN>
-__global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 6) k_merge_rows(
+// a value of a row's old state from the table that holds it
+template <bool FLOAT>
+struct RowValue { using T = double; };
+template <>
+struct RowValue<true> { using T = float; };
+XK_D double row_value(const double* d, const float*, double) { return *d; }
+XK_D float row_value(const double*, const float* f, float) { return *f; }
+XK_D double to_f64(float x) { return xk_f2d(x); }
+XK_D double to_f64(double x) { return x; }
+XK_D float to_f32(float x) { return x; }
+XK_D float to_f32(double x) { return xk_d2f(x); }
+
+// The rows of a merge (merge.cuh): continued state, fresh state, or an old-only row (INACTIVE).  SCREEN: the old
+// state is the float table's, read through its slots (as k_pairs_from32 would bring it to the double one first),
+// and the screened narrowphase of the row is taken on the way, from the old frame in registers, so that what it
+// replaces is neither written nor read again.  Memory bounds it: a row is 95 (double: 178) bytes in and 178 out.
+template <bool SCREEN>
+__global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 2) k_merge_rows(
     const __grid_constant__ xk_mesh m, const __grid_constant__ xk_pairs a, const __grid_constant__ xk_pairs32 q,
     const int32_t* __restrict__ src, const int64_t* __restrict__ count, const __grid_constant__ xk_pairs out,
     const float* __restrict__ n32, float g_on_lo, float g_off_hi, int allow_deact, int32_t* __restrict__ list) {
@@ -1478,34 +1490,48 @@ __global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 6) k_merge_rows(
     const int code = src[i];
     const bool fresh = code == MERGE_NEW, only = code <= MERGE_OLD;
     const long long o = only ? MERGE_OLD - code : code;  // its old row
-    const long long j = FROM32 && !fresh ? q.slot[o] : 0;
-    // a value of the old state, in double or in float (the float table's values are the double one's)
-    auto get = [&](const double* d, const float* f, int c) {
-      return fresh ? 0.0 : (FROM32 ? xk_f2d(f[c * cq + j]) : d[c * ca + o]);
-    };
-    auto getf = [&](const double* d, const float* f, int c) {
-      return fresh ? 0.0f : (FROM32 ? f[c * cq + j] : xk_d2f(d[c * ca + o]));
-    };
-    uint8_t status = fresh || only ? ST_INACTIVE : (FROM32 ? q.status[j] : a.status[o]);
-    const uint8_t stick = fresh ? 1 : (FROM32 ? q.stick[j] : a.stick[o]);
-    out.lambda_n[i] = fresh ? 0.0 : a.lambda_n[o];  // not in the float table
-    out.k_pen[i] = get(a.k_pen, q.k_pen, 0);
-    out.k_t[i] = get(a.k_t, q.k_t, 0);
-    out.p_n[i] = get(a.p_n, q.p_n, 0);
-    out.z_t[i] = get(a.z_t, q.z_t, 0);
-    out.z_t[co + i] = get(a.z_t, q.z_t, 1);
-    out.q_trial_norm[i] = get(a.q_trial_norm, q.q_trial_norm, 0);
-    out.dissipation[i] = get(a.dissipation, q.dissipation, 0);
-    out.stick[i] = stick;
+    const long long j = SCREEN && !fresh ? q.slot[o] : 0;
+    // every load of the row before its first store (the compiler cannot know that the tables are distinct, and a
+    // load that waits for a store before it costs its whole latency: 235 -> 188 us at the 1027-wire strand)
+    using V = typename RowValue<SCREEN>::T;
+    auto get = [&](const double* d, const float* f, int c) { return fresh ? V(0) : row_value(d + c * ca + o, f + c * cq + j, V()); };
+    const double lambda = fresh ? 0.0 : a.lambda_n[o];  // not in the float table
+    const V v[7] = {get(a.k_pen, q.k_pen, 0), get(a.k_t, q.k_t, 0), get(a.p_n, q.p_n, 0), get(a.z_t, q.z_t, 0),
+                    get(a.z_t, q.z_t, 1), get(a.q_trial_norm, q.q_trial_norm, 0), get(a.dissipation, q.dissipation, 0)};
+    V vn[3], vt1[3], g[6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      vn[c] = get(a.normal, q.normal, c);
+      vt1[c] = get(a.t1, q.t1, c);
+      if (!SCREEN) g[3 + c] = get(a.t2, q.t2, c);
+    }
+    if (!SCREEN) {
+      g[0] = get(a.s, q.s, 0);
+      g[1] = get(a.t, q.t, 0);
+      g[2] = get(a.gap, q.gap, 0);
+    }
+    uint8_t status = fresh || only ? ST_INACTIVE : (SCREEN ? q.status[j] : a.status[o]);
+    const uint8_t stick = fresh ? 1 : (SCREEN ? q.stick[j] : a.stick[o]);
     bool exact = false;
+    float nf[3], t1f[3], t2f[3], s, t, gap, lo, hi;
     if (SCREEN) {
-      float nf[3], t1f[3], t2f[3], s, t, gap, lo, hi;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        nf[c] = getf(a.normal, q.normal, c);
-        t1f[c] = getf(a.t1, q.t1, c);
+        nf[c] = to_f32(vn[c]);
+        t1f[c] = to_f32(vt1[c]);
       }
       exact = screen32(m, n32, out.ea[i], out.eb[i], g_on_lo, g_off_hi, nf, t1f, t2f, s, t, gap, lo, hi);
+    }
+    out.lambda_n[i] = lambda;
+    out.k_pen[i] = to_f64(v[0]);
+    out.k_t[i] = to_f64(v[1]);
+    out.p_n[i] = to_f64(v[2]);
+    out.z_t[i] = to_f64(v[3]);
+    out.z_t[co + i] = to_f64(v[4]);
+    out.q_trial_norm[i] = to_f64(v[5]);
+    out.dissipation[i] = to_f64(v[6]);
+    out.stick[i] = stick;
+    if (SCREEN) {
       if (!exact) {
         store_screened(out, (int)i, s, t, gap, nf, t1f, t2f);
         status = screened_status(status, gap, lo, hi, allow_deact);
@@ -1515,15 +1541,17 @@ __global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 6) k_merge_rows(
     }
     out.status[i] = status;
     if (!SCREEN) {
-      out.s[i] = get(a.s, q.s, 0);
-      out.t[i] = get(a.t, q.t, 0);
-      out.gap[i] = get(a.gap, q.gap, 0);
-      for (int c = 0; c < 3; ++c) out.t2[c * co + i] = get(a.t2, q.t2, c);
+      out.s[i] = to_f64(g[0]);
+      out.t[i] = to_f64(g[1]);
+      out.gap[i] = to_f64(g[2]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) out.t2[c * co + i] = to_f64(g[3 + c]);
     }
     if (!SCREEN || exact) {  // the exact routine reads the old frame here and writes the rest
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
-        out.normal[c * co + i] = get(a.normal, q.normal, c);
-        out.t1[c * co + i] = get(a.t1, q.t1, c);
+        out.normal[c * co + i] = to_f64(vn[c]);
+        out.t1[c * co + i] = to_f64(vt1[c]);
       }
     }
     if (!SCREEN && out.coat_cc) {  // coated wires: the coating state travels with the pair (fresh if the source has none)
@@ -1825,16 +1853,12 @@ xk_status xk_merge_rows(const xk_mesh* m, const xk_pairs* old, const int32_t* sr
     const xk_pairs32 none = {};
     float on_lo = 0.0f, off_hi = 0.0f;
     if (!screen) {
-      k_merge_rows<false, false><<<nb, PAIR_T, 0, st>>>(*m, *old, none, src, n, *out, nullptr, on_lo, off_hi, 0, nullptr);
+      k_merge_rows<false><<<nb, PAIR_T, 0, st>>>(*m, *old, none, src, n, *out, nullptr, on_lo, off_hi, 0, nullptr);
     } else {
       const xk_contact_params& cp = *screen->cp;
       screen_band(cp, &on_lo, &off_hi);
-      if (screen->old32)
-        k_merge_rows<true, true><<<nb, PAIR_T, 0, st>>>(*m, *old, *screen->old32, src, n, *out, screen->node32, on_lo,
-                                                        off_hi, cp.allow_deactivation, list);
-      else
-        k_merge_rows<false, true><<<nb, PAIR_T, 0, st>>>(*m, *old, none, src, n, *out, screen->node32, on_lo, off_hi,
-                                                         cp.allow_deactivation, list);
+      k_merge_rows<true><<<nb, PAIR_T, 0, st>>>(*m, *old, *screen->old32, src, n, *out, screen->node32, on_lo, off_hi,
+                                                cp.allow_deactivation, list);
       k_narrow_exact_list<<<2 * xk_sm_count(), PAIR_T, 0, st>>>(*m, *out, screen->u, cp.g_on, cp.g_off,
                                                                 cp.allow_deactivation, list);
     }
