@@ -112,12 +112,14 @@ XK_D void make_grid(const Words& w, long long ne, long long cap_cells, double ce
 // the prescreen of a pair reads these 32 bytes of each segment and gives the same values; midf: the same in
 // float parts.  The extremes and sums go over the block, then by one atomic each into w; the last block forms
 // the grid.
-constexpr int AABB_T = 256, AABB_W = AABB_T / 32;
+// AABB_T: some 60 FP64 operations a segment, so few segments go in small CTAs to many SMs' pipes.
+template <int AABB_T>
 __global__ void __launch_bounds__(AABB_T) k_aabb(xk_mesh m, const double* __restrict__ u, double margin,
                                                  double* __restrict__ box, float4* __restrict__ boxf,
                                                  double4_32a* __restrict__ mid, MidF* __restrict__ midf,
                                                  Words* __restrict__ w, long long cap_cells, double cell_size,
                                                  Grid* __restrict__ grid) {
+  constexpr int AABB_W = AABB_T / 32;
   __shared__ unsigned long long s_max[11][AABB_W];
   __shared__ double s_sum[3][AABB_W];
   __shared__ bool s_last;
@@ -781,10 +783,14 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
   XK_TRY(S.get(&rsum, ne));
   XK_TRY(S.get(&part, RED_BLOCKS));
   XK_CUDA(cudaMemsetAsync(zero, 0, zero_bytes, st));
-  k_aabb<<<xk_blocks(ne, AABB_T), AABB_T, 0, st>>>(*m, u, bp->margin, box, boxf, mid, midf, words, cap_cells,
-                                                   bp->cell_size, grid);
+  if (ne >= 2LL * xk_sm_count() * 256)
+    k_aabb<256><<<xk_blocks(ne, 256), 256, 0, st>>>(*m, u, bp->margin, box, boxf, mid, midf, words, cap_cells,
+                                                    bp->cell_size, grid);
+  else
+    k_aabb<64><<<xk_blocks(ne, 64), 64, 0, st>>>(*m, u, bp->margin, box, boxf, mid, midf, words, cap_cells,
+                                                 bp->cell_size, grid);
   // segments sorted by the cell of their lower corner
-  k_cell_count<<<xk_blocks(ne, 256), 256, 0, st>>>(box, ne, grid, ecell, ccnt, range);
+  k_cell_count<<<xk_blocks(ne, 64), 64, 0, st>>>(box, ne, grid, ecell, ccnt, range);
   XK_CHECK_LAUNCH();
   XK_TRY(xk_exclusive_scan_i32(ccnt, cstart, cap_cells + 1, nullptr, st, &S));
   k_cell_scatter<<<xk_blocks(ne, 256), 256, 0, st>>>(ne, ecell, cstart, ccnt, segs);

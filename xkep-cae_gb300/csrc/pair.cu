@@ -236,18 +236,93 @@ __noinline__ __device__ void closest_exact_call(const double* y, double* o) {
   closest_exact(y, y + 3, y + 6, y + 9, o[0], o[1], o[2], o + 3, diff);
 }
 
+XK_D double fdot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
+
+// What the pairs of a segment share, formed once per segment and iteration (k_seg64) instead of in every pair
+// (24 of the 132 FP64 operations of a pair without force, 46 of a contributing one): its first point X + u, the
+// difference to its second point and the squared length, in fused order (a) and in the reference's (ae); the
+// displacement since u_ref of its first point and the difference to that of its second one.  The pairs' values
+// keep their bits.  Measured at the 1027-wire strand: assembly 1785 -> 1558 us.
+struct Seg64 {
+  double x[3], a, d[3], ae;
+};
+constexpr int SEG64_STRIDE = XK_SEG64_STRIDE;
+static_assert(SEG64_STRIDE == 16, "four vectors of four doubles");
+XK_D void ldg4(const double* p, double* v) {  // p 32-byte aligned
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+XK_D Seg64 load_seg(const double* __restrict__ seg, int e) {
+  Seg64 r;
+  double v[8];
+  ldg4(seg + (long long)SEG64_STRIDE * e, v);
+  ldg4(seg + (long long)SEG64_STRIDE * e + 4, v + 4);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r.x[i] = v[i];
+    r.d[i] = v[4 + i];
+  }
+  r.a = v[3];
+  r.ae = v[7];
+  return r;
+}
+// the same from the nodes' positions (the square in the order that is asked for only)
+template <bool EXACT>
+XK_D Seg64 seg_of(const xk_mesh& m, const double* __restrict__ u, int n0, int n1) {
+  Seg64 r;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r.x[i] = xadd(m.X[3LL * n0 + i], u[6LL * n0 + i]);
+    r.d[i] = xsub(xadd(m.X[3LL * n1 + i], u[6LL * n1 + i]), r.x[i]);
+  }
+  if (EXACT) r.ae = xdot_es(r.d, r.d); else r.a = fdot3(r.d, r.d);
+  return r;
+}
+
+// DU: the displacements too
+template <bool DU>
+__global__ void k_seg64(xk_mesh m, const double* __restrict__ u, const double* __restrict__ u_ref,
+                        double* __restrict__ seg) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= m.n_elems) return;
+  const int n0 = m.conn[2LL * e], n1 = m.conn[2LL * e + 1];
+  const Seg64 r = seg_of<false>(m, u, n0, n1);
+  double o[16] = {r.x[0], r.x[1], r.x[2], r.a, r.d[0], r.d[1], r.d[2], xdot_es(r.d, r.d)};
+#pragma unroll
+  for (int c = 0; DU && c < 3; ++c) {
+    const long long d0 = 6LL * n0 + c, d1 = 6LL * n1 + c;
+    const double du0 = u_ref ? u[d0] - u_ref[d0] : u[d0], du1 = u_ref ? u[d1] - u_ref[d1] : u[d1];
+    o[8 + c] = du0;
+    o[12 + c] = du1 - du0;
+  }
+  o[11] = o[15] = 0.0;
+  double2* w = reinterpret_cast<double2*>(seg + (long long)SEG64_STRIDE * e);
+#pragma unroll
+  for (int k = 0; k < (DU ? 8 : 4); ++k) w[k] = make_double2(o[2 * k], o[2 * k + 1]);
+}
+
+// SEG: the segments' records of this u are in seg (the same bits)
+template <bool SEG>
 XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __restrict__ u, double g_on,
-                           double g_off, int allow_deact, int update_active, int i) {
+                           double g_off, int allow_deact, int update_active, int i,
+                           const double* __restrict__ seg = nullptr) {
   const long long cap = p.cap;
-  PairNodes nd = pair_nodes(m, p.ea[i], p.eb[i]);
-  double x[4][3];
-  for (int k = 0; k < 4; ++k) deformed(m, u, nd.n[k], x[k]);
+  const int ea = p.ea[i], eb = p.eb[i];
   double s, t, dist, nrm[3];
-  if (!closest_exact_fast(x, s, t, dist, nrm)) {
+  Seg64 A, B;
+  if (SEG) {
+    A = load_seg(seg, ea);
+    B = load_seg(seg, eb);
+  } else {
+    const PairNodes nd = pair_nodes(m, ea, eb);
+    A = seg_of<true>(m, u, nd.n[0], nd.n[1]);
+    B = seg_of<true>(m, u, nd.n[2], nd.n[3]);
+  }
+  if (!closest_exact_fast(A.x, A.d, A.ae, B.x, B.d, B.ae, s, t, dist, nrm)) {
     // near-parallel or degenerate: every branch of the routine, out of line on its own copies, so that they
     // neither hold registers here nor send this path's arrays to memory
+    const PairNodes nd = pair_nodes(m, ea, eb);
     double y[12], o[6];
-    for (int k = 0; k < 12; ++k) y[k] = x[k / 3][k % 3];
+    for (int k = 0; k < 4; ++k) deformed(m, u, nd.n[k], y + 3 * k);
     closest_exact_call(y, o);
     s = o[0];
     t = o[1];
@@ -281,11 +356,13 @@ XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __
 }
 
 // Bounded by the FP64 pipe: 328 operations a pair with div64 / sqrt64 in place of the operators (430 before),
-// 255 with the unit-vector forms in the frame.  632,000 pairs: 518 -> 331 us.
+// 255 with the unit-vector forms in the frame, 227 with the segments' records.  632,000 pairs: 518 -> 331 us,
+// then 281 us.
+template <bool SEG>
 __global__ void k_narrow_exact(xk_mesh m, xk_pairs p, const double* __restrict__ u, double g_on, double g_off,
-                               int allow_deact, int update_active) {
+                               int allow_deact, int update_active, const double* __restrict__ seg) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < p.n) narrow_exact_one(m, p, u, g_on, g_off, allow_deact, update_active, i);
+  if (i < p.n) narrow_exact_one<SEG>(m, p, u, g_on, g_off, allow_deact, update_active, i, seg);
 }
 
 XK_HD double huber(double x, double d) {  // contact_force/strategy.py:104-113
@@ -414,71 +491,10 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
 // clock and SM), contributing pairs 936 -> 572 us (393 us if these were fused throughout).
 // ===========================================================================
 
-XK_D double fdot3(const double* a, const double* b) { return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0])); }
 XK_D void fcross3(const double* a, const double* b, double* c) {
   c[0] = fma(a[1], b[2], -(a[2] * b[1]));
   c[1] = fma(a[2], b[0], -(a[0] * b[2]));
   c[2] = fma(a[0], b[1], -(a[1] * b[0]));
-}
-
-// What the pairs of a segment share, formed once per segment and iteration (k_seg64) instead of in every pair
-// (24 of the 132 FP64 operations of a pair without force, 46 of a contributing one): its first point X + u, the
-// difference to its second point and the squared length, in fused order (a) and in the reference's (ae); the
-// displacement since u_ref of its first point and the difference to that of its second one.  The pairs' values
-// keep their bits.  Measured at the 1027-wire strand: assembly 1785 -> 1558 us.
-struct Seg64 {
-  double x[3], a, d[3], ae;
-};
-constexpr int SEG64_STRIDE = XK_SEG64_STRIDE;
-static_assert(SEG64_STRIDE == 16, "four vectors of four doubles");
-XK_D void ldg4(const double* p, double* v) {  // p 32-byte aligned
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
-}
-XK_D Seg64 load_seg(const double* __restrict__ seg, int e) {
-  Seg64 r;
-  double v[8];
-  ldg4(seg + (long long)SEG64_STRIDE * e, v);
-  ldg4(seg + (long long)SEG64_STRIDE * e + 4, v + 4);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    r.x[i] = v[i];
-    r.d[i] = v[4 + i];
-  }
-  r.a = v[3];
-  r.ae = v[7];
-  return r;
-}
-// the same from the nodes' positions (the square in the order that is asked for only)
-template <bool EXACT>
-XK_D Seg64 seg_of(const xk_mesh& m, const double* __restrict__ u, int n0, int n1) {
-  Seg64 r;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    r.x[i] = xadd(m.X[3LL * n0 + i], u[6LL * n0 + i]);
-    r.d[i] = xsub(xadd(m.X[3LL * n1 + i], u[6LL * n1 + i]), r.x[i]);
-  }
-  if (EXACT) r.ae = xdot_es(r.d, r.d); else r.a = fdot3(r.d, r.d);
-  return r;
-}
-
-__global__ void k_seg64(xk_mesh m, const double* __restrict__ u, const double* __restrict__ u_ref,
-                        double* __restrict__ seg) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.n_elems) return;
-  const int n0 = m.conn[2LL * e], n1 = m.conn[2LL * e + 1];
-  const Seg64 r = seg_of<false>(m, u, n0, n1);
-  double o[16] = {r.x[0], r.x[1], r.x[2], r.a, r.d[0], r.d[1], r.d[2], xdot_es(r.d, r.d)};
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const long long d0 = 6LL * n0 + c, d1 = 6LL * n1 + c;
-    const double du0 = u_ref ? u[d0] - u_ref[d0] : u[d0], du1 = u_ref ? u[d1] - u_ref[d1] : u[d1];
-    o[8 + c] = du0;
-    o[12 + c] = du1 - du0;
-  }
-  o[11] = o[15] = 0.0;
-  double2* w = reinterpret_cast<double2*>(seg + (long long)SEG64_STRIDE * e);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) w[k] = make_double2(o[2 * k], o[2 * k + 1]);
 }
 
 // Closest point, distance and unit normal of one pair of segments, in fused operations.  False (nothing
@@ -550,7 +566,7 @@ XK_D bool frame64(const double* n, const double* pn, const double* pt1, double* 
 
 // the exact routine, out of line so that its registers stay out of the common path; it writes the table
 __noinline__ __device__ void narrow64_exact(const xk_mesh& m, const xk_pairs& p, const double* __restrict__ u, int i) {
-  narrow_exact_one(m, p, u, 0.0, 0.0, 0, 0, i);
+  narrow_exact_one<false>(m, p, u, 0.0, 0.0, 0, 0, i);
 }
 
 // Narrowphase of pair i (segments A and B, radius sum rs: the cores' on coated wires), written to the table.
@@ -1567,12 +1583,13 @@ __global__ void __launch_bounds__(PAIR_T, SCREEN ? 4 : 2) k_merge_rows(
   }
 }
 
-// The exact detection narrowphase of the pairs the screen listed (list[0] of them), grid-stride.
+// The exact detection narrowphase of the pairs the screen listed (list[0] of them), grid-stride.  (A short
+// list's time is one pair's chain of operations: 17 us at 37 wires, the same in CTAs of one warp.)
 __global__ void k_narrow_exact_list(xk_mesh m, xk_pairs p, const double* __restrict__ u, double g_on, double g_off,
                                     int allow_deact, const int32_t* __restrict__ list) {
   const int n = list[0];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    narrow_exact_one(m, p, u, g_on, g_off, allow_deact, 1, list[1 + k]);
+    narrow_exact_one<false>(m, p, u, g_on, g_off, allow_deact, 1, list[1 + k]);
 }
 
 // A deferral list: [count, done, slots...].  The pair kernel appends to it; its deferred kernel
@@ -1625,6 +1642,7 @@ XK_D bool last_cta_done(int32_t* done) {
 __global__ void __launch_bounds__(PAIR_T) k_pair_other32_deferred(xk_pairs32 q, const float* __restrict__ n32) {
   int32_t* list = q.defer;
   const int cnt = *(volatile int32_t*)list;
+  if (cnt == 0) return;  // the same in every CTA: the count goes back to zero only after all have read it
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < cnt; x += gridDim.x * blockDim.x)
     other32<false>(q, n32, list[DEFER_SLOTS + x]);
   if (last_cta_done(list + 1) && threadIdx.x == 0) {
@@ -1791,6 +1809,7 @@ __global__ void __launch_bounds__(PAIR_T) k_pair_member32_deferred(xk_pairs32 q,
                                                                    xk_contact_params cp, float* __restrict__ rec) {
   int32_t* list = q.defer + ((long long)q.cap + DEFER_SLOTS);
   const int cnt = *(volatile const int32_t*)list;
+  if (cnt == 0) return;  // the same in every CTA: the count goes back to zero only after all have read it
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < cnt; x += gridDim.x * blockDim.x)
     member32<false>(q, n32, cp, rec, list[DEFER_SLOTS + x]);
   if (last_cta_done(list + 1) && threadIdx.x == 0) {
@@ -1829,8 +1848,20 @@ extern "C" xk_status xk_narrowphase(const xk_mesh* m, xk_pairs* p, const double*
                                     int update_active, xk_stream s) {
   if (!m || !p || !u || !cp) return xk_set_error(XK_ERR_ARG, "xk_narrowphase: null argument");
   if (p->n == 0) return XK_OK;
-  k_narrow_exact<<<xk_blocks(p->n, PAIR_T), PAIR_T, 0, (cudaStream_t)s>>>(*m, *p, u, cp->g_on, cp->g_off,
-                                                                          cp->allow_deactivation, update_active);
+  cudaStream_t st = (cudaStream_t)s;
+  const int bs = pair64_block(p->n), nb = xk_blocks(p->n, bs);
+  // records per segment (30 FP64 operations each) pay from some two pairs a segment on, 28 operations saved in each
+  if (p->n < 2LL * m->n_elems) {
+    k_narrow_exact<false><<<nb, bs, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation, update_active,
+                                             nullptr);
+    XK_CHECK_LAUNCH();
+    return XK_OK;
+  }
+  XkScratch S(st);
+  double* seg;
+  XK_TRY(S.get(&seg, (long long)SEG64_STRIDE * m->n_elems));
+  k_seg64<false><<<xk_blocks(m->n_elems, 64), 64, 0, st>>>(*m, u, nullptr, seg);
+  k_narrow_exact<true><<<nb, bs, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation, update_active, seg);
   XK_CHECK_LAUNCH();
   return XK_OK;
 }
@@ -1900,7 +1931,7 @@ extern "C" xk_status xk_segments64(const xk_mesh* m, const double* u, const doub
   if ((uintptr_t)seg64 & 31) return xk_set_error(XK_ERR_ARG, "xk_segments64: seg64 must be 32-byte aligned");
   if (m->n_elems <= 0) return XK_OK;
   // FP64 work of a few operations a segment: small CTAs reach all SMs
-  k_seg64<<<xk_blocks(m->n_elems, 64), 64, 0, (cudaStream_t)s>>>(*m, u, u_ref, seg64);
+  k_seg64<true><<<xk_blocks(m->n_elems, 64), 64, 0, (cudaStream_t)s>>>(*m, u, u_ref, seg64);
   XK_CHECK_LAUNCH();
   return XK_OK;
 }
@@ -2185,9 +2216,9 @@ extern "C" xk_status xk_nodes_prepare(const xk_mesh* m, const double* u, const d
   if (((uintptr_t)node32 & 15) != 0) return xk_set_error(XK_ERR_ARG, "xk_nodes_prepare: node32 must be 16-byte aligned");
   const bool vec = ((uintptr_t)u & 15) == 0 && ((uintptr_t)u_ref & 15) == 0;
   if (vec)
-    k_nodes_prepare<true><<<xk_blocks(m->n_nodes, 128), 128, 0, (cudaStream_t)s>>>(*m, u, u_ref, node32);
+    k_nodes_prepare<true><<<xk_blocks(m->n_nodes, 64), 64, 0, (cudaStream_t)s>>>(*m, u, u_ref, node32);
   else
-    k_nodes_prepare<false><<<xk_blocks(m->n_nodes, 128), 128, 0, (cudaStream_t)s>>>(*m, u, u_ref, node32);
+    k_nodes_prepare<false><<<xk_blocks(m->n_nodes, 64), 64, 0, (cudaStream_t)s>>>(*m, u, u_ref, node32);
   XK_CHECK_LAUNCH();
   return XK_OK;
 }
@@ -2228,8 +2259,12 @@ extern "C" xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk
   cudaStream_t st = (cudaStream_t)s;
   const int n_o = q->n - q->n_members;
   // the CTA size of the common kernels: a launch-shape choice only (each thread owns one slot)
-  const int bs = (q->block >= 32 && q->block <= PAIR_T && q->block % 32 == 0) ? q->block : PAIR_T;
+  const bool set = q->block >= 32 && q->block <= PAIR_T && q->block % 32 == 0;
+  // unless one is set: small CTAs where the table does not fill the SMs twice over in large ones (7 wires:
+  // k_pair_member32 7.4 -> 6.7 us)
+  auto cta = [&](int n) { return set ? q->block : (n >= 2LL * xk_sm_count() * PAIR_T ? PAIR_T : 64); };
   if ((parts & XK_PAIRS_OTHERS) && n_o > 0) {
+    const int bs = cta(n_o);
     if (q->defer) {
       k_pair_other32<true><<<xk_blocks(n_o, bs), bs, 0, st>>>(*q, node32);
       k_pair_other32_deferred<<<152, PAIR_T, 0, st>>>(*q, node32);
@@ -2238,6 +2273,7 @@ extern "C" xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk
     }
   }
   if ((parts & XK_PAIRS_MEMBERS) && q->n_members > 0) {
+    const int bs = cta(q->n_members);
     if (q->defer) {
       k_pair_member32<true><<<xk_blocks(q->n_members, bs), bs, 0, st>>>(*q, node32, *cp, rec);
       k_pair_member32_deferred<<<152, PAIR_T, 0, st>>>(*q, node32, *cp, rec);
