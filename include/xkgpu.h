@@ -221,8 +221,9 @@ xk_status xk_narrowphase(const xk_mesh* m, xk_pairs* p, const double* u, const x
  * reference arithmetic (as xk_narrowphase) every pair whose float gap lies
  * within a bound of its error from [g_on, g_off], or that is near-parallel,
  * or on coated wires.  The status of every pair is the exact one; the stored
- * s, t, gap and frame of the others carry float rounding.  *n_exact (device,
- * nullable): how many pairs took the exact routine. */
+ * s, t, gap and frame of the others carry float rounding.  *n_exact (device or
+ * pinned host memory, nullable): how many pairs took the exact routine, written
+ * in stream order. */
 xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, const double* u, const float* node32,
                                   const xk_contact_params* cp, int32_t* n_exact, xk_stream s);
 
@@ -444,7 +445,8 @@ xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk_contact_pa
 /* xk_pairs_merge (drop: xk_pairs_merge_pruned), then xk_narrowphase_screened on out; not for coated wires.  With
  * old32 (nullable, only without drop) both are one pass over the merged rows, and the old state is read from this
  * float table, whose rows and slots are old's, as after xk_pairs_from32(old32, old); old keeps its values.
- * n_exact: as there, required. */
+ * n_exact: as there, required.  With old32 it waits for the number of rows only: out's values follow in stream
+ * order. */
 xk_status xk_pairs_merge_screened(const xk_mesh* m, const xk_pairs* old, const xk_pairs32* old32,
                                   const int32_t* cands, int64_t n_cands, xk_pairs* out, int drop, const double* u,
                                   const float* node32, const xk_contact_params* cp, int32_t* n_exact, xk_stream s);

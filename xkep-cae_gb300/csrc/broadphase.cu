@@ -872,11 +872,12 @@ static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t
       k_merge_count<false><<<warp_blocks, BP_T, 0, st>>>(*old, cands, ostart, cstart, ne, stay, cnt);
     XK_CHECK_LAUNCH();
     XK_TRY(xk_exclusive_scan_i32(cnt, off, ne, tot, st, &S));
+    XK_TRY(xk_read_begin(tot, 1, st));
     k_merge_order<<<warp_blocks, BP_T, 0, st>>>(*old, cands, ostart, cstart, ne, stay, off, out->ea, out->eb, src);
     XK_CHECK_LAUNCH();
     XK_TRY(xk_merge_rows(m, old, src, tot, most, out, screen, list, st));
-    XK_CUDA(cudaMemcpyAsync(&h, tot, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    XK_CUDA(cudaStreamSynchronize(st));
+    XK_TRY(xk_read_end(&h, 1));
+    if (!screen) XK_CUDA(cudaStreamSynchronize(st));  // these entry points return with their work done
   }
   out->n = (int32_t)h;
   return XK_OK;

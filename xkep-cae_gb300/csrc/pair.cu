@@ -1895,7 +1895,7 @@ xk_status xk_merge_rows(const xk_mesh* m, const xk_pairs* old, const int32_t* sr
     }
     XK_CHECK_LAUNCH();
   }
-  if (screen) XK_CUDA(cudaMemcpyAsync(screen->n_exact, list, sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+  if (screen) XK_CUDA(cudaMemcpyAsync(screen->n_exact, list, sizeof(int32_t), cudaMemcpyDefault, st));
   return XK_OK;
 }
 
@@ -1919,7 +1919,7 @@ extern "C" xk_status xk_narrowphase_screened(const xk_mesh* m, xk_pairs* p, cons
     k_narrow_exact_list<<<2 * xk_sm_count(), PAIR_T, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation,
                                                               list);
     e = cudaGetLastError();
-    if (e == cudaSuccess && n_exact) e = cudaMemcpyAsync(n_exact, list, sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && n_exact) e = cudaMemcpyAsync(n_exact, list, sizeof(int32_t), cudaMemcpyDefault, st);
   }
   if (e != cudaSuccess) r = xk_set_cuda_error(e, __FILE__, __LINE__);
   cudaFreeAsync(list, st);

@@ -6,6 +6,8 @@
 #include <cstring>
 #include <mutex>
 
+#include <map>
+
 #include "scan.cuh"
 
 static thread_local char g_err[512] = "";
@@ -131,6 +133,45 @@ extern "C" xk_status xk_scratch_trim(int64_t keep_bytes) {
     RelaxedCapture relaxed;
     XK_CUDA(cudaMemPoolTrimTo(pool, (size_t)keep_bytes));
   }
+  return XK_OK;
+}
+
+// --------------------------------------------------------------------------- read-back
+
+namespace {
+// a pinned buffer per thread, an event per thread and device
+struct Readback {
+  int64_t* host = nullptr;
+  std::map<int, cudaEvent_t> events;
+  cudaEvent_t pending = nullptr;
+  ~Readback() {
+    for (auto& e : events) cudaEventDestroy(e.second);
+    if (host) cudaFreeHost(host);
+  }
+};
+thread_local Readback g_read;
+}  // namespace
+
+xk_status xk_read_begin(const int64_t* dev, int words, cudaStream_t s) {
+  Readback& r = g_read;
+  if (words > XK_READ_WORDS) return xk_set_error(XK_ERR_ARG, "xk_read_begin: words");
+  int id = 0;
+  XK_CUDA(cudaGetDevice(&id));
+  cudaEvent_t& e = r.events[id];
+  if (!r.host || !e) {
+    RelaxedCapture relaxed;
+    if (!r.host) XK_CUDA(cudaHostAlloc((void**)&r.host, sizeof(int64_t) * XK_READ_WORDS, cudaHostAllocPortable));
+    if (!e) XK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  XK_CUDA(cudaMemcpyAsync(r.host, dev, sizeof(int64_t) * words, cudaMemcpyDeviceToHost, s));
+  XK_CUDA(cudaEventRecord(e, s));
+  r.pending = e;
+  return XK_OK;
+}
+
+xk_status xk_read_end(int64_t* host, int words) {
+  XK_CUDA(cudaEventSynchronize(g_read.pending));
+  for (int k = 0; k < words; ++k) host[k] = g_read.host[k];
   return XK_OK;
 }
 

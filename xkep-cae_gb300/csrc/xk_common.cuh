@@ -246,6 +246,13 @@ struct XkScratch {
     if (r__ != XK_OK) return r__; \
   } while (0)
 
+// Up to XK_READ_WORDS words of device memory to the host in two steps, so that the kernels queued in between run
+// while the host waits for the words and prepares what follows (a wait for the whole stream leaves the GPU idle
+// for as long as the host needs to come back).  Each begin is followed by its end, on the same thread and device.
+constexpr int XK_READ_WORDS = 8;
+xk_status xk_read_begin(const int64_t* dev, int words, cudaStream_t s);
+xk_status xk_read_end(int64_t* host, int words);
+
 // Device-wide exclusive scan (util.cu), its scratch from S or of its own.
 xk_status xk_exclusive_scan_i32(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
                                 cudaStream_t s, XkScratch* S = nullptr);

@@ -96,7 +96,7 @@ class AssemblyEngine:
         # mixed engine: detection narrowphase in float with the exact routine for the pairs near the
         # active-set thresholds (xk_narrowphase_screened); the active set is the exact one either way
         self.screened_detection = True
-        self._n_exact = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self._n_exact = torch.zeros(1, dtype=torch.int32, pin_memory=True)  # written in stream order
         self._n_detect = 0
         self.prune_stats = {"detections": 0, "verified": 0, "candidates": 0, "kept": 0, "missed": 0}
         self._verify_tables = None  # scratch pair tables of the pruner's verification, kept across detections
@@ -298,9 +298,9 @@ class AssemblyEngine:
         self._mark("narrowphase", stream)
         self.pattern.build(self.pairs, stream)
         self._mark("pattern", stream)
-        # read while the stream is idle after the pattern build, before the float copy is queued, so that
-        # detect returns without waiting for it
-        n_exact = int(self._n_exact.item()) if screened else self.pairs.n
+        # the pattern build has waited for the stream: the count is there, and detect returns without waiting for
+        # the float copy
+        n_exact = int(self._n_exact.item()) if screened and self.pairs.n else self.pairs.n
         if self.precision == L.XK_MIXED:
             self._to32(s)
             self._mark("float_table", stream)
