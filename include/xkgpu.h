@@ -442,11 +442,17 @@ xk_status xk_pairs_from32(const xk_pairs32* q, xk_pairs* p, xk_stream s);
 xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk_contact_params* cp, float* rec, int parts,
                          xk_stream s);
 
+/* xk_broadphase and xk_pairs_merge (drop: xk_pairs_merge_pruned) for a caller that goes on in stream order: they
+ * wait for their counts only, and the rows follow in s. */
+xk_status xk_broadphase_queued(const xk_mesh* m, const double* u, const xk_bp_params* bp, int32_t* out_pairs,
+                               int64_t cap, int64_t* n_out, int64_t* n_raw, int64_t* n_prefilter, xk_stream s);
+xk_status xk_pairs_merge_queued(const xk_mesh* m, const xk_pairs* old, const int32_t* cands, int64_t n_cands,
+                                xk_pairs* out, int drop, xk_stream s);
+
 /* xk_pairs_merge (drop: xk_pairs_merge_pruned), then xk_narrowphase_screened on out; not for coated wires.  With
  * old32 (nullable, only without drop) both are one pass over the merged rows, and the old state is read from this
  * float table, whose rows and slots are old's, as after xk_pairs_from32(old32, old); old keeps its values.
- * n_exact: as there, required.  With old32 it waits for the number of rows only: out's values follow in stream
- * order. */
+ * n_exact: as there, required.  It waits for the number of rows only: out's values follow in stream order. */
 xk_status xk_pairs_merge_screened(const xk_mesh* m, const xk_pairs* old, const xk_pairs32* old32,
                                   const int32_t* cands, int64_t n_cands, xk_pairs* out, int drop, const double* u,
                                   const float* node32, const xk_contact_params* cp, int32_t* n_exact, xk_stream s);

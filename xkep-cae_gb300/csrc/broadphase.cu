@@ -23,6 +23,7 @@
 // lane there: most of the walk's 558 us at 98,592 segments, 189 us now); the radius sums of the margin are skipped
 // where every radius is the same; the prescreen decides in float from split midpoints (slot ranking 96 -> 58 us).
 #include <atomic>
+#include <cstddef>
 #include <cstdio>
 
 #include "merge.cuh"
@@ -735,8 +736,9 @@ __global__ void __launch_bounds__(BP_T) k_merge_order(xk_pairs old, const int32_
 // slot-list length of the walk: grows to the longest list seen (a power of two), kept for later calls
 std::atomic<int> g_slot_cap{32};
 
-extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_bp_params* bp, int32_t* out_pairs,
-                                   int64_t cap, int64_t* n_out, int64_t* n_raw, int64_t* n_prefilter, xk_stream s) {
+extern "C" xk_status xk_broadphase_queued(const xk_mesh* m, const double* u, const xk_bp_params* bp,
+                                          int32_t* out_pairs, int64_t cap, int64_t* n_out, int64_t* n_raw,
+                                          int64_t* n_prefilter, xk_stream s) {
   if (!m || !bp || !n_out) return xk_set_error(XK_ERR_ARG, "xk_broadphase: null argument");
   cudaStream_t st = (cudaStream_t)s;
   *n_out = 0;
@@ -812,11 +814,12 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
                                                words, srt, cnt2);
     XK_CHECK_LAUNCH();
     XK_TRY(xk_exclusive_scan_i32(cnt2, off2, ne, reinterpret_cast<int64_t*>(&words->kept), st, &S));
+    int64_t h[4];  // raw, pre, longest, kept
+    static_assert(offsetof(Words, kept) - offsetof(Words, raw) == 3 * sizeof(int64_t), "four words in a row");
+    XK_TRY(xk_read_begin(reinterpret_cast<const int64_t*>(&words->raw), 4, st));
     k_slots_emit<<<warp_blocks, BP_T, 0, st>>>(ne, srt, cnt, slot_cap, off2, cap, out_pairs);
     XK_CHECK_LAUNCH();
-    long long h[4];  // raw, pre, longest, kept
-    XK_CUDA(cudaMemcpyAsync(h, &words->raw, sizeof(h), cudaMemcpyDeviceToHost, st));
-    XK_CUDA(cudaStreamSynchronize(st));
+    XK_TRY(xk_read_end(h, 4));
     const int longest = (int)h[2];
     if (longest > slot_cap) {  // some lists were cut short: walk again with lists long enough for all
       if (attempt > 0) return xk_set_error(XK_ERR_OVERFLOW, "xk_broadphase: slot lists overflowed twice");
@@ -832,9 +835,19 @@ extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_b
     if (n_raw) *n_raw = h[0];
     if (n_prefilter) *n_prefilter = h[1];
     *n_out = h[3];
-    if (h[3] > cap) return xk_set_error(XK_ERR_CAPACITY, "xk_broadphase: output capacity too small");
+    if (h[3] > cap) {
+      XK_CUDA(cudaStreamSynchronize(st));  // the caller may free the rows
+      return xk_set_error(XK_ERR_CAPACITY, "xk_broadphase: output capacity too small");
+    }
     return XK_OK;
   }
+}
+
+extern "C" xk_status xk_broadphase(const xk_mesh* m, const double* u, const xk_bp_params* bp, int32_t* out_pairs,
+                                   int64_t cap, int64_t* n_out, int64_t* n_raw, int64_t* n_prefilter, xk_stream s) {
+  const xk_status r = xk_broadphase_queued(m, u, bp, out_pairs, cap, n_out, n_raw, n_prefilter, s);
+  if (r == XK_OK) XK_CUDA(cudaStreamSynchronize((cudaStream_t)s));
+  return r;
 }
 
 // The merged rows' order first (two lists of a few dozen rows per segment), then one kernel moves every row's state
@@ -877,20 +890,28 @@ static xk_status merge_impl(const xk_mesh* m, const xk_pairs* old, const int32_t
     XK_CHECK_LAUNCH();
     XK_TRY(xk_merge_rows(m, old, src, tot, most, out, screen, list, st));
     XK_TRY(xk_read_end(&h, 1));
-    if (!screen) XK_CUDA(cudaStreamSynchronize(st));  // these entry points return with their work done
   }
   out->n = (int32_t)h;
   return XK_OK;
 }
 
+extern "C" xk_status xk_pairs_merge_queued(const xk_mesh* m, const xk_pairs* old, const int32_t* cands,
+                                           int64_t n_cands, xk_pairs* out, int drop, xk_stream s) {
+  return merge_impl(m, old, cands, n_cands, out, s, drop != 0);
+}
+
 extern "C" xk_status xk_pairs_merge(const xk_mesh* m, const xk_pairs* old, const int32_t* cands, int64_t n_cands,
                                     xk_pairs* out, xk_stream s) {
-  return merge_impl(m, old, cands, n_cands, out, s, false);
+  XK_TRY(merge_impl(m, old, cands, n_cands, out, s, false));
+  XK_CUDA(cudaStreamSynchronize((cudaStream_t)s));
+  return XK_OK;
 }
 
 extern "C" xk_status xk_pairs_merge_pruned(const xk_mesh* m, const xk_pairs* old, const int32_t* cands,
                                            int64_t n_cands, xk_pairs* out, xk_stream s) {
-  return merge_impl(m, old, cands, n_cands, out, s, true);
+  XK_TRY(merge_impl(m, old, cands, n_cands, out, s, true));
+  XK_CUDA(cudaStreamSynchronize((cudaStream_t)s));
+  return XK_OK;
 }
 
 extern "C" xk_status xk_pairs_merge_screened(const xk_mesh* m, const xk_pairs* old, const xk_pairs32* old32,

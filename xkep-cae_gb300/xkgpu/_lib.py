@@ -124,6 +124,8 @@ SIGNATURES = {
     "xk_broadphase": [P(Mesh), vp, P(BPParams), vp, C.c_int64, i64p, i64p, i64p, vp],
     "xk_pairs_merge": [P(Mesh), P(Pairs), vp, C.c_int64, P(Pairs), vp],
     "xk_pairs_merge_pruned": [P(Mesh), P(Pairs), vp, C.c_int64, P(Pairs), vp],
+    "xk_broadphase_queued": [P(Mesh), vp, P(BPParams), vp, C.c_int64, i64p, i64p, i64p, vp],
+    "xk_pairs_merge_queued": [P(Mesh), P(Pairs), vp, C.c_int64, P(Pairs), C.c_int, vp],
     "xk_pairs_merge_screened": [P(Mesh), P(Pairs), P(Pairs32), vp, C.c_int64, P(Pairs), C.c_int, vp, vp,
                                 P(ContactParams), vp, vp],
     "xk_narrowphase": [P(Mesh), P(Pairs), vp, P(ContactParams), C.c_int, vp],

@@ -148,10 +148,13 @@ class AssemblyEngine:
     # ------------------------------------------------------------------ per increment
     def candidates(self, u: torch.Tensor, stream=None):
         """Broadphase + filters at X + u: (candidate rows int32 [2n] on the device, n)."""
+        return self._candidates("xk_broadphase", u, stream)
+
+    def _candidates(self, entry: str, u: torch.Tensor, stream):
         s = stream_handle(stream)
         n_out, n_raw, n_pre = C.c_int64(0), C.c_int64(0), C.c_int64(0)
         for _ in range(3):
-            code = L.call("xk_broadphase", C.byref(self.mesh.c), ptr(u), C.byref(self.bp), ptr(self.cands),
+            code = L.call(entry, C.byref(self.mesh.c), ptr(u), C.byref(self.bp), ptr(self.cands),
                           self.cands.numel() // 2, C.byref(n_out), C.byref(n_raw), C.byref(n_pre), s,
                           allow=(L.XK_ERR_CAPACITY,))
             if code == L.XK_OK:
@@ -268,7 +271,7 @@ class AssemblyEngine:
         if not from32:
             self.sync_state(stream)
         self._mark("table_back", stream)
-        cands, nc = self.candidates(u, stream)
+        cands, nc = self._candidates("xk_broadphase_queued", u, stream)  # the rows follow in stream order
         self._mark("broadphase", stream)
         n_raw, n_pre = self._bp_counts
         n_all = nc
@@ -287,8 +290,8 @@ class AssemblyEngine:
                    C.byref(self.pairs32.c) if from32 else None, ptr(cands), nc, C.byref(self._spare.c),
                    int(self._merge_pruned), ptr(u), ptr(self.node32), C.byref(self.cp), ptr(self._n_exact), s)
         else:
-            L.call("xk_pairs_merge_pruned" if self._merge_pruned else "xk_pairs_merge", C.byref(self.mesh.c),
-                   C.byref(self.pairs.c), ptr(cands), nc, C.byref(self._spare.c), s)
+            L.call("xk_pairs_merge_queued", C.byref(self.mesh.c), C.byref(self.pairs.c), ptr(cands), nc,
+                   C.byref(self._spare.c), int(self._merge_pruned), s)
         self._state_in32 = False
         self._spare.set_n(self._spare.c.n)
         self.pairs, self._spare = self._spare, self.pairs
