@@ -165,6 +165,13 @@ XK_D void ldg8(const float* __restrict__ p, float* v) {
       : "l"(p));
 }
 
+// Eight floats to a 32-byte aligned address in one 256-bit store.
+XK_D void stg8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Launch helpers
 // ---------------------------------------------------------------------------
