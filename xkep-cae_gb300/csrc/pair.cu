@@ -487,8 +487,8 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
 // frame and friction are fused too.  Pairs outside the ordinary case (near-parallel, degenerate, without a
 // unit frame, NaN) take the exact routine.
 // Measured at the 1027-wire strand (2.46M other pairs, 0.75M contributing ones), exact routine for every
-// pair against this: other pairs 1757 -> 652 us (132 FP64 operations a pair at the pipe's measured 1.64 per
-// clock and SM), contributing pairs 936 -> 572 us (393 us if these were fused throughout).
+// pair against this: other pairs 1757 -> 515 us (100 FP64 operations a pair at the pipe's measured 1.64 per
+// clock and SM), contributing pairs 936 -> 430 us.
 // ===========================================================================
 
 XK_D void fcross3(const double* a, const double* b, double* c) {
@@ -539,15 +539,19 @@ XK_D bool closest64(const Seg64& A, const Seg64& B, double& s, double& t, double
 // The frame at unit normal n transported from the previous one (pn, pt1).  False (nothing written) unless the
 // previous normal is a unit vector within 120 degrees of n and the tangent is one to speak of.
 XK_D bool frame64(const double* n, const double* pn, const double* pt1, double* t1, double* t2) {
-  const double pp = fdot3(pt1, pt1), qq = fdot3(pn, pn);
-  if (!(near_one64(qq) && in_range64<-60, 60>(pp))) return false;
+  // a tangent to speak of: its largest component in [2^-29, 2^29), on the exponents
+  unsigned top = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) top = max(top, (unsigned)__double2hiint(pt1[i]) & 0x7fffffffu);
+  const double qq = fdot3(pn, pn);
+  if (!(near_one64(qq) && top - (994u << 20) < (58u << 20))) return false;
   double no[3], v[3], vx[3], tr[3];
   const double iq = fma(-0.5, qq, 1.5);
 #pragma unroll
   for (int i = 0; i < 3; ++i) no[i] = pn[i] * iq;
   fcross3(no, n, v);
   const double cv = fdot3(no, n);
-  if (!(__double2hiint(cv + 0.5) > 0)) return false;
+  if (!((unsigned)__double2hiint(cv) < 0xbfe00000u)) return false;  // cv > -1/2 on the bits: a NaN here fails rr below
   fcross3(v, pt1, vx);
   const double f = fdot3(v, pt1) * rcp64(1.0 + cv);
 #pragma unroll

@@ -106,20 +106,20 @@ XK_D double xk_f2d(float v) {
 }
 
 // FP64 on the FP64 pipe is scarce (about two operations per clock and SM; a divide or a square root takes some
-// ten of them).  1/x and 1/sqrt(x) for x in the ordinary range: the approximate instruction and two Newton-Raphson steps
-// (r <- r + r (1 - x r); y <- y + y (1/2 - x y^2 / 2)), within a few units of the last place.
+// ten of them).  1/x and 1/sqrt(x) for x in the ordinary range: the approximate instruction (relative error e about
+// 2^-23 for both) and one step of third order, r + r (e + e^2) and y + y e (1/2 + 3/8 e), which leaves 2^-66 before
+// its last rounding: three and five operations, where two Newton-Raphson steps take four and seven.
 XK_D double rcp64(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 XK_D double rsqrt64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = 0.5 * x;
-  y = fma(y, fma(-h * y, y, 0.5), y);
-  return fma(y, fma(-h * y, y, 0.5), y);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 // x in [2^lo, 2^hi), tested on the high word: false for zero, negative values, infinities and NaN
 template <int LO, int HI>
