@@ -868,8 +868,9 @@ constexpr int BEAMW_T = 128;
 constexpr int BEAM_ORDERED = 0, BEAM_ATOMIC = 1, BEAM_COLOUR = 2;
 
 // One element of the launch (t: the thread's logical index), its outputs staged in the slots.
-// elem(e, a, b, o) computes element e between nodes a and b into its slot o.
-template <typename T, typename Elem>
+// elem(e, a, b, o) computes element e between nodes a and b into its slot o.  LANES 2 (ordered mode): two
+// neighbouring lanes to an element, which elem divides between them, and 15 elements to a warp.
+template <typename T, int LANES = 1, typename Elem>
 XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __restrict__ order, int k0, int k1,
                     const int32_t* __restrict__ blk, const uint8_t* __restrict__ first, double* __restrict__ f_int,
                     T* __restrict__ Kv, bool vec, T* slots, Elem elem) {
@@ -879,7 +880,7 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __re
   long long e;
   bool live;
   if (mode == BEAM_ORDERED) {
-    e = 31 * (t >> 5) + lane - 1;
+    e = (32 / LANES - 1) * (t >> 5) + lane / LANES - 1;
     live = e >= 0 && e < ne;
   } else {
     const long long k = k0 + t;
@@ -888,7 +889,7 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __re
     e = mode == BEAM_COLOUR ? order[k] : k;
   }
   const bool want_K = Kv != nullptr;
-  T* o = slots + threadIdx.x * STRIDE;
+  T* o = slots + threadIdx.x / LANES * STRIDE;
   int a = -1, b = -1;
   int* ob = reinterpret_cast<int*>(o + EL_BLK);
   if (live) {
@@ -913,18 +914,20 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __re
     elem(e, a, b, o);
   }
   if (mode == BEAM_ORDERED) {
-    const int bp = __shfl_up_sync(0xffffffffu, b, 1);  // the predecessor's node b
+    const int bp = __shfl_up_sync(0xffffffffu, b, LANES);  // the predecessor's node b
     __syncwarp();
-    if (lane == 0 || e > ne) return;
+    if (lane < LANES || e > ne) return;
+    // of two lanes the second writes the off-diagonal block, the first the rest
+    const bool diag = lane % LANES == 0, off = lane % LANES == LANES - 1;
     const T* p = o - STRIDE;          // the predecessor's slot
     const bool pred = e >= 1;                // the predecessor exists (e <= ne here)
     const bool joined = live && pred && bp == a;
-    if (pred && !joined) {                   // the predecessor ends its wire: its node b alone
+    if (diag && pred && !joined) {           // the predecessor ends its wire: its node b alone
       if (f_int) put_rows<0, T>(f_int, bp, p + EL_G0, p + EL_G3, true);
       if (want_K) put_block<3, 0, T>(Kv + 36LL * reinterpret_cast<const int*>(p + EL_BLK)[3], p, p, vec);
     }
     if (!live) return;
-    if (f_int) {
+    if (diag && f_int) {
       double v[6];
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
@@ -945,8 +948,9 @@ XK_D void beam_item(int mode, long long t, const xk_mesh& m, const int32_t* __re
       }
     }
     if (!want_K) return;
-    if (joined) put_block<4, 0, T>(Kv + 36LL * ob[0], o, p, vec);
-    else put_block<0, 0, T>(Kv + 36LL * ob[0], o, o, vec);
+    if (diag && joined) put_block<4, 0, T>(Kv + 36LL * ob[0], o, p, vec);
+    else if (diag) put_block<0, 0, T>(Kv + 36LL * ob[0], o, o, vec);
+    if (!off) return;
     if (ob[1] >= 0) put_block<1, 0, T>(Kv + 36LL * ob[1], o, o, vec);
     else put_block<2, 0, T>(Kv + 36LL * ob[2], o, o, vec);
     return;
@@ -1212,6 +1216,171 @@ XK_D void beam_elem64(const xk_mesh& m, const double* __restrict__ ref, const do
   for (int i = 0; i < 9; ++i) o[EL_S13 + i] = fma(0.5, X[i], o[EL_S13 + i]);
 }
 
+// beam_elem64 by two lanes, lane `side` of an element taking its node's part: the node's rotation, P and Q, the
+// blocks G1, H0, H1, H3 (node a) or G3, J0, J3, J1 (node b), which are the same operations on other data.  What the
+// nodes share is formed by both.  Some 710 FP64 operations in a row instead of 1,290, in the same order (to the last
+// place, as the contraction is the compiler's; bit for bit at u = 0); 10% more of them in all, so it is for meshes
+// that leave the SMs' FP64 pipes idle (k_beam64s).
+XK_D void beam_elem64_side(const xk_mesh& m, const double* __restrict__ ref, const double* __restrict__ u,
+                           const xk_section& sec, long long e, int a, int b, bool want_K, double* o, int side) {
+  const unsigned pair = 3u << (threadIdx.x & 30);
+  const long long ne = m.n_elems;
+  const double L0 = ref[e];
+  double R0[9], ua[3], ub[3], th[3], dx[3];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) R0[i] = ref[(1 + i) * ne + e];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    ua[i] = u[6LL * a + i];
+    ub[i] = u[6LL * b + i];
+    th[i] = u[6LL * (side ? b : a) + 3 + i];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) dx[i] = (m.X[3LL * b + i] + ub[i]) - (m.X[3LL * a + i] + ua[i]);
+  const double L = sqrt64(dot3(dx, dx));
+  const double iL = div64(1.0, L);
+  const double ex[3] = {dx[0] * iL, dx[1] * iL, dx[2] * iL};
+  double qr[4];
+  quat_between(R0, ex, qr);  // R0 row 0 is e_x of the reference frame
+  const double qrc[4] = {qr[0], -qr[1], -qr[2], -qr[3]};
+  double t[3], t1[3], t2[3];
+  {
+    double qn[4], qx[4], tx[3];
+    quat_of_rotvec(th, qn);
+    qmul(qrc, qn, qx);
+    rotvec_of_quat(qx, tx);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) t[i] = R0[3 * i] * tx[0] + R0[3 * i + 1] * tx[1] + R0[3 * i + 2] * tx[2];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double other = __shfl_xor_sync(pair, t[i], 1);
+    t1[i] = side ? other : t[i];
+    t2[i] = side ? t[i] : other;
+  }
+  const double dax = L - L0;
+  double Rrod[9], R[9];
+  rotmat_of_quat<double>(qr, Rrod);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      R[3 * i + j] = R0[3 * i] * Rrod[3 * j] + R0[3 * i + 1] * Rrod[3 * j + 1] + R0[3 * i + 2] * Rrod[3 * j + 2];
+  const KeCoef<double> k = ke_coef<double>(sec, L0);
+  // the stiffness rows of this node's rotation: (gj, c1, c1') against node a's, (-gj, c2, c2') against node b's
+  const double gs = side ? -k.gj : k.gj, c1y = side ? k.k1by : k.k1ay, c2y = side ? k.k1ay : k.k1by,
+               c1z = side ? k.k1bz : k.k1az, c2z = side ? k.k1az : k.k1bz;
+  const double f0[3] = {-k.ea * dax, k.k2z * (t1[2] + t2[2]), -k.k2y * (t1[1] + t2[1])};
+  const double fs[3] = {gs * (t1[0] - t2[0]), c1y * t1[1] + c2y * t2[1], c1z * t1[2] + c2z * t2[2]};
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double g0 = R[i] * f0[0] + R[3 + i] * f0[1] + R[6 + i] * f0[2];
+    if (!side) o[EL_G0 + i] = g0;
+    o[(side ? EL_G3 : EL_G1) + i] = R[i] * fs[0] + R[3 + i] * fs[1] + R[6 + i] * fs[2];
+  }
+  if (!want_K) return;
+  double D[9], P1[9], P2[9], Q[9];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const double* r = R + 3 * i;
+    D[3 * i] = fma(r[2], -ex[1], r[1] * ex[2]) * iL;
+    D[3 * i + 1] = fma(r[2], ex[0], r[0] * -ex[2]) * iL;
+    D[3 * i + 2] = fma(r[0], ex[1], r[1] * -ex[0]) * iL;
+  }
+  {
+    double Ti[9], Ts[9], M[9], P[9];
+    tangent_ops<double>(t, true, Ti);
+    tangent_ops<double>(th, false, Ts);
+    mm3(Ti, D, P);
+    mm3(Ti, R, M);
+    mm3(M, Ts, Q);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const double other = __shfl_xor_sync(pair, P[i], 1);
+      P1[i] = side ? other : P[i];
+      P2[i] = side ? P[i] : other;
+    }
+  }
+  double a0[3], a1[3], a2[3], X[9], S[6];
+  double* const h = o + (side ? EL_S03 : EL_S01);
+  // G1 or G3
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = fma(gs, P1[c], -gs * P2[c]);
+    a1[c] = fma(c1y, P1[3 + c], c2y * P2[3 + c]);
+    a2[c] = fma(c1z, P1[6 + c], c2z * P2[6 + c]);
+  }
+  add_skew(fs, D, a0, a1, a2);
+  rta3(R, a0, a1, a2, X);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) h[3 * c + i] = 0.5 * X[3 * i + c];
+  // G0
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = k.ea * ex[c];
+    a1[c] = fma(k.k2z, P1[6 + c], k.k2z * P2[6 + c]);
+    a2[c] = fma(-k.k2y, P1[3 + c], -k.k2y * P2[3 + c]);
+  }
+  add_skew(f0, D, a0, a1, a2);
+  rta3(R, a0, a1, a2, X);
+  sym6d(X, S);
+  if (!side)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) o[EL_S00 + i] = S[i];
+  // H0 or J0
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a1[c] = k.k2z * Q[6 + c];
+    a2[c] = -k.k2y * Q[3 + c];
+  }
+  rta2(R, a1, a2, X);
+#pragma unroll
+  for (int i = 0; i < 9; ++i) h[i] = fma(0.5, X[i], h[i]);
+  // H1 or J3
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = k.gj * Q[c];
+    a1[c] = k.k1ay * Q[3 + c];
+    a2[c] = k.k1az * Q[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);
+  sym6d(X, S);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) o[(side ? EL_S33 : EL_S11) + i] = S[i];
+  // H3, to whose half the other lane adds its J1's
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    a0[c] = -k.gj * Q[c];
+    a1[c] = k.k1by * Q[3 + c];
+    a2[c] = k.k1bz * Q[6 + c];
+  }
+  rta3(R, a0, a1, a2, X);
+  if (!side)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[EL_S13 + 3 * c + i] = 0.5 * X[3 * i + c];
+  __syncwarp(pair);
+  if (side)
+#pragma unroll
+    for (int i = 0; i < 9; ++i) o[EL_S13 + i] = fma(0.5, X[i], o[EL_S13 + i]);
+}
+
+// Ordered meshes of a few thousand elements, two lanes to an element.  A warp has the FP64 pipe of its SM quarter,
+// which takes an instruction of 32 lanes in some 64 clocks; one warp per SM leaves three quarters idle while it
+// works through its elements' chain.  Measured at 4,736 elements (37 wires, eager assembly): 67 -> 60 us.
+__global__ void __launch_bounds__(BEAM64_T) k_beam64s(xk_mesh m, xk_section sec, const double* __restrict__ ref,
+                                                      const int32_t* __restrict__ blk, const double* __restrict__ u,
+                                                      double* __restrict__ f_int, double* __restrict__ Kv, int vec) {
+  __shared__ double slots[BEAM64_T / 2 * EL_STRIDE64];
+  beam_item<double, 2>(BEAM_ORDERED, (long long)blockIdx.x * BEAM64_T + threadIdx.x, m, nullptr, 0, 0, blk, nullptr,
+                       f_int, Kv, vec != 0, slots, [&](long long e, int a, int b, double* o) {
+                         beam_elem64_side(m, ref, u, sec, e, a, b, Kv != nullptr, o, threadIdx.x & 1);
+                       });
+}
+
 __global__ void __launch_bounds__(BEAM64_T) k_beam64(int mode, xk_mesh m, xk_section sec,
                                                      const double* __restrict__ ref, const int32_t* __restrict__ order,
                                                      int k0, int k1, const int32_t* __restrict__ blk,
@@ -1307,6 +1476,12 @@ extern "C" xk_status xk_beam_assemble(const xk_mesh* m, const xk_section* sec, c
   const int vec = ((uintptr_t)K_vals & 15) == 0;
   if (precision == XK_FP64 && plan->node_diag && plan->chain_ordered) {  // one launch, one writer per block
     if (m->n_elems == 0) return XK_OK;
+    // up to two warps per SM by elements: the four of two lanes to an element have an SM quarter each
+    if (m->n_elems / 31 + 1 <= 2 * xk_sm_count()) {
+      k_beam64s<<<m->n_elems / 15 + 1, BEAM64_T, 0, st>>>(*m, *sec, elem_ref, plan->blk, u, f_int, (double*)K_vals, vec);
+      XK_CHECK_LAUNCH();
+      return XK_OK;
+    }
     const long long threads = 32 * ((long long)m->n_elems / 31 + 1);
     k_beam64<<<xk_blocks(threads, BEAM64_T), BEAM64_T, 0, st>>>(BEAM_ORDERED, *m, *sec, elem_ref, nullptr, 0, 0, plan->blk,
                                                                plan->first, u, f_int, (double*)K_vals, vec, threads);
