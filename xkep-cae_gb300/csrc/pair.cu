@@ -1861,16 +1861,23 @@ extern "C" xk_status xk_narrowphase(const xk_mesh* m, xk_pairs* p, const double*
   if (p->n == 0) return XK_OK;
   cudaStream_t st = (cudaStream_t)s;
   const int bs = pair64_block(p->n), nb = xk_blocks(p->n, bs);
-  // records per segment (30 FP64 operations each) pay from some two pairs a segment on, 28 operations saved in each
-  if (p->n < 2LL * m->n_elems) {
+  // records per segment (30 FP64 operations each) pay from some two pairs a segment on, 28 operations saved in each;
+  // under capture, or where their scratch cannot be had, the pairs go without (the same bits)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  XK_CUDA(cudaStreamIsCapturing(st, &cap));
+  XkScratch S(st);
+  double* seg = nullptr;
+  if (p->n >= 2LL * m->n_elems && cap == cudaStreamCaptureStatusNone &&
+      S.get(&seg, (long long)SEG64_STRIDE * m->n_elems) != XK_OK) {
+    cudaGetLastError();
+    seg = nullptr;
+  }
+  if (!seg) {
     k_narrow_exact<false><<<nb, bs, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation, update_active,
                                              nullptr);
     XK_CHECK_LAUNCH();
     return XK_OK;
   }
-  XkScratch S(st);
-  double* seg;
-  XK_TRY(S.get(&seg, (long long)SEG64_STRIDE * m->n_elems));
   k_seg64<false><<<xk_blocks(m->n_elems, 64), 64, 0, st>>>(*m, u, nullptr, seg);
   k_narrow_exact<true><<<nb, bs, 0, st>>>(*m, *p, u, cp->g_on, cp->g_off, cp->allow_deactivation, update_active, seg);
   XK_CHECK_LAUNCH();
