@@ -1004,13 +1004,12 @@ extern "C" xk_status xk_prune_features(const xk_mesh* m, const float* node32, co
   if (n == 0) return XK_OK;
   cudaStream_t st = (cudaStream_t)s;
   const long long ne = m->n_elems;
-  int32_t* ostart = nullptr;
-  XK_CUDA(cudaMallocAsync((void**)&ostart, sizeof(int32_t) * (ne + 2), st));
+  XkScratch S(st);  // the library's pool: the default one maps its memory again after every synchronisation (0.1 ms)
+  int32_t* ostart;
+  XK_TRY(S.get(&ostart, ne + 2));
   k_table_seg_start<<<xk_blocks(ne + 1, 256), 256, 0, st>>>(*old, ne, ostart);
   k_features<<<xk_blocks(n, 256), 256, 0, st>>>(*m, node32, cands, n, *old, ostart, feat, hist);
-  cudaError_t e = cudaGetLastError();
-  cudaFreeAsync(ostart, st);
-  if (e != cudaSuccess) return xk_set_cuda_error(e, __FILE__, __LINE__);
+  XK_CHECK_LAUNCH();
   return XK_OK;
 }
 
@@ -1110,17 +1109,16 @@ extern "C" xk_status xk_prune_select(const int32_t* cands, int64_t n, const floa
   if (score_failed) *score_failed = 0;
   if (n == 0) return XK_OK;
   cudaStream_t st = (cudaStream_t)s;
-  int32_t* flag = nullptr;
-  int64_t* tot = nullptr;  // [count, scoring error word]
-  XK_CUDA(cudaMallocAsync((void**)&flag, sizeof(int32_t) * 2 * n, st));
-  cudaError_t e = cudaMallocAsync((void**)&tot, 2 * sizeof(int64_t), st);
-  if (e != cudaSuccess) {
-    cudaFreeAsync(flag, st);
-    return xk_set_cuda_error(e, __FILE__, __LINE__);
-  }
+  XkScratch S(st);
+  int32_t* flag;
+  int64_t* tot;  // [count, scoring error word]
+  XK_TRY(S.reserve(8 * (size_t)n + 8 * (size_t)(n / 256) + 8192));
+  XK_TRY(S.get(&flag, 2 * n));
+  XK_TRY(S.get(&tot, 2));
+  cudaError_t e = cudaSuccess;
   int32_t* off = flag + n;
   k_keep_flags<<<xk_blocks(n, 256), 256, 0, st>>>(n, logit, hist, threshold, invert, score_error, flag);
-  xk_status r = xk_exclusive_scan_i32(flag, off, n, tot, st);
+  xk_status r = xk_exclusive_scan_i32(flag, off, n, tot, st, &S);
   if (r == XK_OK) {
     k_scatter_cands<<<xk_blocks(n, 256), 256, 0, st>>>(n, cands, flag, off, kept);
     int64_t h[2] = {0, 0};
@@ -1137,8 +1135,6 @@ extern "C" xk_status xk_prune_select(const int32_t* cands, int64_t n, const floa
       if (score_failed && score_error) *score_failed = (int32_t)(h[1] & 0xffffffff);
     }
   }
-  cudaFreeAsync(flag, st);
-  cudaFreeAsync(tot, st);
   return r;
 }
 
