@@ -5,7 +5,7 @@
 // selection / pair-table compaction that apply it at detection time.
 //
 // Inference runs on the tensor cores, in two forms: tcgen05.mma with the
-// accumulator in TMEM, 128 candidates per CTA tile (the default), and
+// activations and accumulators in TMEM, five tiles of 128 candidates per SM (the default), and
 // mma.sync m16n8k16 (BF16 -> FP32), where a warp takes 16 candidates and each
 // layer's accumulator fragments are re-packed in registers as the next layer's
 // A operand.  Training runs
