@@ -106,9 +106,11 @@ XK_D double xk_f2d(float v) {
 }
 
 // FP64 on the FP64 pipe is scarce (about two operations per clock and SM; a divide or a square root takes some
-// ten of them).  1/x and 1/sqrt(x) for x in the ordinary range: the approximate instruction (relative error e about
-// 2^-23 for both) and one step of third order, r + r (e + e^2) and y + y e (1/2 + 3/8 e), which leaves 2^-66 before
-// its last rounding: three and five operations, where two Newton-Raphson steps take four and seven.
+// ten of them).  1/x and 1/sqrt(x) for x in the ordinary range: the approximate instruction, which sees the upper 32
+// bits of x (1 - x r and 1 - x y^2 below 2^-19.9 and 2^-19.0 over 2^32 operands on this GPU), and one step of third
+// order, r + r (e + e^2) and y + y e (1/2 + 3/8 e): three and five operations, where two Newton-Raphson steps take
+// four and seven.  Not correctly rounded: the step leaves 2^-59.8 of r, and of y 2^-58 and half the rounding of x y;
+// measured over those operands, at most 0.508 units of the last place of r and 1.0 of y.
 XK_D double rcp64(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -133,9 +135,13 @@ XK_D bool near_one64(double x) {
 
 // The correctly rounded quotient and square root (the bits of the operators) on fewer FP64 operations, after
 // Markstein ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r the
-// reciprocal to the last place, q = RN(x r) leaves an exact remainder x - d q, and RN(q + rem r) is x / d;
-// the square root likewise from g = RN(x y) and its exact remainder.  A divisor's reciprocal serves several
-// quotients.  Operands outside the range where the remainders are exact take the operators, out of line.
+// correctly rounded reciprocal, q = RN(x r) leaves an exact remainder x - d q, and RN(q + rem r) is x / d.  One step
+// r + r (1 - d r) from a reciprocal within a unit of the last place rounds correctly (rcp64 alone does not for one
+// divisor in sixty), but for a mantissa of ones only, 2^k (2 - 2^-52), whose reciprocal lies 2^-106 above a tie.
+// The square root likewise from g = RN(x y) and its exact remainder: near a tie the step's error is below 2^-52.7
+// units, and the few operands whose root lies that close (x = N (N + 1) - c, c small, N (N + 1) = c modulo a power of
+// two) have been tried one by one.  A divisor's reciprocal serves several quotients.  Operands outside the range
+// where the remainders are exact, and divisors of ones, take the operators, out of line.
 __noinline__ static __device__ double div64_plain(double x, double d) { return x / d; }
 __noinline__ static __device__ double sqrt64_plain(double x) { return sqrt(x); }
 struct Divisor64 {
@@ -145,7 +151,11 @@ struct Divisor64 {
 XK_D bool mag_in64(double x) {  // |x| in [2^-300, 2^300)
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (723u << 20) < (600u << 20);
 }
-XK_D Divisor64 divisor64(double d) { return {d, rcp64(d), mag_in64(d)}; }
+XK_D Divisor64 divisor64(double d) {
+  const double r = rcp64(d);
+  const bool ones = ((unsigned)__double2loint(d) & ((unsigned)__double2hiint(d) | 0xfff00000u)) == 0xffffffffu;
+  return {d, fma(fma(-d, r, 1.0), r, r), mag_in64(d) && !ones};
+}
 XK_D double div64(double x, const Divisor64& q) {
   if (!(q.ok && mag_in64(x))) return x == 0.0 && q.ok ? x : div64_plain(x, q.d);
   const double y = x * q.r;
