@@ -37,6 +37,16 @@ __global__ void k_sqrt(long long n, const double* x, double* q, double* want) {
   q[i] = sqrt64(x[i]);
   want[i] = sqrt(x[i]);
 }
+__global__ void k_div_unit(long long n, const double* x, const double* d, double* q, double* want) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  q[i] = next_to_one64(d[i]) ? div_next_to_one64(x[i], d[i]) : -1.0;
+  want[i] = x[i] / d[i];
+}
+extern "C" int t_div_unit(long long n, const double* x, const double* d, double* q, double* want) {
+  k_div_unit<<<(unsigned)((n + 255) / 256), 256>>>(n, x, d, q, want);
+  return (int)cudaDeviceSynchronize();
+}
 extern "C" int t_div(long long n, const double* x, const double* d, double* q, double* want) {
   k_div<<<(unsigned)((n + 255) / 256), 256>>>(n, x, d, q, want);
   return (int)cudaDeviceSynchronize();
@@ -104,6 +114,24 @@ def test_quotients_of_special_operands(lib):
     # a zero over a negative divisor is not asked for: every divisor of the kernels is positive
     keep &= ~((x == 0) & (d < 0))
     _run(lib.t_div, x[keep], d[keep])
+
+
+def test_divisors_next_to_one(lib):
+    """Every divisor of the range over values of few bits (which tie), neighbours of ties, powers of two and their
+    neighbours, values at random and at the ends of the double range."""
+    rng = np.random.default_rng(5)
+    m = [np.arange(1 << 52, (1 << 53) + 1, 1 << 40), (1 << 52) + np.arange(100), (1 << 53) - np.arange(100),
+         rng.integers(1 << 52, 1 << 53, 20000)]
+    for n in range(1, 17):  # m n = 2^52 + j modulo 2^53: within j units of a tie
+        for j in (0, 1, -1, 2, -2, 15, -15, 255, -255, 256, -256, 257, -257, 511, 513, -511, -513):
+            t = ((np.arange(n, 2 * n + 2, dtype=object) << 53) + (1 << 52) + j) // n
+            m.append(np.array([x + y for x in t for y in (-1, 0, 1) if 1 << 52 <= x + y <= 1 << 53], dtype=np.int64))
+    v = np.concatenate(m).astype(np.float64) * 2.0**-53
+    v = np.concatenate([v, -v, v * 2.0**-900, v * 2.0**-1000, v * 2.0**-1040, v * 2.0**1000, v * 2.0**1023 * (2.0 - 2.0**-52),
+                        [0.0, -0.0, 2.0**-1074, 2.0**-1022]])
+    v = v[np.isfinite(v)]
+    for d in [1.0 - k * 2.0**-53 for k in range(17)] + [1.0 + k * 2.0**-52 for k in range(8)]:
+        _run(lib.t_div_unit, v, np.full_like(v, d))
 
 
 def test_square_roots_next_to_ties(lib):

@@ -42,13 +42,12 @@ XK_D double sqrt_unit64(double x) {
   return sqrt64(x);
 }
 
-// v / d by components, each correctly rounded, on one reciprocal; for d = 1 + e, |e| < 2^-49, as v - v e (the
-// quotient's further terms are below 2^-98 of it)
+// v / d by components, each correctly rounded, on one reciprocal or (a vector that is a unit vector up to rounding)
+// without one
 XK_D void div3(const double* v, double d, double* out) {
-  if ((unsigned long long)(__double_as_longlong(d) - 0x3feffffffffffff0LL) < 0x18ULL) {
-    const double e = d - 1.0;
+  if (next_to_one64(d)) {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) out[i] = fma(-v[i], e, v[i]);
+    for (int i = 0; i < 3; ++i) out[i] = div_next_to_one64(v[i], d);
     return;
   }
   const Divisor64 q = divisor64(d);

@@ -162,6 +162,25 @@ XK_D double div64(double x, const Divisor64& q) {
   return fma(fma(-q.d, y, x), q.r, y);
 }
 XK_D double div64(double x, double d) { return div64(x, divisor64(d)); }
+// v / d for a divisor next to one, d = 1 - k 2^-53 (k <= 16) or 1 + k 2^-52 (k < 8): as RN(v + v (1 - d)), one
+// operation, which leaves out v (1 - d)^2, below 2^-45 units of the last place of v.  That decides the rounding where
+// v (1 - d) lies on a tie or within 2^-45 of one (v = 1/2, d = 1 - 2^-53: a contact at 60 degrees), so there, and
+// where v is so close to a power of two that the quotient may change binade, the divide is taken; whole arithmetic on
+// the bits finds these.
+XK_D bool next_to_one64(double d) {
+  return (unsigned long long)(__double_as_longlong(d) - 0x3feffffffffffff0LL) < 0x18ULL;
+}
+XK_D double div_next_to_one64(double v, double d) {
+  const long long k = __double_as_longlong(d) - 0x3ff0000000000000LL, b = __double_as_longlong(v);
+  const unsigned long long n = (unsigned long long)(k < 0 ? -k : 2 * k);  // |1 - d| in units of 2^-53
+  if (n == 0 || (b << 1) == 0) return v;
+  const unsigned long long one = 1ULL << 52, m = ((unsigned long long)b & (one - 1)) | one;
+  const bool tie = ((m * n + one + 512) & (2 * one - 1)) < 1024;  // the fraction of v (1 - d) within 2^-44 of a half
+  const bool edge = m - (one + 32) >= one - 64;
+  const bool range = ((unsigned)__double2hiint(v) & 0x7ff00000u) - (24u << 20) < (2020u << 20);
+  if (tie || edge || !range) return div64(v, d);
+  return fma(v, 1.0 - d, v);
+}
 XK_D double sqrt64(double x) {
   if (!in_range64<-300, 300>(x)) return x == 0.0 ? x : sqrt64_plain(x);
   const double y = rsqrt64(x), g = x * y;
