@@ -76,3 +76,31 @@ def test_candidates_against_the_oracle(shape, n, radii):
         assert (nr.value, np_.value) == (len(raw), len(before))
         got = out[: 2 * nk.value].view(-1, 2).cpu().numpy()
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("offset", [1e6, 1e8, 1e10, 1e12, 1e14])
+@pytest.mark.parametrize("radii", ["equal", "different"])
+def test_candidates_far_from_the_origin(offset, radii):
+    """The prescreen decides as the exact routine wherever the cloud lies: the float midpoints resolve 2^-48 of the
+    position, which passes the width of the undecided band from some 10^8 separations on."""
+    n = 700
+    rng = np.random.default_rng(int(np.log10(offset)))
+    X, conn = _cloud(n, "cube", rng)
+    X = X + offset * np.array([1.0, -0.7, 0.3])
+    r = np.full(n, 0.3) if radii == "equal" else rng.uniform(0.05, 0.4, n)
+    mesh = DeviceMesh(X, conn, r)
+    u = 0.1 * rng.normal(size=6 * len(X))
+    x = oc.deformed_coords(X, u)
+    ud = torch.as_tensor(u, device="cuda")
+    out = torch.zeros(2 * n * n, dtype=torch.int32, device="cuda")
+    for margin, pre_margin in ((1.0, 0.0), (1.0, 0.07)):  # wide boxes, so that many candidates meet the prescreen's line
+        bp = L.BPParams(margin, 1, 0, 1, pre_margin)
+        nk, nr, np_ = C.c_int64(), C.c_int64(), C.c_int64()
+        L.call("xk_broadphase", C.byref(mesh.c), ptr(ud), C.byref(bp), ptr(out), n * n, C.byref(nk), C.byref(nr),
+               C.byref(np_), stream_handle())
+        lo, hi = oc.segment_aabbs(x, conn, r, margin)
+        i, j = np.triu_indices(n, 1)
+        raw = np.stack([i, j], 1)[np.all((lo[i] <= hi[j]) & (lo[j] <= hi[i]), axis=1)]
+        want = oc.filter_candidates(raw, x, conn, r, midpoint_prescreening=True, prescreening_margin=pre_margin)
+        assert nr.value == len(raw)
+        assert np.array_equal(out[: 2 * nk.value].view(-1, 2).cpu().numpy(), want)

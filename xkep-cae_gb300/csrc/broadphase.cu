@@ -501,17 +501,23 @@ XK_D bool midpoint_keep(const double4_32a a, const double4_32a b, double ra, dou
 }
 
 // The same decision with a float screen first: the separation |m_i - m_j| from the split midpoints against the
-// threshold r_i + r_j + extra + h_i + h_j in float decides every pair farther than a relative 1e-5 from it
-// (the roundings of both stay below 1e-6 relative); the rest, and what is not finite, take the exact routine,
-// so the decision is the exact one.
-XK_D bool midpoint_keep_fast(const MidF& a, const MidF& b, float extra, const double4_32a* __restrict__ mid, int i,
-                             int j, const double* __restrict__ radii, double extra64) {
+// threshold r_i + r_j + extra + h_i + h_j in float decides every pair farther from it than a relative 1e-5 (the
+// float roundings of both stay below 1e-6) and than `slack`; the rest, and what is not finite, take the exact
+// routine, so the decision is the exact one.  slack: what the split midpoints do not resolve.  A low part is rounded
+// at 2^-48 of its position and the difference of two at 2^-47 of the larger, 2^-46 a component in all, so 2^-45 of
+// m_i's largest component covers the three (m_j's exceeds it by the separation at most, far below the relative part).
+XK_D float split_slack(const MidF& a) {
+  return 2.8421709e-14f * fmaxf(fabsf(a.hi[0]), fmaxf(fabsf(a.hi[1]), fabsf(a.hi[2])));
+}
+XK_D bool midpoint_keep_fast(const MidF& a, const MidF& b, float extra, float slack,
+                             const double4_32a* __restrict__ mid, int i, int j, const double* __restrict__ radii,
+                             double extra64) {
   const float dx = (a.hi[0] - b.hi[0]) + (a.lo[0] - b.lo[0]), dy = (a.hi[1] - b.hi[1]) + (a.lo[1] - b.lo[1]),
               dz = (a.hi[2] - b.hi[2]) + (a.lo[2] - b.lo[2]);
   const float md = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
   const float thr = ((a.r + b.r) + extra) + (a.half + b.half);
-  if (md < thr * 0.99999f) return true;
-  if (md > thr * 1.00001f) return false;
+  if (md < fmaf(thr, 0.99999f, -slack)) return true;
+  if (md > fmaf(thr, 1.00001f, slack)) return false;
   return midpoint_keep(mid[i], mid[j], radii[i], radii[j], extra64);
 }
 
@@ -532,9 +538,9 @@ __global__ void __launch_bounds__(BP_T) k_slots_rank(xk_mesh m, const double4_32
   int32_t* const out = srt + (long long)i * cap;
   const MidF mi = midf[i];
   const double ex = words->margin;
-  const float exf = xk_d2f(ex);
+  const float exf = xk_d2f(ex), slack = split_slack(mi);
   auto keep = [&](int j) {
-    return !prescreen || midpoint_keep_fast(mi, midf[j], exf, mid, i, j, m.radii, ex);
+    return !prescreen || midpoint_keep_fast(mi, midf[j], exf, slack, mid, i, j, m.radii, ex);
   };
   int kept = 0;
   if (n <= 64) {  // two entries per lane, ranked by shuffle-broadcast comparisons
