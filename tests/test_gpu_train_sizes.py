@@ -36,3 +36,27 @@ def test_gradient_against_the_oracle(n):
     p = grad.cpu().numpy()
     b4 = float(np.sum(w * (1.0 / (1.0 + np.exp(-logit.cpu().numpy().astype(np.float64))) - y)) / n)
     assert abs(p[-1] - b4) <= 1e-5 * max(abs(b4), 1e-3)
+
+
+def test_gradient_sums_of_many_samples():
+    """No gradient is a longer chain of float additions than 1,024 samples and the chunks of a group.
+
+    Every sample adds the same value, c up to a power of two (a zero network: sigmoid 1/2, label 0, weight c).  It
+    loses almost half a last place in every addition to a sum between 4,096 c and 8,192 c: chains that go on that far
+    are off by 1.3e-4.  Bound: a chain of k additions is off by at most k 2^-24 of its sum.
+    """
+    n = 1 << 22
+    th = np.zeros(P.NPARAM, np.float32)
+    th[-129:-65] = 1.0  # the last activations: 1
+    pr = P.PairPruner(th)
+    c = np.float32(1.0 + 2.0**-12 - 2.0**-23)
+    X = torch.zeros(8 * n, device="cuda")
+    y = torch.zeros(n, device="cuda")
+    w = torch.full((n,), float(c), device="cuda")
+    _, grad, _ = pr.gradient(X, y, w, n)
+    g = grad.cpu().numpy()
+    want = 0.5 * float(c)  # the mean of c / 2
+    chunks = n // 1024
+    tol = (1024 + chunks // 8 + 8) * 2.0**-24
+    assert abs(g[-1] - want) <= tol * want  # b4
+    assert np.max(np.abs(g[-65:-1] - want)) <= tol * want

@@ -746,9 +746,12 @@ __global__ void __launch_bounds__(TR_T, 3) k_mlp_train_bwd(const float* __restri
 // Weight gradients: a CTA sums a chunk of samples for every parameter in sample order, two warps with the 64 x 64
 // products d2 a1^T and two with d3 a2^T as 8 x 8 tiles a thread (four samples at a time from [value][sample] rows
 // in shared memory), then its share of the small ones; a second kernel adds the chunks' sums in a fixed order.
-// The chunk follows from n alone: the samples dealt out to WG_CTAS CTAs (three per SM of 152), in whole tiles.
-// Chunks of 1024 whatever n left a few thousand samples to one or two CTAs (1,200 samples: 600 us).
-constexpr int WG_T = 128, WG_S = 32, WG_LD = 36, WG_CTAS = 456;
+// The chunk follows from n alone, so that the sums' order does too: the samples dealt out in whole tiles to WG_CTAS
+// CTAs (what this GPU's 152 SMs hold, three each), or to as many rounds of them as leave no chunk above WG_MOST
+// samples, which bounds the float chains of additions.  Chunks of 1,024 whatever n left a few thousand samples to one
+// or two CTAs (1,200 samples: 600 us) and fill the last round by chance (500,001 samples: the gradient 1,100 us).
+constexpr int WG_T = 128, WG_S = 32, WG_LD = 36, WG_CTAS = 456, WG_MOST = 1024;
+static_assert(WG_MOST % WG_S == 0, "whole tiles");
 static_assert(NA % 64 == 0 && WG_T == 128, "row loads: 16 rows a warp and round");
 constexpr int WG_A = MF + NA;  // rows x0 a1 a2 a3
 struct WgradSmem {
@@ -757,7 +760,8 @@ struct WgradSmem {
   float g[WG_LD];
 };
 long long wgrad_chunk(long long n) {
-  const long long per = (n + WG_CTAS - 1) / WG_CTAS;
+  const long long rounds = (n + WG_CTAS * WG_MOST - 1) / (WG_CTAS * WG_MOST);
+  const long long per = (n + WG_CTAS * rounds - 1) / (WG_CTAS * rounds);
   return (per + WG_S - 1) / WG_S * WG_S;
 }
 
