@@ -2107,12 +2107,13 @@ extern "C" xk_status xk_constraint_jacobian(const xk_mesh* m, const xk_pairs* p,
   cudaStream_t st = (cudaStream_t)s;
   *n_rows = 0;
   if (p->n == 0) return XK_OK;
-  int32_t* flag = nullptr;
+  int32_t* flag = nullptr;  // then the rows' positions
   int64_t* tot = nullptr;
-  XK_CUDA(cudaMallocAsync((void**)&flag, sizeof(int32_t) * p->n, st));
+  XK_CUDA(cudaMallocAsync((void**)&flag, sizeof(int32_t) * 2 * (size_t)p->n, st));
+  int32_t* const off = flag + p->n;
   XK_CUDA(cudaMallocAsync((void**)&tot, sizeof(int64_t), st));
   k_active_flags<<<xk_blocks(p->n, 256), 256, 0, st>>>(*p, flag);
-  xk_status r = xk_exclusive_scan_i32(flag, flag, p->n, tot, st);
+  xk_status r = xk_exclusive_scan_i32(flag, off, p->n, tot, st);
   int64_t h = 0;
   if (r == XK_OK) {
     cudaError_t e = cudaMemcpyAsync(&h, tot, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
@@ -2124,7 +2125,7 @@ extern "C" xk_status xk_constraint_jacobian(const xk_mesh* m, const xk_pairs* p,
     if (h > cap) {
       r = xk_set_error(XK_ERR_CAPACITY, "xk_constraint_jacobian: capacity below the number of active pairs");
     } else if (h > 0) {
-      k_jacobian<<<xk_blocks(p->n, 256), 256, 0, st>>>(*m, *p, flag, rows, cols, vals, pair_index);
+      k_jacobian<<<xk_blocks(p->n, 256), 256, 0, st>>>(*m, *p, off, rows, cols, vals, pair_index);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) r = xk_set_cuda_error(e, __FILE__, __LINE__);
     }

@@ -8,8 +8,9 @@
 // 32 predecessors at a time (one flag per lane, ballots to find the nearest inclusive prefix, flag 2, and
 // any predecessor that has not published), adds the window's aggregates up to that prefix with a warp sum,
 // and publishes the tile's inclusive prefix.  The wait on a predecessor that has not published yet is
-// bounded: past SCAN_SPIN_LIMIT polls the tile sums the inputs before it itself (the same prefix: integer
-// sums do not depend on their order), so the result never depends on the wait.
+// bounded: past SPIN polls the tile sums the inputs before it itself (the same prefix: integer
+// sums do not depend on their order), so the result never depends on the wait.  Earlier tiles may have stored by
+// then: what an operation stores must not be what its one() reads.
 //
 // One launch runs up to SCAN_CHANNELS independent scans (blockIdx.y).  An operation has, per channel c,
 //   long long size(int c) const                      how many values
@@ -60,7 +61,7 @@ XK_D int scan_flag(const int* p) {
   return v;
 }
 
-template <typename Op>
+template <typename Op, int SPIN>
 __global__ void __launch_bounds__(SCAN_T) k_scan_onepass(const __grid_constant__ Op op, long long nb_max,
                                                          int64_t* __restrict__ sums, int* __restrict__ words) {
   __shared__ int64_t wt[SCAN_T / 32];
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_onepass(const __grid_constant__
         const int stop = m_inc ? __ffs(m_inc) - 1 : 32;  // nearest inclusive prefix in the window
         const unsigned need = stop == 32 ? 0xffffffffu : ((1u << stop) - 1u);
         if (__ballot_sync(0xffffffffu, f == 0) & need) {  // a nearer predecessor has not published
-          if (++spins > SCAN_SPIN_LIMIT) {
+          if (++spins > SPIN) {
             fell_back = true;
             break;
           }
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_onepass(const __grid_constant__
   if (t == nb - 1 && threadIdx.x == 0) op.total(c, s_prefix + tile_tot);
 }
 
-// int32 array in, exclusive prefixes out (in place allowed); *sum (nullable) = the sum of all
+// int32 array in, exclusive prefixes out (another array); *sum (nullable) = the sum of all
 struct ScanI32 {
   const int32_t* in;
   int32_t* out;
@@ -207,10 +208,10 @@ inline long long scan_sums(long long n, int channels) { return 2 * scan_tiles(n)
 inline long long scan_words(long long n, int channels) { return (scan_tiles(n) + 1) * channels; }
 
 // n = the longest channel's size (> 0).
-template <typename Op>
+template <typename Op, int SPIN = SCAN_SPIN_LIMIT>
 xk_status scan_launch(const Op& op, long long n, int channels, int64_t* sums, int* zeroed_words, cudaStream_t s) {
   const long long nb = scan_tiles(n);
-  k_scan_onepass<Op><<<dim3((unsigned)nb, channels), SCAN_T, 0, s>>>(op, nb, sums, zeroed_words);
+  k_scan_onepass<Op, SPIN><<<dim3((unsigned)nb, channels), SCAN_T, 0, s>>>(op, nb, sums, zeroed_words);
   XK_CHECK_LAUNCH();
   return XK_OK;
 }

@@ -238,6 +238,7 @@ xk_status xk_exclusive_scan_i32(const int32_t* in, int32_t* out, long long n, in
     if (total_dev) XK_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(int64_t), s));
     return XK_OK;
   }
+  if (in < out + n && out < in + n) return xk_set_error(XK_ERR_ARG, "scan: input and output overlap");
   XkScratch own(s);
   const size_t sums = sizeof(int64_t) * (size_t)scan_sums(n, 1), words = sizeof(int) * (size_t)scan_words(n, 1);
   char* buf = nullptr;

@@ -289,11 +289,11 @@ constexpr int XK_READ_WORDS = 8;
 xk_status xk_read_begin(const int64_t* dev, int words, cudaStream_t s);
 xk_status xk_read_end(int64_t* host, int words);
 
-// Device-wide exclusive scan (util.cu), its scratch from S or of its own.
+// Device-wide exclusive scan (util.cu) into another array, its scratch from S or of its own.
 xk_status xk_exclusive_scan_i32(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
                                 cudaStream_t s, XkScratch* S = nullptr);
 // Number of block sums the scans use for n elements, and the int32 scan with a
-// caller-provided block-sum array of bsum_cap words (same kernels, same result;
+// caller-provided block-sum array of bsum_cap words (same result, in place allowed;
 // allocates nothing).
 long long xk_scan_tiles(long long n);
 xk_status xk_exclusive_scan_i32_scratch(const int32_t* in, int32_t* out, long long n, int64_t* total_dev,
