@@ -5,9 +5,7 @@
 // arguments and streams marshalled, and some ten stream waits took the caller's interpreter longer than the
 // kernels of an ordinary strand take the GPU.
 // Measured eagerly at the 37-wire strand in double: 125 -> 75 us (the segments' records of pair.cu included).
-#include <map>
-
-#include "xk_common.cuh"
+#include "context.cuh"
 
 xk_status xk_pair_step_seg(const xk_mesh* m, xk_pairs* p, const xk_contact_pattern* pat, const double* u,
                            const double* u_ref, const xk_contact_params* cp, int stages, int precision, int out_mode,
@@ -20,24 +18,24 @@ namespace {
 
 constexpr int STAGES = XK_STAGE_NARROW | XK_STAGE_NORMAL | XK_STAGE_FRICTION | XK_STAGE_TANGENT;
 
-// The events of the forks and joins, per thread and device.  A wait takes what its event holds when it is issued,
+// The events of the forks and joins, per thread and context.  A wait takes what its event holds when it is issued,
 // so they serve one call after the other; threads have their own.
 enum { EV_START, EV_NODES, EV_BEAM, EV_OTHERS, EV_MEMBERS, EV_SUMS, EV_TANGENT, EV_N };
 struct Events {
   cudaEvent_t e[EV_N] = {};
-  ~Events() {
+  void drop() {
     for (cudaEvent_t x : e)
       if (x) cudaEventDestroy(x);
   }
 };
 xk_status events_here(Events** out) {
-  thread_local std::map<int, Events> sets;
-  int dev = 0;
-  XK_CUDA(cudaGetDevice(&dev));
-  Events& s = sets[dev];
-  for (cudaEvent_t& x : s.e)
-    if (!x) XK_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
-  *out = &s;
+  thread_local PerContext<Events> sets;
+  XK_TRY(sets.here(out));
+  for (cudaEvent_t& x : (*out)->e)
+    if (!x) {
+      RelaxedCapture relaxed;
+      XK_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+    }
   return XK_OK;
 }
 

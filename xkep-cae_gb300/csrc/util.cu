@@ -6,8 +6,7 @@
 #include <cstring>
 #include <mutex>
 
-#include <map>
-
+#include "context.cuh"
 #include "scan.cuh"
 
 static thread_local char g_err[512] = "";
@@ -71,33 +70,38 @@ bool xk_context_id(unsigned long long* id) {
   return get_id(c, id) == CUDA_SUCCESS;
 }
 
-// The pool of each device, with the context it was made in: a context made later on the device (after
-// cudaDeviceReset) gets its own.
+xk_status xk_context_here(unsigned long long* id) {
+  if (xk_context_id(id)) return XK_OK;
+  RelaxedCapture relaxed;
+  XK_CUDA(cudaFree(nullptr));
+  if (xk_context_id(id)) return XK_OK;
+  int dev = 0;  // a driver without ids: one context per device
+  XK_CUDA(cudaGetDevice(&dev));
+  *id = ~0ULL - (unsigned long long)dev;
+  return XK_OK;
+}
+
 namespace {
+// the pool of each context, never given back: calls on other threads may be using it
 struct ScratchPool {
-  unsigned long long ctx = 0;
   cudaMemPool_t pool = nullptr;
+  void drop() {}
 };
 std::mutex g_pool_mutex;
-ScratchPool g_pool[64];
-
-// Making and trimming a pool are no stream operations: a capture that another thread has under way must not
-// forbid them, nor end by them.
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
+PerContext<ScratchPool>& scratch_pools() {
+  static PerContext<ScratchPool>* const pools = new PerContext<ScratchPool>;
+  return *pools;
+}
 
 // the current device's pool, made on first use; null if there is none to be had
 cudaMemPool_t scratch_pool(bool make) {
   int dev = 0;
   unsigned long long id = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !xk_context_id(&id)) return nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess || !xk_context_id(&id)) return nullptr;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  ScratchPool& g = g_pool[dev];
-  if (g.pool && g.ctx == id) return g.pool;
-  if (!make) return nullptr;
+  ScratchPool* g = scratch_pools().find(id);
+  if (g && g->pool) return g->pool;
+  if (!make || (!g && !(g = scratch_pools().add(id)))) return nullptr;
   RelaxedCapture relaxed;
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
@@ -112,9 +116,7 @@ cudaMemPool_t scratch_pool(bool make) {
     cudaGetLastError();
     return nullptr;
   }
-  g.pool = pool;
-  g.ctx = id;
-  return pool;
+  return g->pool = pool;
 }
 }  // namespace
 
@@ -139,39 +141,45 @@ extern "C" xk_status xk_scratch_trim(int64_t keep_bytes) {
 // --------------------------------------------------------------------------- read-back
 
 namespace {
-// a pinned buffer per thread, an event per thread and device
+// a pinned buffer and an event per thread and context
 struct Readback {
   int64_t* host = nullptr;
-  std::map<int, cudaEvent_t> events;
-  cudaEvent_t pending = nullptr;
-  ~Readback() {
-    for (auto& e : events) cudaEventDestroy(e.second);
+  cudaEvent_t event = nullptr;
+  bool pending = false;  // begun and not ended
+  void drop() {
+    if (event) cudaEventDestroy(event);
     if (host) cudaFreeHost(host);
   }
 };
-thread_local Readback g_read;
+thread_local PerContext<Readback> g_reads;
+thread_local Readback* g_begun = nullptr;
 }  // namespace
 
 xk_status xk_read_begin(const int64_t* dev, int words, cudaStream_t s) {
-  Readback& r = g_read;
   if (words > XK_READ_WORDS) return xk_set_error(XK_ERR_ARG, "xk_read_begin: words");
-  int id = 0;
-  XK_CUDA(cudaGetDevice(&id));
-  cudaEvent_t& e = r.events[id];
-  if (!r.host || !e) {
+  Readback* r;
+  XK_TRY(g_reads.here(&r));
+  if (!r->host || !r->event) {
     RelaxedCapture relaxed;
-    if (!r.host) XK_CUDA(cudaHostAlloc((void**)&r.host, sizeof(int64_t) * XK_READ_WORDS, cudaHostAllocPortable));
-    if (!e) XK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (!r->host) XK_CUDA(cudaHostAlloc((void**)&r->host, sizeof(int64_t) * XK_READ_WORDS, cudaHostAllocDefault));
+    if (!r->event) XK_CUDA(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming));
   }
-  XK_CUDA(cudaMemcpyAsync(r.host, dev, sizeof(int64_t) * words, cudaMemcpyDeviceToHost, s));
-  XK_CUDA(cudaEventRecord(e, s));
-  r.pending = e;
+  if (r->pending) {  // a call failed in between: its copy may still be on its way into the buffer
+    XK_CUDA(cudaEventSynchronize(r->event));
+    r->pending = false;
+  }
+  XK_CUDA(cudaMemcpyAsync(r->host, dev, sizeof(int64_t) * words, cudaMemcpyDeviceToHost, s));
+  XK_CUDA(cudaEventRecord(r->event, s));
+  r->pending = true;
+  g_begun = r;
   return XK_OK;
 }
 
 xk_status xk_read_end(int64_t* host, int words) {
-  XK_CUDA(cudaEventSynchronize(g_read.pending));
-  for (int k = 0; k < words; ++k) host[k] = g_read.host[k];
+  Readback* r = g_begun;
+  XK_CUDA(cudaEventSynchronize(r->event));
+  r->pending = false;
+  for (int k = 0; k < words; ++k) host[k] = r->host[k];
   return XK_OK;
 }
 
