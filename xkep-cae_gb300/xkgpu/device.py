@@ -7,7 +7,7 @@ xkgpu kernels behind the C ABI.
 from __future__ import annotations
 
 import ctypes as C
-import threading
+import itertools
 import weakref
 from dataclasses import dataclass
 
@@ -44,24 +44,25 @@ def as_dev(x, dtype, device) -> torch.Tensor:
 
 # ----------------------------------------------------------------------------- mesh
 
-_meshes: dict[int, int] = {}  # meshes alive per device
-_meshes_lock = threading.Lock()
+# Meshes alive per device, by number.  No lock: a finalizer runs wherever the collector does, so also within
+# _count_mesh on the same thread, and each step here is one indivisible dict operation.
+_meshes: dict[int, dict[int, None]] = {}
+_mesh_numbers = itertools.count()
 
 
-def _mesh_gone(index: int) -> None:
-    with _meshes_lock:
-        _meshes[index] -= 1
-        last = _meshes[index] == 0
-    if last:  # the detection's scratch goes back to the system with the last mesh of the device
+def _mesh_gone(index: int, number: int) -> None:
+    alive = _meshes[index]
+    alive.pop(number, None)
+    if not alive:  # the detection's scratch goes back to the system with the last mesh of the device
         with torch.cuda.device(index):
             L.call("xk_scratch_trim", 0)
 
 
 def _count_mesh(mesh: "DeviceMesh") -> None:
     index = mesh.device.index if mesh.device.index is not None else torch.cuda.current_device()
-    with _meshes_lock:
-        _meshes[index] = _meshes.get(index, 0) + 1
-    weakref.finalize(mesh, _mesh_gone, index).atexit = False
+    number = next(_mesh_numbers)
+    _meshes.setdefault(index, {})[number] = None
+    weakref.finalize(mesh, _mesh_gone, index, number).atexit = False
 
 
 class DeviceMesh:
