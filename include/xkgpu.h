@@ -408,7 +408,8 @@ typedef struct {
                               defer[cap + 2]), which keeps the exact double routine out of the common
                               kernels; each list is back at zero after its kernel */
   int32_t block;           /* threads per CTA of the other-pair and member kernels: a multiple of 32 up to
-                              256, 0 = 256.  Results do not depend on it; an autotuner may choose it. */
+                              256; 0 = 256, or 64 for a kernel of less than two CTAs of 256 per SM.
+                              Results do not depend on it; an autotuner may choose it. */
   int32_t pad_launch;
   int32_t* slot;           /* [cap] or NULL: the slot of each pair of the FP64 table (the inverse of pair),
                               written by xk_pairs_to32, so that xk_pairs_from32 walks the table in its own

@@ -408,14 +408,14 @@ class AssemblyEngine:
         if self.precision == L.XK_MIXED and self._state_in32:
             q = self.pairs32.c
             t = {}
-            for bs in (128, 256):
+            for bs in (0, 128, 256):  # 0: by the tables' sizes (xk_pairs32.block)
                 q.block = bs
                 t[bs] = self._time_calls(lambda s: L.call("xk_pair_step32", C.byref(q), ptr(self.node32),
                                                           C.byref(self.cp), ptr(self.rec), L.XK_PAIRS_ALL,
                                                           stream_handle(s)), reps)
             q.block = min(t, key=t.get)
             self._pair_block = q.block
-            out["pair_block"] = {"times_ms": t, "chosen": q.block, "default": 256}
+            out["pair_block"] = {"times_ms": t, "chosen": q.block, "default": 0}
         if self.gather_variant == L.XK_GATHER_SIDES:
             pat = self.pattern.c
             t = {}
