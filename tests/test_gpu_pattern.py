@@ -132,6 +132,33 @@ def test_lists_against_direct_construction(kind, ne, n, hub, share, optional):
         assert pat.bcodes[: 4 * nb].cpu().numpy().reshape(-1, 4).tolist() == x["terms"]
 
 
+def test_more_cross_terms_than_a_byte_counts():
+    """A block with 256 cross contributions (elements of no length, both ends one node): its list is whole, the
+    inline terms are refused, and those of the rows before it stay."""
+    conn = np.array([(2 * e, 2 * e + 1) for e in range(24)] + [(48, 49 + e) for e in range(8)] + [(57, 57)] * 16)
+    ne, nn = len(conn), 58
+    mesh = DeviceMesh(np.random.default_rng(1).normal(size=(nn, 3)), conn, np.full(ne, 0.1))
+    ea = np.array([2 * k for k in range(12)] + [24 + e for e in range(8) for _ in range(16)])
+    eb = np.array([2 * k + 1 for k in range(12)] + [32 + f for _ in range(8) for f in range(16)])
+    n = len(ea)
+    pairs = DevicePairTable(mesh.device, n)
+    for k, a in (("ea", ea), ("eb", eb), ("status", np.ones(n))):
+        pairs.t[k][:n] = torch.as_tensor(a).to(pairs.t[k])
+    pairs.set_n(n)
+    pat = DeviceContactPattern(mesh)
+    for _ in range(2):
+        pat.build(pairs)
+        x = _expected(conn, ea, eb, np.ones(n, bool), nn)
+        nb = len(x["keys"])
+        assert pat.nnzb == nb and not x["fits"] and not pat.c.sides_ok
+        assert len(x["contrib"][x["keys"].index((48, 57))]) == 256
+        assert _split(pat.blk_ptr[: nb + 1], pat.contrib) == x["contrib"]
+        codes = pat.bcodes[: 4 * nb].cpu().numpy().reshape(-1, 4).tolist()
+        for (v, _), got, want in zip(x["keys"], codes, x["terms"]):
+            if v < 48:
+                assert got == want
+
+
 def test_a_row_over_256_columns_is_refused():
     ne = 400
     conn = np.arange(2 * ne).reshape(-1, 2)

@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(32 * PR_WARPS, 8) k_pat_rows(const __grid_cons
       __syncwarp();
       if (r >= 0 && (same & below) == 0) {  // the first of its block moves the block on
         sp[r] += __popc(same);
-        if (g.bcodes) sx[r] += __popc(crosses);
+        if (g.bcodes) sx[r] = min(sx[r] + __popc(crosses), 4);  // 4: full (a count would overrun its 8 bits)
       }
       __syncwarp();
     }
