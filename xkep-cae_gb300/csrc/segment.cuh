@@ -83,12 +83,3 @@ XK_D bool closest_exact_fast(const double* xA, const double* dA, double a, const
   for (int i = 0; i < 3; ++i) normal[i] = div64(diff[i], q);
   return true;
 }
-XK_D bool closest_exact_fast(const double (*x)[3], double& s, double& t, double& dist, double* normal) {
-  double dA[3], dB[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    dA[i] = xsub(x[1][i], x[0][i]);
-    dB[i] = xsub(x[3][i], x[2][i]);
-  }
-  return closest_exact_fast(x[0], dA, xdot_es(dA, dA), x[2], dB, xdot_es(dB, dB), s, t, dist, normal);
-}
