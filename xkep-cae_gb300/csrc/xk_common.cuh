@@ -134,10 +134,12 @@ XK_D bool near_one64(double x) {
 }
 
 // The correctly rounded quotient and square root (the bits of the operators) on fewer FP64 operations, after
-// Markstein ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): with r the
-// correctly rounded reciprocal, q = RN(x r) leaves an exact remainder x - d q, and RN(q + rem r) is x / d.  One step
-// r + r (1 - d r) from a reciprocal within a unit of the last place rounds correctly (rcp64 alone does not for one
-// divisor in sixty), but for a mantissa of ones only, 2^k (2 - 2^-52), whose reciprocal lies 2^-106 above a tie.
+// Markstein ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): q = RN(x r), r the
+// reciprocal, leaves the remainder x - d q, and RN(q + rem r) is x / d.  With D, R the mantissas of d and r as whole
+// numbers (R D = 2^105) and r off by t units of its last place: a quotient next to a tie is at least 1 / (2 D) units
+// from it, q half a unit, and the last step is off by t / (2 R), so it rounds correctly for t < R / D = 2^105 / D^2.
+// Two Newton-Raphson steps give t < 1/2 + 2^-26 (rcp64 alone 0.508, too much for one divisor in a hundred), and
+// 2^105 / D^2 is above 1/2 + 2^-21 unless the upper 20 bits of the mantissa are ones.
 // The square root likewise from g = RN(x y) and its exact remainder: near a tie the step's error is below 2^-52.7
 // units, and the few operands whose root lies that close (x = N (N + 1) - c, c small, N (N + 1) = c modulo a power of
 // two) have been tried one by one.  A divisor's reciprocal serves several quotients.  Operands outside the range
@@ -152,9 +154,11 @@ XK_D bool mag_in64(double x) {  // |x| in [2^-300, 2^300)
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) - (723u << 20) < (600u << 20);
 }
 XK_D Divisor64 divisor64(double d) {
-  const double r = rcp64(d);
-  const bool ones = ((unsigned)__double2loint(d) & ((unsigned)__double2hiint(d) | 0xfff00000u)) == 0xffffffffu;
-  return {d, fma(fma(-d, r, 1.0), r, r), mag_in64(d) && !ones};
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  return {d, r, mag_in64(d) && (__double2hiint(d) & 0xfffff) != 0xfffff};
 }
 XK_D double div64(double x, const Divisor64& q) {
   if (!(q.ok && mag_in64(x))) return x == 0.0 && q.ok ? x : div64_plain(x, q.d);
