@@ -40,7 +40,9 @@ __global__ void k_sqrt(long long n, const double* x, double* q, double* want) {
 __global__ void k_div_unit(long long n, const double* x, const double* d, double* q, double* want) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  q[i] = next_to_one64(d[i]) ? div_next_to_one64(x[i], d[i]) : -1.0;
+  bool sure;
+  const double y = div_next_to_one64(x[i], d[i], units_from_one64(d[i]), sure);
+  q[i] = !next_to_one64(d[i]) ? -1.0 : sure ? y : x[i] / d[i];
   want[i] = x[i] / d[i];
 }
 extern "C" int t_div_unit(long long n, const double* x, const double* d, double* q, double* want) {

@@ -46,8 +46,18 @@ XK_D double sqrt_unit64(double x) {
 // without one
 XK_D void div3(const double* v, double d, double* out) {
   if (next_to_one64(d)) {
+    const unsigned n = units_from_one64(d);
+    bool sure[3];
+    double q[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) out[i] = div_next_to_one64(v[i], d);
+    for (int i = 0; i < 3; ++i) q[i] = div_next_to_one64(v[i], d, n, sure[i]);
+    if (!(sure[0] && sure[1] && sure[2])) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        if (!sure[i]) q[i] = v[i] == 0.0 ? v[i] : div64_plain(v[i], d);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[i] = q[i];
     return;
   }
   const Divisor64 q = divisor64(d);

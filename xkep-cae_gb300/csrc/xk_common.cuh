@@ -168,21 +168,20 @@ XK_D double div64(double x, const Divisor64& q) {
 XK_D double div64(double x, double d) { return div64(x, divisor64(d)); }
 // v / d for a divisor next to one, d = 1 - k 2^-53 (k <= 16) or 1 + k 2^-52 (k < 8): as RN(v + v (1 - d)), one
 // operation, which leaves out v (1 - d)^2, below 2^-45 units of the last place of v.  That decides the rounding where
-// v (1 - d) lies on a tie or within 2^-45 of one (v = 1/2, d = 1 - 2^-53: a contact at 60 degrees), so there, and
-// where v is so close to a power of two that the quotient may change binade, the divide is taken; whole arithmetic on
-// the bits finds these.
+// v (1 - d) lies on a tie or within 2^-45 of one (v = 1/2, d = 1 - 2^-53: a contact at 60 degrees), and v may be so
+// close to a power of two that the quotient changes binade.  With m the mantissa of v and n = |1 - d| 2^53 <= 16, the
+// product m n is within 512 of a multiple of 2^32 in both cases; where its lower word says so (one value in four
+// million, and those of few bits, zeros, infinities) `sure` falls, and the caller takes the operator.  The whole test
+// of m n takes ten times the integer operations: 632,000 exact narrowphases 299 us, this 277.
 XK_D bool next_to_one64(double d) {
   return (unsigned long long)(__double_as_longlong(d) - 0x3feffffffffffff0LL) < 0x18ULL;
 }
-XK_D double div_next_to_one64(double v, double d) {
-  const long long k = __double_as_longlong(d) - 0x3ff0000000000000LL, b = __double_as_longlong(v);
-  const unsigned long long n = (unsigned long long)(k < 0 ? -k : 2 * k);  // |1 - d| in units of 2^-53
-  if (n == 0 || (b << 1) == 0) return v;
-  const unsigned long long one = 1ULL << 52, m = ((unsigned long long)b & (one - 1)) | one;
-  const bool tie = ((m * n + one + 512) & (2 * one - 1)) < 1024;  // the fraction of v (1 - d) within 2^-44 of a half
-  const bool edge = m - (one + 32) >= one - 64;
-  const bool range = ((unsigned)__double2hiint(v) & 0x7ff00000u) - (24u << 20) < (2020u << 20);
-  if (tie || edge || !range) return div64(v, d);
+XK_D unsigned units_from_one64(double d) {
+  const int k = (int)(__double_as_longlong(d) - 0x3ff0000000000000LL);
+  return (unsigned)(k < 0 ? -k : 2 * k);
+}
+XK_D double div_next_to_one64(double v, double d, unsigned n, bool& sure) {
+  sure = n == 0 || (unsigned)__double2loint(v) * n + 512u >= 1024u;
   return fma(v, 1.0 - d, v);
 }
 XK_D double sqrt64(double x) {
