@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(BEAMW_T, 6) k_beam32e(int mode, xk_mesh m, xk_
 // instead of one per colour.
 // CTAs of one warp: a small mesh then reaches every SM (4,736 elements: 153 CTAs), where CTAs of 128 threads,
 // one launch after another, left most of them idle.
-// Measured, colour launches of beam_tail against this: 98,592 elements 406 -> 265 us, 4,736 elements
+// Measured, colour launches of beam_tail against this: 98,592 elements 406 -> 270 us, 4,736 elements
 // 157 -> 52 us (a warp issues one FP64 instruction in 64 clocks, and that mesh has one warp per SM).
 constexpr int BEAM64_T = 32;
 

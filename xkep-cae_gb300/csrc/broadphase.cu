@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(BP_T, 8) k_sweep(xk_mesh m, const double* __re
 // prescreen margin: mean(r_a + r_b) / 2 over the candidates after the shared-node and same-layer filters
 // (_manager_process.py:275-279) from the per-segment sums, in a fixed order (a tree in every block, the last
 // block over the blocks), or the common radius.
+// RED_BLOCKS is this GPU's number of SMs, but fixed: the order of the sums follows from it.
 constexpr int RED_BLOCKS = 152, RED_T = 256;
 __global__ void __launch_bounds__(RED_T) k_totals(const int32_t* __restrict__ cnt, const int32_t* __restrict__ raw,
                                                   const double* __restrict__ rsum, long long ne,

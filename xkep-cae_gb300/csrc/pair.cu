@@ -365,8 +365,8 @@ XK_D void narrow_exact_one(const xk_mesh& m, const xk_pairs& p, const double* __
 }
 
 // Bounded by the FP64 pipe: 328 operations a pair with div64 / sqrt64 in place of the operators (430 before),
-// 255 with the unit-vector forms in the frame, 227 with the segments' records.  632,000 pairs: 518 -> 331 us,
-// then 281 us.
+// 255 with the unit-vector forms in the frame, 227 with the segments' records (some 230 with the reciprocals that
+// div64 needs).  632,000 pairs: 518 -> 331 us, then 271 us, 277 with every tie decided.
 template <bool SEG>
 __global__ void k_narrow_exact(xk_mesh m, xk_pairs p, const double* __restrict__ u, double g_on, double g_off,
                                int allow_deact, int update_active, const double* __restrict__ seg) {
@@ -490,7 +490,7 @@ XK_D void coating_epilogue(const xk_contact_params& cp, const ST* __restrict__ p
 // double divide and square root costs some ten of them, and a dot product with separately rounded terms
 // five instead of three.  A pair that carries no force needs double precision only, so its narrowphase is
 // written for the fewest FP64 operations: fused multiply-adds, one reciprocal or reciprocal square root per
-// normalisation (two Newton-Raphson steps from the approximate PTX instruction), range tests on the high word
+// normalisation (one step of third order from the approximate PTX instruction), range tests on the high word
 // in the integer pipe, and the frame transported as R p = c p + v x p + v (v.p) / (1 + c).  A contributing
 // pair keeps the reference's operation order up to its normal, with cheaper correctly rounded divides; its
 // frame and friction are fused too.  Pairs outside the ordinary case (near-parallel, degenerate, without a
@@ -1651,7 +1651,9 @@ XK_D bool last_cta_done(int32_t* done) {
   return last;
 }
 
-// The deferred (near-parallel) other pairs, grid-stride over the list.
+// The deferred (near-parallel) other pairs, grid-stride over the list, in DEFER_CTAS CTAs: one for each of this
+// GPU's SMs (any number is right; the list is empty but for near-parallel wires).
+constexpr int DEFER_CTAS = 152;
 __global__ void __launch_bounds__(PAIR_T) k_pair_other32_deferred(xk_pairs32 q, const float* __restrict__ n32) {
   int32_t* list = q.defer;
   const int cnt = *(volatile int32_t*)list;
@@ -2295,7 +2297,7 @@ extern "C" xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk
     const int bs = cta(n_o);
     if (q->defer) {
       k_pair_other32<true><<<xk_blocks(n_o, bs), bs, 0, st>>>(*q, node32);
-      k_pair_other32_deferred<<<152, PAIR_T, 0, st>>>(*q, node32);
+      k_pair_other32_deferred<<<DEFER_CTAS, PAIR_T, 0, st>>>(*q, node32);
     } else {
       k_pair_other32<false><<<xk_blocks(n_o, bs), bs, 0, st>>>(*q, node32);
     }
@@ -2304,7 +2306,7 @@ extern "C" xk_status xk_pair_step32(xk_pairs32* q, const float* node32, const xk
     const int bs = cta(q->n_members);
     if (q->defer) {
       k_pair_member32<true><<<xk_blocks(q->n_members, bs), bs, 0, st>>>(*q, node32, *cp, rec);
-      k_pair_member32_deferred<<<152, PAIR_T, 0, st>>>(*q, node32, *cp, rec);
+      k_pair_member32_deferred<<<DEFER_CTAS, PAIR_T, 0, st>>>(*q, node32, *cp, rec);
     } else {
       k_pair_member32<false><<<xk_blocks(q->n_members, bs), bs, 0, st>>>(*q, node32, *cp, rec);
     }

@@ -5,9 +5,10 @@ solves ``K du = -R`` with the Dirichlet DOFs' rows and columns replaced by the
 identity, by a direct sparse factorisation on the host.  ``DeviceLinearSolver``
 keeps ``K = K_beam + K_c`` in the engine's block matrices and runs BiCGStab
 with a block-Jacobi preconditioner (each node's 6x6 diagonal block) in the
-``xk_bicgstab`` kernels: no matrix leaves the device, and the only host
-synchronisations are the convergence checks (each check interval of
-iterations replays as one CUDA graph).
+``xk_bicgstab`` kernels: no matrix leaves the device.  Systems of up to 4,032
+unknowns run in one thread-block cluster, which checks the convergence itself
+and comes back to the host once per launch of some 500 iterations; larger ones
+replay each check interval as one CUDA graph and synchronise at the checks.
 """
 
 from __future__ import annotations
